@@ -14,6 +14,7 @@ namespace hteno {
 namespace {
 
 __constant__ DevConst c_dev;
+__device__ DevConst g_dev;  // the same in global memory (double: par::ldk)
 unsigned long long g_mask = 0;
 std::mutex g_mu;
 
@@ -46,10 +47,9 @@ __global__ void k1_init(Geo1 G, const double* __restrict__ q, StepState* st) {
   block_max_to(ms, &st->maxbits);
 }
 
-// face f in [0, nx] between cells f-1 and f (FV_System1D.cpp:194-235)
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k1_flux(Geo1 G, const double* __restrict__ q,
-                                                    T* __restrict__ F, const StepState* st) {
+// face f in [0, nx] between cells f-1 and f (FV_System1D.cpp:194-235), mixed precision
+__global__ void __launch_bounds__(kThreads) k1_flux_f(Geo1 G, const double* __restrict__ q,
+                                                      float* __restrict__ F, const StepState* st) {
   if (st->done) return;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f > G.nx) return;
@@ -62,39 +62,21 @@ __global__ void __launch_bounds__(kThreads) k1_flux(Geo1 G, const double* __rest
   }
   cell_prim1(G.g1, qa, wa, ha, sa);
   cell_prim1(G.g1, qb, wb, hb, sb);
-  T Ff[3];
-  if constexpr (std::is_same<T, double>::value) {
-    double R[9], L[9], ch[3][6];
-    par::eig1(G.g1, sa, wa[1], ha, sb, wb[1], hb, R, L);
-    for (int m = 0; m < 6; ++m) {
-      const int c = bmap(f - 3 + m, n, G.bc);
-      const double qq[3] = {q[c], q[n + c], q[2 * n + c]};
-      double cc[3];
-      par::mv3(L, qq, cc);
-      for (int r = 0; r < 3; ++r) ch[r][m] = cc[r];
-    }
-    double cl[3], cr[3], ql[3], qr[3];
-    for (int r = 0; r < 3; ++r) par::lagrange_recon(c_dev, G.recon, ch[r], cl[r], cr[r]);
-    par::mv3(R, cl, ql);  // transformToConservative (FV_System1D.h:48-51)
-    par::mv3(R, cr, qr);
-    if (G.flux == HTENO_FLUX_HLLC) par::hllc1(G.g1, ql, qr, Ff);
-    else par::rusanov1(G.gamma, G.g1, L, R, ql, qr, Ff);
-  } else {
-    const Roe1<T> R = roe1<T>(T(G.g1), T(sa), T(wa[1]), T(ha), T(sb), T(wb[1]), T(hb));
-    T ch[3][6];
-    for (int m = 0; m < 6; ++m) {
-      const int c = bmap(f - 3 + m, n, G.bc);
-      T qq[3] = {T(q[c]), T(q[n + c]), T(q[2 * n + c])}, cc[3];
-      roe1_left(R, qq, cc);
-      for (int r = 0; r < 3; ++r) ch[r][m] = cc[r];
-    }
-    T cl[3], cr[3], ql[3], qr[3];
-    for (int r = 0; r < 3; ++r) lagrange_recon(c_dev, G.recon, ch[r], cl[r], cr[r]);
-    roe1_right(R, cl, ql);
-    roe1_right(R, cr, qr);
-    if (G.flux == HTENO_FLUX_HLLC) hllc1(T(G.g1), ql, qr, Ff);
-    else rusanov1(T(G.gamma), T(G.g1), R, ql, qr, Ff);
+  float Ff[3];
+  const Roe1<float> R = roe1<float>(float(G.g1), float(sa), float(wa[1]), float(ha), float(sb), float(wb[1]), float(hb));
+  float ch[3][6];
+  for (int m = 0; m < 6; ++m) {
+    const int c = bmap(f - 3 + m, n, G.bc);
+    float qq[3] = {float(q[c]), float(q[n + c]), float(q[2 * n + c])}, cc[3];
+    roe1_left(R, qq, cc);
+    for (int r = 0; r < 3; ++r) ch[r][m] = cc[r];
   }
+  float cl[3], cr[3], ql[3], qr[3];
+  for (int r = 0; r < 3; ++r) lagrange_recon(c_dev, G.recon, ch[r], cl[r], cr[r]);
+  roe1_right(R, cl, ql);
+  roe1_right(R, cr, qr);
+  if (G.flux == HTENO_FLUX_HLLC) hllc1(float(G.g1), ql, qr, Ff);
+  else rusanov1(float(G.gamma), float(G.g1), R, ql, qr, Ff);
   for (int v = 0; v < 3; ++v) F[v * (n + 1) + f] = Ff[v];
 }
 
@@ -102,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) k1_flux(Geo1 G, const double* __rest
 // characteristic field, s the side) projects its field's 6-cell stencil and reconstructs one side;
 // the group's lane 0 gathers the six values, projects back and computes the flux.  A 1D grid has
 // a few hundred faces: spreading each face's FP64 work over more lanes and warps (hence SMs)
-// shortens the step; every value is computed with the same operations as in k1_flux.
+// shortens the step.
 __global__ void __launch_bounds__(kThreads) k1_flux_lanes(Geo1 G, const double* __restrict__ q,
                                                           double* __restrict__ F,
                                                           const StepState* st) {
@@ -120,7 +102,7 @@ __global__ void __launch_bounds__(kThreads) k1_flux_lanes(Geo1 G, const double* 
   }
   cell_prim1(G.g1, qa, wa, ha, sa);
   cell_prim1(G.g1, qb, wb, hb, sb);
-  double R[9], L[9];
+  par::fp R[9], L[9];
   par::eig1(G.g1, sa, wa[1], ha, sb, wb[1], hb, R, L);
   const int r = l & 3, side = l >> 2;
   double val = 0.0;
@@ -128,27 +110,27 @@ __global__ void __launch_bounds__(kThreads) k1_flux_lanes(Geo1 G, const double* 
     double ch[6];
     for (int m = 0; m < 6; ++m) {
       const int c = bmap(fc - 3 + m, n, G.bc);
-      double sum = L[3 * r] * q[c];  // row r of par::mv3
+      par::fp sum = L[3 * r] * q[c];  // row r of par::mv3
       sum = sum + L[3 * r + 1] * q[n + c];
       sum = sum + L[3 * r + 2] * q[2 * n + c];
-      ch[m] = sum;
+      ch[m] = sum.v;
     }
-    val = par::lagrange_side(c_dev, G.recon, ch, side);
+    val = par::lagrange_side(g_dev, G.recon, ch, side);
   }
   const int base = int(threadIdx.x & 31u) & ~7;
-  double cl[3], cr[3];
+  par::fp cl[3], cr[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     cl[k] = __shfl_sync(0xffffffffu, val, base + k);
     cr[k] = __shfl_sync(0xffffffffu, val, base + 4 + k);
   }
   if (l != 0 || !live) return;
-  double ql[3], qr[3], Ff[3];
+  par::fp ql[3], qr[3], Ff[3];
   par::mv3(R, cl, ql);  // transformToConservative (FV_System1D.h:48-51)
   par::mv3(R, cr, qr);
   if (G.flux == HTENO_FLUX_HLLC) par::hllc1(G.g1, ql, qr, Ff);
   else par::rusanov1(G.gamma, G.g1, L, R, ql, qr, Ff);
-  for (int v = 0; v < 3; ++v) F[v * (n + 1) + f] = Ff[v];
+  for (int v = 0; v < 3; ++v) F[v * (n + 1) + f] = Ff[v].v;
 }
 
 // rhs (FV_System1D.cpp:237-240) + RungeKutta3 (:243-272); max wave speed on the last stage
@@ -202,14 +184,15 @@ __global__ void __launch_bounds__(kThreads) k1_harvest(Geo1 G, const double* __r
   }
   cell_prim1(G.g1, qa, wa, ha, sa);
   cell_prim1(G.g1, qb, wb, hb, sb);
-  double R[9], L[9], ch[3][6];
+  par::fp R[9], L[9];
+  double ch[3][6];
   par::eig1(G.g1, sa, wa[1], ha, sb, wb[1], hb, R, L);
   for (int m = 0; m < 6; ++m) {
     const int c = bmap(f - 3 + m, n, G.bc);
-    const double qq[3] = {q[c], q[n + c], q[2 * n + c]};
-    double cc[3];
+    const par::fp qq[3] = {q[c], q[n + c], q[2 * n + c]};
+    par::fp cc[3];
     par::mv3(L, qq, cc);
-    for (int r = 0; r < 3; ++r) ch[r][m] = cc[r];
+    for (int r = 0; r < 3; ++r) ch[r][m] = cc[r].v;
   }
   for (int r = 0; r < 3; ++r)
     harvest::emit_both(ch[r], G.recon == HTENO_RECON_TENO5I, seed, (uint64_t(r) << 40) + uint64_t(f),
@@ -261,7 +244,7 @@ void launch_step(hteno_solver* s, const Geo1& G, cudaStream_t cs) {
     if constexpr (std::is_same<T, double>::value)
       k1_flux_lanes<<<gl, kThreads, 0, cs>>>(G, s->q, F, s->dstate);
     else
-      k1_flux<T><<<gf, kThreads, 0, cs>>>(G, s->q, F, s->dstate);
+      k1_flux_f<<<gf, kThreads, 0, cs>>>(G, s->q, F, s->dstate);
     k1_update<T><<<gc, kThreads, 0, cs>>>(G, stage, F, s->q, s->q0, s->dstate);
   }
   k_end_step<<<1, 1, 0, cs>>>(s->dstate);
@@ -298,7 +281,7 @@ cudaError_t ensure_graph(hteno_solver* s, const Geo1& G) {
 }  // namespace
 
 int fv1d_setup(hteno_solver* s) {
-  if (upload_const(c_dev, &g_mask, &g_mu) != cudaSuccess)
+  if (upload_const(&g_mask, &g_mu, c_dev, g_dev) != cudaSuccess)
     return set_error(s, HTENO_ERR_CUDA, "constant upload failed");
   s->work_bytes = 3 * size_t(s->cfg.nx + 1) * sizeof(double);
   cudaError_t e = cudaMalloc(&s->work, s->work_bytes);

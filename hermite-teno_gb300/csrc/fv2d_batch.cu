@@ -324,7 +324,7 @@ int hteno_batch_create(const hteno_config* cfgs, int n, hteno_batch** out) {
   };
   b->n = n;
   b->cfg.assign(cfgs, cfgs + n);
-  if (upload_const(c_dev, &g_mask, &g_mu) != cudaSuccess) return fail(HTENO_ERR_CUDA);
+  if (upload_const(&g_mask, &g_mu, c_dev) != cudaSuccess) return fail(HTENO_ERR_CUDA);
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(HTENO_ERR_CUDA);
   b->own_stream = true;

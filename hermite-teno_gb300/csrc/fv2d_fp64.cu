@@ -13,7 +13,7 @@
 namespace hteno {
 namespace {
 
-__constant__ DevConst c_dev;
+__device__ DevConst g_dev;  // in global memory: par::ldk
 unsigned long long g_mask = 0;
 std::mutex g_mu;
 
@@ -22,15 +22,18 @@ std::mutex g_mu;
 // primitives: calcPrimitiveVariable (FV_System2D.cpp:226-263)
 // The three divisions by rho share one correctly rounded reciprocal (par::quot: the same bits as
 // the divisions, Markstein).
-__device__ __forceinline__ void cell_prim(double g1, const double* q, double* w, double& h,
+__device__ __forceinline__ void cell_prim(double g1, const double* qd, double* w, double& h,
                                           double& sr) {
+  const par::fp q[4] = {qd[0], qd[1], qd[2], qd[3]};
   const par::Den d = par::den_of(q[0]);
-  w[0] = q[0];
-  w[1] = par::quot(q[1], d);
-  w[2] = par::quot(q[2], d);
-  w[3] = (q[3] - 0.5 * (q[1] * w[1] + q[2] * w[2])) * g1;  // par::primitive's pressure
+  const par::fp u = par::quot(q[1], d), v = par::quot(q[2], d);
+  const par::fp p = par::scaled(par::kNegHalf, q[1] * u + q[2] * v, q[3]) * g1;  // par::primitive's pressure
+  w[0] = qd[0];
+  w[1] = u.v;
+  w[2] = v.v;
+  w[3] = p.v;
   sr = sqrt(fabs(w[0]));
-  h = par::quot(q[3] + w[3], d);
+  h = par::quot(q[3] + p, d).v;
 }
 
 __global__ void kp_prim(Geo G, const double* __restrict__ q, double* __restrict__ prim,
@@ -173,17 +176,11 @@ __global__ void __launch_bounds__(kFaceThreads) kp_faces(Geo G, const double* __
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     double a, b;
-    par::lagrange_recon(c_dev, G.recon, ch[r], a, b);
+    par::lagrange_recon(g_dev, G.recon, ch[r], a, b);
     fc[r * nface + o] = a;
     fc[(4 + r) * nface + o] = b;
   }
-  froe[0 * nface + o] = E.vxm;
-  froe[1 * nface + o] = E.vym;
-  froe[2 * nface + o] = E.hm;
-  froe[3 * nface + o] = E.qm;
-  froe[4 * nface + o] = E.cm;
-  froe[5 * nface + o] = E.rcm;
-  froe[6 * nface + o] = E.b1;
+  par::eig_store(E, froe + o, nface);
 }
 
 // Training stencils of the learned classifier from the current state (see harvest.cuh): every
@@ -275,9 +272,10 @@ __global__ void __launch_bounds__(kFaceThreads) kp_audit64(Geo G, const double* 
       for (int b = 0; b < 8; ++b) {
         if (!((route >> b) & 1)) continue;
         const double* v = ch[b >> 1] + (b & 1);  // side 1 reconstructs from cells 1..5
-        double SI[3];
-        par::lagrange_si(v, SI);
-        const int bad = par::teno_decide(v, SI, G.recon == HTENO_RECON_TENO5I) != 7;
+        const par::fp vf[5] = {v[0], v[1], v[2], v[3], v[4]};
+        par::fp SI[3];
+        par::lagrange_si(vf, SI);
+        const int bad = par::teno_decide(vf, SI, G.recon == HTENO_RECON_TENO5I) != 7;
         double lo = v[0], hi = v[0];
         for (int m = 1; m < 5; ++m) {
           lo = fmin(lo, v[m]);
@@ -368,7 +366,7 @@ __global__ void __launch_bounds__(kFaceThreads) kp_faces_g(Geo G, const double* 
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     double va, vb;
-    par::lagrange_recon(c_dev, G.recon, ch[r], va, vb);
+    par::lagrange_recon(g_dev, G.recon, ch[r], va, vb);
     if (interior) {
       fc[r * nface + o] = va;
       fc[(4 + r) * nface + o] = vb;
@@ -378,13 +376,29 @@ __global__ void __launch_bounds__(kFaceThreads) kp_faces_g(Geo G, const double* 
     }
   }
   if (!interior) return;
-  froe[0 * nface + o] = E.vxm;
-  froe[1 * nface + o] = E.vym;
-  froe[2 * nface + o] = E.hm;
-  froe[3 * nface + o] = E.qm;
-  froe[4 * nface + o] = E.cm;
-  froe[5 * nface + o] = E.rcm;
-  froe[6 * nface + o] = E.b1;
+  par::eig_store(E, froe + o, nface);
+}
+
+// The flux of a face from the GL3 values g[array][Gauss point] of its 8 face arrays: R
+// back-projection, HLLC or Rusanov at the three Gauss points, quadrature (FV_System2D.cpp:432-497).
+template <int DIR>
+__device__ __forceinline__ void face_flux(const Geo& G, const par::Eig& E, const double (&g)[8][3], double* F) {
+  par::fp acc[4];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const par::fp cl[4] = {g[0][m], g[1][m], g[2][m], g[3][m]};
+    const par::fp cr[4] = {g[4][m], g[5][m], g[6][m], g[7][m]};
+    par::fp ql[4], qr[4], Fl[4];
+    par::right(E, DIR, cl, ql);
+    par::right(E, DIR, cr, qr);
+    if (G.flux == HTENO_FLUX_HLLC) par::hllc(G.g1, DIR, ql, qr, Fl);
+    else par::rusanov(G.gamma, G.g1, DIR, E, ql, qr, Fl);
+    const par::fp w = par::ldk(g_dev.gl3w[m]);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) acc[v] = m == 0 ? w * Fl[v] : acc[v] + w * Fl[v];
+  }
+#pragma unroll
+  for (int v = 0; v < 4; ++v) F[v] = acc[v].v;
 }
 
 template <int DIR>
@@ -428,38 +442,14 @@ __global__ void __launch_bounds__(kFaceThreads) kp_flux(Geo G, const double* __r
       else
         u5[m] = fc[r * nface + nb[m]];
     }
-    par::gl3(c_dev, u5, g[r]);
+    par::gl3(g_dev, u5, g[r]);
   }
   const size_t o = nb[2];
-  par::Eig E;
-  E.vxm = froe[o];
-  E.vym = froe[nface + o];
-  E.hm = froe[2 * nface + o];
-  E.qm = froe[3 * nface + o];
-  E.cm = froe[4 * nface + o];
-  E.rcm = froe[5 * nface + o];
-  E.b1 = froe[6 * nface + o];
-  const double vn = DIR == 1 ? E.vxm : E.vym;  // derived scalars, recomputed bit-identically
-  E.t0r = vn * E.cm;
-  E.b2 = E.qm * E.b1;
-  E.s0 = vn * E.rcm;
-  E.s1 = E.b1 * vn;
-  E.t2 = 0.5 * E.b1;
-  double Fm[3][4];
+  const par::Eig E = par::eig_load(DIR, froe + o, nface);
+  double Ff[4];
+  face_flux<DIR>(G, E, g, Ff);
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const double cl[4] = {g[0][m], g[1][m], g[2][m], g[3][m]};
-    const double cr[4] = {g[4][m], g[5][m], g[6][m], g[7][m]};
-    double ql[4], qr[4], Fl[4];
-    par::right(E, DIR, cl, ql);
-    par::right(E, DIR, cr, qr);
-    if (G.flux == HTENO_FLUX_HLLC) par::hllc(G.g1, DIR, ql, qr, Fl);
-    else par::rusanov(G.gamma, G.g1, DIR, E, ql, qr, Fl);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) Fm[m][v] = c_dev.gl3w[m] * Fl[v];
-  }
-#pragma unroll
-  for (int v = 0; v < 4; ++v) F[v * nface + o] = (Fm[0][v] + Fm[1][v]) + Fm[2][v];
+  for (int v = 0; v < 4; ++v) F[v * nface + o] = Ff[v];
 }
 
 // rhs (FV_System2D.cpp:562-572) + RungeKutta3 (:575-612); stage 0 writes the residual
@@ -482,9 +472,9 @@ __global__ void kp_update(Geo G, int stage, const double* __restrict__ fx,
       const par::Den da = par::den_of(G.area);  // the four divisions by the cell area
 #pragma unroll
       for (int v = 0; v < 4; ++v)
-        rhs[v] = par::quot((fx[v * nxf + ox] - fx[v * nxf + ox + 1]) * G.dy +
-                               (fy[v * nyf + oy] - fy[v * nyf + oy + G.nx]) * G.dx,
-                           da) + 0.0;
+        rhs[v] = par::quot((par::fp(fx[v * nxf + ox]) - fx[v * nxf + ox + 1]) * G.dy +
+                               (par::fp(fy[v * nyf + oy]) - fy[v * nyf + oy + G.nx]) * G.dx,
+                           da).v + 0.0;
     }
     if (stage == 0) {
 #pragma unroll
@@ -633,7 +623,7 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
         double lo, hi;
-        par::lagrange_recon(c_dev, G.recon, ch[a], lo, hi);
+        par::lagrange_recon(g_dev, G.recon, ch[a], lo, hi);
         S.c[a][it] = lo;
         S.c[4 + a][it] = hi;
       }
@@ -649,26 +639,15 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
         double u5[5];
 #pragma unroll
         for (int m = 0; m < 5; ++m) u5[m] = S.c[a][(t + m) * XF + f];
-        par::gl3(c_dev, u5, g[a]);
+        par::gl3(g_dev, u5, g[a]);
       }
       const size_t ca = size_t(row(t)) * G.nx + col(f - 1), cb = size_t(row(t)) * G.nx + col(f);
       const par::Eig E = par::eig(G.g1, 1, pin[3 * nc + ca], pin[ca], pin[nc + ca], pin[2 * nc + ca],
                                   pin[3 * nc + cb], pin[cb], pin[nc + cb], pin[2 * nc + cb]);
-      double Fm[3][4];
+      double Ff[4];
+      face_flux<1>(G, E, g, Ff);
 #pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        const double cl[4] = {g[0][m], g[1][m], g[2][m], g[3][m]};
-        const double cr[4] = {g[4][m], g[5][m], g[6][m], g[7][m]};
-        double ql[4], qr[4], Fl[4];
-        par::right(E, 1, cl, ql);
-        par::right(E, 1, cr, qr);
-        if (G.flux == HTENO_FLUX_HLLC) par::hllc(G.g1, 1, ql, qr, Fl);
-        else par::rusanov(G.gamma, G.g1, 1, E, ql, qr, Fl);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) Fm[m][v] = c_dev.gl3w[m] * Fl[v];
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) S.f[v][it] = (Fm[0][v] + Fm[1][v]) + Fm[2][v];
+      for (int v = 0; v < 4; ++v) S.f[v][it] = Ff[v];
     }
     __syncthreads();
     // E: x flux difference times dy of each non-uniform cell (kp_update's first term)
@@ -713,7 +692,7 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
         double lo, hi;
-        par::lagrange_recon(c_dev, G.recon, ch[a], lo, hi);
+        par::lagrange_recon(g_dev, G.recon, ch[a], lo, hi);
         S.c[a][it] = lo;
         S.c[4 + a][it] = hi;
       }
@@ -729,26 +708,15 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
         double u5[5];
 #pragma unroll
         for (int m = 0; m < 5; ++m) u5[m] = S.c[a][g * YC + t + m];
-        par::gl3(c_dev, u5, gg[a]);
+        par::gl3(g_dev, u5, gg[a]);
       }
       const size_t ca = size_t(row(g - 1)) * G.nx + col(t), cb = size_t(row(g)) * G.nx + col(t);
       const par::Eig E = par::eig(G.g1, 2, pin[3 * nc + ca], pin[ca], pin[nc + ca], pin[2 * nc + ca],
                                   pin[3 * nc + cb], pin[cb], pin[nc + cb], pin[2 * nc + cb]);
-      double Fm[3][4];
+      double Ff[4];
+      face_flux<2>(G, E, gg, Ff);
 #pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        const double cl[4] = {gg[0][m], gg[1][m], gg[2][m], gg[3][m]};
-        const double cr[4] = {gg[4][m], gg[5][m], gg[6][m], gg[7][m]};
-        double ql[4], qr[4], Fl[4];
-        par::right(E, 2, cl, ql);
-        par::right(E, 2, cr, qr);
-        if (G.flux == HTENO_FLUX_HLLC) par::hllc(G.g1, 2, ql, qr, Fl);
-        else par::rusanov(G.gamma, G.g1, 2, E, ql, qr, Fl);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) Fm[m][v] = c_dev.gl3w[m] * Fl[v];
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) S.f[v][it] = (Fm[0][v] + Fm[1][v]) + Fm[2][v];
+      for (int v = 0; v < 4; ++v) S.f[v][it] = Ff[v];
     }
     __syncthreads();
   }
@@ -765,8 +733,8 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
       const par::Den da = par::den_of(G.area);
 #pragma unroll
       for (int v = 0; v < 4; ++v)
-        rhs[v] = par::quot(S.rx[v][t][i] + (S.f[v][t * TX + i] - S.f[v][(t + 1) * TX + i]) * G.dx,
-                           da) + 0.0;
+        rhs[v] = par::quot(par::fp(S.rx[v][t][i]) + (par::fp(S.f[v][t * TX + i]) - S.f[v][(t + 1) * TX + i]) * G.dx,
+                           da).v + 0.0;
     }
     double qn[4];
 #pragma unroll
@@ -793,7 +761,7 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
 }  // namespace
 
 int fv2d_fp64_setup(hteno_solver* s) {
-  if (upload_const(c_dev, &g_mask, &g_mu) != cudaSuccess)
+  if (upload_const(&g_mask, &g_mu, g_dev) != cudaSuccess)
     return set_error(s, HTENO_ERR_CUDA, "constant upload failed");
   if (s->cfg.precision == HTENO_PREC_FP64 && !s->deep) {
     const cudaError_t e = cudaMalloc(&s->deep, size_t(s->cfg.nx) * s->cfg.ny);
@@ -1022,7 +990,7 @@ extern "C" int hteno_residual_noalloc(const hteno_config* cfg, const double* q, 
     }
     scratch = g_noalloc_ptr[dev];
   }
-  if (upload_const(c_dev, &g_noalloc_const, &g_mu) != cudaSuccess) return HTENO_ERR_CUDA;
+  if (upload_const(&g_noalloc_const, &g_mu, g_dev) != cudaSuccess) return HTENO_ERR_CUDA;
 
   Geo G{};  // every field set, as geo_of() sets them for a solver
   G.nx = c.nx;

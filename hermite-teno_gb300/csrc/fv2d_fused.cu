@@ -188,7 +188,7 @@ bool fused::encode_box_map(CUtensorMap* m, const double* base, int nx, int ny, i
 size_t fv2d_fused_work_bytes(int nx, int ny) { return 4 * size_t(nx) * ny * sizeof(double) + 256; }
 
 int fv2d_fused_setup(hteno_solver* s) {
-  if (upload_const(c_dev, &g_mask, &g_mu) != cudaSuccess)
+  if (upload_const(&g_mask, &g_mu, c_dev) != cudaSuccess)
     return set_error(s, HTENO_ERR_CUDA, "constant upload failed");
   for (int v = 0; v < kNumVariants; ++v) {
     const cudaError_t e = kVariants[v].prepare();

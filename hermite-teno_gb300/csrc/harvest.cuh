@@ -26,18 +26,18 @@ __device__ __forceinline__ bool keep(uint64_t seed, uint64_t id, double p) {
 }
 
 // Cut-off bits of the left-biased side of stencil w[0..5] (teno5, or teno5i when improved).
-__device__ __forceinline__ int label(const double* w, bool improved) {
-  double SI[3];
+__device__ __forceinline__ int label(const double* wd, bool improved) {
+  const par::fp w[5] = {wd[0], wd[1], wd[2], wd[3], wd[4]};
+  par::fp SI[3];
   par::lagrange_si(w, SI);
   double tau;
   if (!improved) {
-    tau = fabs(par::lagrange_b35(w) - (SI[0] + SI[2] + 4.0 * SI[1]) / 6.0);
+    const par::fp mean = par::quot(par::scaled(par::kFour, SI[1], SI[0] + SI[2]), par::den_lit(6.0, par::kRcp6));
+    tau = fabs((par::lagrange_b35(w) - mean).v);
   } else {
-    tau = SI[0];
-    tau = (tau < SI[1]) ? SI[1] : tau;
-    tau = (tau < SI[2]) ? SI[2] : tau;
+    tau = par::maxof3(SI);
   }
-  return par::cutoff_pattern(SI, tau, HTENO_LAG_EPSZ, HTENO_LAG_CT);
+  return par::cutoff_pattern(SI, tau, HTENO_LAG_CT);
 }
 
 // A stencil whose six values are equal once rounded to float is "flat": the float

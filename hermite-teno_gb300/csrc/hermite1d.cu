@@ -19,6 +19,7 @@ namespace hteno {
 namespace {
 
 __constant__ DevConst c_dev;
+__device__ DevConst g_dev;  // the same in global memory (double: par::ldk)
 unsigned long long g_mask = 0;
 std::mutex g_mu;
 
@@ -126,6 +127,7 @@ __global__ void kh1_sensor(GeoH1 G, HermiteK<T> K, const double* __restrict__ q,
   }
   __syncthreads();
   if (!any || e >= 3) return;
+  const par::Den dif = par::den_of(double(K.dif));
   // padded moments with periodic ghosts, then the in-place sweep over [k-1, nxx-k+1)
   double* vp = W.vpad + size_t(e) * nxx;
   for (int i = 0; i < nxx; ++i) vp[i] = v[size_t(e) * n + wrap(i, n)];
@@ -133,7 +135,7 @@ __global__ void kh1_sensor(GeoH1 G, HermiteK<T> K, const double* __restrict__ q,
   for (int i = kGhost - 1; i < nxx - kGhost + 1; ++i) {
     T uu[3] = {T(u[wrap(i - 1, n)]), T(u[wrap(i, n)]), T(u[wrap(i + 1, n)])};
     T dd[3] = {T(vp[i - 1]), T(vp[i]), T(vp[i + 1])};
-    if constexpr (std::is_same<T, double>::value) vp[i] = par::hermite_limiter(K, uu, dd);
+    if constexpr (std::is_same<T, double>::value) vp[i] = par::hermite_limiter(dif, uu, dd);
     else vp[i] = double(hermite_limiter(K, uu, dd));
   }
   for (int i = 0; i < n; ++i) v[size_t(e) * n + i] = vp[i + kGhost];
@@ -158,30 +160,35 @@ __global__ void kh1_faces(GeoH1 G, HermiteK<T> K, const double* __restrict__ q,
   prim1(G.g1, qb, wb, hb, sb);
   T fu[3], fv[3];
   if constexpr (std::is_same<T, double>::value) {
-    double R[9], L[9], A[3][4], B[3][4];
+    par::fp R[9], L[9];
+    double A[3][4], B[3][4];
     par::eig1(G.g1, sa, wa[1], ha, sb, wb[1], hb, R, L);
     for (int m = 0; m < 4; ++m) {
       const int c = wrap(ip - 1 + m, n);
-      const double a3[3] = {q[c], q[n + c], q[2 * n + c]};
-      const double b3[3] = {v[c], v[n + c], v[2 * n + c]};
-      double ca3[3], cb3[3];
+      const par::fp a3[3] = {q[c], q[n + c], q[2 * n + c]};
+      const par::fp b3[3] = {v[c], v[n + c], v[2 * n + c]};
+      par::fp ca3[3], cb3[3];
       par::mv3(L, a3, ca3);
       par::mv3(L, b3, cb3);
       for (int r = 0; r < 3; ++r) {
-        A[r][m] = ca3[r];
-        B[r][m] = cb3[r];
+        A[r][m] = ca3[r].v;
+        B[r][m] = cb3[r].v;
       }
     }
-    double cl[4][3];
+    par::fp cl[4][3];
     for (int r = 0; r < 3; ++r) {
       double o[4];
-      par::hermite_recon(c_dev, K, W.flags[3 * ip + r] ? 1 : 2, A[r], B[r], o);
+      par::hermite_recon(g_dev, K, W.flags[3 * ip + r] ? 1 : 2, A[r], B[r], o);
       for (int a = 0; a < 4; ++a) cl[a][r] = o[a];
     }
-    double X[4][3];
+    par::fp X[4][3], Fu[3], Fv[3];
     for (int a = 0; a < 4; ++a) par::mv3(R, cl[a], X[a]);
-    par::rusanov1(G.gamma, G.g1, L, R, X[0], X[1], fu);
-    par::drusanov1(G.gamma, G.g1, G.g3, L, R, X[0], X[1], X[2], X[3], fv);
+    par::rusanov1(G.gamma, G.g1, L, R, X[0], X[1], Fu);
+    par::drusanov1(G.gamma, G.g1, G.g3, L, R, X[0], X[1], X[2], X[3], Fv);
+    for (int c = 0; c < 3; ++c) {
+      fu[c] = Fu[c].v;
+      fv[c] = Fv[c].v;
+    }
   } else {
     const Roe1<T> R = roe1<T>(T(G.g1), T(sa), T(wa[1]), T(ha), T(sb), T(wb[1]), T(hb));
     T A[3][4], B[3][4];
@@ -285,7 +292,7 @@ void launch_step(hteno_solver* s, const GeoH1& G) {
 }  // namespace
 
 int hermite1d_setup(hteno_solver* s) {
-  if (upload_const(c_dev, &g_mask, &g_mu) != cudaSuccess)
+  if (upload_const(&g_mask, &g_mu, c_dev, g_dev) != cudaSuccess)
     return set_error(s, HTENO_ERR_CUDA, "constant upload failed");
   s->work_bytes = s->cfg.precision == HTENO_PREC_MIXED ? work_bytes_h1<float>(s->cfg.nx)
                                                        : work_bytes_h1<double>(s->cfg.nx);

@@ -16,7 +16,7 @@
 namespace hteno {
 
 int hermite2d_setup(hteno_solver* s) {
-  if (upload_const(c_dev, &g_mask, &g_mu) != cudaSuccess || hermite2d_fp64_setup(s) != HTENO_OK)
+  if (upload_const(&g_mask, &g_mu, c_dev, g_dev) != cudaSuccess || hermite2d_fp64_setup(s) != HTENO_OK)
     return set_error(s, HTENO_ERR_CUDA, "constant upload failed");
   if (s->cfg.bc != HTENO_BC_ZEROGRAD)
     return set_error(s, HTENO_ERR_UNSUPPORTED, "the Hermite 2D scheme uses zero-gradient boundaries");

@@ -6,7 +6,7 @@
 namespace hteno {
 
 int hermite2d_fp64_setup(hteno_solver* s) {
-  if (upload_const(c_dev, &g_mask, &g_mu) != cudaSuccess)
+  if (upload_const(&g_mask, &g_mu, c_dev, g_dev) != cudaSuccess)
     return set_error(s, HTENO_ERR_CUDA, "constant upload failed");
   return HTENO_OK;
 }

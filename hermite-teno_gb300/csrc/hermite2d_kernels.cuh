@@ -100,6 +100,7 @@ void hermite2d_fp64_prim(hteno_solver* s, const GeoH& G);
 namespace {
 
 __constant__ DevConst c_dev;
+__device__ DevConst g_dev;  // the same in global memory (double: par::ldk)
 unsigned long long g_mask = 0;
 std::mutex g_mu;
 
@@ -195,6 +196,7 @@ __global__ void __launch_bounds__(kLimThreads) kh_limit(GeoH G, HermiteK<T> K,
   };
   const int tid = threadIdx.x;
   const bool sweeper = tid < L && l0 + tid < nl;
+  const par::Den dif = par::den_of(double(K.dif));
   T um = T(0), u0 = T(0), dm = T(0), dcur = T(0);
   if (sweeper) {
     um = from_d<T>(q[at(l0 + tid, 0)]);
@@ -224,7 +226,7 @@ __global__ void __launch_bounds__(kLimThreads) kh_limit(GeoH G, HermiteK<T> K,
         T uu[3] = {um, u0, up};
         T dd[3] = {dm, dcur, dn};
         T lim;
-        if constexpr (std::is_same<T, double>::value) lim = par::hermite_limiter(K, uu, dd);
+        if constexpr (std::is_same<T, double>::value) lim = par::hermite_limiter(dif, uu, dd);
         else lim = hermite_limiter(K, uu, dd);
         sd[k][tid] = to_d<T>(lim);
         dm = lim;
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(kHFaceThreads) kh_faces(GeoH G, HermiteK<T> K,
       }
       for (int r = 0; r < 4; ++r) {
         double h[4];
-        par::hermite_recon(c_dev, K, 0, A[r], B[r], h);
+        par::hermite_recon(g_dev, K, 0, A[r], B[r], h);
         for (int a = 0; a < 4; ++a) fc[(a * 4 + r) * nface + o] = h[a];
       }
     }
@@ -473,18 +475,12 @@ __global__ void __launch_bounds__(kHFaceThreads) kh_faces(GeoH G, HermiteK<T> K,
       }
       for (int r = 0; r < 4; ++r) {
         double a, b;
-        par::lagrange_recon(c_dev, HTENO_RECON_TENO5, C[r], a, b);
+        par::lagrange_recon(g_dev, HTENO_RECON_TENO5, C[r], a, b);
         fc[(4 * 4 + r) * nface + o] = a;
         fc[(5 * 4 + r) * nface + o] = b;
       }
     }
-    froe[0 * nface + o] = E.vxm;
-    froe[1 * nface + o] = E.vym;
-    froe[2 * nface + o] = E.hm;
-    froe[3 * nface + o] = E.qm;
-    froe[4 * nface + o] = E.cm;
-    froe[5 * nface + o] = E.rcm;
-    froe[6 * nface + o] = E.b1;
+    par::eig_store(E, froe + o, nface);
     return;
   }
   const Roe2<T> R = roe2<T>(T(G.g1), prim[3 * nc + ca], prim[ca], prim[nc + ca], prim[2 * nc + ca],
@@ -580,45 +576,34 @@ __global__ void __launch_bounds__(kHFluxThreads) kh_flux(GeoH G, const T* __rest
     T u5[5];
 #pragma unroll
     for (int m = 0; m < 5; ++m) u5[m] = fc[size_t(a) * nface + nb[m]];
-    if constexpr (std::is_same<T, double>::value) par::gl3(c_dev, u5, &gat(a, 0));
+    if constexpr (std::is_same<T, double>::value) par::gl3(g_dev, u5, &gat(a, 0));
     else gl3(c_dev, u5, gat(a, 0), gat(a, 1), gat(a, 2));
   }
   const size_t o = nb[2];
   T acc[12];
   if constexpr (std::is_same<T, double>::value) {
-    par::Eig E;
-    E.vxm = froe[o];
-    E.vym = froe[nface + o];
-    E.hm = froe[2 * nface + o];
-    E.qm = froe[3 * nface + o];
-    E.cm = froe[4 * nface + o];
-    E.rcm = froe[5 * nface + o];
-    E.b1 = froe[6 * nface + o];
-    const double vn = DIR == 1 ? E.vxm : E.vym;
-    E.t0r = vn * E.cm;
-    E.b2 = E.qm * E.b1;
-    E.s0 = vn * E.rcm;
-    E.s1 = E.b1 * vn;
-    E.t2 = 0.5 * E.b1;
-    double Fk[3][12];
+    const par::Eig E = par::eig_load(DIR, froe + o, nface);
+    par::fp Fk[12];
     for (int m = 0; m < 3; ++m) {
-      double X[6][4];
+      par::fp X[6][4];
       for (int a = 0; a < 6; ++a) {
-        const double c[4] = {gat(4 * a + 0, m), gat(4 * a + 1, m), gat(4 * a + 2, m), gat(4 * a + 3, m)};
+        const par::fp c[4] = {gat(4 * a + 0, m), gat(4 * a + 1, m), gat(4 * a + 2, m), gat(4 * a + 3, m)};
         par::right(E, DIR, c, X[a]);
       }
-      double fu[4], fn[4], ft[4];
+      par::fp fu[4], fn[4], ft[4];
       par::rusanov(G.gamma, G.g1, DIR, E, X[0], X[1], fu);
       par::drusanov(G.gamma, G.g1, G.g3, DIR, E, X[0], X[1], X[2], X[3], fn);
       par::drusanov(G.gamma, G.g1, G.g3, DIR, E, X[0], X[1], X[4], X[5], ft);
-      const double wm = c_dev.gl3w[m];
+      const par::fp wm = par::ldk(g_dev.gl3w[m]);
+#pragma unroll
       for (int k = 0; k < 4; ++k) {
-        Fk[m][k] = wm * fu[k];
-        Fk[m][4 + k] = wm * fn[k];
-        Fk[m][8 + k] = wm * ft[k];
+        Fk[k] = m == 0 ? wm * fu[k] : Fk[k] + wm * fu[k];
+        Fk[4 + k] = m == 0 ? wm * fn[k] : Fk[4 + k] + wm * fn[k];
+        Fk[8 + k] = m == 0 ? wm * ft[k] : Fk[8 + k] + wm * ft[k];
       }
     }
-    for (int k = 0; k < 12; ++k) acc[k] = (Fk[0][k] + Fk[1][k]) + Fk[2][k];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k] = Fk[k].v;
   } else {
     Roe2<T> R;
     R.vxm = froe[o];

@@ -29,9 +29,10 @@ struct StepState {
   unsigned long long tma_tiles;  // mixed FV 2D tiles staged by a TMA box copy
 };
 
-// Per-device upload of the constant block of one translation unit.
-template <typename Sym>
-inline cudaError_t upload_const(const Sym& sym, unsigned long long* mask, std::mutex* mu) {
+// Per-device upload of the constant block of one translation unit (a __constant__ or __device__
+// variable, or one of each).
+template <typename... Sym>
+inline cudaError_t upload_const(unsigned long long* mask, std::mutex* mu, const Sym&... sym) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -39,7 +40,8 @@ inline cudaError_t upload_const(const Sym& sym, unsigned long long* mask, std::m
   if (dev < 64 && (*mask & (1ull << dev))) return cudaSuccess;
   DevConst h;
   fill_dev_const(&h);
-  e = cudaMemcpyToSymbol(sym, &h, sizeof(DevConst));
+  for (cudaError_t r : {cudaMemcpyToSymbol(sym, &h, sizeof(DevConst))...})
+    if (r != cudaSuccess) e = r;
   if (e == cudaSuccess && dev < 64) *mask |= (1ull << dev);
   return e;
 }

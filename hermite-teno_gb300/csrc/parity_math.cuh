@@ -19,6 +19,7 @@
 #pragma once
 
 #include "device_math.cuh"
+#include "fp3.cuh"
 #include "mixed_conv.cuh"
 #include "hermite_math.cuh"
 
@@ -37,17 +38,27 @@ __device__ __forceinline__ bool nan_bits(double x) {
 __device__ __forceinline__ double catchnan(double x) { return nan_bits(x) ? 1e-15 : x; }
 
 // dot of a 3-vector of coefficients with u[0..2], left to right (Eigen .dot in the reference)
-__device__ __forceinline__ double dot3(double c0, double c1, double c2, const double* u) {
-  double s = c0 * u[0];
+__device__ __forceinline__ fp dot3(fp c0, fp c1, fp c2, const fp* u) {
+  fp s = c0 * u[0];
   s = s + c1 * u[1];
   s = s + c2 * u[2];
   return s;
 }
-__device__ __forceinline__ double dot3v(const double* p, const double* w) {
-  double s = p[0] * w[0];
+__device__ __forceinline__ fp dot3v(const fp* p, const fp* w) {
+  fp s = p[0] * w[0];
   s = s + p[1] * w[1];
   s = s + p[2] * w[2];
   return s;
+}
+// column k of a coefficient table in global memory . u
+template <int N>
+__device__ __forceinline__ fp dot3t(const double (&t)[3][N], int k, const fp* u) {
+  return dot3(ldk(t[0][k]), ldk(t[1][k]), ldk(t[2][k]), u);
+}
+// p . the three weights at w (global memory)
+__device__ __forceinline__ fp dot3w(const fp* p, const double* w) {
+  const fp ww[3] = {ldk(w[0]), ldk(w[1]), ldk(w[2])};
+  return dot3v(p, ww);
 }
 
 // Correctly rounded a / b for several numerators over one denominator: y = RN(1/b) once, then per
@@ -55,53 +66,53 @@ __device__ __forceinline__ double dot3v(const double* p, const double* w) {
 // (Markstein, IBM J. Res. Dev. 34(1), 1990; Muller et al., Handbook of Floating-Point Arithmetic,
 // 2018, Sec. 4.7) q is a / b correctly rounded when y is within half an ulp of 1/b and q0 within
 // one ulp of a / b, barring underflow and overflow: 3 FP64 operations per quotient instead of a
-// division's ~10.  Operands outside [2^-500, 2^501) in magnitude (zeros, subnormals, infinities,
-// NaN) take the division itself, so the theorem's conditions hold wherever the short form is used.
+// division's ~10.  Operands outside [2^-500, 2^501) in magnitude (subnormals, infinities, NaN) take
+// the division itself, so the theorem's conditions hold wherever the short form is used; a
+// numerator of +0 gives q0 = r = q = 0 with the division's sign, so it takes the short form too.
 struct Den {
-  double b, y;
+  fp b, y;
   bool ok;
 };
 __device__ __forceinline__ bool mid_range(double x) {
   const unsigned e = (unsigned(__double2hiint(x)) >> 20) & 0x7ffu;
   return e - 523u <= 1000u;  // biased exponent in [523, 1523]
 }
-__device__ __forceinline__ Den den_of(double b) { return Den{b, __drcp_rn(b), mid_range(b)}; }
-__device__ __forceinline__ double quot(double a, const Den& d) {
-  if (d.ok && mid_range(a)) {
-    const double q0 = a * d.y;
-    const double r = fma(-d.b, q0, a);
-    return fma(r, d.y, q0);
+__device__ __forceinline__ Den den_of(fp b) { return Den{b, __drcp_rn(b.v), mid_range(b.v)}; }
+// a denominator known at compile time, from its value and RN(1 / value) in the table
+__device__ __forceinline__ Den den_lit(double b, Lit y) { return Den{b, lit(y), true}; }
+__device__ __forceinline__ fp quot(fp a, const Den& d) {
+  if (d.ok && (mid_range(a.v) || __double_as_longlong(a.v) == 0ll)) {
+    const fp q0 = a * d.y;
+    const double r = fma(-d.b.v, q0.v, a.v);
+    return fma(r, d.y.v, q0.v);
   }
-  return a / d.b;
+  return a.v / d.b.v;
 }
-constexpr double kRcp24 = 1.0 / 24.0;  // RN(1/24), RN(1/6), RN(1/5040), folded at compile time
-constexpr double kRcp6 = 1.0 / 6.0;
-constexpr double kRcp5040 = 1.0 / 5040.0;
 
 // ---- Schemes::Lagrange ----------------------------------------------------------------------
 
-// smoothnessMeasure (Schemes_Lagrange.cpp:1013-1026)
-__device__ __forceinline__ void lagrange_si(const double* v, double* SI) {
-  double c[3], b[3];
-  c[0] = v[2] - 2.0 * v[3] + v[4];
-  b[0] = 3.0 * v[2] - 4.0 * v[3] + v[4];
-  c[1] = v[1] - 2.0 * v[2] + v[3];
-  b[1] = v[1] - v[3];
-  c[2] = v[0] - 2.0 * v[1] + v[2];
-  b[2] = v[0] - 4.0 * v[1] + 3.0 * v[2];
+// smoothnessMeasure (Schemes_Lagrange.cpp:1013-1026).  The b are halved term by term (exact
+// scalings by powers of two of the reference's b / 2).
+__device__ __forceinline__ void lagrange_si(const fp* v, fp* SI) {
+  fp c[3], b[3];
+  const fp m2 = lit(kThreeHalves) * v[2];
+  c[0] = scaled(kNegTwo, v[3], v[2]) + v[4];
+  b[0] = scaled(kHalf, v[4], scaled(kNegTwo, v[3], m2));
+  c[1] = scaled(kNegTwo, v[2], v[1]) + v[3];
+  b[1] = scaled(kNegHalf, v[3], lit(kHalf) * v[1]);
+  c[2] = scaled(kNegTwo, v[1], v[0]) + v[2];
+  b[2] = scaled(kNegTwo, v[1], lit(kHalf) * v[0]) + m2;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) b[k] = b[k] / 2.0;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) SI[k] = b[k] * b[k] + (13.0 / 12.0) * c[k] * c[k];
+  for (int k = 0; k < 3; ++k) SI[k] = b[k] * b[k] + lit(kThirteenTwelfths) * c[k] * c[k];
 }
 // fullpointsSmootness (:1029-1034)
-__device__ __forceinline__ double lagrange_b35(const double* v) {
-  double r = v[4] * (6908.0 * v[4] - 51001.0 * v[3] + 67923.0 * v[2] - 38947.0 * v[1] +
-                     8209.0 * v[0]) +
-             v[3] * (104963.0 * v[3] - 299076.0 * v[2] + 179098.0 * v[1] - 38947.0 * v[0]) +
-             v[2] * (231153.0 * v[2] - 299076.0 * v[1] + 67923.0 * v[0]) +
-             v[1] * (104963.0 * v[1] - 51001.0 * v[0]) + 6908.0 * v[0] * v[0];
-  return quot(r, Den{5040.0, kRcp5040, true});  // r / 5040
+__device__ __forceinline__ fp lagrange_b35(const fp* v) {
+  const fp r = v[4] * (lit(k6908) * v[4] - lit(k51001) * v[3] + lit(k67923) * v[2] - lit(k38947) * v[1] +
+                       lit(k8209) * v[0]) +
+               v[3] * (lit(k104963) * v[3] - lit(k299076) * v[2] + lit(k179098) * v[1] - lit(k38947) * v[0]) +
+               v[2] * (lit(k231153) * v[2] - lit(k299076) * v[1] + lit(k67923) * v[0]) +
+               v[1] * (lit(k104963) * v[1] - lit(k51001) * v[0]) + lit(k6908) * v[0] * v[0];
+  return quot(r, den_lit(5040.0, kRcp5040));  // r / 5040
 }
 
 // 1/x to a relative 2^-45 for the cut-off decision only (never for a value that is kept): a
@@ -201,8 +212,9 @@ __device__ __forceinline__ bool scaled_ratios(const double* d, double tau, float
 // ratios in float from d_k = SI_k + epsz and tau (scaled_ratios, guard band 2^-13 relative, eight
 // times its error bound), or in double where the scaling cannot reach (guard band 1e-5); inside
 // the band the reference's arithmetic decides.
-__device__ __forceinline__ int cutoff_pattern(const double* SI, double tau, double epsz, double ct) {
-  const double d[3] = {SI[0] + epsz, SI[1] + epsz, SI[2] + epsz};
+__device__ __forceinline__ int cutoff_pattern(const fp* SI, double tau, double ct) {
+  constexpr double epsz = HTENO_LAG_EPSZ;  // of the Hermite schemes too
+  const double d[3] = {(SI[0] + lit(kEpsz)).v, (SI[1] + lit(kEpsz)).v, (SI[2] + lit(kEpsz)).v};
   float xf[3];
   bool near;
   int pat;
@@ -224,7 +236,7 @@ __device__ __forceinline__ int cutoff_pattern(const double* SI, double tau, doub
   if (near) {  // reference arithmetic: w_k = pow(1 + tau/(SI_k + epsz), 6) / sum
     double w[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) w[k] = pow(1.0 + tau / (SI[k] + epsz), 6.0);
+    for (int k = 0; k < 3; ++k) w[k] = pow(1.0 + tau / (SI[k].v + epsz), 6.0);
     const double s = (w[0] + w[1]) + w[2];
     pat = 0;
 #pragma unroll
@@ -235,36 +247,36 @@ __device__ __forceinline__ int cutoff_pattern(const double* SI, double tau, doub
 
 // The cut-off pattern of one side of teno5 (:481-511) / teno5i (:1235-1263) for the window v with
 // indicators SI (bit k set: candidate k kept).
-__device__ __forceinline__ int teno_decide(const double* v, const double* SI, bool improved) {
+__device__ __forceinline__ int teno_decide(const fp* v, const fp* SI, bool improved) {
   // All three indicators exactly zero (constant data): the three ratios 1 + tau/(0 + epsz) are
   // equal whatever tau is, and the cut-off keeps all candidates (pattern 7) -- decided without
   // tau, same bits.  (Equal values alone do not suffice: 3u - 4u + u can leave a rounding
   // residue in one indicator.)
   // The full arithmetic below gives pattern 7 on such a window too (three equal ratios), so the
   // shortcut is taken only when every active lane of the warp can take it: a warp never runs both.
-  if (zero_bits(SI[0]) && zero_bits(SI[1]) && zero_bits(SI[2])) return 7;
+  if (zero_bits(SI[0].v) && zero_bits(SI[1].v) && zero_bits(SI[2].v)) return 7;
   double tau;
   if (!improved) {
-    const double b35 = lagrange_b35(v);
-    tau = fabs(b35 - quot(SI[0] + SI[2] + 4.0 * SI[1], Den{6.0, kRcp6, true}));  // ... / 6.0
+    const fp b35 = lagrange_b35(v);
+    const fp mean = quot(scaled(kFour, SI[1], SI[0] + SI[2]), den_lit(6.0, kRcp6));  // ... / 6.0
+    tau = fabs((b35 - mean).v);
   } else {
-    tau = SI[0];
-    tau = (tau < SI[1]) ? SI[1] : tau;
-    tau = (tau < SI[2]) ? SI[2] : tau;
+    tau = SI[0].v;
+    tau = (tau < SI[1].v) ? SI[1].v : tau;
+    tau = (tau < SI[2].v) ? SI[2].v : tau;
   }
-  return cutoff_pattern(SI, tau, HTENO_LAG_EPSZ, HTENO_LAG_CT);
+  return cutoff_pattern(SI, tau, HTENO_LAG_CT);
 }
 
 // One side of teno5 / teno5i given the candidates p and stencil v.
-__device__ __forceinline__ double teno_side_si(const DevConst& C, const double* p, const double* v,
-                                               const double* SI, int side, bool improved) {
+__device__ __forceinline__ double teno_side_si(const DevConst& C, const fp* p, const fp* v,
+                                               const fp* SI, int side, bool improved) {
   const int pat = teno_decide(v, SI, improved);
-  const double* w = side ? C.wtab_p[pat] : C.wtab_m[pat];
-  return catchnan(dot3v(p, w));
+  return catchnan(dot3w(p, side ? C.wtab_p[pat] : C.wtab_m[pat]).v);
 }
-__device__ __forceinline__ double teno_side(const DevConst& C, const double* p, const double* v,
+__device__ __forceinline__ double teno_side(const DevConst& C, const fp* p, const fp* v,
                                             int side, bool improved) {
-  double SI[3];
+  fp SI[3];
   lagrange_si(v, SI);
   return teno_side_si(C, p, v, SI, side, improved);
 }
@@ -297,7 +309,10 @@ __device__ __forceinline__ double normalised(const double* p, double* w) {
   const double s = (w[0] + w[1]) + w[2];
 #pragma unroll
   for (int k = 0; k < 3; ++k) w[k] = w[k] / s;
-  return catchnan(dot3v(p, w));
+  double o = p[0] * w[0];
+  o = o + p[1] * w[1];
+  o = o + p[2] * w[2];
+  return catchnan(o);
 }
 
 // weno5N / teno5N indicators (:445-450) on the side's window v[0..4]; returns the 5-point
@@ -314,7 +329,13 @@ __device__ __forceinline__ double alt_side(const DevConst& C, int kind, const do
                                            const double* v, int side) {
   const double* d = side ? C.dkp : C.dkm;
   double SI[3], w[3];
-  if (kind == 3 || kind == 4 || kind == 7) lagrange_si(v, SI);
+  if (kind == 3 || kind == 4 || kind == 7) {
+    const fp vf[5] = {v[0], v[1], v[2], v[3], v[4]};
+    fp S[3];
+    lagrange_si(vf, S);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) SI[k] = S[k].v;
+  }
   if (kind == 3) {  // w_k = d_k / (eps + SI_k)^2
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -352,36 +373,48 @@ __device__ __forceinline__ double alt_side(const DevConst& C, int kind, const do
     for (int k = 0; k < 3; ++k) r[k] = 1.0 / (SI[k] + HTENO_LAG_EPSZ);
   }
   const int pat = cutoff_from_r(r, HTENO_LAG_CT);
-  const double* tw = side ? C.wtab_p[pat] : C.wtab_m[pat];
-  return catchnan(dot3v(p, tw));
+  const fp pf[3] = {p[0], p[1], p[2]};
+  return catchnan(dot3w(pf, side ? C.wtab_p[pat] : C.wtab_m[pat]).v);
 }
 
-// kind 0 teno5, 1 teno5i, 2 linear (:1219-1233), 3..7 the alternatives above
-__device__ __forceinline__ void lagrange_recon(const DevConst& C, int kind, const double* u,
+// kind 2 linear (:1219-1233) or an alternative (3..7), one side, from its candidates and window
+__device__ __forceinline__ double other_side(const DevConst& C, int kind, const fp* p, const fp* v, int side) {
+  if (kind == 2) return dot3w(p, side ? C.dkp : C.dkm).v;
+  const double pd[3] = {p[0].v, p[1].v, p[2].v};
+  const double vd[5] = {v[0].v, v[1].v, v[2].v, v[3].v, v[4].v};
+  return alt_side(C, kind, pd, vd, side);
+}
+
+// kind 0 teno5, 1 teno5i, 2 linear (:1219-1233), 3..7 the alternatives above.  C in global memory.
+__device__ __forceinline__ void lagrange_recon(const DevConst& C, int kind, const double* ud,
                                                double& outm, double& outp) {
-  double p[3];
-  p[0] = dot3(C.crj[0][1], C.crj[1][1], C.crj[2][1], u + 2);
-  p[1] = dot3(C.crj[0][2], C.crj[1][2], C.crj[2][2], u + 1);
-  p[2] = dot3(C.crj[0][3], C.crj[1][3], C.crj[2][3], u + 0);
+  const fp u[6] = {ud[0], ud[1], ud[2], ud[3], ud[4], ud[5]};
+  fp p[3], pp[3];
+  p[0] = dot3t(C.crj, 1, u + 2);
+  p[1] = dot3t(C.crj, 2, u + 1);
+  p[2] = dot3t(C.crj, 3, u + 0);
+  // the two sides' windows overlap in 5 cells: p1+ = p0-, p2+ = p1- (the same expressions on the
+  // same operands, the same bits)
+  pp[0] = dot3t(C.crj, 0, u + 3);
+  pp[1] = p[0];
+  pp[2] = p[1];
   if (kind <= 1) {
-    // teno5 / teno5i: the two sides' windows overlap in 5 cells, so the + side reuses two of the
-    // - side's candidates (p1+ = p0-, p2+ = p1-) and two of its indicator terms: the same
-    // expressions on the same operands, the same bits
-    double c[4], SIm[3], SIp[3];
-    c[0] = u[2] - 2.0 * u[3] + u[4];
-    c[1] = u[1] - 2.0 * u[2] + u[3];
-    c[2] = u[0] - 2.0 * u[1] + u[2];
-    c[3] = u[3] - 2.0 * u[4] + u[5];  // c0 of the + side
-    double t[4];
+    // teno5 / teno5i: two of the indicators' second-difference terms are shared as well
+    fp c[4], t[4], SIm[3], SIp[3], bm[3], bp[3];
+    c[0] = scaled(kNegTwo, u[3], u[2]) + u[4];
+    c[1] = scaled(kNegTwo, u[2], u[1]) + u[3];
+    c[2] = scaled(kNegTwo, u[1], u[0]) + u[2];
+    c[3] = scaled(kNegTwo, u[4], u[3]) + u[5];  // c0 of the + side
 #pragma unroll
-    for (int k = 0; k < 4; ++k) t[k] = (13.0 / 12.0) * c[k] * c[k];
-    double bm[3], bp[3];
-    bm[0] = (3.0 * u[2] - 4.0 * u[3] + u[4]) / 2.0;
-    bm[1] = (u[1] - u[3]) / 2.0;
-    bm[2] = (u[0] - 4.0 * u[1] + 3.0 * u[2]) / 2.0;
-    bp[0] = (3.0 * u[3] - 4.0 * u[4] + u[5]) / 2.0;
-    bp[1] = (u[2] - u[4]) / 2.0;
-    bp[2] = (u[1] - 4.0 * u[2] + 3.0 * u[3]) / 2.0;
+    for (int k = 0; k < 4; ++k) t[k] = lit(kThirteenTwelfths) * c[k] * c[k];
+    const fp m2 = lit(kThreeHalves) * u[2], m3 = lit(kThreeHalves) * u[3];
+    const fp h1 = lit(kHalf) * u[1];
+    bm[0] = scaled(kHalf, u[4], scaled(kNegTwo, u[3], m2));
+    bm[1] = scaled(kNegHalf, u[3], h1);
+    bm[2] = scaled(kNegTwo, u[1], lit(kHalf) * u[0]) + m2;
+    bp[0] = scaled(kHalf, u[5], scaled(kNegTwo, u[4], m3));
+    bp[1] = scaled(kNegHalf, u[4], lit(kHalf) * u[2]);
+    bp[2] = scaled(kNegTwo, u[2], h1) + m3;
     SIm[0] = bm[0] * bm[0] + t[0];
     SIm[1] = bm[1] * bm[1] + t[1];
     SIm[2] = bm[2] * bm[2] + t[2];
@@ -389,120 +422,116 @@ __device__ __forceinline__ void lagrange_recon(const DevConst& C, int kind, cons
     SIp[1] = bp[1] * bp[1] + t[0];
     SIp[2] = bp[2] * bp[2] + t[1];
     outm = teno_side_si(C, p, u, SIm, 0, kind == 1);
-    double pp[3];
-    pp[0] = dot3(C.crj[0][0], C.crj[1][0], C.crj[2][0], u + 3);
-    pp[1] = p[0];
-    pp[2] = p[1];
     outp = teno_side_si(C, pp, u + 1, SIp, 1, kind == 1);
     return;
   }
-  outm = kind == 2 ? dot3v(p, C.dkm) : alt_side(C, kind, p, u, 0);
-  p[0] = dot3(C.crj[0][0], C.crj[1][0], C.crj[2][0], u + 3);
-  p[1] = dot3(C.crj[0][1], C.crj[1][1], C.crj[2][1], u + 2);
-  p[2] = dot3(C.crj[0][2], C.crj[1][2], C.crj[2][2], u + 1);
-  outp = kind == 2 ? dot3v(p, C.dkp) : alt_side(C, kind, p, u + 1, 1);
+  outm = other_side(C, kind, p, u, 0);
+  outp = other_side(C, kind, pp, u + 1, 1);
 }
 
 // One side of lagrange_recon (side 0: u^-, side 1: u^+), the same arithmetic.
-__device__ __forceinline__ double lagrange_side(const DevConst& C, int kind, const double* u, int side) {
-  double p[3];
-  if (side == 0) {
-    p[0] = dot3(C.crj[0][1], C.crj[1][1], C.crj[2][1], u + 2);
-    p[1] = dot3(C.crj[0][2], C.crj[1][2], C.crj[2][2], u + 1);
-    p[2] = dot3(C.crj[0][3], C.crj[1][3], C.crj[2][3], u + 0);
-    return kind == 2 ? dot3v(p, C.dkm) : kind >= 3 ? alt_side(C, kind, p, u, 0)
-                                                   : teno_side(C, p, u, 0, kind == 1);
-  }
-  p[0] = dot3(C.crj[0][0], C.crj[1][0], C.crj[2][0], u + 3);
-  p[1] = dot3(C.crj[0][1], C.crj[1][1], C.crj[2][1], u + 2);
-  p[2] = dot3(C.crj[0][2], C.crj[1][2], C.crj[2][2], u + 1);
-  return kind == 2 ? dot3v(p, C.dkp) : kind >= 3 ? alt_side(C, kind, p, u + 1, 1)
-                                                 : teno_side(C, p, u + 1, 1, kind == 1);
+__device__ __forceinline__ double lagrange_side(const DevConst& C, int kind, const double* ud, int side) {
+  const fp v[5] = {side ? ud[1] : ud[0], side ? ud[2] : ud[1], side ? ud[3] : ud[2], side ? ud[4] : ud[3],
+                   side ? ud[5] : ud[4]};
+  // candidate k is column 1 + k - side of crj on the cells from 2 - k of the window
+  fp p[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p[k] = dot3t(C.crj, 1 + k - side, v + 2 - k);
+  return kind <= 1 ? teno_side(C, p, v, side, kind == 1) : other_side(C, kind, p, v, side);
 }
 
 
 // weno5JS3PointsQuadrature (Schemes_Lagrange.cpp:1155-1217).  Not inlined: the flux kernels call
-// it 8 times per face, and eight inlined copies overflow the instruction cache.
-static __device__ __noinline__ void gl3(const DevConst& C, const double* u, double* out) {
-  double bg[3], cg[3], s2[3];
-  bg[0] = u[0] - 4.0 * u[1] + 3.0 * u[2];
-  cg[0] = u[0] - 2.0 * u[1] + u[2];
+// it 8 times per face, and eight inlined copies overflow the instruction cache.  C in global memory.
+static __device__ __noinline__ void gl3(const DevConst& C, const double* ud, double* out) {
+  const fp u[5] = {ud[0], ud[1], ud[2], ud[3], ud[4]};
+  fp bg[3], cg[3], s2[3];
+  const fp m2 = lit(kThree) * u[2];
+  bg[0] = scaled(kNegFour, u[1], u[0]) + m2;
+  cg[0] = scaled(kNegTwo, u[1], u[0]) + u[2];
   bg[1] = u[1] - u[3];
-  cg[1] = u[1] - 2.0 * u[2] + u[3];
-  bg[2] = 3.0 * u[2] - 4.0 * u[3] + u[4];
-  cg[2] = u[2] - 2.0 * u[3] + u[4];
+  cg[1] = scaled(kNegTwo, u[2], u[1]) + u[3];
+  bg[2] = scaled(kNegFour, u[3], m2) + u[4];
+  cg[2] = scaled(kNegTwo, u[3], u[2]) + u[4];
+  const Den d24 = den_lit(24.0, kRcp24);
+  const fp n2 = lit(k23) * u[2];
+  fp p[3];
   // (taken only when every active lane of the warp can take it: the full arithmetic gives the same
   // bits on constant data, and a warp then never runs both)
-  if (__all_sync(__activemask(), zero_bits(bg[0]) && zero_bits(bg[1]) && zero_bits(bg[2]) &&
-                                     zero_bits(cg[0]) && zero_bits(cg[1]) && zero_bits(cg[2]))) {
+  if (__all_sync(__activemask(), zero_bits(bg[0].v) && zero_bits(bg[1].v) && zero_bits(bg[2].v) &&
+                                     zero_bits(cg[0].v) && zero_bits(cg[1].v) && zero_bits(cg[2].v))) {
     // every indicator is zero: the normalised weights are the constants gl3flat, which the host
     // computed with these same operations -- the same bits without the 24 divisions
-    double p[3];
-    p[0] = dot3(C.gp[0][0], C.gp[1][0], C.gp[2][0], u + 0);
-    p[1] = dot3(C.gp[0][1], C.gp[1][1], C.gp[2][1], u + 1);
-    p[2] = dot3(C.gp[0][2], C.gp[1][2], C.gp[2][2], u + 2);
-    out[0] = dot3v(p, C.gl3flat[0]);
-    const Den d24{24.0, kRcp24, true};
-    p[0] = quot(-u[0] + 2.0 * u[1] + 23.0 * u[2], d24);
-    p[1] = quot(-u[1] + 26.0 * u[2] - u[3], d24);
-    p[2] = quot(23.0 * u[2] + 2.0 * u[3] - u[4], d24);
-    double c = C.sumw0p * dot3v(p, C.gl3flat[1]);
-    c = c - C.sumw0m * dot3v(p, C.gl3flat[2]);
-    out[1] = c;
-    p[0] = dot3(C.gm[0][0], C.gm[1][0], C.gm[2][0], u + 0);
-    p[1] = dot3(C.gm[0][1], C.gm[1][1], C.gm[2][1], u + 1);
-    p[2] = dot3(C.gm[0][2], C.gm[1][2], C.gm[2][2], u + 2);
-    out[2] = dot3v(p, C.gl3flat[3]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) p[k] = dot3t(C.gp, k, u + k);
+    out[0] = dot3w(p, C.gl3flat[0]).v;
+    p[0] = quot(scaled(kTwo, u[1], -u[0]) + n2, d24);
+    p[1] = quot(-u[1] + lit(k26) * u[2] - u[3], d24);
+    p[2] = quot(scaled(kTwo, u[3], n2) - u[4], d24);
+    fp c = fp(ldk(C.sumw0p)) * dot3w(p, C.gl3flat[1]);
+    c = c - fp(ldk(C.sumw0m)) * dot3w(p, C.gl3flat[2]);
+    out[1] = c.v;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) p[k] = dot3t(C.gm, k, u + k);
+    out[2] = dot3w(p, C.gl3flat[3]).v;
 #pragma unroll
     for (int k = 0; k < 3; ++k) out[k] = catchnan(out[k]);
     return;
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const double si = 0.25 * (bg[k] * bg[k]) + (13.0 / 12.0) * (cg[k] * cg[k]);
-    const double e = 1e-6 + si;
+    // 0.25 bg^2 + 13/12 cg^2, the first product exact
+    const fp si = scaled(kQuarter, bg[k] * bg[k], lit(kThirteenTwelfths) * (cg[k] * cg[k]));
+    const fp e = lit(kEps6) + si;
     s2[k] = e * e;  // pow(eps + SI, 2)
   }
-  double p[3], w[3];
   const Den ds[3] = {den_of(s2[0]), den_of(s2[1]), den_of(s2[2])};  // each serves 4 weight sets
   auto weighted = [&](const double* lw) {
+    fp w[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) w[k] = quot(lw[k], ds[k]);
-    const double s = (w[0] + w[1]) + w[2];
-    const Den dn = den_of(s);
+    for (int k = 0; k < 3; ++k) w[k] = quot(ldk(lw[k]), ds[k]);
+    const Den dn = den_of((w[0] + w[1]) + w[2]);
 #pragma unroll
     for (int k = 0; k < 3; ++k) w[k] = quot(w[k], dn);
     return dot3v(p, w);
   };
-  p[0] = dot3(C.gp[0][0], C.gp[1][0], C.gp[2][0], u + 0);
-  p[1] = dot3(C.gp[0][1], C.gp[1][1], C.gp[2][1], u + 1);
-  p[2] = dot3(C.gp[0][2], C.gp[1][2], C.gp[2][2], u + 2);
-  out[0] = weighted(C.linwp);
-  const Den d24{24.0, kRcp24, true};
-  p[0] = quot(-u[0] + 2.0 * u[1] + 23.0 * u[2], d24);
-  p[1] = quot(-u[1] + 26.0 * u[2] - u[3], d24);
-  p[2] = quot(23.0 * u[2] + 2.0 * u[3] - u[4], d24);
-  double c = C.sumw0p * weighted(C.linw0p);
-  c = c - C.sumw0m * weighted(C.linw0m);
-  out[1] = c;
-  p[0] = dot3(C.gm[0][0], C.gm[1][0], C.gm[2][0], u + 0);
-  p[1] = dot3(C.gm[0][1], C.gm[1][1], C.gm[2][1], u + 1);
-  p[2] = dot3(C.gm[0][2], C.gm[1][2], C.gm[2][2], u + 2);
-  out[2] = weighted(C.linwm);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p[k] = dot3t(C.gp, k, u + k);
+  out[0] = weighted(C.linwp).v;
+  p[0] = quot(scaled(kTwo, u[1], -u[0]) + n2, d24);
+  p[1] = quot(-u[1] + lit(k26) * u[2] - u[3], d24);
+  p[2] = quot(scaled(kTwo, u[3], n2) - u[4], d24);
+  fp c = fp(ldk(C.sumw0p)) * weighted(C.linw0p);
+  c = c - fp(ldk(C.sumw0m)) * weighted(C.linw0m);
+  out[1] = c.v;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) p[k] = dot3t(C.gm, k, u + k);
+  out[2] = weighted(C.linwm).v;
 #pragma unroll
   for (int k = 0; k < 3; ++k) out[k] = catchnan(out[k]);
 }
 
 // ---- Equations::Euler2D ---------------------------------------------------------------------
 
-__device__ __forceinline__ void primitive(double g1, const double* q, double* w) {  // :20-26
+__device__ __forceinline__ fp operator/(fp a, fp b) { return fp(a.v / b.v); }
+__device__ __forceinline__ fp sqrt_abs(fp a) { return fp(sqrt(fabs(a.v))); }
+__device__ __forceinline__ fp max_(fp a, fp b) { return fp(fmax(a.v, b.v)); }
+
+__device__ __forceinline__ void primitive(double g1, const fp* q, fp* w) {  // :20-26
   w[0] = q[0];
   w[1] = q[1] / q[0];
   w[2] = q[2] / q[0];
-  w[3] = (q[3] - 0.5 * (q[1] * w[1] + q[2] * w[2])) * g1;
+  w[3] = scaled(kNegHalf, q[1] * w[1] + q[2] * w[2], q[3]) * g1;
+}
+__device__ __forceinline__ void primitive(double g1, const double* q, double* w) {
+  const fp qf[4] = {q[0], q[1], q[2], q[3]};
+  fp wf[4];
+  primitive(g1, qf, wf);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = wf[k].v;
 }
 
-__device__ __forceinline__ void flux(int dir, const double* q, const double* w, double* f) {
+__device__ __forceinline__ void flux(int dir, const fp* q, const fp* w, fp* f) {
   if (dir == 1) {
     f[0] = q[1];
     f[1] = q[1] * w[1] + w[3];
@@ -519,55 +548,92 @@ __device__ __forceinline__ void flux(int dir, const double* q, const double* w, 
 // Face eigensystem (eigen2DEuler, FV_System2D.cpp:265-361): the entries of R and L are kept as
 // the scalars the reference's matrices are built from.
 struct Eig {
-  double vxm, vym, hm, qm, cm, t0r;  // t0r = vn * cm (right eigenvectors)
-  double rcm, b1, b2, s0, s1, t2;    // left eigenvectors
+  fp vxm, vym, hm, qm, cm, t0r;  // t0r = vn * cm (right eigenvectors)
+  fp rcm, b1, b2, s0, s1, t2;    // left eigenvectors
 };
 
-__device__ __forceinline__ Eig eig(double g1, int dir, double sra, double ua, double va, double ha,
-                                   double srb, double ub, double vb, double hb) {
+__device__ __forceinline__ Eig eig(double g1, int dir, fp sra, fp ua, fp va, fp ha, fp srb, fp ub,
+                                   fp vb, fp hb) {
   Eig e;
-  double t0 = sra / (sra + srb);
-  const double t1 = 1.0 - t0;
+  const fp t0 = sra / (sra + srb);
+  const fp t1 = lit(kOne) - t0;
   e.vxm = t0 * ua + t1 * ub;
   e.vym = t0 * va + t1 * vb;
   e.hm = t0 * ha + t1 * hb;
-  e.qm = 0.5 * (e.vxm * e.vxm + e.vym * e.vym);
-  e.cm = sqrt(fabs(g1 * (e.hm - e.qm)));
-  const double vn = dir == 1 ? e.vxm : e.vym;
+  e.qm = lit(kHalf) * (e.vxm * e.vxm + e.vym * e.vym);
+  e.cm = sqrt_abs(fp(g1) * (e.hm - e.qm));
+  const fp vn = dir == 1 ? e.vxm : e.vym;
   e.t0r = vn * e.cm;
-  e.rcm = 1.0 / e.cm;
-  e.b1 = g1 * e.rcm * e.rcm;
+  e.rcm = lit(kOne) / e.cm;
+  e.b1 = fp(g1) * e.rcm * e.rcm;
   e.b2 = e.qm * e.b1;
   e.s0 = vn * e.rcm;
   e.s1 = e.b1 * vn;
-  e.t2 = 0.5 * e.b1;
+  e.t2 = lit(kHalf) * e.b1;
   return e;
+}
+
+// The eigensystem from its seven stored scalars (vxm, vym, hm, qm, cm, rcm, b1 with `stride`
+// between them), the derived ones recomputed with the same operations.
+__device__ __forceinline__ Eig eig_load(int dir, const double* f, size_t stride) {
+  Eig e;
+  e.vxm = f[0];
+  e.vym = f[stride];
+  e.hm = f[2 * stride];
+  e.qm = f[3 * stride];
+  e.cm = f[4 * stride];
+  e.rcm = f[5 * stride];
+  e.b1 = f[6 * stride];
+  const fp vn = dir == 1 ? e.vxm : e.vym;
+  e.t0r = vn * e.cm;
+  e.b2 = e.qm * e.b1;
+  e.s0 = vn * e.rcm;
+  e.s1 = e.b1 * vn;
+  e.t2 = lit(kHalf) * e.b1;
+  return e;
+}
+__device__ __forceinline__ void eig_store(const Eig& e, double* f, size_t stride) {
+  f[0] = e.vxm.v;
+  f[stride] = e.vym.v;
+  f[2 * stride] = e.hm.v;
+  f[3 * stride] = e.qm.v;
+  f[4 * stride] = e.cm.v;
+  f[5 * stride] = e.rcm.v;
+  f[6 * stride] = e.b1.v;
 }
 
 // L * q with the reference's left-to-right row sums (leftEigenVectorx/y, :133-205).  Zero entries
 // of L add exact zeros in the reference and are skipped; unit entries multiply exactly.
-__device__ __forceinline__ void left(const Eig& e, int dir, const double* q, double* c) {
-  const double l00 = 0.5 * (e.b2 + e.s0), l0n = -0.5 * (e.s1 + e.rcm);
-  const double l30 = 0.5 * (e.b2 - e.s0), l3n = -0.5 * (e.s1 - e.rcm);
-  const double l20 = 1.0 - e.b2;
+__device__ __forceinline__ void left(const Eig& e, int dir, const fp* q, fp* c) {
+  const fp half = lit(kHalf), nhalf = lit(kNegHalf);
+  const fp l00 = half * (e.b2 + e.s0), l0n = nhalf * (e.s1 + e.rcm);
+  const fp l30 = half * (e.b2 - e.s0), l3n = nhalf * (e.s1 - e.rcm);
+  const fp l20 = lit(kOne) - e.b2;
   if (dir == 1) {
-    const double lt = -e.t2 * e.vym, l2t = e.b1 * e.vym;
-    double s = l00 * q[0]; s = s + l0n * q[1]; s = s + lt * q[2]; s = s + e.t2 * q[3]; c[0] = s;
+    const fp lt = -e.t2 * e.vym, l2t = e.b1 * e.vym;
+    fp s = l00 * q[0]; s = s + l0n * q[1]; s = s + lt * q[2]; s = s + e.t2 * q[3]; c[0] = s;
     s = -e.vym * q[0]; s = s + q[2]; c[1] = s;
     s = l20 * q[0]; s = s + e.s1 * q[1]; s = s + l2t * q[2]; s = s + (-e.b1) * q[3]; c[2] = s;
     s = l30 * q[0]; s = s + l3n * q[1]; s = s + lt * q[2]; s = s + e.t2 * q[3]; c[3] = s;
   } else {
-    const double lt = -e.t2 * e.vxm, l2t = e.b1 * e.vxm;
-    double s = l00 * q[0]; s = s + lt * q[1]; s = s + l0n * q[2]; s = s + e.t2 * q[3]; c[0] = s;
+    const fp lt = -e.t2 * e.vxm, l2t = e.b1 * e.vxm;
+    fp s = l00 * q[0]; s = s + lt * q[1]; s = s + l0n * q[2]; s = s + e.t2 * q[3]; c[0] = s;
     s = -e.vxm * q[0]; s = s + q[1]; c[1] = s;
     s = l20 * q[0]; s = s + l2t * q[1]; s = s + e.s1 * q[2]; s = s + (-e.b1) * q[3]; c[2] = s;
     s = l30 * q[0]; s = s + lt * q[1]; s = s + l3n * q[2]; s = s + e.t2 * q[3]; c[3] = s;
   }
 }
+__device__ __forceinline__ void left(const Eig& e, int dir, const double* q, double* c) {
+  const fp qf[4] = {q[0], q[1], q[2], q[3]};
+  fp cf[4];
+  left(e, dir, qf, cf);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) c[k] = cf[k].v;
+}
 
 // R * c (rightEigenVectorx/y, :100-131, 169-180)
-__device__ __forceinline__ void right(const Eig& e, int dir, const double* c, double* q) {
-  double s = c[0]; s = s + c[2]; s = s + c[3]; q[0] = s;
+__device__ __forceinline__ void right(const Eig& e, int dir, const fp* c, fp* q) {
+  fp s = c[0]; s = s + c[2]; s = s + c[3]; q[0] = s;
   if (dir == 1) {
     s = (e.vxm - e.cm) * c[0]; s = s + e.vxm * c[2]; s = s + (e.vxm + e.cm) * c[3]; q[1] = s;
     s = e.vym * c[0]; s = s + c[1]; s = s + e.vym * c[2]; s = s + e.vym * c[3]; q[2] = s;
@@ -580,39 +646,38 @@ __device__ __forceinline__ void right(const Eig& e, int dir, const double* c, do
 }
 
 // HLLC (Equations_Euler2D.cpp:372-428)
-__device__ __forceinline__ void hllc(double g1, int dir, const double* ql, const double* qr,
-                                     double* F) {
+__device__ __forceinline__ void hllc(double g1, int dir, const fp* ql, const fp* qr, fp* F) {
   const int d1 = dir - 1;
-  double wl[4], wr[4], fl[4], qs[4];
+  fp wl[4], wr[4], fl[4], qs[4];
   primitive(g1, ql, wl);
   primitive(g1, qr, wr);
-  const double hl = (ql[3] + wl[3]) / wl[0];
-  const double hr = (qr[3] + wr[3]) / wr[0];
-  const double rr = sqrt(fabs(wr[0] / wl[0]));
-  const double rrr = 1.0 / (1.0 + rr);
-  double vm[2];
+  const fp hl = (ql[3] + wl[3]) / wl[0];
+  const fp hr = (qr[3] + wr[3]) / wr[0];
+  const fp rr = sqrt_abs(wr[0] / wl[0]);
+  const fp rrr = lit(kOne) / (lit(kOne) + rr);
+  fp vm[2];
   vm[0] = (wl[1] + wr[1] * rr) * rrr;
   vm[1] = (wl[2] + wr[2] * rr) * rrr;
-  const double qm = 0.5 * (vm[0] * vm[0] + vm[1] * vm[1]);
-  const double hm = (hl + hr * rr) * rrr;
-  const double cm = sqrt(fabs(g1 * (hm - qm)));
-  const double cl = sqrt(fabs(wl[3] / wl[0]));
-  const double cr = sqrt(fabs(wr[3] / wr[0]));
-  const double sl = fmin(wl[dir] - cl, vm[d1] - cm);
-  const double sr = fmax(wr[dir] + cr, vm[d1] + cm);
-  const double sm = (qr[dir] * (sr - wr[dir]) - ql[dir] * (sl - wl[dir]) + wl[3] - wr[3]) /
-                    (wr[0] * (sr - wr[dir]) - wl[0] * (sl - wl[dir]));
-  const double ps = wl[3] + wl[0] * (wl[dir] - sl) * (wl[dir] - sm);
+  const fp qm = lit(kHalf) * (vm[0] * vm[0] + vm[1] * vm[1]);
+  const fp hm = (hl + hr * rr) * rrr;
+  const fp cm = sqrt_abs(fp(g1) * (hm - qm));
+  const fp cl = sqrt_abs(wl[3] / wl[0]);
+  const fp cr = sqrt_abs(wr[3] / wr[0]);
+  const fp sl = fmin((wl[dir] - cl).v, (vm[d1] - cm).v);
+  const fp sr = fmax((wr[dir] + cr).v, (vm[d1] + cm).v);
+  const fp dl = sl - wl[dir], dr = sr - wr[dir];
+  const fp sm = (qr[dir] * dr - ql[dir] * dl + wl[3] - wr[3]) / (wr[0] * dr - wl[0] * dl);
+  const fp ps = wl[3] + wl[0] * (wl[dir] - sl) * (wl[dir] - sm);
   // The reference's four regions (:408-427).  The two star regions run the same expressions on
   // the left or the right operands (the energy term keeps the left pressure in both, as the
   // reference does), and so do the two outer regions, so the operands are selected first and
   // one copy of the arithmetic runs: a warp whose faces fall in different regions does not pay
   // for both.  Same operations in the same order on the same values: the same bits.
-  const bool outer_l = sl > 0.0;
-  const bool star_l = !outer_l && sl <= 0.0 && sm > 0.0;
-  const bool star_r = !outer_l && !star_l && sm <= 0.0 && sr >= 0.0;
+  const bool outer_l = sl.v > 0.0;
+  const bool star_l = !outer_l && sl.v <= 0.0 && sm.v > 0.0;
+  const bool star_r = !outer_l && !star_l && sm.v <= 0.0 && sr.v >= 0.0;
   const bool use_l = outer_l || star_l;
-  double q[4], w[4];
+  fp q[4], w[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     q[k] = use_l ? ql[k] : qr[k];
@@ -620,8 +685,8 @@ __device__ __forceinline__ void hllc(double g1, int dir, const double* ql, const
   }
   flux(dir, q, w, fl);
   if (star_l || star_r) {
-    const double s = use_l ? sl : sr;
-    const double nom = s - w[dir], den = s - sm;
+    const fp s = use_l ? sl : sr;
+    const fp nom = use_l ? dl : dr, den = s - sm;
     qs[0] = w[0] * nom / den;
     qs[1] = dir == 1 ? (nom * q[1] + ps - w[3]) / den : nom * q[1] / den;
     qs[2] = dir == 2 ? (nom * q[2] + ps - w[3]) / den : nom * q[2] / den;
@@ -634,19 +699,24 @@ __device__ __forceinline__ void hllc(double g1, int dir, const double* ql, const
   }
 }
 
-// characteristic Rusanov (:310-330) with maxLocalWaveSpeed (:221-246)
+// maxLocalWaveSpeed (:221-246): the four characteristic speeds' maxima of the two sides
+__device__ __forceinline__ void local_speeds(double g, int dir, const fp* wl, const fp* wr, fp* a) {
+  const fp cl = sqrt_abs(fp(g) * wl[3] / wl[0]);
+  const fp cr = sqrt_abs(fp(g) * wr[3] / wr[0]);
+  const fp vl = wl[dir], vr = wr[dir];
+  a[0] = max_(abs_(vl - cl), abs_(vr - cr));
+  a[1] = max_(abs_(vl), abs_(vr));
+  a[2] = a[1];
+  a[3] = max_(abs_(vl + cl), abs_(vr + cr));
+}
+
+// characteristic Rusanov (:310-330) with maxLocalWaveSpeed
 __device__ __forceinline__ void rusanov(double g, double g1, int dir, const Eig& e,
-                                        const double* ql, const double* qr, double* F) {
-  double wl[4], wr[4], a[4], fl[4], fr[4], d[4], m[4], rm[4];
+                                        const fp* ql, const fp* qr, fp* F) {
+  fp wl[4], wr[4], a[4], fl[4], fr[4], d[4], m[4], rm[4];
   primitive(g1, ql, wl);
   primitive(g1, qr, wr);
-  const double cl = sqrt(fabs(g * wl[3] / wl[0]));
-  const double cr = sqrt(fabs(g * wr[3] / wr[0]));
-  const double vl = wl[dir], vr = wr[dir];
-  a[0] = fmax(fabs(vl - cl), fabs(vr - cr));
-  a[1] = fmax(fabs(vl), fabs(vr));
-  a[2] = a[1];
-  a[3] = fmax(fabs(vl + cl), fabs(vr + cr));
+  local_speeds(g, dir, wl, wr, a);
   flux(dir, ql, wl, fl);
   flux(dir, qr, wr, fr);
 #pragma unroll
@@ -656,7 +726,7 @@ __device__ __forceinline__ void rusanov(double g, double g1, int dir, const Eig&
   for (int k = 0; k < 4; ++k) m[k] = a[k] * m[k];
   right(e, dir, m, rm);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) F[k] = 0.5 * (fl[k] + fr[k] - rm[k]);
+  for (int k = 0; k < 4; ++k) F[k] = lit(kHalf) * (fl[k] + fr[k] - rm[k]);
 }
 
 // maxSpeed over both directions (Equations_Euler2D.cpp:207-219)
@@ -667,63 +737,68 @@ __device__ __forceinline__ double max_speed2(double g, const double* w) {
 
 // ---- Equations::Euler1D (Equations_Euler1D.cpp) --------------------------------------------
 
-__device__ __forceinline__ void primitive1(double g1, const double* q, double* w) {  // :18-23
+__device__ __forceinline__ void primitive1(double g1, const fp* q, fp* w) {  // :18-23
   w[0] = q[0];
   w[1] = q[1] / q[0];
-  w[2] = (q[2] - 0.5 * q[1] * w[1]) * g1;
+  w[2] = scaled(kNegHalf, q[1] * w[1], q[2]) * g1;
 }
 
 // eigen1DEuler (FV_System1D.cpp:121-156), eigenvectors :55-89 as full row-major 3x3 matrices
-__device__ __forceinline__ void eig1(double g1, double sra, double ua, double ha, double srb,
-                                     double ub, double hb, double* R, double* L) {
-  double t0 = sra / (sra + srb);
-  const double t1 = 1.0 - t0;
-  const double vxm = t0 * ua + t1 * ub;
-  const double hm = t0 * ha + t1 * hb;
-  const double qm = 0.5 * vxm * vxm;
-  const double cm = sqrt(fabs(g1 * (hm - qm)));
+__device__ __forceinline__ void eig1(double g1, fp sra, fp ua, fp ha, fp srb, fp ub, fp hb, fp* R, fp* L) {
+  const fp one = lit(kOne), half = lit(kHalf), nhalf = lit(kNegHalf);
+  fp t0 = sra / (sra + srb);
+  const fp t1 = one - t0;
+  const fp vxm = t0 * ua + t1 * ub;
+  const fp hm = t0 * ha + t1 * hb;
+  const fp qm = half * vxm * vxm;
+  const fp cm = sqrt_abs(fp(g1) * (hm - qm));
   t0 = vxm * cm;
-  R[0] = 1.0; R[1] = 1.0; R[2] = 1.0;
+  R[0] = one; R[1] = one; R[2] = one;
   R[3] = vxm - cm; R[4] = vxm; R[5] = vxm + cm;
   R[6] = hm - t0; R[7] = qm; R[8] = hm + t0;
-  const double rcm = 1.0 / cm;
-  const double b1 = g1 * rcm * rcm;
-  const double b2 = qm * b1;
-  const double s0 = vxm * rcm;
-  const double s1 = b1 * vxm;
-  const double t2 = 0.5 * b1;
-  L[0] = 0.5 * (b2 + s0); L[1] = -0.5 * (s1 + rcm); L[2] = t2;
-  L[3] = 1.0 - b2; L[4] = s1; L[5] = -b1;
-  L[6] = 0.5 * (b2 - s0); L[7] = -0.5 * (s1 - rcm); L[8] = t2;
+  const fp rcm = one / cm;
+  const fp b1 = fp(g1) * rcm * rcm;
+  const fp b2 = qm * b1;
+  const fp s0 = vxm * rcm;
+  const fp s1 = b1 * vxm;
+  const fp t2 = half * b1;
+  L[0] = half * (b2 + s0); L[1] = nhalf * (s1 + rcm); L[2] = t2;
+  L[3] = one - b2; L[4] = s1; L[5] = -b1;
+  L[6] = half * (b2 - s0); L[7] = nhalf * (s1 - rcm); L[8] = t2;
 }
 
-__device__ __forceinline__ void mv3(const double* M, const double* x, double* y) {
+__device__ __forceinline__ void mv3(const fp* M, const fp* x, fp* y) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    double s = M[3 * i] * x[0];
+    fp s = M[3 * i] * x[0];
     s = s + M[3 * i + 1] * x[1];
     s = s + M[3 * i + 2] * x[2];
     y[i] = s;
   }
 }
 
-__device__ __forceinline__ void flux1(const double* q, const double* w, double* f) {
+__device__ __forceinline__ void flux1(const fp* q, const fp* w, fp* f) {
   f[0] = q[1];
   f[1] = q[1] * w[1] + w[2];
   f[2] = w[1] * (q[2] + w[2]);
 }
 
-// Rusanov (Equations_Euler1D.cpp:129-135) with maxLocalWaveSpeed (:96-107)
-__device__ __forceinline__ void rusanov1(double g, double g1, const double* L, const double* R,
-                                         const double* ql, const double* qr, double* F) {
-  double wl[3], wr[3], a[3], fl[3], fr[3], d[3], m[3], rm[3];
+// maxLocalWaveSpeed (Equations_Euler1D.cpp:96-107)
+__device__ __forceinline__ void local_speeds1(double g, const fp* wl, const fp* wr, fp* a) {
+  const fp cl = sqrt_abs(fp(g) * wl[2] / wl[0]);
+  const fp cr = sqrt_abs(fp(g) * wr[2] / wr[0]);
+  a[0] = max_(abs_(wl[1] - cl), abs_(wr[1] - cr));
+  a[1] = max_(abs_(wl[1]), abs_(wr[1]));
+  a[2] = max_(abs_(wl[1] + cl), abs_(wr[1] + cr));
+}
+
+// Rusanov (Equations_Euler1D.cpp:129-135) with maxLocalWaveSpeed
+__device__ __forceinline__ void rusanov1(double g, double g1, const fp* L, const fp* R,
+                                         const fp* ql, const fp* qr, fp* F) {
+  fp wl[3], wr[3], a[3], fl[3], fr[3], d[3], m[3], rm[3];
   primitive1(g1, ql, wl);
   primitive1(g1, qr, wr);
-  const double cl = sqrt(fabs(g * wl[2] / wl[0]));
-  const double cr = sqrt(fabs(g * wr[2] / wr[0]));
-  a[0] = fmax(fabs(wl[1] - cl), fabs(wr[1] - cr));
-  a[1] = fmax(fabs(wl[1]), fabs(wr[1]));
-  a[2] = fmax(fabs(wl[1] + cl), fabs(wr[1] + cr));
+  local_speeds1(g, wl, wr, a);
   flux1(ql, wl, fl);
   flux1(qr, wr, fr);
 #pragma unroll
@@ -733,51 +808,52 @@ __device__ __forceinline__ void rusanov1(double g, double g1, const double* L, c
   for (int k = 0; k < 3; ++k) m[k] = a[k] * m[k];
   mv3(R, m, rm);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) F[k] = 0.5 * (fl[k] + fr[k] - rm[k]);
+  for (int k = 0; k < 3; ++k) F[k] = lit(kHalf) * (fl[k] + fr[k] - rm[k]);
 }
 
-// HLLC (Equations_Euler1D.cpp:156-210)
-__device__ __forceinline__ void hllc1(double g1, const double* ql, const double* qr, double* F) {
-  double wl[3], wr[3], fl[3], fr[3], qs[3];
+// HLLC (Equations_Euler1D.cpp:156-210).  As in 2D the operands of the left or right region are
+// selected first and one copy of the arithmetic runs.
+__device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp* F) {
+  fp wl[3], wr[3], fl[3], qs[3];
   primitive1(g1, ql, wl);
   primitive1(g1, qr, wr);
-  const double hl = (ql[2] + wl[2]) / wl[0];
-  const double hr = (qr[2] + wr[2]) / wr[0];
-  const double rr = sqrt(fabs(wr[0] / wl[0]));
-  const double rrr = 1.0 / (1.0 + rr);
-  const double vm = (wl[1] + wr[1] * rr) * rrr;
-  const double qm = 0.5 * vm * vm;
-  const double hm = (hl + hr * rr) * rrr;
-  const double cm = sqrt(fabs(g1 * (hm - qm)));
-  const double cl = sqrt(fabs(wl[2] / wl[0]));
-  const double cr = sqrt(fabs(wr[2] / wr[0]));
-  const double sl = fmin(wl[1] - cl, vm - cm);
-  const double sr = fmax(wr[1] + cr, vm + cm);
-  const double sm = (qr[1] * (sr - wr[1]) - ql[1] * (sl - wl[1]) + wl[2] - wr[2]) /
-                    (wr[0] * (sr - wr[1]) - wl[0] * (sl - wl[1]));
-  const double ps = wl[2] + wl[0] * (wl[1] - sl) * (wl[1] - sm);
-  flux1(ql, wl, fl);
-  flux1(qr, wr, fr);
-  if (sl > 0.0) {
+  const fp hl = (ql[2] + wl[2]) / wl[0];
+  const fp hr = (qr[2] + wr[2]) / wr[0];
+  const fp rr = sqrt_abs(wr[0] / wl[0]);
+  const fp rrr = lit(kOne) / (lit(kOne) + rr);
+  const fp vm = (wl[1] + wr[1] * rr) * rrr;
+  const fp qm = lit(kHalf) * vm * vm;
+  const fp hm = (hl + hr * rr) * rrr;
+  const fp cm = sqrt_abs(fp(g1) * (hm - qm));
+  const fp cl = sqrt_abs(wl[2] / wl[0]);
+  const fp cr = sqrt_abs(wr[2] / wr[0]);
+  const fp sl = fmin((wl[1] - cl).v, (vm - cm).v);
+  const fp sr = fmax((wr[1] + cr).v, (vm + cm).v);
+  const fp dl = sl - wl[1], dr = sr - wr[1];
+  const fp sm = (qr[1] * dr - ql[1] * dl + wl[2] - wr[2]) / (wr[0] * dr - wl[0] * dl);
+  const fp ps = wl[2] + wl[0] * (wl[1] - sl) * (wl[1] - sm);
+  const bool outer_l = sl.v > 0.0;
+  const bool star_l = !outer_l && sl.v <= 0.0 && sm.v > 0.0;
+  const bool star_r = !outer_l && !star_l && sm.v <= 0.0 && sr.v >= 0.0;
+  const bool use_l = outer_l || star_l;
+  fp q[3], w[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) F[k] = fl[k];
-  } else if (sl <= 0.0 && sm > 0.0) {
-    const double nom = sl - wl[1], den = sl - sm;
-    qs[0] = wl[0] * nom / den;
-    qs[1] = (nom * ql[1] + ps - wl[2]) / den;
-    qs[2] = (nom * ql[2] - wl[2] * wl[1] + ps * sm) / den;
+  for (int k = 0; k < 3; ++k) {
+    q[k] = use_l ? ql[k] : qr[k];
+    w[k] = use_l ? wl[k] : wr[k];
+  }
+  flux1(q, w, fl);
+  if (star_l || star_r) {
+    const fp s = use_l ? sl : sr;
+    const fp nom = use_l ? dl : dr, den = s - sm;
+    qs[0] = w[0] * nom / den;
+    qs[1] = (nom * q[1] + ps - w[2]) / den;
+    qs[2] = (nom * q[2] - wl[2] * w[1] + ps * sm) / den;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) F[k] = fl[k] + sl * (qs[k] - ql[k]);
-  } else if (sm <= 0.0 && sr >= 0.0) {
-    const double nom = sr - wr[1], den = sr - sm;
-    qs[0] = wr[0] * nom / den;
-    qs[1] = (nom * qr[1] + ps - wr[2]) / den;
-    qs[2] = (nom * qr[2] - wl[2] * wr[1] + ps * sm) / den;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) F[k] = fr[k] + sr * (qs[k] - qr[k]);
+    for (int k = 0; k < 3; ++k) F[k] = fl[k] + s * (qs[k] - q[k]);
   } else {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) F[k] = fr[k];
+    for (int k = 0; k < 3; ++k) F[k] = fl[k];
   }
 }
 
@@ -788,162 +864,165 @@ __device__ __forceinline__ double max_speed1(double g, const double* w) {  // :9
 
 // ---- Schemes::Hermite (Schemes_Hermite.cpp) -------------------------------------------------
 
-// smoothnessMeasure (:515-526)
-__device__ __forceinline__ void hermite_si(const double* u, const double* v, double* SI) {
-  double b[3], c[3];
-  b[0] = -2.0 * (u[0] - u[1]) - v[0];
-  c[0] = -2.0 * (u[0] - u[1] + v[0]);
-  b[1] = -2.0 * (u[1] - u[2]) - v[2];
-  c[1] = 2.0 * (u[1] - u[2]) + 2.0 * v[2];
-  b[2] = (-u[0] + u[2]) / 2.0;
-  c[2] = u[0] - 2.0 * u[1] + u[2];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) SI[k] = (13.0 / 12.0) * (c[k] * c[k]) + b[k] * b[k];
+// smoothnessMeasure (:515-526).  The reference's c0, c1 are twice the sums kept here and its b2
+// half of the difference: the factors 4 and 1/4 of their squares are exact and ride in the sum.
+__device__ __forceinline__ void hermite_si(const fp* u, const fp* v, fp* SI) {
+  const fp u01 = u[0] - u[1], u12 = u[1] - u[2], c1 = lit(kThirteenTwelfths);
+  const fp b0 = scaled(kNegTwo, u01, -v[0]), x0 = u01 + v[0];
+  const fp b1 = scaled(kNegTwo, u12, -v[2]), x1 = u12 + v[2];
+  const fp b2 = u[2] - u[0], x2 = scaled(kNegTwo, u[1], u[0]) + u[2];
+  SI[0] = scaled(kFour, c1 * (x0 * x0), b0 * b0);
+  SI[1] = scaled(kFour, c1 * (x1 * x1), b1 * b1);
+  SI[2] = scaled(kQuarter, b2 * b2, c1 * (x2 * x2));
 }
-// smoothnessMeasureDerivative (:528-541)
-__device__ __forceinline__ void hermite_sid(const double* u, const double* d, double* SI) {
-  double b[3], c[3];
-  b[0] = 6.0 * (u[0] - u[1]) + (2.0 * d[0] + 4.0 * d[1]);
-  c[0] = 12.0 * (u[0] - u[1]) + 6.0 * (d[0] + d[1]);
-  b[1] = 6.0 * (u[2] - u[1]) - (4.0 * d[1] + 2.0 * d[2]);
-  c[1] = 12.0 * (u[1] - u[2]) + 6.0 * (d[1] + d[2]);
-  b[2] = u[0] - 2.0 * u[1] + u[2];
-  c[2] = 3.0 * (u[2] - u[0]) - 6.0 * d[1];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) SI[k] = (13.0 / 12.0) * (c[k] * c[k]) + b[k] * b[k];
+// smoothnessMeasureDerivative (:528-541); c0 and c1 as half the reference's
+__device__ __forceinline__ void hermite_sid(const fp* u, const fp* d, fp* SI) {
+  const fp c1 = lit(kThirteenTwelfths), six = lit(kSix), three = lit(kThree);
+  const fp s01 = six * (u[0] - u[1]), s21 = six * (u[2] - u[1]);
+  const fp b0 = scaled(kTwo, scaled(kTwo, d[1], d[0]), s01), x0 = s01 + three * (d[0] + d[1]);
+  const fp b1 = scaled(kNegTwo, scaled(kTwo, d[1], d[2]), s21), x1 = three * (d[1] + d[2]) - s21;
+  const fp b2 = scaled(kNegTwo, u[1], u[0]) + u[2], x2 = three * (u[2] - u[0]) - six * d[1];
+  SI[0] = scaled(kFour, c1 * (x0 * x0), b0 * b0);
+  SI[1] = scaled(kFour, c1 * (x1 * x1), b1 * b1);
+  SI[2] = c1 * (x2 * x2) + b2 * b2;
 }
 // fullPointsSI (:597-603)
-__device__ __forceinline__ double hermite_brk(const double* u, const double* d) {
-  return fabs((1029270.0 * u[2] - 2129184.0 * u[1] + 1099914.0 * u[0] + 281121.0 * d[0] -
-               494958.0 * d[2]) * d[0] +
-              (-1029270.0 * u[0] + 2129184.0 * u[1] - 1099914.0 * u[2] + 281121.0 * d[2]) * d[2] +
-              (1099445.0 * u[2] - 4317056.0 * u[1] + 2118166.0 * u[0]) * u[2] +
-              4317056.0 * (u[1] - u[0]) * u[1] + 1099445.0 * u[0] * u[0]) /
-         6720.0;
+__device__ __forceinline__ fp hermite_brk(const fp* u, const fp* d) {
+  const fp r = (lit(k1029270) * u[2] - lit(k2129184) * u[1] + lit(k1099914) * u[0] + lit(k281121) * d[0] -
+                lit(k494958) * d[2]) * d[0] +
+               (lit(k2129184) * u[1] - lit(k1029270) * u[0] - lit(k1099914) * u[2] + lit(k281121) * d[2]) * d[2] +
+               (lit(k1099445) * u[2] - lit(k4317056) * u[1] + lit(k2118166) * u[0]) * u[2] +
+               lit(k4317056) * (u[1] - u[0]) * u[1] + lit(k1099445) * u[0] * u[0];
+  return quot(abs_(r), den_lit(6720.0, kRcp6720));
 }
 // fullPointsSId (:605-612)
-__device__ __forceinline__ double hermite_brkd(const double* u, const double* d) {
-  return fabs((3156862.0 * d[2] + 13189240.0 * d[1] + 1710479.0 * d[0] - 9617754.0 * u[2] -
-               531552.0 * u[1] + 10149306.0 * u[0]) * d[0] +
-              (13189240.0 * d[2] + 26511200.0 * d[1] - 39700440.0 * u[2] + 39700440.0 * u[0]) * d[1] +
-              (1710479.0 * d[2] - 10149306.0 * u[2] + 531552.0 * u[1] + 9617754.0 * u[0]) * d[2] +
-              (15136011.0 * u[2] - 1076544.0 * u[1] - 29195478.0 * u[0]) * u[2] +
-              1076544.0 * (u[1] - u[0]) * u[1] + 15136011.0 * u[0] * u[0]) /
-         1680.0;
+__device__ __forceinline__ fp hermite_brkd(const fp* u, const fp* d) {
+  const fp r = (lit(k3156862) * d[2] + lit(k13189240) * d[1] + lit(k1710479) * d[0] - lit(k9617754) * u[2] -
+                lit(k531552) * u[1] + lit(k10149306) * u[0]) * d[0] +
+               (lit(k13189240) * d[2] + lit(k26511200) * d[1] - lit(k39700440) * u[2] + lit(k39700440) * u[0]) * d[1] +
+               (lit(k1710479) * d[2] - lit(k10149306) * u[2] + lit(k531552) * u[1] + lit(k9617754) * u[0]) * d[2] +
+               (lit(k15136011) * u[2] - lit(k1076544) * u[1] - lit(k29195478) * u[0]) * u[2] +
+               lit(k1076544) * (u[1] - u[0]) * u[1] + lit(k15136011) * u[0] * u[0];
+  return quot(abs_(r), den_lit(1680.0, kRcp1680));
 }
-__device__ __forceinline__ double maxof3(const double* s) {
-  double t = s[0];
-  t = (t < s[1]) ? s[1] : t;
-  t = (t < s[2]) ? s[2] : t;
+__device__ __forceinline__ double maxof3(const fp* s) {
+  double t = s[0].v;
+  t = (t < s[1].v) ? s[1].v : t;
+  t = (t < s[2].v) ? s[2].v : t;
   return t;
 }
+// tau of hteno (full: the full-stencil indicator) or htenoi (improved)
+__device__ __forceinline__ double hermite_tau(bool improved, fp full, const fp* SI) {
+  if (improved) return maxof3(SI);
+  return fabs(scaled(kNegQuarter, scaled(kTwo, SI[2], SI[0] + SI[1]), full).v);
+}
 // one hteno/htenoi output: cut-off (cutOff/cutOffd, :614-628) and the table weights
-__device__ __forceinline__ double hermite_weighted(const DevConst& C, int which, const double* p,
-                                                   const double* SI, double tau) {
-  const int pat = cutoff_pattern(SI, tau, 1e-40, 1e-3);
+__device__ __forceinline__ double hermite_weighted(const DevConst& C, int which, const fp* p,
+                                                   const fp* SI, double tau) {
+  const int pat = cutoff_pattern(SI, tau, HTENO_HER_CT);
   const double* w = which == 0 ? C.hwtab_m[pat] : which == 1 ? C.hwtab_p[pat]
                   : which == 2 ? C.hwtab_md[pat] : C.hwtab_pd[pat];
-  return catchnan(dot3v(p, w));
+  return catchnan(dot3w(p, w).v);
 }
 
 // kind 0 hteno (:295-379), 1 htenoi (:670-758), 2 linear (:760-812);
-// out = {u^-, u^+, d^-, d^+} at x_{i+1/2}
+// out = {u^-, u^+, d^-, d^+} at x_{i+1/2}.  C in global memory.
 __device__ __forceinline__ void hermite_recon(const DevConst& C, const HermiteK<double>& K,
-                                              int kind, const double* u, const double* d,
+                                              int kind, const double* uin, const double* din,
                                               double* out) {
+  const fp u[4] = {uin[0], uin[1], uin[2], uin[3]}, d[4] = {din[0], din[1], din[2], din[3]};
+  auto k = [](double c) { return fp(c); };
   if (kind == 2) {
-    out[0] = dot3(K.crjlin[0][0], K.crjlin[1][0], K.crjlin[2][0], u) + K.crjlin[3][0] * d[0] +
-             K.crjlin[4][0] * d[2];
-    out[1] = dot3(K.crjlin[0][1], K.crjlin[1][1], K.crjlin[2][1], u + 1) + K.crjlin[3][1] * d[1] +
-             K.crjlin[4][1] * d[3];
-    out[2] = dot3(K.crjlind[0][0], K.crjlind[1][0], K.crjlind[2][0], u) +
-             dot3(K.crjlind[3][0], K.crjlind[4][0], K.crjlind[5][0], d);
-    out[3] = dot3(K.crjlind[0][1], K.crjlind[1][1], K.crjlind[2][1], u + 1) +
-             dot3(K.crjlind[3][1], K.crjlind[4][1], K.crjlind[5][1], d + 1);
+    out[0] = (dot3(K.crjlin[0][0], K.crjlin[1][0], K.crjlin[2][0], u) + k(K.crjlin[3][0]) * d[0] +
+              k(K.crjlin[4][0]) * d[2]).v;
+    out[1] = (dot3(K.crjlin[0][1], K.crjlin[1][1], K.crjlin[2][1], u + 1) + k(K.crjlin[3][1]) * d[1] +
+              k(K.crjlin[4][1]) * d[3]).v;
+    out[2] = (dot3(K.crjlind[0][0], K.crjlind[1][0], K.crjlind[2][0], u) +
+              dot3(K.crjlind[3][0], K.crjlind[4][0], K.crjlind[5][0], d)).v;
+    out[3] = (dot3(K.crjlind[0][1], K.crjlind[1][1], K.crjlind[2][1], u + 1) +
+              dot3(K.crjlind[3][1], K.crjlind[4][1], K.crjlind[5][1], d + 1)).v;
     return;
   }
   const bool imp = kind == 1;
-  double ud[4];
+  fp ud[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) ud[k] = d[k] * K.dif;
-  double p[3], SI[3], tau;
-  p[0] = K.crj[0][0] * u[0] + K.crj[1][0] * u[1] + K.crj[2][0] * d[0];
-  p[1] = K.crj[0][1] * u[1] + K.crj[1][1] * u[2] + K.crj[2][1] * d[2];
-  p[2] = K.crj[0][2] * u[0] + K.crj[1][2] * u[1] + K.crj[2][2] * u[2];
+  for (int m = 0; m < 4; ++m) ud[m] = d[m] * k(K.dif);
+  fp p[3], SI[3];
+  p[0] = k(K.crj[0][0]) * u[0] + k(K.crj[1][0]) * u[1] + k(K.crj[2][0]) * d[0];
+  p[1] = k(K.crj[0][1]) * u[1] + k(K.crj[1][1]) * u[2] + k(K.crj[2][1]) * d[2];
+  p[2] = k(K.crj[0][2]) * u[0] + k(K.crj[1][2]) * u[1] + k(K.crj[2][2]) * u[2];
   hermite_si(u, ud, SI);
-  tau = imp ? maxof3(SI) : fabs(hermite_brk(u, ud) - 0.25 * (SI[0] + SI[1] + 2.0 * SI[2]));
-  out[0] = hermite_weighted(C, 0, p, SI, tau);
+  out[0] = hermite_weighted(C, 0, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brk(u, ud), SI));
 
-  p[0] = K.crjd[0][0] * u[0] + K.crjd[1][0] * u[1] + K.crjd[2][0] * d[0] + K.crjd[3][0] * d[1];
-  p[1] = K.crjd[0][1] * u[1] + K.crjd[1][1] * u[2] + K.crjd[2][1] * d[1] + K.crjd[3][1] * d[2];
-  p[2] = K.crjd[0][2] * u[0] + K.crjd[1][2] * u[1] + K.crjd[2][2] * u[2] + K.crjd[3][2] * d[1];
+  p[0] = k(K.crjd[0][0]) * u[0] + k(K.crjd[1][0]) * u[1] + k(K.crjd[2][0]) * d[0] + k(K.crjd[3][0]) * d[1];
+  p[1] = k(K.crjd[0][1]) * u[1] + k(K.crjd[1][1]) * u[2] + k(K.crjd[2][1]) * d[1] + k(K.crjd[3][1]) * d[2];
+  p[2] = k(K.crjd[0][2]) * u[0] + k(K.crjd[1][2]) * u[1] + k(K.crjd[2][2]) * u[2] + k(K.crjd[3][2]) * d[1];
   hermite_sid(u, ud, SI);
-  tau = imp ? maxof3(SI) : fabs(hermite_brkd(u, ud) - 0.25 * (SI[0] + SI[1] + 2.0 * SI[2]));
-  out[2] = hermite_weighted(C, 2, p, SI, tau);
+  out[2] = hermite_weighted(C, 2, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brkd(u, ud), SI));
 
-  p[0] = K.crj[1][1] * u[1] + K.crj[0][1] * u[2] - K.crj[2][1] * d[1];
-  p[1] = K.crj[1][0] * u[2] + K.crj[0][0] * u[3] - K.crj[2][0] * d[3];
-  p[2] = K.crj[2][2] * u[1] + K.crj[1][2] * u[2] + K.crj[0][2] * u[3];
+  p[0] = k(K.crj[1][1]) * u[1] + k(K.crj[0][1]) * u[2] - k(K.crj[2][1]) * d[1];
+  p[1] = k(K.crj[1][0]) * u[2] + k(K.crj[0][0]) * u[3] - k(K.crj[2][0]) * d[3];
+  p[2] = k(K.crj[2][2]) * u[1] + k(K.crj[1][2]) * u[2] + k(K.crj[0][2]) * u[3];
   hermite_si(u + 1, ud + 1, SI);
-  tau = imp ? maxof3(SI) : fabs(hermite_brk(u + 1, ud + 1) - 0.25 * (SI[0] + SI[1] + 2.0 * SI[2]));
-  out[1] = hermite_weighted(C, 1, p, SI, tau);
+  out[1] = hermite_weighted(C, 1, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brk(u + 1, ud + 1), SI));
 
-  p[0] = K.crjd[0][1] * u[1] + K.crjd[1][1] * u[2] + K.crjd[3][1] * d[1] + K.crjd[2][1] * d[2];
-  p[1] = K.crjd[0][0] * u[2] + K.crjd[1][0] * u[3] + K.crjd[3][0] * d[2] + K.crjd[2][0] * d[3];
-  p[2] = -(K.crjd[2][2] * u[1] + K.crjd[1][2] * u[2] + K.crjd[0][2] * u[3]) + K.crjd[3][2] * d[2];
+  p[0] = k(K.crjd[0][1]) * u[1] + k(K.crjd[1][1]) * u[2] + k(K.crjd[3][1]) * d[1] + k(K.crjd[2][1]) * d[2];
+  p[1] = k(K.crjd[0][0]) * u[2] + k(K.crjd[1][0]) * u[3] + k(K.crjd[3][0]) * d[2] + k(K.crjd[2][0]) * d[3];
+  p[2] = -(k(K.crjd[2][2]) * u[1] + k(K.crjd[1][2]) * u[2] + k(K.crjd[0][2]) * u[3]) + k(K.crjd[3][2]) * d[2];
   hermite_sid(u + 1, ud + 1, SI);
-  tau = imp ? maxof3(SI) : fabs(hermite_brkd(u + 1, ud + 1) - 0.25 * (SI[0] + SI[1] + 2.0 * SI[2]));
-  out[3] = hermite_weighted(C, 3, p, SI, tau);
+  out[3] = hermite_weighted(C, 3, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brkd(u + 1, ud + 1), SI));
 }
 
-// hermiteLimiter (Schemes_Hermite.cpp:634-662)
-__device__ __forceinline__ double hermite_limiter(const HermiteK<double>& K, const double* u,
-                                                  const double* d) {
-  double p[3];
-  p[0] = 0.75 * (u[2] - u[0]) / K.dif - 0.25 * (d[0] + d[2]);
-  p[1] = (u[1] - u[0]) / K.dif;
-  p[2] = (u[2] - u[1]) / K.dif;
-  const double lw[3] = {1.0 - 2E-5, 1E-5, 1E-5};
-  const double ud[3] = {d[0] * K.dif, d[1] * K.dif, d[2] * K.dif};
-  double sm[3];
+// hermiteLimiter (Schemes_Hermite.cpp:634-662); dif: the cell size, as a shared denominator
+__device__ __forceinline__ double hermite_limiter(const Den& dif, const double* uin, const double* din) {
+  const fp u[3] = {uin[0], uin[1], uin[2]}, d[3] = {din[0], din[1], din[2]};
+  fp p[3], sm[3], w[3];
+  p[0] = scaled(kNegQuarter, d[0] + d[2], quot(lit(kThreeQuarters) * (u[2] - u[0]), dif));
+  p[1] = quot(u[1] - u[0], dif);
+  p[2] = quot(u[2] - u[1], dif);
+  const fp ud[3] = {d[0] * dif.b, d[1] * dif.b, d[2] * dif.b};
   sm[0] = hermite_brk(u, ud);
   sm[1] = (u[0] - u[1]) * (u[0] - u[1]);
   sm[2] = (u[1] - u[2]) * (u[1] - u[2]);
-  const double ta = fabs(sm[0] - sm[1]) + fabs(sm[0] - sm[2]);
-  const double tau = ta * ta / 4.0;
-  double w[3];
+  const fp ta = abs_(sm[0] - sm[1]) + abs_(sm[0] - sm[2]);
+  const fp tau = lit(kQuarter) * (ta * ta);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) w[k] = lw[k] * (1.0 + tau / (sm[k] + 1e-6));
-  const double s = (w[0] + w[1]) + w[2];
+  for (int k = 0; k < 3; ++k)
+    w[k] = lit(k == 0 ? kLw0 : kLw1) * (lit(kOne) + tau / (sm[k] + lit(kEps6)));
+  const Den ds = den_of((w[0] + w[1]) + w[2]);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) w[k] = w[k] / s;
-  const double r1 = lw[1] / lw[0], r2 = lw[2] / lw[0];
-  double inner = r1 * p[1];
-  inner = inner + r2 * p[2];
-  double w12 = w[1] * p[1];
+  for (int k = 0; k < 3; ++k) w[k] = quot(w[k], ds);
+  const fp r12 = lit(kLw1OverLw0);
+  fp inner = r12 * p[1];
+  inner = inner + r12 * p[2];
+  fp w12 = w[1] * p[1];
   w12 = w12 + w[2] * p[2];
-  return w[0] * (p[0] / lw[0] - inner) + w12;
+  return (w[0] * (quot(p[0], den_lit(1.0 - 2E-5, kRcpLw0)) - inner) + w12).v;
+}
+__device__ __forceinline__ double hermite_limiter(const HermiteK<double>& K, const double* u, const double* d) {
+  return hermite_limiter(den_of(K.dif), u, d);
 }
 
 // A(q) * x with the Jacobians dfluxx / dfluxy (Equations_Euler2D.cpp:52-98), row sums left to
 // right; zero and unit entries as in the reference's matrices.
-__device__ __forceinline__ void dflux_apply(double g, double g1, double g3, int dir, const double* q,
-                                            const double* w, const double* x, double* y) {
+__device__ __forceinline__ void dflux_apply(fp g, fp g1, fp g3, int dir, const fp* q, const fp* w,
+                                            const fp* x, fp* y) {
+  const fp half = lit(kHalf);
   if (dir == 1) {
-    const double sv = w[1] * w[1];
-    const double dv = 0.5 * g1 * (sv + w[2] * w[2]);
-    const double h = (q[3] + w[3]) / w[0];
+    const fp sv = w[1] * w[1];
+    const fp dv = half * g1 * (sv + w[2] * w[2]);
+    const fp h = (q[3] + w[3]) / w[0];
     y[0] = x[1];
-    double s = (dv - sv) * x[0]; s = s + (-g3 * w[1]) * x[1]; s = s + (-g1 * w[2]) * x[2]; s = s + g1 * x[3]; y[1] = s;
+    fp s = (dv - sv) * x[0]; s = s + (-g3 * w[1]) * x[1]; s = s + (-g1 * w[2]) * x[2]; s = s + g1 * x[3]; y[1] = s;
     s = (-w[1] * w[2]) * x[0]; s = s + w[2] * x[1]; s = s + w[1] * x[2]; y[2] = s;
     s = ((dv - h) * w[1]) * x[0]; s = s + (h - g1 * sv) * x[1]; s = s + (-g1 * w[1] * w[2]) * x[2];
     s = s + (g * w[1]) * x[3]; y[3] = s;
   } else {
-    const double sv = w[2] * w[2];
-    const double dv = 0.5 * g1 * (sv + w[1] * w[1]);
-    const double h = (q[3] + w[3]) / w[0];
+    const fp sv = w[2] * w[2];
+    const fp dv = half * g1 * (sv + w[1] * w[1]);
+    const fp h = (q[3] + w[3]) / w[0];
     y[0] = x[2];
-    double s = (-w[1] * w[2]) * x[0]; s = s + w[2] * x[1]; s = s + w[1] * x[2]; y[1] = s;
+    fp s = (-w[1] * w[2]) * x[0]; s = s + w[2] * x[1]; s = s + w[1] * x[2]; y[1] = s;
     s = (dv - sv) * x[0]; s = s + (-g1 * w[1]) * x[1]; s = s + (-g3 * w[2]) * x[2]; s = s + g1 * x[3]; y[2] = s;
     s = ((dv - h) * w[2]) * x[0]; s = s + (-g1 * w[1] * w[2]) * x[1]; s = s + (h - g1 * sv) * x[2];
     s = s + (g * w[2]) * x[3]; y[3] = s;
@@ -952,20 +1031,13 @@ __device__ __forceinline__ void dflux_apply(double g, double g1, double g3, int 
 
 // dRusanov (Equations_Euler2D.cpp:352-360) as called in FVHermite_System2D.cpp:553-589
 __device__ __forceinline__ void drusanov(double g, double g1, double g3, int dir, const Eig& e,
-                                         const double* ql, const double* qr, const double* dql,
-                                         const double* dqr, double* F) {
-  double wl[4], wr[4], a[4], d[4], m[4], al[4], ar[4], rm[4];
+                                         const fp* ql, const fp* qr, const fp* dql, const fp* dqr, fp* F) {
+  fp wl[4], wr[4], a[4], d[4], m[4], al[4], ar[4], rm[4];
   primitive(g1, ql, wl);
   primitive(g1, qr, wr);
   dflux_apply(g, g1, g3, dir, ql, wl, dql, al);
   dflux_apply(g, g1, g3, dir, qr, wr, dqr, ar);
-  const double cl = sqrt(fabs(g * wl[3] / wl[0]));
-  const double cr = sqrt(fabs(g * wr[3] / wr[0]));
-  const double vl = wl[dir], vr = wr[dir];
-  a[0] = fmax(fabs(vl - cl), fabs(vr - cr));
-  a[1] = fmax(fabs(vl), fabs(vr));
-  a[2] = a[1];
-  a[3] = fmax(fabs(vl + cl), fabs(vr + cr));
+  local_speeds(g, dir, wl, wr, a);
 #pragma unroll
   for (int k = 0; k < 4; ++k) d[k] = dqr[k] - dql[k];
   left(e, dir, d, m);
@@ -973,36 +1045,30 @@ __device__ __forceinline__ void drusanov(double g, double g1, double g3, int dir
   for (int k = 0; k < 4; ++k) m[k] = a[k] * m[k];
   right(e, dir, m, rm);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) F[k] = 0.5 * (al[k] + ar[k] - rm[k]);
+  for (int k = 0; k < 4; ++k) F[k] = lit(kHalf) * (al[k] + ar[k] - rm[k]);
 }
 
 // dflux 1D (Equations_Euler1D.cpp:39-53) applied to x; dRusanov 1D (:212-220)
-__device__ __forceinline__ void drusanov1(double g, double g1, double g3, const double* L,
-                                          const double* R, const double* ql, const double* qr,
-                                          const double* dql, const double* dqr, double* F) {
-  double wl[3], wr[3], a[3], d[3], m[3], rm[3], al[3], ar[3];
+__device__ __forceinline__ void drusanov1(double g, double g1, double g3, const fp* L, const fp* R,
+                                          const fp* ql, const fp* qr, const fp* dql, const fp* dqr, fp* F) {
+  fp wl[3], wr[3], a[3], d[3], m[3], rm[3], al[3], ar[3];
   primitive1(g1, ql, wl);
   primitive1(g1, qr, wr);
-  auto apply = [&](const double* q, const double* w, const double* x, double* y) {
-    double A[9];
-    A[0] = 0.0; A[1] = 1.0; A[2] = 0.0;
-    A[3] = 0.5 * g3 * w[1] * w[1];
-    A[4] = -g3 * w[1];
-    A[5] = g1;
-    A[6] = (g1 * (w[1] * w[1]) - g * q[2] / w[0]) * w[1];
-    A[7] = g * q[2] / w[0] - 1.5 * g1 * w[1] * w[1];
-    A[8] = g * w[1];
+  auto apply = [&](const fp* q, const fp* w, const fp* x, fp* y) {
+    const fp G(g), G1(g1), G3(g3);
+    const fp a3 = lit(kHalf) * G3 * w[1] * w[1];
+    const fp a4 = -G3 * w[1];
+    const fp e = G * q[2] / w[0];
+    const fp a6 = (G1 * (w[1] * w[1]) - e) * w[1];
+    const fp a7 = e - lit(kThreeHalves) * G1 * w[1] * w[1];
+    const fp a8 = G * w[1];
     y[0] = x[1];
-    double s = A[3] * x[0]; s = s + A[4] * x[1]; s = s + A[5] * x[2]; y[1] = s;
-    s = A[6] * x[0]; s = s + A[7] * x[1]; s = s + A[8] * x[2]; y[2] = s;
+    fp s = a3 * x[0]; s = s + a4 * x[1]; s = s + G1 * x[2]; y[1] = s;
+    s = a6 * x[0]; s = s + a7 * x[1]; s = s + a8 * x[2]; y[2] = s;
   };
   apply(ql, wl, dql, al);
   apply(qr, wr, dqr, ar);
-  const double cl = sqrt(fabs(g * wl[2] / wl[0]));
-  const double cr = sqrt(fabs(g * wr[2] / wr[0]));
-  a[0] = fmax(fabs(wl[1] - cl), fabs(wr[1] - cr));
-  a[1] = fmax(fabs(wl[1]), fabs(wr[1]));
-  a[2] = fmax(fabs(wl[1] + cl), fabs(wr[1] + cr));
+  local_speeds1(g, wl, wr, a);
 #pragma unroll
   for (int k = 0; k < 3; ++k) d[k] = dqr[k] - dql[k];
   mv3(L, d, m);
@@ -1010,7 +1076,7 @@ __device__ __forceinline__ void drusanov1(double g, double g1, double g3, const 
   for (int k = 0; k < 3; ++k) m[k] = a[k] * m[k];
   mv3(R, m, rm);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) F[k] = 0.5 * (al[k] + ar[k] - rm[k]);
+  for (int k = 0; k < 3; ++k) F[k] = lit(kHalf) * (al[k] + ar[k] - rm[k]);
 }
 
 }  // namespace par

@@ -15,12 +15,13 @@ namespace hteno {
 namespace {
 
 __constant__ DevConst c_dev;
+__device__ DevConst g_dev;  // the same in global memory (double: par::ldk)
 unsigned long long g_mask = 0;
 std::mutex g_mu;
 
 inline int prep(void* stream, cudaStream_t* st) {
   *st = static_cast<cudaStream_t>(stream);
-  return upload_const(c_dev, &g_mask, &g_mu) == cudaSuccess ? HTENO_OK : HTENO_ERR_CUDA;
+  return upload_const(&g_mask, &g_mu, c_dev, g_dev) == cudaSuccess ? HTENO_OK : HTENO_ERR_CUDA;
 }
 inline int finish() {
   cudaError_t e = cudaGetLastError();
@@ -35,7 +36,7 @@ __global__ void k_lagrange(int kind, const double* __restrict__ u, double* __res
   T v[6];
   for (int m = 0; m < 6; ++m) v[m] = static_cast<T>(u[6 * k + m]);
   T a, b;
-  if constexpr (std::is_same<T, double>::value) par::lagrange_recon(c_dev, kind, v, a, b);
+  if constexpr (std::is_same<T, double>::value) par::lagrange_recon(g_dev, kind, v, a, b);
   else lagrange_recon(c_dev, kind, v, a, b);
   out[2 * k] = a;
   out[2 * k + 1] = b;
@@ -50,7 +51,7 @@ __global__ void k_gl3(const double* __restrict__ u, double* __restrict__ out, lo
   T a, b, c;
   if constexpr (std::is_same<T, double>::value) {
     double o[3];
-    par::gl3(c_dev, v, o);
+    par::gl3(g_dev, v, o);
     a = o[0]; b = o[1]; c = o[2];
   } else {
     gl3(c_dev, v, a, b, c);
@@ -70,7 +71,7 @@ __global__ void k_hermite(int kind, HermiteK<T> K, const double* __restrict__ u,
     uu[m] = static_cast<T>(u[4 * k + m]);
     dd[m] = static_cast<T>(d[4 * k + m]);
   }
-  if constexpr (std::is_same<T, double>::value) par::hermite_recon(c_dev, K, kind, uu, dd, o);
+  if constexpr (std::is_same<T, double>::value) par::hermite_recon(g_dev, K, kind, uu, dd, o);
   else hermite_recon(c_dev, K, kind, uu, dd, o);
   for (int m = 0; m < 4; ++m) out[4 * k + m] = o[m];
 }
@@ -99,8 +100,14 @@ __global__ void k_hllc2(T g1, int dir, const double* __restrict__ ql, const doub
     a[m] = static_cast<T>(ql[4 * k + m]);
     b[m] = static_cast<T>(qr[4 * k + m]);
   }
-  if constexpr (std::is_same<T, double>::value) par::hllc(g1, dir, a, b, F);
-  else hllc2(g1, dir, a, b, F);
+  if constexpr (std::is_same<T, double>::value) {
+    const par::fp l[4] = {a[0], a[1], a[2], a[3]}, r[4] = {b[0], b[1], b[2], b[3]};
+    par::fp f[4];
+    par::hllc(g1, dir, l, r, f);
+    for (int m = 0; m < 4; ++m) F[m] = f[m].v;
+  } else {
+    hllc2(g1, dir, a, b, F);
+  }
   for (int m = 0; m < 4; ++m) out[4 * k + m] = F[m];
 }
 
@@ -114,8 +121,14 @@ __global__ void k_hllc1(T g1, const double* __restrict__ ql, const double* __res
     a[m] = static_cast<T>(ql[3 * k + m]);
     b[m] = static_cast<T>(qr[3 * k + m]);
   }
-  if constexpr (std::is_same<T, double>::value) par::hllc1(g1, a, b, F);
-  else hllc1(g1, a, b, F);
+  if constexpr (std::is_same<T, double>::value) {
+    const par::fp l[3] = {a[0], a[1], a[2]}, r[3] = {b[0], b[1], b[2]};
+    par::fp f[3];
+    par::hllc1(g1, l, r, f);
+    for (int m = 0; m < 3; ++m) F[m] = f[m].v;
+  } else {
+    hllc1(g1, a, b, F);
+  }
   for (int m = 0; m < 3; ++m) out[3 * k + m] = F[m];
 }
 
@@ -147,7 +160,10 @@ __global__ void k_rusanov2(T g, T g1, int dir, const double* __restrict__ qa,
     par::primitive(g1, qb + 4 * k, wb);
     const par::Eig E = par::eig(g1, dir, sqrt(fabs(wa[0])), wa[1], wa[2], (qa[4 * k + 3] + wa[3]) / wa[0],
                                 sqrt(fabs(wb[0])), wb[1], wb[2], (qb[4 * k + 3] + wb[3]) / wb[0]);
-    par::rusanov(g, g1, dir, E, a, b, F);
+    const par::fp l[4] = {a[0], a[1], a[2], a[3]}, r[4] = {b[0], b[1], b[2], b[3]};
+    par::fp f[4];
+    par::rusanov(g, g1, dir, E, l, r, f);
+    for (int m = 0; m < 4; ++m) F[m] = f[m].v;
   } else {
     Roe2<T> s = roe_of_pair(g1, qa + 4 * k, qb + 4 * k);
     rusanov2(g, g1, dir, s, a, b, F);
@@ -175,7 +191,11 @@ __global__ void k_drusanov2(T g, T g1, T g3, int dir, const double* __restrict__
     par::primitive(g1, qb + 4 * k, wb);
     const par::Eig E = par::eig(g1, dir, sqrt(fabs(wa[0])), wa[1], wa[2], (qa[4 * k + 3] + wa[3]) / wa[0],
                                 sqrt(fabs(wb[0])), wb[1], wb[2], (qb[4 * k + 3] + wb[3]) / wb[0]);
-    par::drusanov(g, g1, g3, dir, E, a, b, da, db, F);
+    const par::fp l[4] = {a[0], a[1], a[2], a[3]}, r[4] = {b[0], b[1], b[2], b[3]};
+    const par::fp dl[4] = {da[0], da[1], da[2], da[3]}, dr[4] = {db[0], db[1], db[2], db[3]};
+    par::fp f[4];
+    par::drusanov(g, g1, g3, dir, E, l, r, dl, dr, f);
+    for (int m = 0; m < 4; ++m) F[m] = f[m].v;
   } else {
     Roe2<T> s = roe_of_pair(g1, qa + 4 * k, qb + 4 * k);
     drusanov2(g, g1, dir, s, a, b, da, db, F);
