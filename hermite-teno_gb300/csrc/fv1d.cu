@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kThreads) k1_flux_lanes(Geo1 G, const double* 
   par::mv3(R, cl, ql);  // transformToConservative (FV_System1D.h:48-51)
   par::mv3(R, cr, qr);
   if (G.flux == HTENO_FLUX_HLLC) par::hllc1(G.g1, ql, qr, Ff);
-  else par::rusanov1(G.gamma, G.g1, L, R, ql, qr, Ff);
+  else par::rusanov1(par::sides1_of(G.gamma, G.g1, ql, qr), L, R, ql, qr, Ff);
   for (int v = 0; v < 3; ++v) F[v * (n + 1) + f] = Ff[v].v;
 }
 

@@ -392,7 +392,7 @@ __device__ __forceinline__ void face_flux(const Geo& G, const par::Eig& E, const
     par::right(E, DIR, cl, ql);
     par::right(E, DIR, cr, qr);
     if (G.flux == HTENO_FLUX_HLLC) par::hllc(G.g1, DIR, ql, qr, Fl);
-    else par::rusanov(G.gamma, G.g1, DIR, E, ql, qr, Fl);
+    else par::rusanov(DIR, E, par::sides_of(G.gamma, G.g1, DIR, ql, qr), ql, qr, Fl);
     const par::fp w = par::ldk(g_dev.gl3w[m]);
 #pragma unroll
     for (int v = 0; v < 4; ++v) acc[v] = m == 0 ? w * Fl[v] : acc[v] + w * Fl[v];

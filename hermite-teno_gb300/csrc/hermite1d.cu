@@ -183,8 +183,9 @@ __global__ void kh1_faces(GeoH1 G, HermiteK<T> K, const double* __restrict__ q,
     }
     par::fp X[4][3], Fu[3], Fv[3];
     for (int a = 0; a < 4; ++a) par::mv3(R, cl[a], X[a]);
-    par::rusanov1(G.gamma, G.g1, L, R, X[0], X[1], Fu);
-    par::drusanov1(G.gamma, G.g1, G.g3, L, R, X[0], X[1], X[2], X[3], Fv);
+    const par::Sides1 S = par::sides1_of(G.gamma, G.g1, X[0], X[1]);
+    par::rusanov1(S, L, R, X[0], X[1], Fu);
+    par::drusanov1(G.gamma, G.g1, G.g3, S, L, R, X[0], X[1], X[2], X[3], Fv);
     for (int c = 0; c < 3; ++c) {
       fu[c] = Fu[c].v;
       fv[c] = Fv[c].v;

@@ -591,9 +591,10 @@ __global__ void __launch_bounds__(kHFluxThreads) kh_flux(GeoH G, const T* __rest
         par::right(E, DIR, c, X[a]);
       }
       par::fp fu[4], fn[4], ft[4];
-      par::rusanov(G.gamma, G.g1, DIR, E, X[0], X[1], fu);
-      par::drusanov(G.gamma, G.g1, G.g3, DIR, E, X[0], X[1], X[2], X[3], fn);
-      par::drusanov(G.gamma, G.g1, G.g3, DIR, E, X[0], X[1], X[4], X[5], ft);
+      const par::Sides S = par::sides_of(G.gamma, G.g1, DIR, X[0], X[1]);
+      par::rusanov(DIR, E, S, X[0], X[1], fu);
+      par::drusanov(G.gamma, G.g1, G.g3, DIR, E, S, X[0], X[1], X[2], X[3], fn);
+      par::drusanov(G.gamma, G.g1, G.g3, DIR, E, S, X[0], X[1], X[4], X[5], ft);
       const par::fp wm = par::ldk(g_dev.gl3w[m]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {

@@ -517,16 +517,17 @@ __device__ __forceinline__ fp operator/(fp a, fp b) { return fp(a.v / b.v); }
 __device__ __forceinline__ fp sqrt_abs(fp a) { return fp(sqrt(fabs(a.v))); }
 __device__ __forceinline__ fp max_(fp a, fp b) { return fp(fmax(a.v, b.v)); }
 
-__device__ __forceinline__ void primitive(double g1, const fp* q, fp* w) {  // :20-26
+// The divisions by a density share one correctly rounded reciprocal: d = den_of(q[0]).
+__device__ __forceinline__ void primitive(double g1, const fp* q, const Den& d, fp* w) {  // :20-26
   w[0] = q[0];
-  w[1] = q[1] / q[0];
-  w[2] = q[2] / q[0];
+  w[1] = quot(q[1], d);
+  w[2] = quot(q[2], d);
   w[3] = scaled(kNegHalf, q[1] * w[1] + q[2] * w[2], q[3]) * g1;
 }
 __device__ __forceinline__ void primitive(double g1, const double* q, double* w) {
   const fp qf[4] = {q[0], q[1], q[2], q[3]};
   fp wf[4];
-  primitive(g1, qf, wf);
+  primitive(g1, qf, den_of(qf[0]), wf);
 #pragma unroll
   for (int k = 0; k < 4; ++k) w[k] = wf[k].v;
 }
@@ -649,11 +650,12 @@ __device__ __forceinline__ void right(const Eig& e, int dir, const fp* c, fp* q)
 __device__ __forceinline__ void hllc(double g1, int dir, const fp* ql, const fp* qr, fp* F) {
   const int d1 = dir - 1;
   fp wl[4], wr[4], fl[4], qs[4];
-  primitive(g1, ql, wl);
-  primitive(g1, qr, wr);
-  const fp hl = (ql[3] + wl[3]) / wl[0];
-  const fp hr = (qr[3] + wr[3]) / wr[0];
-  const fp rr = sqrt_abs(wr[0] / wl[0]);
+  const Den rl = den_of(ql[0]), rg = den_of(qr[0]);  // the left and right density
+  primitive(g1, ql, rl, wl);
+  primitive(g1, qr, rg, wr);
+  const fp hl = quot(ql[3] + wl[3], rl);
+  const fp hr = quot(qr[3] + wr[3], rg);
+  const fp rr = sqrt_abs(quot(wr[0], rl));
   const fp rrr = lit(kOne) / (lit(kOne) + rr);
   fp vm[2];
   vm[0] = (wl[1] + wr[1] * rr) * rrr;
@@ -661,8 +663,8 @@ __device__ __forceinline__ void hllc(double g1, int dir, const fp* ql, const fp*
   const fp qm = lit(kHalf) * (vm[0] * vm[0] + vm[1] * vm[1]);
   const fp hm = (hl + hr * rr) * rrr;
   const fp cm = sqrt_abs(fp(g1) * (hm - qm));
-  const fp cl = sqrt_abs(wl[3] / wl[0]);
-  const fp cr = sqrt_abs(wr[3] / wr[0]);
+  const fp cl = sqrt_abs(quot(wl[3], rl));
+  const fp cr = sqrt_abs(quot(wr[3], rg));
   const fp sl = fmin((wl[dir] - cl).v, (vm[d1] - cm).v);
   const fp sr = fmax((wr[dir] + cr).v, (vm[d1] + cm).v);
   const fp dl = sl - wl[dir], dr = sr - wr[dir];
@@ -686,11 +688,12 @@ __device__ __forceinline__ void hllc(double g1, int dir, const fp* ql, const fp*
   flux(dir, q, w, fl);
   if (star_l || star_r) {
     const fp s = use_l ? sl : sr;
-    const fp nom = use_l ? dl : dr, den = s - sm;
-    qs[0] = w[0] * nom / den;
-    qs[1] = dir == 1 ? (nom * q[1] + ps - w[3]) / den : nom * q[1] / den;
-    qs[2] = dir == 2 ? (nom * q[2] + ps - w[3]) / den : nom * q[2] / den;
-    qs[3] = (nom * q[3] - wl[3] * w[dir] + ps * sm) / den;
+    const fp nom = use_l ? dl : dr;
+    const Den den = den_of(s - sm);
+    qs[0] = quot(w[0] * nom, den);
+    qs[1] = quot(dir == 1 ? nom * q[1] + ps - w[3] : nom * q[1], den);
+    qs[2] = quot(dir == 2 ? nom * q[2] + ps - w[3] : nom * q[2], den);
+    qs[3] = quot(nom * q[3] - wl[3] * w[dir] + ps * sm, den);
 #pragma unroll
     for (int k = 0; k < 4; ++k) F[k] = fl[k] + s * (qs[k] - q[k]);
   } else {
@@ -699,34 +702,47 @@ __device__ __forceinline__ void hllc(double g1, int dir, const fp* ql, const fp*
   }
 }
 
-// maxLocalWaveSpeed (:221-246): the four characteristic speeds' maxima of the two sides
-__device__ __forceinline__ void local_speeds(double g, int dir, const fp* wl, const fp* wr, fp* a) {
-  const fp cl = sqrt_abs(fp(g) * wl[3] / wl[0]);
-  const fp cr = sqrt_abs(fp(g) * wr[3] / wr[0]);
-  const fp vl = wl[dir], vr = wr[dir];
-  a[0] = max_(abs_(vl - cl), abs_(vr - cr));
-  a[1] = max_(abs_(vl), abs_(vr));
-  a[2] = a[1];
-  a[3] = max_(abs_(vl + cl), abs_(vr + cr));
+// The two sides of a Gauss point with what the Rusanov fluxes share: primitives, the densities as
+// shared denominators, and maxLocalWaveSpeed (:221-246), the four characteristic speeds' maxima.
+struct Sides {
+  fp wl[4], wr[4], a[4];
+  Den rl, rg;
+};
+__device__ __forceinline__ Sides sides_of(double g, double g1, int dir, const fp* ql, const fp* qr) {
+  Sides s;
+  s.rl = den_of(ql[0]);
+  s.rg = den_of(qr[0]);
+  primitive(g1, ql, s.rl, s.wl);
+  primitive(g1, qr, s.rg, s.wr);
+  const fp cl = sqrt_abs(quot(fp(g) * s.wl[3], s.rl));
+  const fp cr = sqrt_abs(quot(fp(g) * s.wr[3], s.rg));
+  const fp vl = s.wl[dir], vr = s.wr[dir];
+  s.a[0] = max_(abs_(vl - cl), abs_(vr - cr));
+  s.a[1] = max_(abs_(vl), abs_(vr));
+  s.a[2] = s.a[1];
+  s.a[3] = max_(abs_(vl + cl), abs_(vr + cr));
+  return s;
 }
-
-// characteristic Rusanov (:310-330) with maxLocalWaveSpeed
-__device__ __forceinline__ void rusanov(double g, double g1, int dir, const Eig& e,
-                                        const fp* ql, const fp* qr, fp* F) {
-  fp wl[4], wr[4], a[4], fl[4], fr[4], d[4], m[4], rm[4];
-  primitive(g1, ql, wl);
-  primitive(g1, qr, wr);
-  local_speeds(g, dir, wl, wr, a);
-  flux(dir, ql, wl, fl);
-  flux(dir, qr, wr, fr);
+// (fl + fr - R (a * L (xr - xl))) / 2
+__device__ __forceinline__ void dissipate(int dir, const Eig& e, const fp* a, const fp* xl, const fp* xr,
+                                          const fp* fl, const fp* fr, fp* F) {
+  fp d[4], m[4], rm[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) d[k] = qr[k] - ql[k];
+  for (int k = 0; k < 4; ++k) d[k] = xr[k] - xl[k];
   left(e, dir, d, m);
 #pragma unroll
   for (int k = 0; k < 4; ++k) m[k] = a[k] * m[k];
   right(e, dir, m, rm);
 #pragma unroll
   for (int k = 0; k < 4; ++k) F[k] = lit(kHalf) * (fl[k] + fr[k] - rm[k]);
+}
+
+// characteristic Rusanov (:310-330)
+__device__ __forceinline__ void rusanov(int dir, const Eig& e, const Sides& s, const fp* ql, const fp* qr, fp* F) {
+  fp fl[4], fr[4];
+  flux(dir, ql, s.wl, fl);
+  flux(dir, qr, s.wr, fr);
+  dissipate(dir, e, s.a, ql, qr, fl, fr, F);
 }
 
 // maxSpeed over both directions (Equations_Euler2D.cpp:207-219)
@@ -737,9 +753,9 @@ __device__ __forceinline__ double max_speed2(double g, const double* w) {
 
 // ---- Equations::Euler1D (Equations_Euler1D.cpp) --------------------------------------------
 
-__device__ __forceinline__ void primitive1(double g1, const fp* q, fp* w) {  // :18-23
+__device__ __forceinline__ void primitive1(double g1, const fp* q, const Den& d, fp* w) {  // :18-23
   w[0] = q[0];
-  w[1] = q[1] / q[0];
+  w[1] = quot(q[1], d);
   w[2] = scaled(kNegHalf, q[1] * w[1], q[2]) * g1;
 }
 
@@ -783,26 +799,29 @@ __device__ __forceinline__ void flux1(const fp* q, const fp* w, fp* f) {
   f[2] = w[1] * (q[2] + w[2]);
 }
 
-// maxLocalWaveSpeed (Equations_Euler1D.cpp:96-107)
-__device__ __forceinline__ void local_speeds1(double g, const fp* wl, const fp* wr, fp* a) {
-  const fp cl = sqrt_abs(fp(g) * wl[2] / wl[0]);
-  const fp cr = sqrt_abs(fp(g) * wr[2] / wr[0]);
-  a[0] = max_(abs_(wl[1] - cl), abs_(wr[1] - cr));
-  a[1] = max_(abs_(wl[1]), abs_(wr[1]));
-  a[2] = max_(abs_(wl[1] + cl), abs_(wr[1] + cr));
+// The 1D counterpart of Sides; maxLocalWaveSpeed (Equations_Euler1D.cpp:96-107)
+struct Sides1 {
+  fp wl[3], wr[3], a[3];
+  Den rl, rg;
+};
+__device__ __forceinline__ Sides1 sides1_of(double g, double g1, const fp* ql, const fp* qr) {
+  Sides1 s;
+  s.rl = den_of(ql[0]);
+  s.rg = den_of(qr[0]);
+  primitive1(g1, ql, s.rl, s.wl);
+  primitive1(g1, qr, s.rg, s.wr);
+  const fp cl = sqrt_abs(quot(fp(g) * s.wl[2], s.rl));
+  const fp cr = sqrt_abs(quot(fp(g) * s.wr[2], s.rg));
+  s.a[0] = max_(abs_(s.wl[1] - cl), abs_(s.wr[1] - cr));
+  s.a[1] = max_(abs_(s.wl[1]), abs_(s.wr[1]));
+  s.a[2] = max_(abs_(s.wl[1] + cl), abs_(s.wr[1] + cr));
+  return s;
 }
-
-// Rusanov (Equations_Euler1D.cpp:129-135) with maxLocalWaveSpeed
-__device__ __forceinline__ void rusanov1(double g, double g1, const fp* L, const fp* R,
-                                         const fp* ql, const fp* qr, fp* F) {
-  fp wl[3], wr[3], a[3], fl[3], fr[3], d[3], m[3], rm[3];
-  primitive1(g1, ql, wl);
-  primitive1(g1, qr, wr);
-  local_speeds1(g, wl, wr, a);
-  flux1(ql, wl, fl);
-  flux1(qr, wr, fr);
+__device__ __forceinline__ void dissipate1(const fp* L, const fp* R, const fp* a, const fp* xl, const fp* xr,
+                                           const fp* fl, const fp* fr, fp* F) {
+  fp d[3], m[3], rm[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) d[k] = qr[k] - ql[k];
+  for (int k = 0; k < 3; ++k) d[k] = xr[k] - xl[k];
   mv3(L, d, m);
 #pragma unroll
   for (int k = 0; k < 3; ++k) m[k] = a[k] * m[k];
@@ -811,22 +830,31 @@ __device__ __forceinline__ void rusanov1(double g, double g1, const fp* L, const
   for (int k = 0; k < 3; ++k) F[k] = lit(kHalf) * (fl[k] + fr[k] - rm[k]);
 }
 
+// Rusanov (Equations_Euler1D.cpp:129-135)
+__device__ __forceinline__ void rusanov1(const Sides1& s, const fp* L, const fp* R, const fp* ql, const fp* qr, fp* F) {
+  fp fl[3], fr[3];
+  flux1(ql, s.wl, fl);
+  flux1(qr, s.wr, fr);
+  dissipate1(L, R, s.a, ql, qr, fl, fr, F);
+}
+
 // HLLC (Equations_Euler1D.cpp:156-210).  As in 2D the operands of the left or right region are
 // selected first and one copy of the arithmetic runs.
 __device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp* F) {
   fp wl[3], wr[3], fl[3], qs[3];
-  primitive1(g1, ql, wl);
-  primitive1(g1, qr, wr);
-  const fp hl = (ql[2] + wl[2]) / wl[0];
-  const fp hr = (qr[2] + wr[2]) / wr[0];
-  const fp rr = sqrt_abs(wr[0] / wl[0]);
+  const Den rl = den_of(ql[0]), rg = den_of(qr[0]);
+  primitive1(g1, ql, rl, wl);
+  primitive1(g1, qr, rg, wr);
+  const fp hl = quot(ql[2] + wl[2], rl);
+  const fp hr = quot(qr[2] + wr[2], rg);
+  const fp rr = sqrt_abs(quot(wr[0], rl));
   const fp rrr = lit(kOne) / (lit(kOne) + rr);
   const fp vm = (wl[1] + wr[1] * rr) * rrr;
   const fp qm = lit(kHalf) * vm * vm;
   const fp hm = (hl + hr * rr) * rrr;
   const fp cm = sqrt_abs(fp(g1) * (hm - qm));
-  const fp cl = sqrt_abs(wl[2] / wl[0]);
-  const fp cr = sqrt_abs(wr[2] / wr[0]);
+  const fp cl = sqrt_abs(quot(wl[2], rl));
+  const fp cr = sqrt_abs(quot(wr[2], rg));
   const fp sl = fmin((wl[1] - cl).v, (vm - cm).v);
   const fp sr = fmax((wr[1] + cr).v, (vm + cm).v);
   const fp dl = sl - wl[1], dr = sr - wr[1];
@@ -845,10 +873,11 @@ __device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp*
   flux1(q, w, fl);
   if (star_l || star_r) {
     const fp s = use_l ? sl : sr;
-    const fp nom = use_l ? dl : dr, den = s - sm;
-    qs[0] = w[0] * nom / den;
-    qs[1] = (nom * q[1] + ps - w[2]) / den;
-    qs[2] = (nom * q[2] - wl[2] * w[1] + ps * sm) / den;
+    const fp nom = use_l ? dl : dr;
+    const Den den = den_of(s - sm);
+    qs[0] = quot(w[0] * nom, den);
+    qs[1] = quot(nom * q[1] + ps - w[2], den);
+    qs[2] = quot(nom * q[2] - wl[2] * w[1] + ps * sm, den);
 #pragma unroll
     for (int k = 0; k < 3; ++k) F[k] = fl[k] + s * (qs[k] - q[k]);
   } else {
@@ -1006,12 +1035,12 @@ __device__ __forceinline__ double hermite_limiter(const HermiteK<double>& K, con
 // A(q) * x with the Jacobians dfluxx / dfluxy (Equations_Euler2D.cpp:52-98), row sums left to
 // right; zero and unit entries as in the reference's matrices.
 __device__ __forceinline__ void dflux_apply(fp g, fp g1, fp g3, int dir, const fp* q, const fp* w,
-                                            const fp* x, fp* y) {
+                                            const Den& rho, const fp* x, fp* y) {
   const fp half = lit(kHalf);
   if (dir == 1) {
     const fp sv = w[1] * w[1];
     const fp dv = half * g1 * (sv + w[2] * w[2]);
-    const fp h = (q[3] + w[3]) / w[0];
+    const fp h = quot(q[3] + w[3], rho);
     y[0] = x[1];
     fp s = (dv - sv) * x[0]; s = s + (-g3 * w[1]) * x[1]; s = s + (-g1 * w[2]) * x[2]; s = s + g1 * x[3]; y[1] = s;
     s = (-w[1] * w[2]) * x[0]; s = s + w[2] * x[1]; s = s + w[1] * x[2]; y[2] = s;
@@ -1020,7 +1049,7 @@ __device__ __forceinline__ void dflux_apply(fp g, fp g1, fp g3, int dir, const f
   } else {
     const fp sv = w[2] * w[2];
     const fp dv = half * g1 * (sv + w[1] * w[1]);
-    const fp h = (q[3] + w[3]) / w[0];
+    const fp h = quot(q[3] + w[3], rho);
     y[0] = x[2];
     fp s = (-w[1] * w[2]) * x[0]; s = s + w[2] * x[1]; s = s + w[1] * x[2]; y[1] = s;
     s = (dv - sv) * x[0]; s = s + (-g1 * w[1]) * x[1]; s = s + (-g3 * w[2]) * x[2]; s = s + g1 * x[3]; y[2] = s;
@@ -1030,53 +1059,33 @@ __device__ __forceinline__ void dflux_apply(fp g, fp g1, fp g3, int dir, const f
 }
 
 // dRusanov (Equations_Euler2D.cpp:352-360) as called in FVHermite_System2D.cpp:553-589
-__device__ __forceinline__ void drusanov(double g, double g1, double g3, int dir, const Eig& e,
+__device__ __forceinline__ void drusanov(double g, double g1, double g3, int dir, const Eig& e, const Sides& s,
                                          const fp* ql, const fp* qr, const fp* dql, const fp* dqr, fp* F) {
-  fp wl[4], wr[4], a[4], d[4], m[4], al[4], ar[4], rm[4];
-  primitive(g1, ql, wl);
-  primitive(g1, qr, wr);
-  dflux_apply(g, g1, g3, dir, ql, wl, dql, al);
-  dflux_apply(g, g1, g3, dir, qr, wr, dqr, ar);
-  local_speeds(g, dir, wl, wr, a);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) d[k] = dqr[k] - dql[k];
-  left(e, dir, d, m);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) m[k] = a[k] * m[k];
-  right(e, dir, m, rm);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) F[k] = lit(kHalf) * (al[k] + ar[k] - rm[k]);
+  fp al[4], ar[4];
+  dflux_apply(g, g1, g3, dir, ql, s.wl, s.rl, dql, al);
+  dflux_apply(g, g1, g3, dir, qr, s.wr, s.rg, dqr, ar);
+  dissipate(dir, e, s.a, dql, dqr, al, ar, F);
 }
 
 // dflux 1D (Equations_Euler1D.cpp:39-53) applied to x; dRusanov 1D (:212-220)
-__device__ __forceinline__ void drusanov1(double g, double g1, double g3, const fp* L, const fp* R,
+__device__ __forceinline__ void drusanov1(double g, double g1, double g3, const Sides1& s, const fp* L, const fp* R,
                                           const fp* ql, const fp* qr, const fp* dql, const fp* dqr, fp* F) {
-  fp wl[3], wr[3], a[3], d[3], m[3], rm[3], al[3], ar[3];
-  primitive1(g1, ql, wl);
-  primitive1(g1, qr, wr);
-  auto apply = [&](const fp* q, const fp* w, const fp* x, fp* y) {
+  fp al[3], ar[3];
+  auto apply = [&](const fp* q, const fp* w, const Den& rho, const fp* x, fp* y) {
     const fp G(g), G1(g1), G3(g3);
     const fp a3 = lit(kHalf) * G3 * w[1] * w[1];
     const fp a4 = -G3 * w[1];
-    const fp e = G * q[2] / w[0];
+    const fp e = quot(G * q[2], rho);
     const fp a6 = (G1 * (w[1] * w[1]) - e) * w[1];
     const fp a7 = e - lit(kThreeHalves) * G1 * w[1] * w[1];
     const fp a8 = G * w[1];
     y[0] = x[1];
-    fp s = a3 * x[0]; s = s + a4 * x[1]; s = s + G1 * x[2]; y[1] = s;
-    s = a6 * x[0]; s = s + a7 * x[1]; s = s + a8 * x[2]; y[2] = s;
+    fp t = a3 * x[0]; t = t + a4 * x[1]; t = t + G1 * x[2]; y[1] = t;
+    t = a6 * x[0]; t = t + a7 * x[1]; t = t + a8 * x[2]; y[2] = t;
   };
-  apply(ql, wl, dql, al);
-  apply(qr, wr, dqr, ar);
-  local_speeds1(g, wl, wr, a);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) d[k] = dqr[k] - dql[k];
-  mv3(L, d, m);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) m[k] = a[k] * m[k];
-  mv3(R, m, rm);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) F[k] = lit(kHalf) * (al[k] + ar[k] - rm[k]);
+  apply(ql, s.wl, s.rl, dql, al);
+  apply(qr, s.wr, s.rg, dqr, ar);
+  dissipate1(L, R, s.a, dql, dqr, al, ar, F);
 }
 
 }  // namespace par

@@ -162,7 +162,7 @@ __global__ void k_rusanov2(T g, T g1, int dir, const double* __restrict__ qa,
                                 sqrt(fabs(wb[0])), wb[1], wb[2], (qb[4 * k + 3] + wb[3]) / wb[0]);
     const par::fp l[4] = {a[0], a[1], a[2], a[3]}, r[4] = {b[0], b[1], b[2], b[3]};
     par::fp f[4];
-    par::rusanov(g, g1, dir, E, l, r, f);
+    par::rusanov(dir, E, par::sides_of(g, g1, dir, l, r), l, r, f);
     for (int m = 0; m < 4; ++m) F[m] = f[m].v;
   } else {
     Roe2<T> s = roe_of_pair(g1, qa + 4 * k, qb + 4 * k);
@@ -194,7 +194,7 @@ __global__ void k_drusanov2(T g, T g1, T g3, int dir, const double* __restrict__
     const par::fp l[4] = {a[0], a[1], a[2], a[3]}, r[4] = {b[0], b[1], b[2], b[3]};
     const par::fp dl[4] = {da[0], da[1], da[2], da[3]}, dr[4] = {db[0], db[1], db[2], db[3]};
     par::fp f[4];
-    par::drusanov(g, g1, g3, dir, E, l, r, dl, dr, f);
+    par::drusanov(g, g1, g3, dir, E, par::sides_of(g, g1, dir, l, r), l, r, dl, dr, f);
     for (int m = 0; m < 4; ++m) F[m] = f[m].v;
   } else {
     Roe2<T> s = roe_of_pair(g1, qa + 4 * k, qb + 4 * k);
