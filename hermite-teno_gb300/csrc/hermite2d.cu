@@ -2,14 +2,14 @@
 // moments v = du/dx, w = du/dy.  Per stage:
 //   limit             : hermiteLimiter on v along x and on w along y.  The reference updates in
 //                       place while sweeping (limitDerivatives, :393-427), i.e. a Gauss-Seidel
-//                       sweep: one thread per (row, field) resp. (column, field) walks the line.
+//                       sweep; here segments of a line sweep side by side until they agree.
 //   prim              : primitives of u
 //   faces<X>, <Y>     : Roe average; HTENO on (L u, L v_n) over 4 cells, TENO5 on L v_t over 6
 //   flux<X>, <Y>      : GL3 along the face for the 24 face arrays, R back-projection, Rusanov for u
 //                       and dRusanov for the two moments at 3 Gauss points
 //   update            : flux differences and SSP-RK3 for u, v, w.  RungeKutta3 saves v0, w0
 //                       after the first rhs (the limited moments) and combines later stages with
-//                       the unlimited stage values, so those are kept in vs, ws.
+//                       the unlimited stage values, which v, w keep: the limited ones go to vt, wt.
 // Boundaries are zero-gradient (the reference's Hermite 2D rhs).  T = double or float.
 #include "hermite2d_kernels.cuh"
 

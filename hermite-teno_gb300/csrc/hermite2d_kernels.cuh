@@ -4,6 +4,7 @@
 // parity functions).  Each including translation unit owns its constant block.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "hermite_math.cuh"
@@ -36,31 +37,34 @@ __device__ __forceinline__ double to_d(T x) {
   else return x;
 }
 
+// Equality of two values' bits (a NaN equals itself, +0 and -0 differ).
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
+
 template <typename T>
 struct WorkH {
-  double* prim;   // [4][nc] u, v, h, sqrt|rho|
-  double* vs;     // [4][nc] unlimited stage moments
-  double* ws;
+  double* prim;   // [4][nc] u, v, h, sqrt|rho| (double)
   T* xc;          // [24][ny][nx+1]: kind a (0 u-, 1 u+, 2 vn-, 3 vn+, 4 vt-, 5 vt+) x field r
   T* xroe;        // [7][ny][nx+1]
   T* yc;          // [24][ny+1][nx]
   T* yroe;        // [7][ny+1][nx]
   T* fx;          // [12][ny][nx+1]: kind (0 u, 1 moment along the sweep, 2 cross moment) x field
   T* fy;          // [12][ny+1][nx]
-  // the state as the face kernels read it, in the compute type: for double the state arrays
-  // themselves (set by the launcher); for float copies written by the kernels that produce the
-  // state (update, limiter), so each cell is converted once per stage, not once per stencil use
-  T* qt;          // [4][nc]
-  T* vt;          // [4][nc] limited moments
+  T* vt;          // [4][nc] limited moments (the state's v, w keep the unlimited ones)
   T* wt;
+  // the state as the limiter and the face kernels read it, in the compute type: for double the
+  // state array and prim (set by the launcher); for float copies written by the kernels that
+  // produce the state, so each cell is converted once per stage, not once per stencil use
+  T* qt;          // [4][nc]
   T* primt;       // [4][nc] u, v, h, sqrt|rho|
 };
 
 template <typename T>
 size_t work_bytes_h(int nx, int ny) {
   const size_t nc = size_t(nx) * ny, nxf = size_t(nx + 1) * ny, nyf = size_t(ny + 1) * nx;
-  const size_t copies = std::is_same<T, float>::value ? 16 * nc * sizeof(float) + 256 * 4 : 0;
-  return 12 * nc * sizeof(double) + (24 + 7 + 12) * (nxf + nyf) * sizeof(T) + 256 * 12 + copies;
+  return 16 * nc * sizeof(T) + (24 + 7 + 12) * (nxf + nyf) * sizeof(T) + 256 * 12;
 }
 
 template <typename T>
@@ -73,22 +77,22 @@ WorkH<T> carve_h(void* base, int nx, int ny) {
     return r;
   };
   WorkH<T> w;
-  w.prim = reinterpret_cast<double*>(take(4 * nc * sizeof(double)));
-  w.vs = reinterpret_cast<double*>(take(4 * nc * sizeof(double)));
-  w.ws = reinterpret_cast<double*>(take(4 * nc * sizeof(double)));
   w.xc = reinterpret_cast<T*>(take(24 * nxf * sizeof(T)));
   w.xroe = reinterpret_cast<T*>(take(7 * nxf * sizeof(T)));
   w.yc = reinterpret_cast<T*>(take(24 * nyf * sizeof(T)));
   w.yroe = reinterpret_cast<T*>(take(7 * nyf * sizeof(T)));
   w.fx = reinterpret_cast<T*>(take(12 * nxf * sizeof(T)));
   w.fy = reinterpret_cast<T*>(take(12 * nyf * sizeof(T)));
-  w.qt = nullptr;
-  w.vt = w.wt = w.primt = nullptr;
-  if constexpr (std::is_same<T, float>::value) {
+  w.vt = reinterpret_cast<T*>(take(4 * nc * sizeof(T)));
+  w.wt = reinterpret_cast<T*>(take(4 * nc * sizeof(T)));
+  w.prim = nullptr;
+  w.qt = w.primt = nullptr;
+  T* prim = reinterpret_cast<T*>(take(4 * nc * sizeof(T)));
+  if constexpr (std::is_same<T, double>::value) {
+    w.prim = prim;
+  } else {
+    w.primt = prim;
     w.qt = reinterpret_cast<T*>(take(4 * nc * sizeof(T)));
-    w.vt = reinterpret_cast<T*>(take(4 * nc * sizeof(T)));
-    w.wt = reinterpret_cast<T*>(take(4 * nc * sizeof(T)));
-    w.primt = reinterpret_cast<T*>(take(4 * nc * sizeof(T)));
   }
   return w;
 }
@@ -160,256 +164,277 @@ __global__ void kh_prim_f(GeoH G, const double* __restrict__ q, float* __restric
   block_max_to(ms, &st->maxbits);
 }
 
-// Gauss-Seidel hermiteLimiter sweeps of both directions in one launch.  Blocks [0, nbx): x lines
-// (line = row j of field e, walks i, updates v); blocks [nbx, ...): y lines (column i, walks j,
-// updates w).  The two directions touch different arrays, so they run side by side.  The
-// neighbour beyond the last cell is the zero-gradient ghost, which holds the pre-sweep value; the
-// one before the first cell is the first cell (old value).
-//
-// Each block takes 32 lines of one field.  The sweep itself is sequential along a line (each cell
-// reads its left neighbour's limited value), so one thread walks each line; the block stages the
-// lines through shared memory in chunks of kLimChunk cells with coalesced loads and stores (along
-// the rows for x lines, across the columns for y lines), keeping the global-memory latency off
-// the sweep's dependency chain.
-constexpr int kLimLines = 32, kLimChunk = 64, kLimThreads = 128;
-
+// ---- the limiter ---------------------------------------------------------------------------------
+// One cell of hermiteLimiter (Schemes_Hermite.cpp:634-662) as a sweep from left to right sees it:
+// next() takes the right neighbour's average and (unlimited) moment, at() the left neighbour's
+// limited moment.  What the next cell shares with this one is carried over.
 template <typename T>
-__global__ void __launch_bounds__(kLimThreads) kh_limit(GeoH G, HermiteK<T> K,
-                                                        const double* __restrict__ q,
-                                                        double* __restrict__ v,
-                                                        double* __restrict__ w, int nbx,
-                                                        const StepState* st) {
+struct LimitSweep;
+
+// Double: par::hermite_limiter's operations (the same bits); the difference quotient, its square
+// and the latter's reciprocal to the left of a cell are those to the right of the cell before.
+template <>
+struct LimitSweep<double> {
+  par::Den dif, r1, r2;  // r_k: s_k + eps
+  par::fp u0, u1, u2, d2, p1, p2, s1, s2;
+  __device__ __forceinline__ LimitSweep(const HermiteK<double>& K, double ul, double uc)
+      : dif(par::den_of(K.dif)), u1(ul), u2(uc) {
+    flat_ok = false;
+    right();
+  }
+  __device__ __forceinline__ void right() {
+    p2 = par::quot(u2 - u1, dif);
+    s2 = (u1 - u2) * (u1 - u2);
+    r2 = par::den_of(s2 + par::lit(par::kEps6));
+  }
+  __device__ __forceinline__ void next(double ur, double dr) {
+    u0 = u1;
+    u1 = u2;
+    p1 = p2;
+    s1 = s2;
+    r1 = r2;
+    u2 = ur;
+    d2 = dr;
+    if (!(flat_ok && same_bits(u0.v, u1.v) && same_bits(u1.v, u2.v))) right();  // else p2, s2, r2 stay
+  }
+  // A cell on constant data with a zero moment to its right (a tail running out into a flat region:
+  // the limited moment there shrinks by a quarter per cell for hundreds of cells): every operand but
+  // d0 is the flat value's, so the weights are those of the cell before if the full-stencil
+  // indicator before its scaling, r, has the same bits -- or is below 5e-21 in both cells, where
+  // s0 = r / 6720 < 1e-24 is lost in s0 + 1e-6 and tau = s0^2 in 1 + tau / 1e-6 -- and the terms in
+  // p1, p2 are +0.  13 operations instead of ~100.
+  bool flat_ok;
+  par::fp flat_u, flat_a, flat_z, flat_v, flat_r, flat_w;
+  __device__ __forceinline__ bool flat() const {
+    return same_bits(u0.v, u1.v) && same_bits(u1.v, u2.v) && same_bits(d2.v, 0.0);
+  }
+  __device__ __forceinline__ double at_flat(double dl) {
+    using namespace par;
+    const fp d0(dl);
+    if (!flat_ok || !same_bits(flat_u.v, u1.v)) {
+      flat_u = u1;
+      flat_a = lit(k1029270) * u1 - lit(k2129184) * u1 + lit(k1099914) * u1;
+      flat_z = (lit(k1099445) * u1 - lit(k4317056) * u1 + lit(k2118166) * u1) * u1;
+      flat_v = lit(k1099445) * u1 * u1;
+      flat_ok = true;
+      flat_r = flat_indicator(d0);
+      const double lim = at(dl, &flat_w);
+      return lim;
+    }
+    const fp r = flat_indicator(d0);
+    if (!same_bits(r.v, flat_r.v) && !(r.v < 5e-21 && flat_r.v < 5e-21)) {
+      flat_r = r;
+      return at(dl, &flat_w);
+    }
+    const fp p0 = scaled(kNegQuarter, d0 + d2, fp(0.0));
+    return (flat_w * quot(p0, den_lit(1.0 - 2E-5, kRcpLw0)) + fp(0.0)).v;
+  }
+  // |hermite_brk|'s sum on flat data: the terms left out are zeros
+  __device__ __forceinline__ par::fp flat_indicator(par::fp d0) const {
+    const par::fp ud0 = d0 * dif.b;
+    return par::abs_((flat_a + par::lit(par::k281121) * ud0) * ud0 + flat_z + flat_v);
+  }
+  __device__ __forceinline__ double at(double dl, par::fp* w0n = nullptr) const {
+    using namespace par;
+    const fp d0(dl), u[3] = {u0, u1, u2}, ud[3] = {d0 * dif.b, fp(0.0), d2 * dif.b};
+    const fp p0 = scaled(kNegQuarter, d0 + d2, quot(lit(kThreeQuarters) * (u2 - u0), dif));
+    const fp s0 = hermite_brk(u, ud);
+    const fp ta = abs_(s0 - s1) + abs_(s0 - s2), t4 = ta * ta;  // tau = t4 / 4: the factor is exact
+    const fp one = lit(kOne);
+    fp w0 = lit(kLw0) * scaled(kQuarter, quot(t4, den_of(s0 + lit(kEps6))), one);
+    fp w1 = lit(kLw1) * scaled(kQuarter, quot(t4, r1), one);
+    fp w2 = lit(kLw1) * scaled(kQuarter, quot(t4, r2), one);
+    const Den ds = den_of((w0 + w1) + w2);
+    w0 = quot(w0, ds);
+    w1 = quot(w1, ds);
+    w2 = quot(w2, ds);
+    if (w0n) *w0n = w0;
+    const fp r12 = lit(kLw1OverLw0);
+    const fp inner = r12 * p1 + r12 * p2;
+    const fp w12 = w1 * p1 + w2 * p2;
+    return (w0 * (quot(p0, den_lit(1.0 - 2E-5, kRcpLw0)) - inner) + w12).v;
+  }
+};
+
+// Float: restated so that little waits for the left neighbour's limited value d0.  hermiteLimiter's
+// result is
+//   lim = [w0 (p0/lw0 - Q) + w1 p1 + w2 p2] / (w0 + w1 + w2),  w_k = lw_k (1 + tau / (s_k + eps))
+// where only p0 = P - d0/4 and s0 = |(a ud0 + B) ud0 + C|/6720 (ud0 = d0 dif, the smoothness
+// measure fullPointsSI expanded in ud0) depend on d0.  next() computes B, C, s1, s2, E = P/lw0 - Q,
+// M = lw1 r1 + lw2 r2, L = lw1 p1 + lw2 p2, N = lw1 r1 p1 + lw2 r2 p2 with r_k = 1/(s_k + eps); at()
+//   tau = (|s0 - s1| + |s0 - s2|)^2 / 4,  w0 = lw0 (1 + tau / (s0 + eps)),
+//   lim = (w0 (E - d0 / (4 lw0)) + L + tau N) / (w0 + lw1 + lw2 + tau M).
+template <>
+struct LimitSweep<float> {
+  static constexpr float lw0 = 1.0f - 2e-5f, lw1 = 1e-5f, lw2 = 1e-5f, eps = float(HTENO_LAG_EPS);
+  float dif, rdif, u0, u1, u2, B, Cc, p1, p2, r1, r2, s1, s2, E, M, L, N;
+  template <typename T>
+  __device__ __forceinline__ LimitSweep(const HermiteK<T>& K, float ul, float uc)
+      : dif(float(K.dif)), rdif(float(K.rdif)), u1(ul), u2(uc) {
+    right();
+  }
+  __device__ __forceinline__ void right() {
+    p2 = (u2 - u1) * rdif;
+    s2 = (u1 - u2) * (u1 - u2);
+    r2 = 1.0f / (s2 + eps);
+  }
+  __device__ __forceinline__ void next(float ur, float dr) {
+    u0 = u1;
+    u1 = u2;
+    u2 = ur;
+    const float ud2 = dr * dif;
+    p1 = p2;
+    s1 = s2;
+    r1 = r2;
+    right();
+    constexpr float k6720 = 1.0f / 6720.0f;
+    B = (1029270.0f * u2 - 2129184.0f * u1 + 1099914.0f * u0 - 494958.0f * ud2) * k6720;
+    Cc = ((-1029270.0f * u0 + 2129184.0f * u1 - 1099914.0f * u2 + 281121.0f * ud2) * ud2 +
+          (1099445.0f * u2 - 4317056.0f * u1 + 2118166.0f * u0) * u2 +
+          4317056.0f * (u1 - u0) * u1 + 1099445.0f * u0 * u0) * k6720;
+    const float P = 0.75f * (u2 - u0) * rdif - 0.25f * dr;
+    E = P * (1.0f / lw0) - ((lw1 / lw0) * p1 + (lw2 / lw0) * p2);
+    M = lw1 * r1 + lw2 * r2;
+    L = lw1 * p1 + lw2 * p2;
+    N = lw1 * r1 * p1 + lw2 * r2 * p2;
+  }
+  __device__ __forceinline__ float at(float d0) const {
+    constexpr float a = 281121.0f / 6720.0f, c4 = 0.25f / lw0;
+    const float ud0 = d0 * dif;
+    const float s0 = fabsf(fmaf(fmaf(a, ud0, B), ud0, Cc));
+    const float t = fabsf(s0 - s1) + fabsf(s0 - s2);
+    const float tau = 0.25f * t * t;
+    const float w0 = lw0 * fmaf(tau, __fdividef(1.0f, s0 + eps), 1.0f);
+    const float num = fmaf(w0, fmaf(-c4, d0, E), fmaf(tau, N, L));
+    const float den = w0 + fmaf(tau, M, lw1 + lw2);
+    return __fdividef(num, den);
+  }
+};
+
+// The reference's limiter is a Gauss-Seidel sweep along every line (row j of field e walking i on
+// v, column i walking j on w): each cell reads its left neighbour's limited value, so a line is one
+// serial chain, ~110 FP64 operations (64 cycles each) or ~70 dependent float operations per cell.
+// The chain forgets quickly (a cell passes on about a quarter of its left neighbour's change), so
+// a line is cut into segments that sweep side by side: every segment first starts from a guess of its
+// left neighbour's value (the unlimited moment; in double the float sweep of the kLimWarm cells before
+// it, which costs next to nothing beside one cell in double); then, as long as a segment's left
+// neighbour came out with other bits than it was computed from, it sweeps again from its first cell
+// and stops at the first cell whose bits do not change.  When nothing changes any more every cell
+// has been computed from its final left neighbour: the bits of the one sweep, whatever the data.
+// (Segment k is final after k such passes at the latest.  Bits usually agree again after about 15
+// cells in double, 28 without the float guess, and 12-21 in float; a tail that vanishes into constant
+// data takes longer, in double on the short form at_flat.)
+//
+// Threads of a block: `lines` lines (16 or 32, the fast index) x segments.  Blocks [0, nbx): x
+// lines; [nbx, ...): y lines.  The neighbour beyond the last cell is the zero-gradient ghost, the
+// one before the first cell is the first cell (unlimited values).  Limited moments go to vt, wt:
+// the unlimited ones stay where the later stages of a step read them.  A y line's cells are read
+// across the lanes (coalesced); in float an x line's come through shared memory in chunks of kLimC
+// cells of the warp's 32 lines, loaded and stored along the rows (kStaged; in double the arithmetic
+// hides the scattered loads).
+constexpr int kLimC = 16, kLimWarm = 24;
+
+template <typename T, bool kStaged>
+__global__ void __launch_bounds__(256) kh_limit(GeoH G, HermiteK<T> K, const T* __restrict__ q,
+                                                const double* __restrict__ v, const double* __restrict__ w,
+                                                T* __restrict__ vt, T* __restrict__ wt, int lines, int nbx,
+                                                const StepState* st) {
   if (st->done) return;
-  constexpr int L = kLimLines, C = kLimChunk;
-  __shared__ double sq[C + 1][L + 1];
-  __shared__ double sd[C + 1][L + 1];
+  __shared__ T last[256];  // the limited value of each segment's last cell
   const bool xd = int(blockIdx.x) < nbx;
   const int b = xd ? int(blockIdx.x) : int(blockIdx.x) - nbx;
   const int nl = xd ? G.ny : G.nx;  // number of lines
   const int n = xd ? G.nx : G.ny;   // length of a line
-  const int nlb = (nl + L - 1) / L;
-  const int e = b / nlb, l0 = (b - e * nlb) * L;
-  double* __restrict__ d = xd ? v : w;
-  const size_t nc = size_t(G.nx) * G.ny;
-  auto at = [&](int l, int s) -> size_t {
-    return size_t(e) * nc + (xd ? size_t(l) * G.nx + s : size_t(s) * G.nx + l);
-  };
-  const int tid = threadIdx.x;
-  const bool sweeper = tid < L && l0 + tid < nl;
-  const par::Den dif = par::den_of(double(K.dif));
-  T um = T(0), u0 = T(0), dm = T(0), dcur = T(0);
-  if (sweeper) {
-    um = from_d<T>(q[at(l0 + tid, 0)]);
-    u0 = um;
-    dm = from_d<T>(d[at(l0 + tid, 0)]);
-    dcur = dm;
-  }
-  for (int c0 = 0; c0 < n; c0 += C) {
-    const int cnt = min(C, n - c0);
-    // cells c0 .. c0 + cnt of each line (the last is the look-ahead, clamped to the line's end);
-    // every d value read here is a pre-sweep value: the sweep has written cells < c0 only
-    for (int it = tid; it < (cnt + 1) * L; it += kLimThreads) {
-      int l, k;
-      if (xd) { k = it % (cnt + 1); l = it / (cnt + 1); }
-      else { l = it % L; k = it / L; }
-      if (l0 + l < nl) {
-        const size_t o = at(l0 + l, min(c0 + k, n - 1));
-        sq[k][l] = q[o];
-        sd[k][l] = d[o];
+  const int nlb = (nl + lines - 1) / lines;
+  const int e = b / nlb, seg = threadIdx.x / lines, segs = blockDim.x / lines;
+  const int l0 = (b - e * nlb) * lines, line = l0 + int(threadIdx.x) - seg * lines;
+  const int len = (n + segs - 1) / segs, c0 = min(n, seg * len), c1 = min(n, c0 + len);
+  const bool live = line < nl && c0 < c1;
+  const size_t field = size_t(e) * G.nx * G.ny;
+  const size_t base = field + (xd ? size_t(line) * G.nx : size_t(line));
+  const size_t step = xd ? 1 : size_t(G.nx);
+  const double* __restrict__ d = xd ? v : w;
+  T* __restrict__ out = xd ? vt : wt;
+  T used = T(0);  // the left neighbour's value the segment was computed from
+  // cells c0 .. of the segment from the left value dl; with `again` up to the first unchanged cell
+  auto sweep = [&](T dl, bool again) {
+    LimitSweep<T> s(K, q[base + size_t(max(c0 - 1, 0)) * step], q[base + size_t(c0) * step]);
+    size_t k = base + size_t(c0) * step, kr = base + size_t(min(c0 + 1, n - 1)) * step;
+    T ur = q[kr], dr = from_d<T>(d[kr]);
+    for (int i = c0; i < c1; ++i, k += step) {
+      s.next(ur, dr);
+      if (i + 1 < c1) {  // in flight during this cell's arithmetic
+        kr = base + size_t(min(i + 2, n - 1)) * step;
+        ur = q[kr];
+        dr = from_d<T>(d[kr]);
       }
+      if constexpr (std::is_same<T, double>::value) dl = again && s.flat() ? s.at_flat(dl) : s.at(dl);
+      else dl = s.at(dl);
+      if (again && same_bits(dl, out[k])) return;
+      out[k] = dl;
     }
-    __syncthreads();
-    if (sweeper) {
-      for (int k = 0; k < cnt; ++k) {
-        const T up = from_d<T>(sq[k + 1][tid]);
-        const T dn = from_d<T>(sd[k + 1][tid]);  // not yet limited (or the ghost = pre-sweep last value)
-        T uu[3] = {um, u0, up};
-        T dd[3] = {dm, dcur, dn};
-        T lim;
-        if constexpr (std::is_same<T, double>::value) lim = par::hermite_limiter(dif, uu, dd);
-        else lim = hermite_limiter(K, uu, dd);
-        sd[k][tid] = to_d<T>(lim);
-        dm = lim;
-        um = u0;
-        u0 = up;
-        dcur = dn;
+    last[threadIdx.x] = dl;
+  };
+  if (live) used = from_d<T>(d[base + size_t(max(c0 - 1, 0)) * step]);
+  if constexpr (std::is_same<T, double>::value) {
+    if (live && c0 > kLimWarm) {
+      auto uf = [&](int i) { return mix::d2f(q[base + size_t(i) * step]); };
+      auto df = [&](int i) { return mix::d2f(d[base + size_t(i) * step]); };
+      LimitSweep<float> s(K, uf(c0 - kLimWarm - 1), uf(c0 - kLimWarm));
+      float x = df(c0 - kLimWarm - 1);
+      for (int i = c0 - kLimWarm; i < c0; ++i) {  // the limited value of cell i
+        s.next(uf(i + 1), df(i + 1));
+        x = s.at(x);
       }
+      if (fabsf(x) <= 3.4e38f) used = mix::f2d(x);
     }
-    __syncthreads();
-    for (int it = tid; it < cnt * L; it += kLimThreads) {
-      int l, k;
-      if (xd) { k = it % cnt; l = it / cnt; }
-      else { l = it % L; k = it / L; }
-      if (l0 + l < nl) d[at(l0 + l, c0 + k)] = sd[k][l];
-    }
-    __syncthreads();
   }
-}
-
-// Mixed precision: the same sweeps with the float limiter restated so that the part that waits
-// for the left neighbour's limited value d0 is short.  hermiteLimiter's result is
-//   lim = [w0 (p0/lw0 - Q) + w1 p1 + w2 p2] / (w0 + w1 + w2),  w_k = lw_k (1 + tau / (s_k + eps))
-// where only p0 = P - d0/4 and s0 = |(a ud0 + B) ud0 + C|/6720 (ud0 = d0 dif, the smoothness
-// measure fullPointsSI expanded in ud0) depend on d0.  Every other quantity of a cell is computed
-// off the sweep's chain, before the sweep reaches the cell: B, C, s1, s2, E = P/lw0 - Q,
-// M = lw1 r1 + lw2 r2, L = lw1 p1 + lw2 p2, N = lw1 r1 p1 + lw2 r2 p2 with r_k = 1/(s_k + eps).
-// The sweep then evaluates, per cell,
-//   tau = (|s0 - s1| + |s0 - s2|)^2 / 4,  w0 = lw0 (1 + tau / (s0 + eps)),
-//   lim = (w0 (E - d0 / (4 lw0)) + L + tau N) / (w0 + lw1 + lw2 + tau M).
-// The block's four warps work as a pipeline over chunks of kLimChunkF cells: warp 0 sweeps its
-// 32 lines through chunk s while warps 1-3 load chunk s + 1, precompute its per-cell quantities
-// into the other half of a double buffer, and store the limited values of chunk s - 1; one block
-// barrier per chunk hands the buffers over.  The sweep, the only sequential part, so runs back to
-// back instead of waiting for each chunk's loads, precompute and stores.
-constexpr int kLimChunkF = 16;
-
-__global__ void __launch_bounds__(kLimThreads, 4) kh_limit_f(GeoH G, HermiteK<float> K,
-                                                          const double* __restrict__ q,
-                                                          double* __restrict__ v,
-                                                          double* __restrict__ w,
-                                                          float* __restrict__ vt,
-                                                          float* __restrict__ wt, int nbx,
-                                                          const StepState* st) {
-  if (st->done) return;
-  constexpr int L = kLimLines, C = kLimChunkF, NP = kLimThreads - 32;  // NP producer threads
-  constexpr float lw0 = 1.0f - 2e-5f, lw1 = 1e-5f, lw2 = 1e-5f, eps = float(HTENO_LAG_EPS);
-  __shared__ float pre[2][8][C][L + 1];
-  __shared__ float su[C + 2][L + 1];  // cells c0 - 1 .. c0 + C of the chunk being prepared (clamped)
-  __shared__ float sd[C][L + 1];      // pre-sweep d of cells c0 + 1 .. c0 + C (clamped)
-  __shared__ float outf[2][C][L + 1];  // limited values (their double copies are exact)
-  const bool xd = int(blockIdx.x) < nbx;
-  const int b = xd ? int(blockIdx.x) : int(blockIdx.x) - nbx;
-  const int nl = xd ? G.ny : G.nx;
-  const int n = xd ? G.nx : G.ny;
-  const int nlb = (nl + L - 1) / L;
-  const int e = b / nlb, l0 = (b - e * nlb) * L;
-  double* __restrict__ d = xd ? v : w;
-  float* __restrict__ dt = xd ? vt : wt;
-  const size_t nc = size_t(G.nx) * G.ny;
-  auto at = [&](int l, int s) -> size_t {
-    return size_t(e) * nc + (xd ? size_t(l) * G.nx + s : size_t(s) * G.nx + l);
-  };
-  const int tid = threadIdx.x;
-  const bool sweeper_warp = tid < 32;
-  const bool sweeper = sweeper_warp && l0 + tid < nl;
-  const int ptid = tid - 32;
-  const float dif = K.dif, rdif = K.rdif;
-  const int nchunks = (n + C - 1) / C;
-  // x lines: consecutive threads take consecutive cells of a row; y lines: consecutive lines
-  // (columns) of a cell row; both coalesce
-  auto slot = [&](int it, int rows, int& l, int& k) {
-    if (xd) { l = it / rows; k = it - l * rows; }
-    else { l = it % L; k = it / L; }
-  };
-  // producers: the raw inputs of a chunk are loaded into registers one step before they are
-  // staged (bu: cells c0 - 1 .. c0 + C, bd: pre-sweep d of cells c0 + 1 .. c0 + C, clamped), so the
-  // loads are in flight during a whole step
-  constexpr int NU = ((C + 2) * L + NP - 1) / NP, ND = (C * L + NP - 1) / NP;
-  double bu[NU], bd[ND];
-  auto fetch = [&](int c) {
-    const int c0 = c * C, cnt = min(C, n - c0);
-#pragma unroll
-    for (int j = 0; j < NU; ++j) {
-      const int it = ptid + NP * j;
-      int l, k;
-      slot(it, C + 2, l, k);
-      bu[j] = (it < (C + 2) * L && l0 + l < nl && k < cnt + 2)
-                  ? q[at(l0 + l, min(max(c0 - 1 + k, 0), n - 1))] : 0.0;
-    }
-#pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      const int it = ptid + NP * j;
-      int l, k;
-      slot(it, C, l, k);
-      bd[j] = (it < C * L && l0 + l < nl && k < cnt) ? d[at(l0 + l, min(c0 + 1 + k, n - 1))] : 0.0;
-    }
-  };
-  // producers: stage the fetched chunk c, start fetching chunk c + 1, then compute chunk c's
-  // per-cell quantities into pre[buf]
-  auto prepare = [&](int c, int buf) {
-    const int c0 = c * C, cnt = min(C, n - c0);
-#pragma unroll
-    for (int j = 0; j < NU; ++j) {
-      const int it = ptid + NP * j;
-      int l, k;
-      slot(it, C + 2, l, k);
-      if (it < (C + 2) * L && k < cnt + 2) su[k][l] = mix::d2f(bu[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < ND; ++j) {
-      const int it = ptid + NP * j;
-      int l, k;
-      slot(it, C, l, k);
-      if (it < C * L && k < cnt) sd[k][l] = mix::d2f(bd[j]);
-    }
-    if (c + 1 < nchunks) fetch(c + 1);
-    asm volatile("bar.sync 1, %0;" ::"n"(NP));
-    for (int it = ptid; it < cnt * L; it += NP) {
-      const int l = it % L, k = it / L;
-      const float u0 = su[k][l], u1 = su[k + 1][l], u2 = su[k + 2][l];
-      const float ud2 = sd[k][l] * dif;
-      const float p1 = (u1 - u0) * rdif, p2 = (u2 - u1) * rdif;
-      const float s1 = (u0 - u1) * (u0 - u1), s2 = (u1 - u2) * (u1 - u2);
-      const float r1 = 1.0f / (s1 + eps), r2 = 1.0f / (s2 + eps);
-      constexpr float k6720 = 1.0f / 6720.0f;
-      const float B = (1029270.0f * u2 - 2129184.0f * u1 + 1099914.0f * u0 - 494958.0f * ud2) * k6720;
-      const float Cc = ((-1029270.0f * u0 + 2129184.0f * u1 - 1099914.0f * u2 + 281121.0f * ud2) * ud2 +
-                        (1099445.0f * u2 - 4317056.0f * u1 + 2118166.0f * u0) * u2 +
-                        4317056.0f * (u1 - u0) * u1 + 1099445.0f * u0 * u0) * k6720;
-      const float P = 0.75f * (u2 - u0) * rdif - 0.25f * sd[k][l];
-      pre[buf][0][k][l] = B;
-      pre[buf][1][k][l] = Cc;
-      pre[buf][2][k][l] = s1;
-      pre[buf][3][k][l] = s2;
-      pre[buf][4][k][l] = P * (1.0f / lw0) - ((lw1 / lw0) * p1 + (lw2 / lw0) * p2);
-      pre[buf][5][k][l] = lw1 * r1 + lw2 * r2;
-      pre[buf][6][k][l] = lw1 * p1 + lw2 * p2;
-      pre[buf][7][k][l] = lw1 * r1 * p1 + lw2 * r2 * p2;
-    }
-  };
-  // producers: the limited values of chunk c (in outf[buf]) to global memory
-  auto store = [&](int c, int buf) {
-    const int c0 = c * C, cnt = min(C, n - c0);
-    for (int it = ptid; it < cnt * L; it += NP) {
-      int l, k;
-      slot(it, cnt, l, k);
-      if (l0 + l < nl) {
-        const size_t o = at(l0 + l, c0 + k);
-        const float x = outf[buf][k][l];
-        d[o] = mix::f2d(x);
-        dt[o] = x;
-      }
-    }
-  };
-  float d0 = sweeper ? mix::d2f(d[at(l0 + tid, 0)]) : 0.f;  // ghost before the first cell
-  if (!sweeper_warp) {
-    fetch(0);
-    prepare(0, 0);
-  }
-  __syncthreads();
-  for (int s = 0; s <= nchunks; ++s) {
-    if (sweeper_warp) {
-      if (s < nchunks && sweeper) {
-        const int cnt = min(C, n - s * C), buf = s & 1;
-        constexpr float a = 281121.0f / 6720.0f, c4 = 0.25f / lw0;
-        for (int k = 0; k < cnt; ++k) {
-          const float ud0 = d0 * dif;
-          const float s0 = fabsf(fmaf(fmaf(a, ud0, pre[buf][0][k][tid]), ud0, pre[buf][1][k][tid]));
-          const float t = fabsf(s0 - pre[buf][2][k][tid]) + fabsf(s0 - pre[buf][3][k][tid]);
-          const float tau = 0.25f * t * t;
-          const float w0 = lw0 * fmaf(tau, __fdividef(1.0f, s0 + eps), 1.0f);
-          const float num = fmaf(w0, fmaf(-c4, d0, pre[buf][4][k][tid]),
-                                 fmaf(tau, pre[buf][7][k][tid], pre[buf][6][k][tid]));
-          const float den = w0 + fmaf(tau, pre[buf][5][k][tid], lw1 + lw2);
-          d0 = __fdividef(num, den);
-          outf[buf][k][tid] = d0;
+  if constexpr (kStaged) {
+    __shared__ T su[8][kLimC][33], sd[8][kLimC][33];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;  // a warp: 32 lines, one segment
+    if (xd && c0 < c1) {
+      const size_t mine = field + size_t(min(line, nl - 1)) * G.nx;
+      LimitSweep<T> s(K, q[mine + max(c0 - 1, 0)], q[mine + c0]);
+      T dl = used;
+      for (int a = c0; a < c1; a += kLimC) {
+        const int cnt = min(kLimC, c1 - a);
+        __syncwarp();
+#pragma unroll 4
+        for (int j = 0; j < 32 * kLimC / 32; ++j) {  // the right neighbours of cells a .. a + 15
+          const int r = j * (32 / kLimC) + lane / kLimC, c = lane % kLimC;
+          const size_t kr = field + size_t(min(l0 + r, nl - 1)) * G.nx + min(a + c + 1, n - 1);
+          su[wid][c][r] = q[kr];
+          sd[wid][c][r] = from_d<T>(d[kr]);
+        }
+        __syncwarp();
+        for (int c = 0; c < cnt; ++c) {
+          s.next(su[wid][c][lane], sd[wid][c][lane]);
+          dl = s.at(dl);
+          sd[wid][c][lane] = dl;
+        }
+        __syncwarp();
+#pragma unroll 4
+        for (int j = 0; j < 32 * kLimC / 32; ++j) {
+          const int r = j * (32 / kLimC) + lane / kLimC, c = lane % kLimC;
+          if (l0 + r < nl && c < cnt) out[field + size_t(l0 + r) * G.nx + a + c] = sd[wid][c][r];
         }
       }
-    } else {
-      if (s + 1 < nchunks) prepare(s + 1, (s + 1) & 1);
-      if (s >= 1) store(s - 1, (s - 1) & 1);
+      last[threadIdx.x] = dl;
+    } else if (live) {
+      sweep(used, false);
     }
+  } else if (live) {
+    sweep(used, false);
+  }
+  for (int pass = 1; pass < segs; ++pass) {
     __syncthreads();
+    const T left = live && seg ? last[threadIdx.x - lines] : used;
+    const bool redo = live && !same_bits(left, used);
+    if (!__syncthreads_or(redo)) break;
+    if (redo) {
+      used = left;
+      sweep(left, true);
+    }
   }
 }
 
@@ -639,13 +664,14 @@ __global__ void __launch_bounds__(kHFluxThreads) kh_flux(GeoH G, const T* __rest
   for (int k = 0; k < 12; ++k) F[size_t(k) * nface + o] = acc[k];
 }
 
-// rhs (:710-730) and RungeKutta3 (:733-782) for u, v, w
+// rhs (:710-730) and RungeKutta3 (:733-782) for u, v, w: stage 1 starts from the limited moments
+// (vt, wt) and saves them, the later stages combine with the unlimited stage values in v, w.
 template <typename T>
 __global__ void __launch_bounds__(256, 4) kh_update(GeoH G, int stage, const T* __restrict__ fx, const T* __restrict__ fy,
                           double* __restrict__ q, double* __restrict__ q0,
                           double* __restrict__ v, double* __restrict__ v0,
-                          double* __restrict__ vs, double* __restrict__ w,
-                          double* __restrict__ w0, double* __restrict__ ws,
+                          const T* __restrict__ vt, double* __restrict__ w,
+                          double* __restrict__ w0, const T* __restrict__ wt,
                           double* __restrict__ prim, float* __restrict__ qt,
                           float* __restrict__ primt, StepState* st) {
   if (st->done) return;
@@ -676,12 +702,12 @@ __global__ void __launch_bounds__(256, 4) kh_update(GeoH G, int stage, const T* 
         const size_t c = size_t(e) * nc + k;
         double bq, bv, bw, cq = q[c], cv, cw;
         if (stage == 1) {
-          bq = cq; bv = v[c]; bw = w[c];
+          bq = cq; bv = to_d<T>(vt[c]); bw = to_d<T>(wt[c]);
           q0[c] = bq; v0[c] = bv; w0[c] = bw;
           cv = bv; cw = bw;
         } else {
           bq = q0[c]; bv = v0[c]; bw = w0[c];
-          cv = vs[c]; cw = ws[c];
+          cv = v[c]; cw = w[c];
         }
         qn[e] = mix::rk_stage(bq, cq, ru, dt, stage);
         const double nv = mix::rk_stage(bv, cv, rv, dt, stage);
@@ -689,9 +715,7 @@ __global__ void __launch_bounds__(256, 4) kh_update(GeoH G, int stage, const T* 
         q[c] = qn[e];
         qt[c] = mix::d2f(qn[e]);
         v[c] = nv;
-        vs[c] = nv;
         w[c] = nw;
-        ws[c] = nw;
       }
       const float fr = mix::d2f(qn[0]);
       double ir = mix::f2d(__frcp_rn(fr));
@@ -722,21 +746,19 @@ __global__ void __launch_bounds__(256, 4) kh_update(GeoH G, int stage, const T* 
         const size_t c = size_t(e) * nc + k;
         double bq, bv, bw, cq = q[c], cv, cw;
         if (stage == 1) {
-          bq = cq; bv = v[c]; bw = w[c];   // save() after the first rhs: limited moments
+          bq = cq; bv = vt[c]; bw = wt[c];  // save() after the first rhs: limited moments
           q0[c] = bq; v0[c] = bv; w0[c] = bw;
           cv = bv; cw = bw;
         } else {
           bq = q0[c]; bv = v0[c]; bw = w0[c];
-          cv = vs[c]; cw = ws[c];          // unlimited stage values (cell.v1 / cell.v2)
+          cv = v[c]; cw = w[c];            // unlimited stage values (cell.v1 / cell.v2)
         }
         qn[e] = ssprk3(bq, cq, ru, dt, stage);
         const double nv = ssprk3(bv, cv, rv, dt, stage);
         const double nw = ssprk3(bw, cw, rw, dt, stage);
         q[c] = qn[e];
         v[c] = nv;
-        vs[c] = nv;
         w[c] = nw;
-        ws[c] = nw;
       }
       double u, vv, p, h, sr;
       cell_prim(G.g1, qn, u, vv, p, h, sr);
@@ -770,14 +792,36 @@ GeoH geo_of(const hteno_solver* s) {
   return G;
 }
 
+// The limiter's launch: lines per block and segments per line.  32 lines x 8 segments (coalesced)
+// while that gives the chip's 608 sub-partitions two warps each or more; else 16 lines x 8 segments: a
+// small grid is bound by the length of a chain, and twice the blocks, of one warp per sub-partition,
+// put its warps on more of the chip.  Segments have at least 16 cells, about what a repeated sweep takes to agree.
+// Measured at 2048^2 in float 0.55 -> 0.27 ms a launch (one warp per line group before, its block's
+// three other warps staging the lines), at 300 x 211 in double 2.42 -> 0.43 ms.
+template <typename T>
+void launch_limit(hteno_solver* s, const GeoH& G, const HermiteK<T>& K, const WorkH<T>& W) {
+  const int nx = G.nx, ny = G.ny;
+  auto blocks = [&](int nl, int lines) { return 4 * ((nl + lines - 1) / lines); };
+  const bool wide = (blocks(nx, 32) + blocks(ny, 32)) * 8 >= 2 * 608;
+  const int lines = wide ? 32 : 16;
+  const int segs = std::max(2, std::min(8, std::min(nx, ny) / 32 * 2));
+  const int nbx = blocks(ny, lines), nby = blocks(nx, lines);
+  const unsigned threads = unsigned(lines * segs);  // whole warps
+  constexpr bool staged = std::is_same<T, float>::value;
+  if (wide && staged)
+    kh_limit<T, staged><<<unsigned(nbx + nby), threads, 0, s->stream>>>(G, K, W.qt, s->v, s->w, W.vt, W.wt, lines,
+                                                                       nbx, s->dstate);
+  else
+    kh_limit<T, false><<<unsigned(nbx + nby), threads, 0, s->stream>>>(G, K, W.qt, s->v, s->w, W.vt, W.wt, lines,
+                                                                      nbx, s->dstate);
+}
+
 template <typename T>
 void launch_step(hteno_solver* s, const GeoH& G) {
   cudaStream_t cs = s->stream;
   WorkH<T> W = carve_h<T>(s->work, G.nx, G.ny);
   if constexpr (std::is_same<T, double>::value) {
     W.qt = s->q;
-    W.vt = s->v;
-    W.wt = s->w;
     W.primt = W.prim;
   }
   const HermiteK<T> K = make_hermite_k<T>(s->dx);  // setGridSize(dx) for both directions
@@ -786,7 +830,6 @@ void launch_step(hteno_solver* s, const GeoH& G) {
   const size_t nc = size_t(nx) * ny;
   const double ncd = double(nc);
   const int k_l = trace_kind(s, "h_limit", ncd * 4 * 8 * 6, 0);
-  const int nbx = 4 * ((ny + kLimLines - 1) / kLimLines), nby = 4 * ((nx + kLimLines - 1) / kLimLines);
   const int k_fx = trace_kind(s, "h_faces_x", ncd * 128 + double(nxf) * 31 * sizeof(T), 0);
   const int k_fy = trace_kind(s, "h_faces_y", ncd * 128 + double(nyf) * 31 * sizeof(T), 0);
   const int k_x = trace_kind(s, "h_flux_x", double(nxf) * 43 * sizeof(T), 0);
@@ -795,11 +838,7 @@ void launch_step(hteno_solver* s, const GeoH& G) {
   k_begin_step<<<1, 1, 0, cs>>>(s->dstate);
   for (int stage = 1; stage <= 3; ++stage) {
     trace_begin(s, k_l);
-    if constexpr (std::is_same<T, float>::value)
-      kh_limit_f<<<unsigned(nbx + nby), kLimThreads, 0, cs>>>(G, K, s->q, s->v, s->w, W.vt, W.wt, nbx,
-                                                               s->dstate);
-    else
-      kh_limit<T><<<unsigned(nbx + nby), kLimThreads, 0, cs>>>(G, K, s->q, s->v, s->w, nbx, s->dstate);
+    launch_limit<T>(s, G, K, W);
     trace_end(s);
     // the y faces and fluxes beside the x ones on the side stream (one stream while timing)
     // (if the fork cannot be recorded, the y kernels stay on the solver's stream)
@@ -834,7 +873,7 @@ void launch_step(hteno_solver* s, const GeoH& G) {
       primtf = W.primt;
     }
     kh_update<T><<<unsigned((nc + 255) / 256), 256, 0, cs>>>(G, stage, W.fx, W.fy, s->q, s->q0,
-                                                            s->v, s->v0, W.vs, s->w, s->w0, W.ws,
+                                                            s->v, s->v0, W.vt, s->w, s->w0, W.wt,
                                                             W.prim, qtf, primtf, s->dstate);
     trace_end(s);
   }
