@@ -954,52 +954,49 @@ __device__ __forceinline__ double hermite_weighted(const DevConst& C, int which,
   return catchnan(dot3w(p, w).v);
 }
 
-// kind 0 hteno (:295-379), 1 htenoi (:670-758), 2 linear (:760-812);
-// out = {u^-, u^+, d^-, d^+} at x_{i+1/2}.  C in global memory.
+// One side of kind 0 hteno (:295-379), 1 htenoi (:670-758) or 2 linear (:760-812) at x_{i+1/2}: side
+// 0 from the cells u[0..2], d[0..2] (u^-, d^-), side 1 from the three cells one further to the right
+// (u^+, d^+), by the mirrored coefficients in the reference's order.  C in global memory.
+__device__ __forceinline__ void hermite_side(const DevConst& C, const HermiteK<double>& K, int kind, const fp* u,
+                                             const fp* d, int side, double& val, double& der) {
+  auto pick = [&](double c0, double c1) { return fp(side ? c1 : c0); };
+  if (kind == 2) {
+    fp c[6];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) c[m] = pick(K.crjlin[m][0], K.crjlin[m][1]);
+    val = (dot3(c[0], c[1], c[2], u) + c[3] * d[0] + c[4] * d[2]).v;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) c[m] = pick(K.crjlind[m][0], K.crjlind[m][1]);
+    der = (dot3(c[0], c[1], c[2], u) + dot3(c[3], c[4], c[5], d)).v;
+    return;
+  }
+  const bool imp = kind == 1;
+  const fp ud[3] = {d[0] * K.dif, d[1] * K.dif, d[2] * K.dif};
+  fp p[3], SI[3];
+  const auto& a = K.crj;
+  p[0] = pick(a[0][0], a[1][1]) * u[0] + pick(a[1][0], a[0][1]) * u[1] + pick(a[2][0], -a[2][1]) * d[0];
+  p[1] = pick(a[0][1], a[1][0]) * u[1] + pick(a[1][1], a[0][0]) * u[2] + pick(a[2][1], -a[2][0]) * d[2];
+  p[2] = pick(a[0][2], a[2][2]) * u[0] + fp(a[1][2]) * u[1] + pick(a[2][2], a[0][2]) * u[2];
+  hermite_si(u, ud, SI);
+  val = hermite_weighted(C, side, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brk(u, ud), SI));
+
+  const auto& b = K.crjd;
+  p[0] = pick(b[0][0], b[0][1]) * u[0] + pick(b[1][0], b[1][1]) * u[1] + pick(b[2][0], b[3][1]) * d[0] +
+         pick(b[3][0], b[2][1]) * d[1];
+  p[1] = pick(b[0][1], b[0][0]) * u[1] + pick(b[1][1], b[1][0]) * u[2] + pick(b[2][1], b[3][0]) * d[1] +
+         pick(b[3][1], b[2][0]) * d[2];
+  const fp s = pick(b[0][2], b[2][2]) * u[0] + fp(b[1][2]) * u[1] + pick(b[2][2], b[0][2]) * u[2];
+  p[2] = (side ? -s : s) + fp(b[3][2]) * d[1];
+  hermite_sid(u, ud, SI);
+  der = hermite_weighted(C, 2 + side, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brkd(u, ud), SI));
+}
+// Both sides: out = {u^-, u^+, d^-, d^+}
 __device__ __forceinline__ void hermite_recon(const DevConst& C, const HermiteK<double>& K,
                                               int kind, const double* uin, const double* din,
                                               double* out) {
   const fp u[4] = {uin[0], uin[1], uin[2], uin[3]}, d[4] = {din[0], din[1], din[2], din[3]};
-  auto k = [](double c) { return fp(c); };
-  if (kind == 2) {
-    out[0] = (dot3(K.crjlin[0][0], K.crjlin[1][0], K.crjlin[2][0], u) + k(K.crjlin[3][0]) * d[0] +
-              k(K.crjlin[4][0]) * d[2]).v;
-    out[1] = (dot3(K.crjlin[0][1], K.crjlin[1][1], K.crjlin[2][1], u + 1) + k(K.crjlin[3][1]) * d[1] +
-              k(K.crjlin[4][1]) * d[3]).v;
-    out[2] = (dot3(K.crjlind[0][0], K.crjlind[1][0], K.crjlind[2][0], u) +
-              dot3(K.crjlind[3][0], K.crjlind[4][0], K.crjlind[5][0], d)).v;
-    out[3] = (dot3(K.crjlind[0][1], K.crjlind[1][1], K.crjlind[2][1], u + 1) +
-              dot3(K.crjlind[3][1], K.crjlind[4][1], K.crjlind[5][1], d + 1)).v;
-    return;
-  }
-  const bool imp = kind == 1;
-  fp ud[4];
-#pragma unroll
-  for (int m = 0; m < 4; ++m) ud[m] = d[m] * k(K.dif);
-  fp p[3], SI[3];
-  p[0] = k(K.crj[0][0]) * u[0] + k(K.crj[1][0]) * u[1] + k(K.crj[2][0]) * d[0];
-  p[1] = k(K.crj[0][1]) * u[1] + k(K.crj[1][1]) * u[2] + k(K.crj[2][1]) * d[2];
-  p[2] = k(K.crj[0][2]) * u[0] + k(K.crj[1][2]) * u[1] + k(K.crj[2][2]) * u[2];
-  hermite_si(u, ud, SI);
-  out[0] = hermite_weighted(C, 0, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brk(u, ud), SI));
-
-  p[0] = k(K.crjd[0][0]) * u[0] + k(K.crjd[1][0]) * u[1] + k(K.crjd[2][0]) * d[0] + k(K.crjd[3][0]) * d[1];
-  p[1] = k(K.crjd[0][1]) * u[1] + k(K.crjd[1][1]) * u[2] + k(K.crjd[2][1]) * d[1] + k(K.crjd[3][1]) * d[2];
-  p[2] = k(K.crjd[0][2]) * u[0] + k(K.crjd[1][2]) * u[1] + k(K.crjd[2][2]) * u[2] + k(K.crjd[3][2]) * d[1];
-  hermite_sid(u, ud, SI);
-  out[2] = hermite_weighted(C, 2, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brkd(u, ud), SI));
-
-  p[0] = k(K.crj[1][1]) * u[1] + k(K.crj[0][1]) * u[2] - k(K.crj[2][1]) * d[1];
-  p[1] = k(K.crj[1][0]) * u[2] + k(K.crj[0][0]) * u[3] - k(K.crj[2][0]) * d[3];
-  p[2] = k(K.crj[2][2]) * u[1] + k(K.crj[1][2]) * u[2] + k(K.crj[0][2]) * u[3];
-  hermite_si(u + 1, ud + 1, SI);
-  out[1] = hermite_weighted(C, 1, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brk(u + 1, ud + 1), SI));
-
-  p[0] = k(K.crjd[0][1]) * u[1] + k(K.crjd[1][1]) * u[2] + k(K.crjd[3][1]) * d[1] + k(K.crjd[2][1]) * d[2];
-  p[1] = k(K.crjd[0][0]) * u[2] + k(K.crjd[1][0]) * u[3] + k(K.crjd[3][0]) * d[2] + k(K.crjd[2][0]) * d[3];
-  p[2] = -(k(K.crjd[2][2]) * u[1] + k(K.crjd[1][2]) * u[2] + k(K.crjd[0][2]) * u[3]) + k(K.crjd[3][2]) * d[2];
-  hermite_sid(u + 1, ud + 1, SI);
-  out[3] = hermite_weighted(C, 3, p, SI, hermite_tau(imp, imp ? fp(0.0) : hermite_brkd(u + 1, ud + 1), SI));
+  hermite_side(C, K, kind, u, d, 0, out[0], out[2]);
+  hermite_side(C, K, kind, u + 1, d + 1, 1, out[1], out[3]);
 }
 
 // hermiteLimiter (Schemes_Hermite.cpp:634-662); dif: the cell size, as a shared denominator

@@ -62,3 +62,33 @@ def test_limiter_segments_mixed(hteno_lib, cuda, nx, ny):
     got = run2(hteno_lib, q, v, w, 1, precision=hteno_lib.PREC_MIXED)
     for a, b, tol in zip(got, want, (1e-5, 1e-2, 1e-2)):
         assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
+
+
+# fewer cells than segments, one cell a segment and one more, ragged
+@pytest.mark.parametrize("nx", [6, 41, 42, 85, 333, 1500])
+@pytest.mark.parametrize("kind", ["noise", "flat", "waves"])
+def test_hermite1d_sensor_bitwise(hteno_lib, cuda, oracle, nx, kind):
+    """LMPE hits (runs of candidates of every length) and the segmented sweep, several steps, so that
+    flags persist and meet new candidates."""
+    rng = np.random.default_rng(nx)
+    x = (np.arange(nx) + 0.5) / nx
+    if kind == "waves":
+        rho = 1.5 + 0.4 * np.sin(2 * np.pi * x) + np.where((x > 0.3) & (x < 0.6), 0.5, 0.0)
+    elif kind == "flat":
+        rho = np.where(x < 0.4, 1.0, 2.0)
+    else:
+        rho = rng.uniform(0.5, 2.0, nx)
+    q = np.ascontiguousarray(np.stack([rho, 0.3 * rho * (kind != "flat"), 2.5 + 0.1 * rho]))
+    v = rng.normal(size=q.shape) * 0.1
+    if kind == "flat":
+        v *= 0.0
+        v[:, nx // 2] = 1.0
+    v = np.ascontiguousarray(v)
+    want_q, want_v, _, n = oracle.hermite1d_run(q, v, 5)
+    cfg = hteno_lib.config(dims=1, scheme=hteno_lib.SCHEME_HERMITE, nx=nx)
+    with hteno_lib.Solver(cfg) as s:
+        s.set_state(q)
+        s.set_moments(v)
+        s.step(5)
+        np.testing.assert_array_equal(s.get_state(), want_q)
+        np.testing.assert_array_equal(s.get_moments(), want_v)
