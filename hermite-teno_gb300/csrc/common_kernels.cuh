@@ -13,20 +13,21 @@ __device__ __forceinline__ int bmap(int i, int n, int bc) {
 }
 
 // Block-wide max of a non-negative double folded into *bits (NaN is skipped, as fmax skips it
-// in the reference's reduction).  Every thread of the block must call it.
+// in the reference's reduction); on the integer pipes: non-negative doubles order as their bits.
+// Every thread of the block must call it.
 __device__ __forceinline__ void block_max_to(double v, unsigned long long* bits) {
-  __shared__ double red[32];
-  if (isnan(v)) v = 0.0;
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __shared__ unsigned long long red[32];
+  unsigned long long m = static_cast<unsigned long long>(__double_as_longlong(v));
+  if (m > 0x7ff0000000000000ull) m = 0ull;  // NaN, or a sign bit
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) red[wid] = v;
+  if (lane == 0) red[wid] = m;
   __syncthreads();
   if (wid == 0) {
     const int nw = (blockDim.x + 31) >> 5;
-    v = lane < nw ? red[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0 && v > 0.0)
-      atomicMax(bits, static_cast<unsigned long long>(__double_as_longlong(v)));
+    m = lane < nw ? red[lane] : 0ull;
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0 && m) atomicMax(bits, m);
   }
 }
 

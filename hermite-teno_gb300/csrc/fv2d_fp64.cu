@@ -492,7 +492,7 @@ __global__ void kp_update(Geo G, int stage, const double* __restrict__ fx,
         } else {
           base = q0[v * nc + k];
         }
-        qn[v] = ssprk3(base, cur, rhs[v], dt, stage);
+        qn[v] = par::rk3(base, cur, rhs[v], dt, stage);
         q[v * nc + k] = qn[v];
       }
       double w[4], h, sr;
@@ -502,8 +502,8 @@ __global__ void kp_update(Geo G, int stage, const double* __restrict__ fx,
       prim[2 * nc + k] = h;
       prim[3 * nc + k] = sr;
       if (stage == 3) ms = par::max_speed2(G.gamma, w);
-      bad = (isnan(qn[0]) || isnan(qn[1]) || isnan(qn[2]) || isnan(qn[3])) ? 1 : 0;
-      bad |= (qn[0] <= 0.0 || w[3] <= 0.0) ? 2 : 0;
+      bad = (par::nan_bits(qn[0]) || par::nan_bits(qn[1]) || par::nan_bits(qn[2]) || par::nan_bits(qn[3])) ? 1 : 0;
+      bad |= (par::nonpositive_bits(qn[0]) || par::nonpositive_bits(w[3])) ? 2 : 0;
     }
   }
   if (stage == 3) block_max_to(ms, &st->maxbits);
@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
     for (int v = 0; v < 4; ++v) {
       const double cur = S.q[v][t + 3][i + 3];
       const double base = stage == 1 ? cur : qbase[v * nc + k];
-      qn[v] = ssprk3(base, cur, rhs[v], dt, stage);
+      qn[v] = par::rk3(base, cur, rhs[v], dt, stage);
       qout[v * nc + k] = qn[v];
     }
     double w[4], h, sr;
@@ -751,8 +751,8 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
     pout[2 * nc + k] = h;
     pout[3 * nc + k] = sr;
     if (stage == 3) ms = fmax(ms, par::max_speed2(G.gamma, w));
-    bad |= (isnan(qn[0]) || isnan(qn[1]) || isnan(qn[2]) || isnan(qn[3])) ? 1 : 0;
-    bad |= (qn[0] <= 0.0 || w[3] <= 0.0) ? 2 : 0;
+    bad |= (par::nan_bits(qn[0]) || par::nan_bits(qn[1]) || par::nan_bits(qn[2]) || par::nan_bits(qn[3])) ? 1 : 0;
+    bad |= (par::nonpositive_bits(qn[0]) || par::nonpositive_bits(w[3])) ? 2 : 0;
   }
   if (stage == 3) block_max_to(ms, &st->maxbits);
   if (bad) atomicOr(&st->status, bad);

@@ -86,7 +86,7 @@ __global__ void kh1_init(GeoH1 G, const double* __restrict__ q, StepState* st) {
   if (i < G.nx) {
     double qq[3] = {q[i], q[G.nx + i], q[2 * G.nx + i]}, w[3], h, sr;
     prim1(G.g1, qq, w, h, sr);
-    ms = par::max_speed1(G.gamma, w);
+    ms = par::max_speed1(G.gamma, w[1], w[2], par::den_of(w[0]));
   }
   block_max_to(ms, &st->maxbits);
 }
@@ -374,14 +374,14 @@ __global__ void kh1_update(GeoH1 G, int stage, WorkH1<T> W, double* __restrict__
         bq = q0[o]; bv = v0[o];
         cv = v[o];  // the unlimited stage value
       }
-      qn[c] = ssprk3(bq, cq, ru, dt, stage);
-      const double nv = ssprk3(bv, cv, rv, dt, stage);
+      qn[c] = par::rk3(bq, cq, ru, dt, stage);
+      const double nv = par::rk3(bv, cv, rv, dt, stage);
       q[o] = qn[c];
       v[o] = nv;
     }
     double w[3], h, sr;
     prim1(G.g1, qn, w, h, sr);
-    if (stage == 3) ms = par::max_speed1(G.gamma, w);
+    if (stage == 3) ms = par::max_speed1(G.gamma, w[1], w[2], par::den_of(w[0]));
     bad = (isnan(qn[0]) || isnan(qn[1]) || isnan(qn[2])) ? 1 : 0;
     bad |= (qn[0] <= 0.0 || w[2] <= 0.0) ? 2 : 0;
   }

@@ -599,9 +599,9 @@ __global__ void __launch_bounds__(256, 4) kh_update(GeoH G, int stage, const T* 
           bq = q0[c]; bv = v0[c]; bw = w0[c];
           cv = v[c]; cw = w[c];            // unlimited stage values (cell.v1 / cell.v2)
         }
-        qn[e] = ssprk3(bq, cq, ru, dt, stage);
-        const double nv = ssprk3(bv, cv, rv, dt, stage);
-        const double nw = ssprk3(bw, cw, rw, dt, stage);
+        qn[e] = par::rk3(bq, cq, ru, dt, stage);
+        const double nv = par::rk3(bv, cv, rv, dt, stage);
+        const double nw = par::rk3(bw, cw, rw, dt, stage);
         q[c] = qn[e];
         v[c] = nv;
         w[c] = nw;

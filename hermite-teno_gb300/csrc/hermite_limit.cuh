@@ -75,7 +75,7 @@ struct LimitSweep<double> {
       flat_r = r;
       return at(dl, &flat_w);
     }
-    const fp p0 = scaled(kNegQuarter, d0 + d2, fp(0.0));
+    const fp p0 = fp(0.0) - lit(kQuarter) * (d0 + d2);
     return (flat_w * quot(p0, den_lit(1.0 - 2E-5, kRcpLw0)) + fp(0.0)).v;
   }
   // |hermite_brk|'s sum on flat data: the terms left out are zeros
@@ -86,7 +86,7 @@ struct LimitSweep<double> {
   __device__ __forceinline__ double at(double dl, par::fp* w0n = nullptr) const {
     using namespace par;
     const fp d0(dl), u[3] = {u0, u1, u2}, ud[3] = {d0 * dif.b, fp(0.0), d2 * dif.b};
-    const fp p0 = scaled(kNegQuarter, d0 + d2, quot(lit(kThreeQuarters) * (u2 - u0), dif));
+    const fp p0 = quot(lit(kThreeQuarters) * (u2 - u0), dif) - lit(kQuarter) * (d0 + d2);
     const fp s0 = hermite_brk(u, ud);
     const fp ta = abs_(s0 - s1) + abs_(s0 - s2), t4 = ta * ta;  // tau = t4 / 4: the factor is exact
     const fp one = lit(kOne);

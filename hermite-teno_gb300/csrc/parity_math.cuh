@@ -89,6 +89,19 @@ __device__ __forceinline__ fp quot(fp a, const Den& d) {
   return a.v / d.b.v;
 }
 
+// Schemes::SSPRK::RungeKuttaIII (Schemes_SSPRK.cpp:3-15): hteno::ssprk3's operations
+__device__ __forceinline__ double rk3(fp q0, fp qn, fp rhs, fp dt, int stage) {
+  if (stage == 1) return (q0 + dt * rhs).v;
+  const fp x = qn + rhs * dt;
+  // (the quarter rounds where it is subnormal: not folded into the sum)
+  if (stage == 2) return (lit(kThreeQuarters) * q0 + lit(kQuarter) * x).v;
+  return quot(scaled(kTwo, x, q0), den_lit(3.0, kRcp3)).v;
+}
+// x <= 0, on the integer pipes
+__device__ __forceinline__ bool nonpositive_bits(double x) {
+  return __double_as_longlong(x) <= 0ll && !nan_bits(x);
+}
+
 // ---- Schemes::Lagrange ----------------------------------------------------------------------
 
 // smoothnessMeasure (Schemes_Lagrange.cpp:1013-1026).  The b are halved term by term (exact
@@ -747,8 +760,8 @@ __device__ __forceinline__ void rusanov(int dir, const Eig& e, const Sides& s, c
 
 // maxSpeed over both directions (Equations_Euler2D.cpp:207-219)
 __device__ __forceinline__ double max_speed2(double g, const double* w) {
-  const double c = sqrt(fabs(g * w[3] / w[0]));
-  return fmax(fmax(w[1] - c, fabs(w[1] + c)), fmax(w[2] - c, fabs(w[2] + c)));
+  const fp c = sqrt_abs(fp(g) * w[3] / w[0]);
+  return fmax(fmax((fp(w[1]) - c).v, fabs((fp(w[1]) + c).v)), fmax((fp(w[2]) - c).v, fabs((fp(w[2]) + c).v)));
 }
 
 // ---- Equations::Euler1D (Equations_Euler1D.cpp) --------------------------------------------
@@ -838,28 +851,34 @@ __device__ __forceinline__ void rusanov1(const Sides1& s, const fp* L, const fp*
   dissipate1(L, R, s.a, ql, qr, fl, fr, F);
 }
 
-// HLLC (Equations_Euler1D.cpp:156-210).  As in 2D the operands of the left or right region are
-// selected first and one copy of the arithmetic runs.
-__device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp* F) {
-  fp wl[3], wr[3], fl[3], qs[3];
-  const Den rl = den_of(ql[0]), rg = den_of(qr[0]);
-  primitive1(g1, ql, rl, wl);
-  primitive1(g1, qr, rg, wr);
-  const fp hl = quot(ql[2] + wl[2], rl);
-  const fp hr = quot(qr[2] + wr[2], rg);
-  const fp rr = sqrt_abs(quot(wr[0], rl));
+// One side of the 1D HLLC flux (Equations_Euler1D.cpp:156-210): primitives, enthalpy, sound speed.
+struct Hllc1Side {
+  fp q[3], w[3], h, c;
+};
+__device__ __forceinline__ Hllc1Side hllc1_side(double g1, const fp* q, const Den& rho) {
+  Hllc1Side s;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) s.q[k] = q[k];
+  primitive1(g1, q, rho, s.w);
+  s.h = quot(q[2] + s.w[2], rho);
+  s.c = sqrt_abs(quot(s.w[2], rho));
+  return s;
+}
+// The flux from its two sides; rl: the left density.  As in 2D the operands of the left or right
+// region are selected first and one copy of the arithmetic runs.
+__device__ __forceinline__ void hllc1(double g1, const Hllc1Side& l, const Hllc1Side& r, const Den& rl, fp* F) {
+  fp fl[3], qs[3];
+  const fp rr = sqrt_abs(quot(r.w[0], rl));
   const fp rrr = lit(kOne) / (lit(kOne) + rr);
-  const fp vm = (wl[1] + wr[1] * rr) * rrr;
+  const fp vm = (l.w[1] + r.w[1] * rr) * rrr;
   const fp qm = lit(kHalf) * vm * vm;
-  const fp hm = (hl + hr * rr) * rrr;
+  const fp hm = (l.h + r.h * rr) * rrr;
   const fp cm = sqrt_abs(fp(g1) * (hm - qm));
-  const fp cl = sqrt_abs(quot(wl[2], rl));
-  const fp cr = sqrt_abs(quot(wr[2], rg));
-  const fp sl = fmin((wl[1] - cl).v, (vm - cm).v);
-  const fp sr = fmax((wr[1] + cr).v, (vm + cm).v);
-  const fp dl = sl - wl[1], dr = sr - wr[1];
-  const fp sm = (qr[1] * dr - ql[1] * dl + wl[2] - wr[2]) / (wr[0] * dr - wl[0] * dl);
-  const fp ps = wl[2] + wl[0] * (wl[1] - sl) * (wl[1] - sm);
+  const fp sl = fmin((l.w[1] - l.c).v, (vm - cm).v);
+  const fp sr = fmax((r.w[1] + r.c).v, (vm + cm).v);
+  const fp dl = sl - l.w[1], dr = sr - r.w[1];
+  const fp sm = (r.q[1] * dr - l.q[1] * dl + l.w[2] - r.w[2]) / (r.w[0] * dr - l.w[0] * dl);
+  const fp ps = l.w[2] + l.w[0] * (l.w[1] - sl) * (l.w[1] - sm);
   const bool outer_l = sl.v > 0.0;
   const bool star_l = !outer_l && sl.v <= 0.0 && sm.v > 0.0;
   const bool star_r = !outer_l && !star_l && sm.v <= 0.0 && sr.v >= 0.0;
@@ -867,8 +886,8 @@ __device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp*
   fp q[3], w[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    q[k] = use_l ? ql[k] : qr[k];
-    w[k] = use_l ? wl[k] : wr[k];
+    q[k] = use_l ? l.q[k] : r.q[k];
+    w[k] = use_l ? l.w[k] : r.w[k];
   }
   flux1(q, w, fl);
   if (star_l || star_r) {
@@ -877,7 +896,7 @@ __device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp*
     const Den den = den_of(s - sm);
     qs[0] = quot(w[0] * nom, den);
     qs[1] = quot(nom * q[1] + ps - w[2], den);
-    qs[2] = quot(nom * q[2] - wl[2] * w[1] + ps * sm, den);
+    qs[2] = quot(nom * q[2] - l.w[2] * w[1] + ps * sm, den);
 #pragma unroll
     for (int k = 0; k < 3; ++k) F[k] = fl[k] + s * (qs[k] - q[k]);
   } else {
@@ -885,10 +904,14 @@ __device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp*
     for (int k = 0; k < 3; ++k) F[k] = fl[k];
   }
 }
+__device__ __forceinline__ void hllc1(double g1, const fp* ql, const fp* qr, fp* F) {
+  const Den rl = den_of(ql[0]);
+  hllc1(g1, hllc1_side(g1, ql, rl), hllc1_side(g1, qr, den_of(qr[0])), rl, F);
+}
 
-__device__ __forceinline__ double max_speed1(double g, const double* w) {  // :91-94
-  const double c = sqrt(fabs(g * w[2] / w[0]));
-  return fmax(fabs(w[1] - c), fabs(w[1] + c));
+__device__ __forceinline__ double max_speed1(double g, fp u, fp p, const Den& rho) {  // :91-94
+  const fp c = sqrt_abs(quot(fp(g) * p, rho));
+  return fmax(fabs((u - c).v), fabs((u + c).v));
 }
 
 // ---- Schemes::Hermite (Schemes_Hermite.cpp) -------------------------------------------------
@@ -1003,7 +1026,7 @@ __device__ __forceinline__ void hermite_recon(const DevConst& C, const HermiteK<
 __device__ __forceinline__ double hermite_limiter(const Den& dif, const double* uin, const double* din) {
   const fp u[3] = {uin[0], uin[1], uin[2]}, d[3] = {din[0], din[1], din[2]};
   fp p[3], sm[3], w[3];
-  p[0] = scaled(kNegQuarter, d[0] + d[2], quot(lit(kThreeQuarters) * (u[2] - u[0]), dif));
+  p[0] = quot(lit(kThreeQuarters) * (u[2] - u[0]), dif) - lit(kQuarter) * (d[0] + d[2]);
   p[1] = quot(u[1] - u[0], dif);
   p[2] = quot(u[2] - u[1], dif);
   const fp ud[3] = {d[0] * dif.b, d[1] * dif.b, d[2] * dif.b};

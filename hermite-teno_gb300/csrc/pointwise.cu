@@ -208,7 +208,7 @@ __global__ void k_ssprk3(const double* __restrict__ q0, const double* __restrict
                          double* __restrict__ out, long n) {
   long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (k >= n) return;
-  out[k] = ssprk3(q0[k], qn[k], rhs[k], dt, stage);
+  out[k] = par::rk3(q0[k], qn[k], rhs[k], dt, stage);
 }
 
 }  // namespace
