@@ -452,6 +452,159 @@ __global__ void __launch_bounds__(kFaceThreads) kp_flux(Geo G, const double* __r
   for (int v = 0; v < 4; ++v) F[v * nface + o] = Ff[v];
 }
 
+// ---- small grids: 8 lanes per face ---------------------------------------------------------------
+// A grid of a few thousand faces gives the chip's 608 SM sub-partitions less than a warp each, and an
+// FP64 unit takes 64 cycles per warp instruction however many lanes are active: the time of kp_faces
+// and kp_flux is then one thread's ~850 and ~2500 FP64 operations in sequence.  Here 8 lanes share a
+// face, ~180 and ~400 operations each, in 8 times the warps: the same operations on the same values.
+// A warp whose faces are all skipped returns; the others compute all their faces (nothing reads what
+// a skipped neighbour left) and store the ones that are not.
+
+// kp_faces: lane r + 4 s projects characteristic field r and reconstructs side s.
+template <int DIR>
+__global__ void __launch_bounds__(64) kp_faces_lanes(Geo G, const double* __restrict__ q,
+                                                     const double* __restrict__ prim, double* __restrict__ fc,
+                                                     double* __restrict__ froe, const StepState* st,
+                                                     const uint8_t* __restrict__ deep) {
+  if (st && st->done) return;
+  const int nf = DIR == 1 ? G.nx + 1 : G.ny + 1;
+  const int nt = DIR == 1 ? G.ny : G.nx;
+  const long all = long(nf) * nt, gid = (blockIdx.x * 64l + threadIdx.x) >> 3;
+  const long idx = min(gid, all - 1);
+  const int l = threadIdx.x & 7, r = l & 3, side = l >> 2;
+  int f, t;
+  if (DIR == 1) { f = int(idx % nf); t = int(idx / nf); }
+  else { t = int(idx % nt); f = int(idx / nt); }
+  const size_t nc = size_t(G.nx) * G.ny;
+  const int ns = DIR == 1 ? G.nx : G.ny;
+  auto cell = [&](int s) -> size_t {
+    const int m = bmap(s, ns, G.bc);
+    return DIR == 1 ? size_t(t) * G.nx + m : size_t(m) * G.nx + t;
+  };
+  bool skip = gid >= all;
+  if (deep && !skip) {  // as kp_faces
+    const int a = bmap(f - 1, ns, G.bc), b = bmap(f, ns, G.bc);
+    skip = true;
+#pragma unroll
+    for (int m = -2; m <= 2; ++m) {
+      const int tt = bmap(t + m, nt, G.bc);
+      const size_t ka = DIR == 1 ? size_t(tt) * G.nx + a : size_t(a) * G.nx + tt;
+      const size_t kb = DIR == 1 ? size_t(tt) * G.nx + b : size_t(b) * G.nx + tt;
+      skip = skip && deep[ka] && deep[kb];
+    }
+  }
+  if (__all_sync(0xffffffffu, skip)) return;
+  const size_t ca = cell(f - 1), cb = cell(f);
+  const par::Eig E = par::eig(G.g1, DIR, prim[3 * nc + ca], prim[ca], prim[nc + ca],
+                              prim[2 * nc + ca], prim[3 * nc + cb], prim[cb], prim[nc + cb],
+                              prim[2 * nc + cb]);
+  const par::LeftRow L = par::left_row(E, DIR, r);
+  double ch[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    const size_t c = cell(f - 3 + m);
+    ch[m] = L.dot(q[c], q[nc + c], q[2 * nc + c], q[3 * nc + c]).v;
+  }
+  const double val = par::lagrange_side(g_dev, G.recon, ch, side);
+  if (skip) return;
+  const size_t nface = size_t(nf) * nt;
+  const size_t o = DIR == 1 ? size_t(t) * nf + f : size_t(f) * nt + t;
+  fc[size_t(4 * side + r) * nface + o] = val;
+  if (l == 0) par::eig_store(E, froe + o, nface);
+}
+
+// kp_flux: lane k interpolates face array k to the Gauss points (GL3); lane m + 4 s (m < 3) then
+// projects side s back at Gauss point m, the two sides of a point meet by a shuffle, and lane v sums
+// component v over the points.
+template <int DIR>
+__global__ void __launch_bounds__(64) kp_flux_lanes(Geo G, const double* __restrict__ fc,
+                                                    const double* __restrict__ froe, double* __restrict__ F,
+                                                    const StepState* st, const uint8_t* __restrict__ deep,
+                                                    const double* __restrict__ gfc) {
+  using par::fp;
+  if (st && st->done) return;
+  const int nf = DIR == 1 ? G.nx + 1 : G.ny + 1;
+  const int nt = DIR == 1 ? G.ny : G.nx;
+  const long all = long(nf) * nt, gid = (blockIdx.x * 64l + threadIdx.x) >> 3;
+  const long idx = min(gid, all - 1);
+  const int l = threadIdx.x & 7, side = l >> 2, pt = min(l & 3, 2), base = threadIdx.x & 24;
+  int f, t;
+  if (DIR == 1) { f = int(idx % nf); t = int(idx / nf); }
+  else { t = int(idx % nt); f = int(idx / nt); }
+  bool skip = gid >= all;
+  if (deep && !skip) {  // as kp_flux
+    const int ns = DIR == 1 ? G.nx : G.ny;
+    const int a = bmap(f - 1, ns, G.bc), b = bmap(f, ns, G.bc);
+    const size_t ka = DIR == 1 ? size_t(t) * G.nx + a : size_t(a) * G.nx + t;
+    const size_t kb = DIR == 1 ? size_t(t) * G.nx + b : size_t(b) * G.nx + t;
+    skip = deep[ka] && deep[kb];
+  }
+  if (__all_sync(0xffffffffu, skip)) return;
+  const size_t nface = size_t(nf) * nt;
+  auto at = [&](int tt) -> size_t { return DIR == 1 ? size_t(tt) * nf + f : size_t(f) * nt + tt; };
+  double u5[5], g[3];
+#pragma unroll
+  for (int m = 0; m < 5; ++m) {
+    const int tr = t - 2 + m;
+    if (gfc && (tr < 0 || tr >= nt))  // a face row of the ghosts (kp_faces_g)
+      u5[m] = gfc[(size_t(tr < 0 ? tr + 2 : tr - nt + 2) * 8 + l) * nf + f];
+    else
+      u5[m] = fc[l * nface + at(bmap(tr, nt, G.bc))];
+  }
+  par::gl3(g_dev, u5, g);
+  const size_t o = at(t);
+  const par::Eig E = par::eig_load(DIR, froe + o, nface);
+  fp c[4], qs[4], Fl[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int src = base + 4 * side + k;
+    const double a = __shfl_sync(0xffffffffu, g[0], src), b = __shfl_sync(0xffffffffu, g[1], src),
+                 d = __shfl_sync(0xffffffffu, g[2], src);
+    c[k] = pt == 0 ? a : pt == 1 ? b : d;
+  }
+  par::right(E, DIR, c, qs);
+  auto swap = [&](fp x) { return fp(__shfl_xor_sync(0xffffffffu, x.v, 4)); };
+  if (G.flux == HTENO_FLUX_HLLC) {
+    const par::Den rho = par::den_of(qs[0]);
+    const par::HllcSide own = par::hllc_side(G.g1, qs, rho);
+    par::HllcSide other;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) other.q[k] = swap(own.q[k]);
+    other.w[0] = other.q[0];
+#pragma unroll
+    for (int k = 1; k < 4; ++k) other.w[k] = swap(own.w[k]);
+    other.h = swap(own.h);
+    other.c = swap(own.c);
+    const fp oy = swap(rho.y);
+    const par::Den rl = side ? par::Den{other.q[0], oy, par::mid_range(other.q[0].v)} : rho;
+    par::HllcSide a = own, b = other;
+    if (side) {
+      a = other;
+      b = own;
+    }
+    par::hllc(G.g1, DIR, a, b, rl, Fl);
+  } else {
+    fp ql[4], qr[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const fp x = swap(qs[k]);
+      ql[k] = side ? x : qs[k];
+      qr[k] = side ? qs[k] : x;
+    }
+    par::rusanov(DIR, E, par::sides_of(G.gamma, G.g1, DIR, ql, qr), ql, qr, Fl);
+  }
+  const fp w = par::ldk(g_dev.gl3w[pt]);
+  double sum = 0.0;
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {  // (w0 F0 + w1 F1) + w2 F2
+    const double x = (w * Fl[v]).v;
+    const fp a = __shfl_sync(0xffffffffu, x, base), b = __shfl_sync(0xffffffffu, x, base + 1),
+             d = __shfl_sync(0xffffffffu, x, base + 2);
+    if (v == l) sum = (a + b + d).v;
+  }
+  if (!skip && l < 4) F[l * nface + o] = sum;
+}
+
 // rhs (FV_System2D.cpp:562-572) + RungeKutta3 (:575-612); stage 0 writes the residual
 __global__ void kp_update(Geo G, int stage, const double* __restrict__ fx,
                           const double* __restrict__ fy, double* __restrict__ q,
@@ -862,8 +1015,13 @@ void fv2d_fp64_stage(hteno_solver* s, const Geo& G, const Work<double>& W, int s
                     cudaEventRecord(s->fork_ev, cs) == cudaSuccess &&
                     cudaStreamWaitEvent(s->side_stream, s->fork_ev, 0) == cudaSuccess;
   cudaStream_t ys = fork ? s->side_stream : cs;
+  // 8 lanes per face (about 5 times the work in a seventh of the sequence) while the faces of both
+  // directions give the chip's 608 sub-partitions less than three quarters of a warp each
+  const bool lanes = nxf + nyf <= 32l * 456;
   trace_begin(s, kf_x);
-  if (gx) {
+  if (lanes && !gx) {
+    kp_faces_lanes<1><<<unsigned((nxf + 7) / 8), 64, 0, cs>>>(G, q, W.prim, W.xc, W.xroe, st, deep);
+  } else if (gx) {
     const long n = long(nx + 1) * (ny + 4);
     kp_faces_g<1><<<unsigned((n + kFaceThreads - 1) / kFaceThreads), kFaceThreads, 0, cs>>>(
         G, q, W.xc, W.xroe, gx, st, deep);
@@ -873,7 +1031,9 @@ void fv2d_fp64_stage(hteno_solver* s, const Geo& G, const Work<double>& W, int s
   }
   trace_end(s);
   trace_begin(s, kf_y);
-  if (gy) {
+  if (lanes && !gy) {
+    kp_faces_lanes<2><<<unsigned((nyf + 7) / 8), 64, 0, ys>>>(G, q, W.prim, W.yc, W.yroe, st, deep);
+  } else if (gy) {
     const long n = long(ny + 1) * (nx + 4);
     kp_faces_g<2><<<unsigned((n + kFaceThreads - 1) / kFaceThreads), kFaceThreads, 0, ys>>>(
         G, q, W.yc, W.yroe, gy, st, deep);
@@ -883,12 +1043,18 @@ void fv2d_fp64_stage(hteno_solver* s, const Geo& G, const Work<double>& W, int s
   }
   trace_end(s);
   trace_begin(s, kx);
-  kp_flux<1><<<unsigned((nxf + kFaceThreads - 1) / kFaceThreads), kFaceThreads, 0, cs>>>(
-      G, W.xc, W.xroe, W.fx, st, deep, gx);
+  if (lanes)
+    kp_flux_lanes<1><<<unsigned((nxf + 7) / 8), 64, 0, cs>>>(G, W.xc, W.xroe, W.fx, st, deep, gx);
+  else
+    kp_flux<1><<<unsigned((nxf + kFaceThreads - 1) / kFaceThreads), kFaceThreads, 0, cs>>>(
+        G, W.xc, W.xroe, W.fx, st, deep, gx);
   trace_end(s);
   trace_begin(s, ky);
-  kp_flux<2><<<unsigned((nyf + kFaceThreads - 1) / kFaceThreads), kFaceThreads, 0, ys>>>(
-      G, W.yc, W.yroe, W.fy, st, deep, gy);
+  if (lanes)
+    kp_flux_lanes<2><<<unsigned((nyf + 7) / 8), 64, 0, ys>>>(G, W.yc, W.yroe, W.fy, st, deep, gy);
+  else
+    kp_flux<2><<<unsigned((nyf + kFaceThreads - 1) / kFaceThreads), kFaceThreads, 0, ys>>>(
+        G, W.yc, W.yroe, W.fy, st, deep, gy);
   trace_end(s);
   // the join; if it cannot be recorded, wait for the side stream on the host instead
   if (fork && (cudaEventRecord(s->join_ev, ys) != cudaSuccess ||
