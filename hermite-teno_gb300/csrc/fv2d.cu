@@ -44,19 +44,67 @@ int fv2d_prepare(hteno_solver* s) {
   return cuda_error(s, cudaGetLastError(), "primitives");
 }
 
+namespace {
+
+void launch_step(hteno_solver* s, const Geo& G) {
+  k_begin_step<<<1, 1, 0, s->stream>>>(s->dstate);
+  if (s->cfg.precision == HTENO_PREC_MIXED) {
+    fv2d_fused_step(s, G, static_cast<double*>(s->work));
+  } else {
+    const Work<double> W = carve<double>(s->work, G.nx, G.ny);
+    if (s->fused64) fv2d_fp64_fused_step(s, G, W);
+    else for (int stage = 1; stage <= 3; ++stage) fv2d_fp64_stage(s, G, W, stage, s->q, nullptr);
+  }
+  k_end_step<<<1, 1, 0, s->stream>>>(s->dstate);
+}
+
+// A plain FP64 step of a small grid is 20 launches on two streams of ~10-30 us each, which the host
+// issues hardly faster than they run: runs of kGraphSteps steps are captured once into a graph (the
+// solver's buffers are fixed; dt, t and the stop live on the device) and replayed.  Larger grids'
+// launches outlast their issue.  64 x 48, 24 steps with state copies: GRAPH_TIMES.
+constexpr int kGraphSteps = 4;
+constexpr size_t kGraphCells = size_t(1) << 15;
+
+// (a stream that the caller is capturing takes the launches themselves)
+bool graphed(const hteno_solver* s) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  return s->cfg.precision == HTENO_PREC_FP64 && !s->fused64 && !s->timing && s->ncell <= kGraphCells &&
+         cudaStreamIsCapturing(s->stream, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone;
+}
+
+cudaError_t ensure_graph(hteno_solver* s, const Geo& G) {
+  if (s->step_graph) return cudaSuccess;
+  cudaStream_t cap, own = s->stream;
+  cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  cudaGraph_t g = nullptr;
+  e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    s->stream = cap;  // the side stream joins the capture through its fork event
+    for (int k = 0; k < kGraphSteps; ++k) launch_step(s, G);
+    s->stream = own;
+    e = cudaStreamEndCapture(cap, &g);
+  }
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&s->step_graph, g, 0);
+  if (g) cudaGraphDestroy(g);
+  cudaStreamDestroy(cap);
+  return e;
+}
+
+}  // namespace
+
 int fv2d_step_async(hteno_solver* s, int nsteps) {
   const Geo G = geo_of(s);
-  for (int n = 0; n < nsteps; ++n) {
-    k_begin_step<<<1, 1, 0, s->stream>>>(s->dstate);
-    if (s->cfg.precision == HTENO_PREC_MIXED) {
-      fv2d_fused_step(s, G, static_cast<double*>(s->work));
-    } else {
-      const Work<double> W = carve<double>(s->work, G.nx, G.ny);
-      if (s->fused64) fv2d_fp64_fused_step(s, G, W);
-      else for (int stage = 1; stage <= 3; ++stage) fv2d_fp64_stage(s, G, W, stage, s->q, nullptr);
+  int left = nsteps;
+  if (graphed(s) && left >= kGraphSteps) {
+    const cudaError_t e = ensure_graph(s, G);
+    if (e != cudaSuccess) return cuda_error(s, e, "fv2d step graph");
+    for (; left >= kGraphSteps; left -= kGraphSteps) {
+      const cudaError_t el = cudaGraphLaunch(s->step_graph, s->stream);
+      if (el != cudaSuccess) return cuda_error(s, el, "fv2d graph launch");
     }
-    k_end_step<<<1, 1, 0, s->stream>>>(s->dstate);
   }
+  for (; left > 0; --left) launch_step(s, G);
   return cuda_error(s, cudaGetLastError(), "fv2d step launch");
 }
 

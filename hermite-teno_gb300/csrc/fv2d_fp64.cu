@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(256) kp_deep(Geo G, const double* __restrict__
   if (st && st->done) return;
   constexpr int TX = 32, TY = 8, W = TX + 6, H = TY + 6;
   __shared__ unsigned long long key[4][H][W];
+  __shared__ bool row[H][TX];  // the 7 cells of a row around a column hold the middle one's state
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const size_t nc = size_t(G.nx) * G.ny;
   const bool ghosts = G.bc >= HTENO_BC_TAYLOR;  // ghosts that are not copies: compare their states
@@ -94,27 +95,39 @@ __global__ void __launch_bounds__(256) kp_deep(Geo G, const double* __restrict__
     for (int v = 0; v < 4; ++v) key[v][y][x] = static_cast<unsigned long long>(__double_as_longlong(qq[v]));
   }
   __syncthreads();
+  for (int it = threadIdx.x; it < TX * H; it += blockDim.x) {
+    const int y = it / TX, x = it - y * TX;
+    bool same = true;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const unsigned long long c = key[v][y][x + 3];
+#pragma unroll
+      for (int dx = 0; dx < 7; ++dx) same &= key[v][y][x + dx] == c;
+    }
+    row[y][x] = same;
+  }
+  __syncthreads();
   const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
   const int gi = i0 + tx, gj = j0 + ty;
-  bool u = false;
-  if (gi < G.nx && gj < G.ny) {
-    const unsigned long long c0 = key[0][ty + 3][tx + 3], c1 = key[1][ty + 3][tx + 3];
-    const unsigned long long c2 = key[2][ty + 3][tx + 3], c3 = key[3][ty + 3][tx + 3];
-    const double qc[4] = {__longlong_as_double(static_cast<long long>(c0)),
-                          __longlong_as_double(static_cast<long long>(c1)),
-                          __longlong_as_double(static_cast<long long>(c2)),
-                          __longlong_as_double(static_cast<long long>(c3))};
-    double w[4];
-    par::primitive(G.g1, qc, w);
-    constexpr double lo = 0x1p-64, hi = 0x1p64;
-    u = w[0] >= lo && w[0] <= hi && w[3] >= lo && w[3] <= hi &&
-        w[1] * w[1] + w[2] * w[2] <= 64.0 * (G.gamma * w[3] / w[0]);
+  bool u = gi < G.nx && gj < G.ny;
+  if (u) {
+    const unsigned long long c[4] = {key[0][ty + 3][tx + 3], key[1][ty + 3][tx + 3], key[2][ty + 3][tx + 3],
+                                     key[3][ty + 3][tx + 3]};
 #pragma unroll
-    for (int dy = 0; dy < 7; ++dy)
+    for (int dy = 0; dy < 7; ++dy) {
+      u &= row[ty + dy][tx];
 #pragma unroll
-      for (int dx = 0; dx < 7; ++dx)
-        u &= key[0][ty + dy][tx + dx] == c0 && key[1][ty + dy][tx + dx] == c1 &&
-             key[2][ty + dy][tx + dx] == c2 && key[3][ty + dy][tx + dx] == c3;
+      for (int v = 0; v < 4; ++v) u &= key[v][ty + dy][tx + 3] == c[v];
+    }
+    if (u) {  // the FP64 unit only where the cells are equal
+      double qc[4], w[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) qc[v] = __longlong_as_double(static_cast<long long>(c[v]));
+      par::primitive(G.g1, qc, w);
+      constexpr double lo = 0x1p-64, hi = 0x1p64;
+      u = w[0] >= lo && w[0] <= hi && w[3] >= lo && w[3] <= hi &&
+          w[1] * w[1] + w[2] * w[2] <= 64.0 * (G.gamma * w[3] / w[0]);
+    }
     deep[size_t(gj) * G.nx + gi] = u ? 1 : 0;
   }
   // cells given their zero residual this stage (every thread reaches the count)
@@ -622,7 +635,7 @@ __global__ void kp_update(Geo G, int stage, const double* __restrict__ fx,
     const size_t ox = size_t(j) * (G.nx + 1) + i, oy = size_t(j) * G.nx + i;
     double rhs[4] = {0.0, 0.0, 0.0, 0.0};  // a deep cell's flux pairs are equal: residual +0
     if (!(deep && deep[k])) {
-      const par::Den da = par::den_of(G.area);  // the four divisions by the cell area
+      const par::Den da{G.area, G.rarea, par::mid_range(G.area)};  // the four divisions by the cell area
 #pragma unroll
       for (int v = 0; v < 4; ++v)
         rhs[v] = par::quot((par::fp(fx[v * nxf + ox]) - fx[v * nxf + ox + 1]) * G.dy +
@@ -883,7 +896,7 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
     const size_t k = size_t(j0 + t) * G.nx + (i0 + i);
     double rhs[4] = {0.0, 0.0, 0.0, 0.0};  // a uniform cell's flux pairs are equal: residual +0
     if (!S.deep[t][i]) {
-      const par::Den da = par::den_of(G.area);
+      const par::Den da{G.area, G.rarea, par::mid_range(G.area)};
 #pragma unroll
       for (int v = 0; v < 4; ++v)
         rhs[v] = par::quot(par::fp(S.rx[v][t][i]) + (par::fp(S.f[v][t * TX + i]) - S.f[v][(t + 1) * TX + i]) * G.dx,
@@ -912,6 +925,10 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
 }
 
 }  // namespace
+
+// Threads per block of the cell kernels: small blocks while they give each of the chip's 608
+// sub-partitions two warps or fewer (a block of 256 would put two on each of its SM's).
+static unsigned update_threads(size_t nc) { return nc <= size_t(32) * 1216 ? 64 : 256; }
 
 int fv2d_fp64_setup(hteno_solver* s) {
   if (upload_const(&g_mask, &g_mu, g_dev) != cudaSuccess)
@@ -980,7 +997,8 @@ void fv2d_fp64_fused_step(hteno_solver* s, const Geo& G, const Work<double>& W) 
 void fv2d_fp64_prim(hteno_solver* s, const Geo& G, const Work<double>& W, const double* q,
                     StepState* st, int do_max) {
   const size_t nc = size_t(G.nx) * G.ny;
-  kp_prim<<<unsigned((nc + 255) / 256), 256, 0, s->stream>>>(G, q, W.prim, st, do_max);
+  const unsigned ut = update_threads(nc);
+  kp_prim<<<unsigned((nc + ut - 1) / ut), ut, 0, s->stream>>>(G, q, W.prim, st, do_max);
 }
 
 void fv2d_fp64_stage(hteno_solver* s, const Geo& G, const Work<double>& W, int stage,
@@ -1062,8 +1080,8 @@ void fv2d_fp64_stage(hteno_solver* s, const Geo& G, const Work<double>& W, int s
     cudaStreamSynchronize(ys);
   const size_t nc = size_t(nx) * ny;
   trace_begin(s, ku);
-  kp_update<<<unsigned((nc + 255) / 256), 256, 0, cs>>>(G, stage, W.fx, W.fy, s->q, s->q0,
-                                                       W.prim, out, st, deep);
+  const unsigned ut = update_threads(nc);
+  kp_update<<<unsigned((nc + ut - 1) / ut), ut, 0, cs>>>(G, stage, W.fx, W.fy, s->q, s->q0, W.prim, out, st, deep);
   trace_end(s);
 }
 
@@ -1167,6 +1185,7 @@ extern "C" int hteno_residual_noalloc(const hteno_config* cfg, const double* q, 
   G.dx = (c.xr - c.xl) / c.nx;
   G.dy = (c.yt - c.yb) / c.ny;
   G.area = G.dx * G.dy;
+  G.rarea = 1.0 / G.area;
   G.gamma = c.gamma;
   G.g1 = c.gamma - 1.0;
   G.x0 = c.xl;
@@ -1186,7 +1205,7 @@ extern "C" int hteno_residual_noalloc(const hteno_config* cfg, const double* q, 
       G, W.xc, W.xroe, W.fx, nullptr);
   kp_flux<2><<<unsigned((nyf + kFaceThreads - 1) / kFaceThreads), kFaceThreads, 0, cs>>>(
       G, W.yc, W.yroe, W.fy, nullptr);
-  kp_update<<<unsigned((nc + 255) / 256), 256, 0, cs>>>(G, 0, W.fx, W.fy, nullptr, nullptr,
-                                                       W.prim, rhs, nullptr);
+  const unsigned ut = update_threads(nc);
+  kp_update<<<unsigned((nc + ut - 1) / ut), ut, 0, cs>>>(G, 0, W.fx, W.fy, nullptr, nullptr, W.prim, rhs, nullptr);
   return cudaGetLastError() == cudaSuccess ? HTENO_OK : HTENO_ERR_CUDA;
 }
