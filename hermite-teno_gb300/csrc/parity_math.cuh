@@ -445,6 +445,19 @@ __device__ __forceinline__ void lagrange_recon(const DevConst& C, int kind, cons
   outp = other_side(C, kind, pp, u + 1, 1);
 }
 
+// lagrange_recon out of line, the stencil by value: the face kernels reconstruct four fields, and four
+// inlined copies overflow the instruction cache.
+struct SidePair {
+  double m, p;
+};
+static __device__ __noinline__ SidePair recon_call(const DevConst& C, int kind, double u0, double u1, double u2,
+                                                   double u3, double u4, double u5) {
+  const double u[6] = {u0, u1, u2, u3, u4, u5};
+  SidePair o;
+  lagrange_recon(C, kind, u, o.m, o.p);
+  return o;
+}
+
 // One side of lagrange_recon (side 0: u^-, side 1: u^+), the same arithmetic.
 __device__ __forceinline__ double lagrange_side(const DevConst& C, int kind, const double* ud, int side) {
   const fp v[5] = {side ? ud[1] : ud[0], side ? ud[2] : ud[1], side ? ud[3] : ud[2], side ? ud[4] : ud[3],
