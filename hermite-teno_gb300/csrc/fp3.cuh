@@ -30,20 +30,22 @@ namespace par {
 enum Lit : int {
   kOne, kNegZero, kHalf, kNegHalf, kQuarter, kNegQuarter, kThreeQuarters, kThreeHalves, kTwo, kNegTwo, kThree,
   kFour, kNegFour, kSix, kTwelve, kThirteenTwelfths, kEpsz, kEps6, k6908, k51001, k67923, k38947, k8209, k104963,
-  k299076, k179098, k231153, kRcp5040, kRcp6, kRcp24, kRcp3, k23, k26,
+  k299076, k179098, k231153, kDiv5040, kDiv5040Lo, kDiv6, kDiv6Lo, kDiv24, kDiv24Lo, kDiv3, kDiv3Lo, k23, k26,
   // Schemes::Hermite's full-stencil indicators
-  k1029270, k2129184, k1099914, k281121, k494958, k1099445, k4317056, k2118166, kRcp6720, k3156862, k13189240,
-  k1710479, k9617754, k531552, k10149306, k26511200, k39700440, k15136011, k1076544, k29195478, kRcp1680,
+  k1029270, k2129184, k1099914, k281121, k494958, k1099445, k4317056, k2118166, kDiv6720, kDiv6720Lo, k3156862, k13189240,
+  k1710479, k9617754, k531552, k10149306, k26511200, k39700440, k15136011, k1076544, k29195478, kDiv1680, kDiv1680Lo,
   kLw0, kLw1, kRcpLw0, kLw1OverLw0,
   kLitCount
 };
 static __device__ double g_lit[kLitCount] = {
     1.0, -0.0, 0.5, -0.5, 0.25, -0.25, 0.75, 1.5, 2.0, -2.0, 3.0,
     4.0, -4.0, 6.0, 12.0, 13.0 / 12.0, 1e-40, 1e-6, 6908.0, 51001.0, 67923.0, 38947.0, 8209.0, 104963.0,
-    299076.0, 179098.0, 231153.0, 1.0 / 5040.0, 1.0 / 6.0, 1.0 / 24.0, 1.0 / 3.0, 23.0, 26.0,
-    1029270.0, 2129184.0, 1099914.0, 281121.0, 494958.0, 1099445.0, 4317056.0, 2118166.0, 1.0 / 6720.0, 3156862.0,
+    299076.0, 179098.0, 231153.0, 1.0 / 5040.0, 0x1.a01a01a01a01ap-73, 1.0 / 6.0, 0x1.5555555555555p-57,
+    1.0 / 24.0, 0x1.5555555555555p-59, 1.0 / 3.0, 0x1.5555555555555p-56, 23.0, 26.0,
+    1029270.0, 2129184.0, 1099914.0, 281121.0, 494958.0, 1099445.0, 4317056.0, 2118166.0, 1.0 / 6720.0,
+    -0x1.fb1fb1fb1fb20p-67, 3156862.0,
     13189240.0, 1710479.0, 9617754.0, 531552.0, 10149306.0, 26511200.0, 39700440.0, 15136011.0, 1076544.0,
-    29195478.0, 1.0 / 1680.0, 1.0 - 2e-5, 1e-5, 1.0 / (1.0 - 2e-5), 1e-5 / (1.0 - 2e-5)};
+    29195478.0, 1.0 / 1680.0, -0x1.fb1fb1fb1fb20p-65, 1.0 - 2e-5, 1e-5, 1.0 / (1.0 - 2e-5), 1e-5 / (1.0 - 2e-5)};
 
 // A double of global memory that is constant while the kernel runs, in a vector register.
 __device__ __forceinline__ double ldk(const double& x) {

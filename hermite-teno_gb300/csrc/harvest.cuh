@@ -32,7 +32,7 @@ __device__ __forceinline__ int label(const double* wd, bool improved) {
   par::lagrange_si(w, SI);
   double tau;
   if (!improved) {
-    const par::fp mean = par::quot(par::scaled(par::kFour, SI[1], SI[0] + SI[2]), par::den_lit(6.0, par::kRcp6));
+    const par::fp mean = par::quot_lit(par::scaled(par::kFour, SI[1], SI[0] + SI[2]), 6.0, par::kDiv6);
     tau = fabs((par::lagrange_b35(w) - mean).v);
   } else {
     tau = par::maxof3(SI);

@@ -92,13 +92,24 @@ __device__ __forceinline__ fp quot(fp a, const Den& d) {
   return divide(a.v, d.b.v);
 }
 
+// a / c correctly rounded for the integers c whose 1/c is in the table as hi + lo (kDivC, kDivCLo: 1/c
+// rounded, and what that leaves, rounded): RN(a hi + RN(a lo)), two operations.  (Multiplication by a
+// constant in two parts, Brisebarre & Muller, IEEE Trans. Computers 57(2), 2008.)  The value that is
+// rounded is off by less than 2^-104 of itself, 2^-51 ulp, while a / c, a quotient by an integer with
+// the odd part d, lies 1/(2d) ulp or more from every midpoint of two doubles (d <= 315 here): no
+// rounding can differ.  Zeros keep their sign; other operands outside quot's range take the division.
+__device__ __forceinline__ fp quot_lit(fp a, double c, Lit hi) {
+  if (mid_range(a.v) || zero_bits(a.v)) return fma(a.v, lit(hi).v, (a * lit(Lit(hi + 1))).v);
+  return divide(a.v, c);
+}
+
 // Schemes::SSPRK::RungeKuttaIII (Schemes_SSPRK.cpp:3-15): hteno::ssprk3's operations
 __device__ __forceinline__ double rk3(fp q0, fp qn, fp rhs, fp dt, int stage) {
   if (stage == 1) return (q0 + dt * rhs).v;
   const fp x = qn + rhs * dt;
   // (the quarter rounds where it is subnormal: not folded into the sum)
   if (stage == 2) return (lit(kThreeQuarters) * q0 + lit(kQuarter) * x).v;
-  return quot(scaled(kTwo, x, q0), den_lit(3.0, kRcp3)).v;
+  return quot_lit(scaled(kTwo, x, q0), 3.0, kDiv3).v;
 }
 // x <= 0, on the integer pipes
 __device__ __forceinline__ bool nonpositive_bits(double x) {
@@ -128,7 +139,7 @@ __device__ __forceinline__ fp lagrange_b35(const fp* v) {
                v[3] * (lit(k104963) * v[3] - lit(k299076) * v[2] + lit(k179098) * v[1] - lit(k38947) * v[0]) +
                v[2] * (lit(k231153) * v[2] - lit(k299076) * v[1] + lit(k67923) * v[0]) +
                v[1] * (lit(k104963) * v[1] - lit(k51001) * v[0]) + lit(k6908) * v[0] * v[0];
-  return quot(r, den_lit(5040.0, kRcp5040));  // r / 5040
+  return quot_lit(r, 5040.0, kDiv5040);
 }
 
 // 1/x to a relative 2^-45 for the cut-off decision only (never for a value that is kept): a
@@ -274,7 +285,7 @@ __device__ __forceinline__ int teno_decide(const fp* v, const fp* SI, bool impro
   double tau;
   if (!improved) {
     const fp b35 = lagrange_b35(v);
-    const fp mean = quot(scaled(kFour, SI[1], SI[0] + SI[2]), den_lit(6.0, kRcp6));  // ... / 6.0
+    const fp mean = quot_lit(scaled(kFour, SI[1], SI[0] + SI[2]), 6.0, kDiv6);
     tau = fabs((b35 - mean).v);
   } else {
     tau = SI[0].v;
@@ -482,7 +493,6 @@ static __device__ __noinline__ void gl3(const DevConst& C, const double* ud, dou
   cg[1] = scaled(kNegTwo, u[2], u[1]) + u[3];
   bg[2] = scaled(kNegFour, u[3], m2) + u[4];
   cg[2] = scaled(kNegTwo, u[3], u[2]) + u[4];
-  const Den d24 = den_lit(24.0, kRcp24);
   const fp n2 = lit(k23) * u[2];
   fp p[3];
   // (taken only when every active lane of the warp can take it: the full arithmetic gives the same
@@ -494,9 +504,9 @@ static __device__ __noinline__ void gl3(const DevConst& C, const double* ud, dou
 #pragma unroll
     for (int k = 0; k < 3; ++k) p[k] = dot3t(C.gp, k, u + k);
     out[0] = dot3w(p, C.gl3flat[0]).v;
-    p[0] = quot(scaled(kTwo, u[1], -u[0]) + n2, d24);
-    p[1] = quot(-u[1] + lit(k26) * u[2] - u[3], d24);
-    p[2] = quot(scaled(kTwo, u[3], n2) - u[4], d24);
+    p[0] = quot_lit(scaled(kTwo, u[1], -u[0]) + n2, 24.0, kDiv24);
+    p[1] = quot_lit(-u[1] + lit(k26) * u[2] - u[3], 24.0, kDiv24);
+    p[2] = quot_lit(scaled(kTwo, u[3], n2) - u[4], 24.0, kDiv24);
     fp c = fp(ldk(C.sumw0p)) * dot3w(p, C.gl3flat[1]);
     c = c - fp(ldk(C.sumw0m)) * dot3w(p, C.gl3flat[2]);
     out[1] = c.v;
@@ -527,9 +537,9 @@ static __device__ __noinline__ void gl3(const DevConst& C, const double* ud, dou
 #pragma unroll
   for (int k = 0; k < 3; ++k) p[k] = dot3t(C.gp, k, u + k);
   out[0] = weighted(C.linwp).v;
-  p[0] = quot(scaled(kTwo, u[1], -u[0]) + n2, d24);
-  p[1] = quot(-u[1] + lit(k26) * u[2] - u[3], d24);
-  p[2] = quot(scaled(kTwo, u[3], n2) - u[4], d24);
+  p[0] = quot_lit(scaled(kTwo, u[1], -u[0]) + n2, 24.0, kDiv24);
+  p[1] = quot_lit(-u[1] + lit(k26) * u[2] - u[3], 24.0, kDiv24);
+  p[2] = quot_lit(scaled(kTwo, u[3], n2) - u[4], 24.0, kDiv24);
   fp c = fp(ldk(C.sumw0p)) * weighted(C.linw0p);
   c = c - fp(ldk(C.sumw0m)) * weighted(C.linw0m);
   out[1] = c.v;
@@ -1001,7 +1011,7 @@ __device__ __forceinline__ fp hermite_brk(const fp* u, const fp* d) {
                (lit(k2129184) * u[1] - lit(k1029270) * u[0] - lit(k1099914) * u[2] + lit(k281121) * d[2]) * d[2] +
                (lit(k1099445) * u[2] - lit(k4317056) * u[1] + lit(k2118166) * u[0]) * u[2] +
                lit(k4317056) * (u[1] - u[0]) * u[1] + lit(k1099445) * u[0] * u[0];
-  return quot(abs_(r), den_lit(6720.0, kRcp6720));
+  return quot_lit(abs_(r), 6720.0, kDiv6720);
 }
 // fullPointsSId (:605-612)
 __device__ __forceinline__ fp hermite_brkd(const fp* u, const fp* d) {
@@ -1011,7 +1021,7 @@ __device__ __forceinline__ fp hermite_brkd(const fp* u, const fp* d) {
                (lit(k1710479) * d[2] - lit(k10149306) * u[2] + lit(k531552) * u[1] + lit(k9617754) * u[0]) * d[2] +
                (lit(k15136011) * u[2] - lit(k1076544) * u[1] - lit(k29195478) * u[0]) * u[2] +
                lit(k1076544) * (u[1] - u[0]) * u[1] + lit(k15136011) * u[0] * u[0];
-  return quot(abs_(r), den_lit(1680.0, kRcp1680));
+  return quot_lit(abs_(r), 1680.0, kDiv1680);
 }
 __device__ __forceinline__ double maxof3(const fp* s) {
   double t = s[0].v;
