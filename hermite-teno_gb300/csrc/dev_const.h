@@ -24,6 +24,11 @@ struct DevConst {
   float f_linwp[3], f_linwm[3], f_linw0p[3], f_linw0m[3], f_sumw0p, f_sumw0m, f_gl3w[3];
   float f_wtab_m[8][3], f_wtab_p[8][3];
   float f_hwtab_m[8][3], f_hwtab_p[8][3], f_hwtab_md[8][3], f_hwtab_pd[8][3];
+  // pairs for the packed float arithmetic of the fused mixed kernels: candidate k's coefficients of
+  // the minus and the plus side, and the GL3 coefficients twice each
+  alignas(8) float x2_cand[3][3][2];  // [k][cell]: crj[cell][1 + k], crj[cell][k]
+  alignas(8) float x2_gp[3][3][2], x2_gm[3][3][2];  // [k][cell]
+  alignas(8) float x2_linwp[3][2], x2_linwm[3][2], x2_linw0p[3][2], x2_linw0m[3][2], x2_sumw0p[2], x2_sumw0m[2];
 };
 
 void fill_dev_const(DevConst* c);  // host side, device_consts.cpp

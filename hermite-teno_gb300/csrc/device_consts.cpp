@@ -136,6 +136,21 @@ void fill_dev_const(DevConst* c) {
   to_float(c->hwtab_p, c->f_hwtab_p);
   to_float(c->hwtab_md, c->f_hwtab_md);
   to_float(c->hwtab_pd, c->f_hwtab_pd);
+  for (int h = 0; h < 2; ++h) {
+    for (int k = 0; k < 3; ++k) {
+      for (int r = 0; r < 3; ++r) {
+        c->x2_cand[k][r][h] = c->f_crj[r][1 + k - h];
+        c->x2_gp[k][r][h] = c->f_gp[r][k];
+        c->x2_gm[k][r][h] = c->f_gm[r][k];
+      }
+      c->x2_linwp[k][h] = c->f_linwp[k];
+      c->x2_linwm[k][h] = c->f_linwm[k];
+      c->x2_linw0p[k][h] = c->f_linw0p[k];
+      c->x2_linw0m[k][h] = c->f_linw0m[k];
+    }
+    c->x2_sumw0p[h] = c->f_sumw0p;
+    c->x2_sumw0m[h] = c->f_sumw0m;
+  }
 }
 
 }  // namespace hteno

@@ -26,6 +26,7 @@
 
 #include <cuda.h>  // CUtensorMap
 
+#include "f32x2.cuh"
 #include "fv2d_common.cuh"
 #include "mixed_conv.cuh"
 #include "tc_ptx.cuh"
@@ -91,30 +92,10 @@ constexpr size_t smem_bytes() {
   return sizeof(Smem<TX, TY>);
 }
 
-// Cut-off pattern of one side of teno5 / teno5i (float).  With all three indicators exactly zero
-// (constant data) the three ratios are equal and the pattern is 7 whatever tau is.
-__device__ __forceinline__ int teno_pat_s(const float* v, bool improved) {
-  float SI0, SI1, SI2;
-  lagrange_si(v, SI0, SI1, SI2);
-  if (SI0 == 0.f && SI1 == 0.f && SI2 == 0.f) return 7;
-  float tau;
-  if (!improved) tau = fabsf(lagrange_b35(v) - (SI0 + SI2 + 4.0f * SI1) * (1.0f / 6.0f));
-  else tau = fmaxf(fmaxf(SI0, SI1), SI2);
-  const float ez = HTENO_F32_EPSZ;
-  const float r0 = fmaf(tau, Cst<float>::rcp(SI0 + ez), 1.0f);
-  const float r1 = fmaf(tau, Cst<float>::rcp(SI1 + ez), 1.0f);
-  const float r2 = fmaf(tau, Cst<float>::rcp(SI2 + ez), 1.0f);
-  return teno_pattern(r0, r1, r2, float(HTENO_LAG_CT));
-}
-
 // A side's 5-cell window of equal float values, counted by the audit (the classifier hands such
 // stencils to nobody).
 __device__ __forceinline__ bool flat5(const float* v) {
   return v[1] == v[0] && v[2] == v[0] && v[3] == v[0] && v[4] == v[0];
-}
-
-__device__ __forceinline__ float weighted(float p0, float p1, float p2, const float* w) {
-  return catchnan(dot3m(p0, w[0], p1, w[1], p2, w[2]));
 }
 
 // Audit counters of the learned router: stencils seen, routed to the linear weights, routed
@@ -124,82 +105,266 @@ struct RouteCount {
   int seen = 0, routed = 0, misrouted = 0, smooth = 0, flat = 0;
 };
 
-// One side of teno5 (Schemes_Lagrange.cpp:481-511), teno5i (:1235-1263), linear (:1219-1233) or
-// an alternative, u[0..5] -> u^-_{i+1/2} (side 0) or u^+_{i+1/2} (side 1).  With the route bit
-// set (learned routing, TENO kinds) the side takes the linear weights without evaluating the
-// indicators; when auditing, the plain cut-off is evaluated as well and counted.  The weight
-// tables live in shared memory: a per-thread pattern would serialise constant-memory reads.
-struct SideOut {
-  float v;
-  int pat;  // the TENO cut-off pattern evaluated (7 when not evaluated)
+// A constant pair of DevConst.
+__device__ __forceinline__ f2 cpair(const float (&p)[2]) { return pack(p[0], p[1]); }
+
+// Both sides of teno5 (Schemes_Lagrange.cpp:481-511) or teno5i (:1235-1263) at once: the low half of
+// every pair is u^-_{i+1/2} from cells 0..4 of the stencil, the high half u^+_{i+1/2} from cells 1..5,
+// the same expressions on both.  P0, P1, P2: cells (0, 1), (2, 3), (4, 5).  Where a route bit is set
+// (learned routing; bit 0 minus, bit 1 plus) the side takes the linear weights; the indicators are not
+// evaluated when both are, unless the stage is audited.  The weight tables live in shared memory: a
+// per-thread pattern would serialise constant-memory reads.
+struct Sides {
+  float m, p;
+  int pat_m, pat_p;  // the TENO cut-off patterns evaluated (7 when not evaluated)
 };
-// Not inlined (8 calls per face in phases B and D); the stencil comes by value so it stays in
+// Cut-off pattern from the three normalised sixth powers' comparison with the limit; NaN anywhere makes
+// every comparison false -> all candidates kept, as in the reference.
+__device__ __forceinline__ int pattern_of(float a0, float a1, float a2, float lim) {
+  return (a0 < lim ? 0 : 1) | (a1 < lim ? 0 : 2) | (a2 < lim ? 0 : 4);
+}
+// Not inlined (4 calls per face in phases B and D); the stencil comes by value so it stays in
 // registers.  The caller counts the audit.
-static __device__ __noinline__ SideOut side_value(const DevConst& C, int kind,
-                                                  const float (*tab)[8][3], float u0, float u1,
-                                                  float u2, float u3, float u4, float u5, int side,
-                                                  bool routed, bool audit) {
-  float p0, p1, p2;
-  if (side == 0) {
-    p0 = dot3m(C.f_crj[0][1], u2, C.f_crj[1][1], u3, C.f_crj[2][1], u4);
-    p1 = dot3m(C.f_crj[0][2], u1, C.f_crj[1][2], u2, C.f_crj[2][2], u3);
-    p2 = dot3m(C.f_crj[0][3], u0, C.f_crj[1][3], u1, C.f_crj[2][3], u2);
-  } else {
-    p0 = dot3m(C.f_crj[0][0], u3, C.f_crj[1][0], u4, C.f_crj[2][0], u5);
-    p1 = dot3m(C.f_crj[0][1], u2, C.f_crj[1][1], u3, C.f_crj[2][1], u4);
-    p2 = dot3m(C.f_crj[0][2], u1, C.f_crj[1][2], u2, C.f_crj[2][2], u3);
+static __device__ __noinline__ Sides teno_sides(const DevConst& C, bool improved, const float (*tab)[8][3], f2 P0,
+                                                f2 P1, f2 P2, int routed, bool audit) {
+  const f2 v0 = P0, v1 = pack(hi(P0), lo(P1)), v2 = P1, v3 = pack(hi(P1), lo(P2)), v4 = P2;
+  Sides o;
+  o.pat_m = o.pat_p = 7;
+  if (routed != 3 || audit) {
+    const f2 m2 = dup(-2.0f), m4 = dup(-4.0f), half = dup(0.5f), c13 = dup(float(HTENO_C1));
+    const f2 c0 = mad(m2, v3, v2) + v4;
+    const f2 b0 = (mad(m4, v3, dup(3.0f) * v2) + v4) * half;
+    const f2 c1 = mad(m2, v2, v1) + v3;
+    const f2 b1 = (v1 - v3) * half;
+    const f2 c2 = mad(m2, v1, v0) + v2;
+    const f2 b2 = mad(dup(3.0f), v2, mad(m4, v1, v0)) * half;
+    const f2 S0 = mad(c13 * c0, c0, b0 * b0);
+    const f2 S1 = mad(c13 * c1, c1, b1 * b1);
+    const f2 S2 = mad(c13 * c2, c2, b2 * b2);
+    // all indicators exactly zero (constant data): three equal ratios, pattern 7 whatever tau is (they
+    // are sums of squares: zero as bits)
+    if ((S0.b | S1.b | S2.b) != 0ull) {
+      f2 tau;
+      if (!improved) {
+        const f2 a4 = mad(dup(8209.0f), v0, mad(dup(-38947.0f), v1, mad(dup(67923.0f), v2,
+                          mad(dup(-51001.0f), v3, dup(6908.0f) * v4))));
+        const f2 a3 = mad(dup(-38947.0f), v0, mad(dup(179098.0f), v1, mad(dup(-299076.0f), v2, dup(104963.0f) * v3)));
+        const f2 a2 = mad(dup(67923.0f), v0, mad(dup(-299076.0f), v1, dup(231153.0f) * v2));
+        const f2 a1 = mad(dup(-51001.0f), v0, dup(104963.0f) * v1);
+        const f2 r = mad(dup(6908.0f) * v0, v0, mad(v1, a1, mad(v2, a2, mad(v3, a3, v4 * a4))));
+        const f2 mean = mad(dup(4.0f), S1, S0 + S2) * dup(1.0f / 6.0f);  // (4 S1 is exact)
+        tau = abs_(r * dup(1.0f / 5040.0f) - mean);
+      } else {
+        tau = pack(fmaxf(fmaxf(lo(S0), lo(S1)), lo(S2)), fmaxf(fmaxf(hi(S0), hi(S1)), hi(S2)));
+      }
+      const f2 ez = dup(HTENO_F32_EPSZ), one = dup(1.0f);
+      auto rcp2 = [](f2 x) { return pack(Cst<float>::rcp(lo(x)), Cst<float>::rcp(hi(x))); };
+      const f2 r0 = mad(tau, rcp2(S0 + ez), one), r1 = mad(tau, rcp2(S1 + ez), one), r2 = mad(tau, rcp2(S2 + ez), one);
+      // normalised by the largest ratio so that the sixth power cannot overflow
+      const f2 inv = pack(Cst<float>::rcp(fmaxf(fmaxf(lo(r0), lo(r1)), lo(r2))),
+                          Cst<float>::rcp(fmaxf(fmaxf(hi(r0), hi(r1)), hi(r2))));
+      auto sixth = [](f2 x) {
+        const f2 s = x * x;
+        return s * s * s;
+      };
+      const f2 e0 = sixth(r0 * inv), e1 = sixth(r1 * inv), e2 = sixth(r2 * inv);
+      const f2 lim = dup(float(HTENO_LAG_CT)) * ((e0 + e1) + e2);
+      o.pat_m = pattern_of(lo(e0), lo(e1), lo(e2), lo(lim));
+      o.pat_p = pattern_of(hi(e0), hi(e1), hi(e2), hi(lim));
+    }
   }
-  const float v[5] = {side ? u1 : u0, side ? u2 : u1, side ? u3 : u2, side ? u4 : u3, side ? u5 : u4};
-  if (kind == 2) return {dot3m(p0, tab[side][7][0], p1, tab[side][7][1], p2, tab[side][7][2]), 7};
-  if (kind >= 3) return {alt_side(kind, p0, p1, p2, v, tab[side], tab[side][7]), 7};
-  int pat = 7;
-  if (!routed || audit) pat = teno_pat_s(v, kind == 1);
-  return {weighted(p0, p1, p2, tab[side][routed ? 7 : pat]), pat};
+  const float* wm = tab[0][routed & 1 ? 7 : o.pat_m];
+  const float* wp = tab[1][routed & 2 ? 7 : o.pat_p];
+  const f2 p0 = dot3m(cpair(C.x2_cand[0][0]), v2, cpair(C.x2_cand[0][1]), v3, cpair(C.x2_cand[0][2]), v4);
+  const f2 p1 = dot3m(cpair(C.x2_cand[1][0]), v1, cpair(C.x2_cand[1][1]), v2, cpair(C.x2_cand[1][2]), v3);
+  const f2 p2 = dot3m(cpair(C.x2_cand[2][0]), v0, cpair(C.x2_cand[2][1]), v1, cpair(C.x2_cand[2][2]), v2);
+  const f2 s = dot3m(p0, pack(wm[0], wp[0]), p1, pack(wm[1], wp[1]), p2, pack(wm[2], wp[2]));
+  o.m = catchnan(lo(s));
+  o.p = catchnan(hi(s));
+  return o;
 }
 
-// One side of teno5 / teno5i / linear / an alternative for the stencil u[0..5], with the audit
-// of the learned router counted here (TENO kinds).
-__device__ __forceinline__ float side_counted(const DevConst& C, int kind, const float (*tab)[8][3],
-                                              const float* u, int side, bool routed, bool audit,
-                                              RouteCount& rc) {
-  const SideOut o = side_value(C, kind, tab, u[0], u[1], u[2], u[3], u[4], u[5], side, routed, audit);
-  if (audit && kind <= 1) {
-    rc.seen += 1;
-    rc.smooth += o.pat == 7;
-    rc.flat += flat5(u + side);
-    rc.routed += routed;
-    rc.misrouted += routed && o.pat != 7;
-  }
-  return o.v;
+// Both sides by the linear weights (kind 2, Schemes_Lagrange.cpp:1219-1233) or an alternative (kind
+// >= 3) for the stencil u0..u5.
+static __device__ __noinline__ Sides other_sides(const DevConst& C, int kind, const float (*tab)[8][3], float u0,
+                                                 float u1, float u2, float u3, float u4, float u5) {
+  auto one = [&](int side, float v0, float v1, float v2, float v3, float v4) {
+    const int k = 1 - side;
+    const float p0 = hteno::dot3m(C.f_crj[0][k], v2, C.f_crj[1][k], v3, C.f_crj[2][k], v4);
+    const float p1 = hteno::dot3m(C.f_crj[0][k + 1], v1, C.f_crj[1][k + 1], v2, C.f_crj[2][k + 1], v3);
+    const float p2 = hteno::dot3m(C.f_crj[0][k + 2], v0, C.f_crj[1][k + 2], v1, C.f_crj[2][k + 2], v2);
+    if (kind == 2) return hteno::dot3m(p0, tab[side][7][0], p1, tab[side][7][1], p2, tab[side][7][2]);
+    const float v[5] = {v0, v1, v2, v3, v4};
+    return alt_side(kind, p0, p1, p2, v, tab[side], tab[side][7]);
+  };
+  return {one(0, u0, u1, u2, u3, u4), one(1, u1, u2, u3, u4, u5), 7, 7};
 }
 
-// GL3 of one face array, not inlined: phases C and E call it 8 times per face each, and inlined
-// copies crowd the instruction cache.
+// Both sides of one field for the stencil P0, P1, P2 (cell pairs), with the audit of the learned
+// router counted here (TENO kinds).
+__device__ __forceinline__ Sides sides_counted(const DevConst& C, int kind, const float (*tab)[8][3], f2 P0, f2 P1,
+                                               f2 P2, int routed, bool audit, RouteCount& rc) {
+  if (kind > 1) return other_sides(C, kind, tab, lo(P0), hi(P0), lo(P1), hi(P1), lo(P2), hi(P2));
+  const Sides o = teno_sides(C, kind == 1, tab, P0, P1, P2, routed, audit);
+  if (audit) {
+    const float u[6] = {lo(P0), hi(P0), lo(P1), hi(P1), lo(P2), hi(P2)};
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const int pat = side ? o.pat_p : o.pat_m, r = routed >> side & 1;
+      rc.seen += 1;
+      rc.smooth += pat == 7;
+      rc.flat += flat5(u + side);
+      rc.routed += r;
+      rc.misrouted += r && pat != 7;
+    }
+  }
+  return o;
+}
+
+// GL3 (weno5JS3PointsQuadrature, as gl3() of device_math.cuh) of the left (low half) and right (high
+// half) face values of one field at once, not inlined: phases C and E call it 4 times per face each,
+// and inlined copies crowd the instruction cache.
 struct Gl3f {
-  float a, b, c;
+  f2 a, b, c;
 };
-static __device__ __noinline__ Gl3f gl3_f(const DevConst& C, const float* u) {
-  Gl3f g;
-  gl3(C, u, g.a, g.b, g.c);
-  return g;
+static __device__ __noinline__ Gl3f gl3_f(const DevConst& C, f2 u0, f2 u1, f2 u2, f2 u3, f2 u4) {
+  auto rcp2 = [](f2 x) { return pack(Cst<float>::rcp(lo(x)), Cst<float>::rcp(hi(x))); };
+  auto nan2 = [](f2 x) { return pack(catchnan(lo(x)), catchnan(hi(x))); };
+  const f2 m2 = dup(-2.0f), m4 = dup(-4.0f), c13 = dup(float(HTENO_C1)), q4 = dup(0.25f), eps = dup(float(HTENO_LAG_EPS));
+  const f2 bg0 = mad(dup(3.0f), u2, mad(m4, u1, u0));
+  const f2 cg0 = mad(m2, u1, u0) + u2;
+  const f2 bg1 = u1 - u3;
+  const f2 cg1 = mad(m2, u2, u1) + u3;
+  const f2 bg2 = mad(m4, u3, dup(3.0f) * u2) + u4;
+  const f2 cg2 = mad(m2, u3, u2) + u4;
+  f2 s0 = eps + mad(c13 * cg0, cg0, q4 * bg0 * bg0);
+  f2 s1 = eps + mad(c13 * cg1, cg1, q4 * bg1 * bg1);
+  f2 s2 = eps + mad(c13 * cg2, cg2, q4 * bg2 * bg2);
+  s0 = s0 * s0;
+  s1 = s1 * s1;
+  s2 = s2 * s2;
+  // alpha_k = 1 / s_k, scaled by the smallest s to keep float in range
+  const f2 smin = pack(fminf(fminf(lo(s0), lo(s1)), lo(s2)), fminf(fminf(hi(s0), hi(s1)), hi(s2)));
+  const f2 a0 = smin * rcp2(s0), a1 = smin * rcp2(s1), a2 = smin * rcp2(s2);
+  auto mix = [&](const float (&lw)[3][2], f2 q0, f2 q1, f2 q2) {
+    const f2 g0 = cpair(lw[0]) * a0, g1 = cpair(lw[1]) * a1, g2 = cpair(lw[2]) * a2;
+    return dot3m(q0, g0, q1, g1, q2, g2) * rcp2(g0 + g1 + g2);
+  };
+  auto cand = [&](const float (&g)[3][3][2], const float (&lw)[3][2]) {
+    const f2 q0 = dot3m(cpair(g[0][0]), u0, cpair(g[0][1]), u1, cpair(g[0][2]), u2);
+    const f2 q1 = dot3m(cpair(g[1][0]), u1, cpair(g[1][1]), u2, cpair(g[1][2]), u3);
+    const f2 q2 = dot3m(cpair(g[2][0]), u2, cpair(g[2][1]), u3, cpair(g[2][2]), u4);
+    return mix(lw, q0, q1, q2);
+  };
+  Gl3f o;
+  o.a = nan2(cand(C.x2_gp, C.x2_linwp));
+  const f2 r24 = dup(1.0f / 24.0f), two = dup(2.0f), t23 = dup(23.0f);
+  const f2 q0 = mad(t23, u2, mad(two, u1, -u0)) * r24;
+  const f2 q1 = (mad(dup(26.0f), u2, -u1) - u3) * r24;
+  const f2 q2 = (mad(two, u3, t23 * u2) - u4) * r24;
+  const f2 c = cpair(C.x2_sumw0p) * mix(C.x2_linw0p, q0, q1, q2);
+  o.b = nan2(c - cpair(C.x2_sumw0m) * mix(C.x2_linw0m, q0, q1, q2));
+  o.c = nan2(cand(C.x2_gm, C.x2_linwm));
+  return o;
 }
 
-// The flux at one Gauss point of a face: R back-projection of both sides' characteristic values,
-// then HLLC or Rusanov.  Not inlined (3 calls per face in each of phases C and E).
+// Roe projection L q of two cells at once (roe_left of device_math.cuh): q[v] the cells' pair of
+// conserved variable v, c[r] their pair of characteristic field r.
+struct LeftRows {
+  f2 t2, tvt, n0, d0, nvt, nb1, bvt, s1, d2, n3, d3;
+};
+__device__ __forceinline__ LeftRows left_rows(const Roe2<float>& s, int dir) {
+  const float vn = dir == 1 ? s.vxm : s.vym, vt = dir == 1 ? s.vym : s.vxm;
+  const float b2 = s.qm * s.b1, s0 = vn * s.rcm, s1 = s.b1 * vn, t2 = 0.5f * s.b1;
+  LeftRows L;
+  L.t2 = dup(t2);
+  L.tvt = dup(-t2 * vt);
+  L.n0 = dup(-0.5f * (s1 + s.rcm));
+  L.d0 = dup(0.5f * (b2 + s0));
+  L.nvt = dup(-vt);
+  L.nb1 = dup(-s.b1);
+  L.bvt = dup(s.b1 * vt);
+  L.s1 = dup(s1);
+  L.d2 = dup(1.0f - b2);
+  L.n3 = dup(-0.5f * (s1 - s.rcm));
+  L.d3 = dup(0.5f * (b2 - s0));
+  return L;
+}
+__device__ __forceinline__ void project2(const LeftRows& L, int dir, const f2* q, f2* c) {
+  const f2 qn = dir == 1 ? q[1] : q[2], qt = dir == 1 ? q[2] : q[1];
+  c[0] = mad(L.t2, q[3], mad(L.tvt, qt, mad(L.n0, qn, L.d0 * q[0])));
+  c[1] = mad(L.nvt, q[0], qt);
+  c[2] = mad(L.nb1, q[3], mad(L.bvt, qt, mad(L.s1, qn, L.d2 * q[0])));
+  c[3] = mad(L.t2, q[3], mad(L.tvt, qt, mad(L.n3, qn, L.d3 * q[0])));
+}
+
+// The flux at one Gauss point of a face: R back-projection of both sides' characteristic values (pairs
+// left, right), then HLLC (hllc2 of device_math.cuh with the two sides' part packed) or Rusanov.  Not
+// inlined (3 calls per face in each of phases C and E).
 struct F4 {
   float v[4];
 };
 template <int DIR>
-static __device__ __noinline__ F4 gauss_flux(Roe2<float> R, int flux, float g1, float gamma, float l0,
-                                             float l1, float l2, float l3, float r0, float r1,
-                                             float r2, float r3) {
-  const float cl[4] = {l0, l1, l2, l3}, cr[4] = {r0, r1, r2, r3};
-  float ql[4], qr[4];
+static __device__ __noinline__ F4 gauss_flux(Roe2<float> s, int flux, float g1, float gamma, f2 c0, f2 c1, f2 c2,
+                                             f2 c3) {
   F4 F;
-  roe_right(R, DIR, cl, ql);
-  roe_right(R, DIR, cr, qr);
-  if (flux == HTENO_FLUX_HLLC) hllc2(g1, DIR, ql, qr, F.v);
-  else rusanov2(gamma, g1, DIR, R, ql, qr, F.v);
+  const float vn = DIR == 1 ? s.vxm : s.vym, vt = DIR == 1 ? s.vym : s.vxm, t0 = vn * s.cm;
+  f2 q[4];  // (roe_right)
+  q[0] = c0 + c2 + c3;
+  const f2 qn = mad(dup(vn + s.cm), c3, mad(dup(vn), c2, dup(vn - s.cm) * c0));
+  const f2 qt = mad(dup(vt), c3, mad(dup(vt), c2, mad(dup(vt), c0, c1)));
+  q[DIR == 1 ? 1 : 2] = qn;
+  q[DIR == 1 ? 2 : 1] = qt;
+  q[3] = mad(dup(s.hm + t0), c3, mad(dup(s.qm), c2, mad(dup(vt), c1, dup(s.hm - t0) * c0)));
+  if (flux != HTENO_FLUX_HLLC) {
+    const float ql[4] = {lo(q[0]), lo(q[1]), lo(q[2]), lo(q[3])}, qr[4] = {hi(q[0]), hi(q[1]), hi(q[2]), hi(q[3])};
+    rusanov2(gamma, g1, DIR, s, ql, qr, F.v);
+    return F;
+  }
+  const f2 i2 = pack(Cst<float>::rcp(lo(q[0])), Cst<float>::rcp(hi(q[0])));
+  const f2 w1 = q[1] * i2, w2 = q[2] * i2;
+  const f2 p = (q[3] - dup(0.5f) * mad(q[2], w2, q[1] * w1)) * dup(g1);
+  const f2 h = (q[3] + p) * i2, cc = p * i2;
+  const float cl = Cst<float>::sqrt_(fabsf(lo(cc))), cr = Cst<float>::sqrt_(fabsf(hi(cc)));
+  const float rr = Cst<float>::sqrt_(fabsf(hi(q[0]) * lo(i2)));
+  const float rrr = Cst<float>::rcp(1.0f + rr);
+  const float vm0 = hteno::mad(hi(w1), rr, lo(w1)) * rrr;
+  const float vm1 = hteno::mad(hi(w2), rr, lo(w2)) * rrr;
+  const float qm = 0.5f * hteno::mad(vm1, vm1, vm0 * vm0);
+  const float hm = hteno::mad(hi(h), rr, lo(h)) * rrr;
+  const float cm = Cst<float>::sqrt_(fabsf(g1 * (hm - qm)));
+  const float vmd = DIR == 1 ? vm0 : vm1;
+  const f2 wn = DIR == 1 ? w1 : w2, mn = q[DIR];
+  const float ul = lo(wn), ur = hi(wn);
+  const float sl = fminf(ul - cl, vmd - cm);
+  const float sr = fmaxf(ur + cr, vmd + cm);
+  const float sm = (hteno::mad(-lo(mn), sl - ul, hi(mn) * (sr - ur)) + lo(p) - hi(p)) *
+                   Cst<float>::rcp(hteno::mad(-lo(q[0]), sl - ul, hi(q[0]) * (sr - ur)));
+  const float ps = hteno::mad(lo(q[0]) * (ul - sl), ul - sm, lo(p));
+  // the reference's four regions (:408-427), the operands of the left or right ones selected first
+  const bool outer_l = sl > 0.0f;
+  const bool star_l = !outer_l && sl <= 0.0f && sm > 0.0f;
+  const bool star_r = !outer_l && !star_l && sm <= 0.0f && sr >= 0.0f;
+  const bool use_l = outer_l || star_l;
+  float u[4], w[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) u[k] = use_l ? lo(q[k]) : hi(q[k]);
+  w[0] = u[0];
+  w[1] = use_l ? lo(w1) : hi(w1);
+  w[2] = use_l ? lo(w2) : hi(w2);
+  w[3] = use_l ? lo(p) : hi(p);
+  flux2(DIR, u, w, F.v);
+  if (star_l || star_r) {
+    const float sk = use_l ? sl : sr, un = use_l ? ul : ur;
+    const float nom = sk - un, iden = Cst<float>::rcp(sk - sm);
+    float qs[4];
+    qs[0] = w[0] * nom * iden;
+    qs[1] = DIR == 1 ? (hteno::mad(nom, u[1], ps) - w[3]) * iden : nom * u[1] * iden;
+    qs[2] = DIR == 2 ? (hteno::mad(nom, u[2], ps) - w[3]) * iden : nom * u[2] * iden;
+    qs[3] = hteno::mad(ps, sm, hteno::mad(-lo(p), un, nom * u[3])) * iden;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) F.v[k] = hteno::mad(sk, qs[k] - u[k], F.v[k]);
+  }
   return F;
 }
 
@@ -371,14 +536,16 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     const Roe2<float> R = roe2<float>(g1, S.p[3][y][xa], S.p[0][y][xa], S.p[1][y][xa],
                                       S.p[2][y][xa], S.p[3][y][xb], S.p[0][y][xb],
                                       S.p[1][y][xb], S.p[2][y][xb]);
-    float ch[4][6];
+    f2 ch[4][3];  // field r's cells (0, 1), (2, 3), (4, 5)
+    const LeftRows L = left_rows(R, 1);
 #pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const float qq[4] = {S.q[0][y][f + m], S.q[1][y][f + m], S.q[2][y][f + m], S.q[3][y][f + m]};
-      float cc[4];
-      roe_left(R, 1, qq, cc);
+    for (int m = 0; m < 3; ++m) {
+      f2 qq[4], cc2[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) ch[r][m] = cc[r];
+      for (int v = 0; v < 4; ++v) qq[v] = pack(S.q[v][y][f + 2 * m], S.q[v][y][f + 2 * m + 1]);
+      project2(L, 1, qq, cc2);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) ch[r][m] = cc2[r];
     }
     int route = 0;
     bool own = false;
@@ -390,8 +557,9 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      S.c[r][it] = side_counted(C, G.recon, S.wtab, ch[r], 0, (route >> (2 * r)) & 1, own, rc);
-      S.c[4 + r][it] = side_counted(C, G.recon, S.wtab, ch[r], 1, (route >> (2 * r + 1)) & 1, own, rc);
+      const Sides o = sides_counted(C, G.recon, S.wtab, ch[r][0], ch[r][1], ch[r][2], (route >> (2 * r)) & 3, own, rc);
+      S.c[r][it] = o.m;
+      S.c[4 + r][it] = o.p;
     }
   }
   __syncthreads();
@@ -399,16 +567,13 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
   // C: x faces, transverse quadrature and flux
   for (int it = tid; it < Sh::XF * TY; it += NT) {
     const int r = it / Sh::XF, f = it - r * Sh::XF;
-    float g[8][3];
+    Gl3f g[4];  // (left, right) of field k at the three Gauss points
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float u5[5];
+    for (int k = 0; k < 4; ++k) {
+      f2 u5[5];
 #pragma unroll
-      for (int m = 0; m < 5; ++m) u5[m] = S.c[k][(r + m) * Sh::XF + f];
-      const Gl3f o = gl3_f(C, u5);
-      g[k][0] = o.a;
-      g[k][1] = o.b;
-      g[k][2] = o.c;
+      for (int m = 0; m < 5; ++m) u5[m] = pack(S.c[k][(r + m) * Sh::XF + f], S.c[4 + k][(r + m) * Sh::XF + f]);
+      g[k] = gl3_f(C, u5[0], u5[1], u5[2], u5[3], u5[4]);
     }
     const int y = r + 3, xa = f + 2, xb = f + 3;
     const Roe2<float> R = roe2<float>(g1, S.p[3][y][xa], S.p[0][y][xa], S.p[1][y][xa],
@@ -417,8 +582,9 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     float acc[4];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      const F4 Fm = gauss_flux<1>(R, G.flux, g1, float(G.gamma), g[0][m], g[1][m], g[2][m], g[3][m],
-                                   g[4][m], g[5][m], g[6][m], g[7][m]);
+      const F4 Fm = m == 0 ? gauss_flux<1>(R, G.flux, g1, float(G.gamma), g[0].a, g[1].a, g[2].a, g[3].a)
+                    : m == 1 ? gauss_flux<1>(R, G.flux, g1, float(G.gamma), g[0].b, g[1].b, g[2].b, g[3].b)
+                             : gauss_flux<1>(R, G.flux, g1, float(G.gamma), g[0].c, g[1].c, g[2].c, g[3].c);
       const float wm = C.f_gl3w[m];
 #pragma unroll
       for (int v = 0; v < 4; ++v) acc[v] = m == 0 ? wm * Fm.v[v] : fmaf(wm, Fm.v[v], acc[v]);
@@ -436,15 +602,16 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     const Roe2<float> R = roe2<float>(g1, S.p[3][ya][x], S.p[0][ya][x], S.p[1][ya][x],
                                       S.p[2][ya][x], S.p[3][yb][x], S.p[0][yb][x],
                                       S.p[1][yb][x], S.p[2][yb][x]);
-    float ch[4][6];
+    f2 ch[4][3];  // field r's cells (0, 1), (2, 3), (4, 5)
+    const LeftRows L = left_rows(R, 2);
 #pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const float qq[4] = {S.q[0][gg + m][x], S.q[1][gg + m][x], S.q[2][gg + m][x],
-                           S.q[3][gg + m][x]};
-      float cv[4];
-      roe_left(R, 2, qq, cv);
+    for (int m = 0; m < 3; ++m) {
+      f2 qq[4], cc2[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) ch[r][m] = cv[r];
+      for (int v = 0; v < 4; ++v) qq[v] = pack(S.q[v][gg + 2 * m][x], S.q[v][gg + 2 * m + 1][x]);
+      project2(L, 2, qq, cc2);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) ch[r][m] = cc2[r];
     }
     int route = 0;
     bool own = false;
@@ -456,8 +623,9 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      S.c[r][it] = side_counted(C, G.recon, S.wtab, ch[r], 0, (route >> (2 * r)) & 1, own, rc);
-      S.c[4 + r][it] = side_counted(C, G.recon, S.wtab, ch[r], 1, (route >> (2 * r + 1)) & 1, own, rc);
+      const Sides o = sides_counted(C, G.recon, S.wtab, ch[r][0], ch[r][1], ch[r][2], (route >> (2 * r)) & 3, own, rc);
+      S.c[r][it] = o.m;
+      S.c[4 + r][it] = o.p;
     }
   }
   __syncthreads();
@@ -465,16 +633,13 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
   // E: y faces, transverse quadrature and flux
   for (int it = tid; it < Sh::YF * TX; it += NT) {
     const int gg = it / TX, col = it - gg * TX;
-    float g[8][3];
+    Gl3f g[4];  // (left, right) of field k at the three Gauss points
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float u5[5];
+    for (int k = 0; k < 4; ++k) {
+      f2 u5[5];
 #pragma unroll
-      for (int m = 0; m < 5; ++m) u5[m] = S.c[k][gg * Sh::YC + col + m];
-      const Gl3f o = gl3_f(C, u5);
-      g[k][0] = o.a;
-      g[k][1] = o.b;
-      g[k][2] = o.c;
+      for (int m = 0; m < 5; ++m) u5[m] = pack(S.c[k][gg * Sh::YC + col + m], S.c[4 + k][gg * Sh::YC + col + m]);
+      g[k] = gl3_f(C, u5[0], u5[1], u5[2], u5[3], u5[4]);
     }
     const int x = col + 3, ya = gg + 2, yb = gg + 3;
     const Roe2<float> R = roe2<float>(g1, S.p[3][ya][x], S.p[0][ya][x], S.p[1][ya][x],
@@ -483,8 +648,9 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     float acc[4];
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
-      const F4 Fm = gauss_flux<2>(R, G.flux, g1, float(G.gamma), g[0][m], g[1][m], g[2][m], g[3][m],
-                                   g[4][m], g[5][m], g[6][m], g[7][m]);
+      const F4 Fm = m == 0 ? gauss_flux<2>(R, G.flux, g1, float(G.gamma), g[0].a, g[1].a, g[2].a, g[3].a)
+                    : m == 1 ? gauss_flux<2>(R, G.flux, g1, float(G.gamma), g[0].b, g[1].b, g[2].b, g[3].b)
+                             : gauss_flux<2>(R, G.flux, g1, float(G.gamma), g[0].c, g[1].c, g[2].c, g[3].c);
       const float wm = C.f_gl3w[m];
 #pragma unroll
       for (int v = 0; v < 4; ++v) acc[v] = m == 0 ? wm * Fm.v[v] : fmaf(wm, Fm.v[v], acc[v]);
