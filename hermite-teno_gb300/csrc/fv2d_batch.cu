@@ -354,6 +354,9 @@ int hteno_batch_create(const hteno_config* cfgs, int n, hteno_batch** out) {
     I.G.dx = (c.xr - c.xl) / c.nx;
     I.G.dy = (c.yt - c.yb) / c.ny;
     I.G.area = I.G.dx * I.G.dy;
+    I.G.rdx = 1.0 / I.G.dx;
+    I.G.rdy = 1.0 / I.G.dy;
+    I.G.rarea = 1.0 / I.G.area;
     I.G.gamma = c.gamma;
     I.G.g1 = c.gamma - 1.0;
     I.G.x0 = c.xl;

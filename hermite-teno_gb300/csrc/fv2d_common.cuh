@@ -8,7 +8,8 @@ namespace hteno {
 
 struct Geo {
   int nx, ny, bc, recon, flux;
-  double dx, dy, area, rarea, gamma, g1;  // rarea = 1 / area
+  double dx, dy, area, gamma, g1;
+  double rdx, rdy, rarea;  // 1 / dx, 1 / dy, 1 / area
   // boundaries whose ghosts are not copies of interior cells (HTENO_BC_TAYLOR, _DOUBLE_MACH)
   double x0, y0;        // xl, yb: cell centres
   double t0;            // time of a residual evaluation (the stepping kernels read the step state)
@@ -139,6 +140,8 @@ inline Geo geo_of(const hteno_solver* s) {
   G.dx = s->dx;
   G.dy = s->dy;
   G.area = s->dx * s->dy;
+  G.rdx = 1.0 / G.dx;
+  G.rdy = 1.0 / G.dy;
   G.rarea = 1.0 / G.area;
   G.gamma = s->cfg.gamma;
   G.g1 = s->cfg.gamma - 1.0;

@@ -1186,6 +1186,8 @@ extern "C" int hteno_residual_noalloc(const hteno_config* cfg, const double* q, 
   G.dx = (c.xr - c.xl) / c.nx;
   G.dy = (c.yt - c.yb) / c.ny;
   G.area = G.dx * G.dy;
+  G.rdx = 1.0 / G.dx;
+  G.rdy = 1.0 / G.dy;
   G.rarea = 1.0 / G.area;
   G.gamma = c.gamma;
   G.g1 = c.gamma - 1.0;
