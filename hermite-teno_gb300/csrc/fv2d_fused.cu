@@ -32,11 +32,10 @@ __global__ void __launch_bounds__(NT, MINB) k_fused(Geo G, int stage, fused::Sta
   // an audited step that runs (not past the stop time) counts once
   if (stage == 1 && a.audit && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
     atomicAdd(a.audit + 6, 1ull);
-  uint32_t phase = 0;
   if (a.tmap) fused::tma_setup(S);
   int bad = 0;
   const double ms = fused::tile_stage<TX, TY, NT>(c_dev, G, blockIdx.x * TX, blockIdx.y * TY,
-                                                  stage, a, S, bad, phase);
+                                                  stage, a, S, bad);
   if (stage == 3) {
     block_max_to(ms, &a.st->maxbits);
     if (bad) atomicOr(&a.st->status, bad);

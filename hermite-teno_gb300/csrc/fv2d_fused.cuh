@@ -397,8 +397,8 @@ __device__ __forceinline__ bool tame_state(float r, float mx, float my, float e,
   return r >= lo && r <= hi && p >= lo && p <= hi && u * u + v * v <= 64.0f * (gamma * p * ir);
 }
 
-// The block's TMA mbarrier (S.bar), initialised once per launch before its first tile when a
-// tensor map may be used; tma_phase then tracks the parity of the block's next box copy.
+// The block's TMA mbarrier (S.bar), initialised once per launch before its tile when a
+// tensor map may be used.
 template <int TX, int TY>
 __device__ __forceinline__ void tma_setup(Smem<TX, TY>& S) {
   if (threadIdx.x == 0) {
@@ -411,12 +411,11 @@ __device__ __forceinline__ void tma_setup(Smem<TX, TY>& S) {
 // The tile at (i0, j0) of grid G.  Every thread of the block must call it (barriers inside).
 // Returns this thread's max wave speed over the cells it updated (stage 3) and ORs health flags
 // into *bad (bit 2: the tile's TMA copy did not complete within the bounded wait; the tile is
-// left unwritten and the caller must stop using the block's shared memory for box copies).
-// tma_phase: parity of the block's next TMA box copy (tma_setup ran), flipped by each copy.
+// left unwritten).  One tile a block: the box copy's mbarrier (tma_setup ran) is in its first phase.
 template <int TX, int TY, int NT>
 __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, int i0, int j0,
                                              int stage, const StageArgs& a, Smem<TX, TY>& S,
-                                             int& bad, uint32_t& tma_phase) {
+                                             int& bad) {
   typedef Shape<TX, TY> Sh;
   RouteCount rc;
   // routing is a run-time switch (uniform per launch): the same machine code serves the plain and
@@ -443,7 +442,6 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
                        j0 + TY + 3 <= G.ny;
   if (use_tma) {
     auto box = stage_box(S);
-    __syncthreads();  // every thread is done with the box region (a previous tile's fluxes)
     if (tid == 0) {
       tc::fence_proxy_async();  // earlier generic accesses to the box region come first
       tc::mbar_arrive_expect_tx(&S.bar, Box<TX, TY>::kBytes);
@@ -451,15 +449,14 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     }
     // bounded wait; on giving up (never expected) the block flags the step, waits once more
     // for its copy in flight, and leaves this tile unwritten
-    const bool late = __syncthreads_or(!tc::mbar_wait(&S.bar, tma_phase, kTmaWaitLimit));
+    const bool late = __syncthreads_or(!tc::mbar_wait(&S.bar, 0u, kTmaWaitLimit));
     if (late) {
-      tc::mbar_wait(&S.bar, tma_phase, kTmaWaitLimit);
+      tc::mbar_wait(&S.bar, 0u, kTmaWaitLimit);
       if (tid == 0 && a.st) atomicOr(&a.st->status, 4);
       __syncthreads();
       bad |= 4;
       return 0.0;
     }
-    tma_phase ^= 1u;
     if (tid == 0 && a.st) atomicAdd(&a.st->tma_tiles, 1ull);
     for (int it = tid; it < Sh::W * Sh::H; it += NT) {
       const int y = it / Sh::W, x = it - y * Sh::W;
