@@ -102,17 +102,7 @@ __global__ void k_batch_set_target(StepState* st, int n, double t_final) {
 // Max wave speed of one instance's state (the first dt after set_state), double.
 __global__ void k_inst_max_speed(const BInst* __restrict__ inst, int i) {
   const BInst& I = inst[i];
-  const size_t nc = size_t(I.G.nx) * I.G.ny;
-  const double* q = I.q;
-  double ms = 0.0;
-  for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < nc;
-       k += size_t(gridDim.x) * blockDim.x) {
-    const double r = q[k], u = q[nc + k] / r, v = q[2 * nc + k] / r;
-    const double p = (q[3 * nc + k] - 0.5 * (q[nc + k] * u + q[2 * nc + k] * v)) * I.G.g1;
-    const double c = sqrt(fabs(I.G.gamma * p / r));
-    ms = fmax(ms, fmax(fmax(u - c, fabs(u + c)), fmax(v - c, fabs(v + c))));
-  }
-  block_max_to(ms, &I.st->maxbits);
+  block_max_to(fused::grid_max_speed(I.G, I.q, &I.st->maxbits), &I.st->maxbits);
 }
 
 struct BVariant {
@@ -439,7 +429,7 @@ int hteno_batch_set_state(hteno_batch* b, int i, const double* q, int where) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->dstate + i, &s, sizeof(StepState), cudaMemcpyHostToDevice, b->stream);
   if (e == cudaSuccess) {
-    k_inst_max_speed<<<64, 256, 0, b->stream>>>(b->dinst, i);
+    k_inst_max_speed<<<unsigned(std::min<size_t>(8 * 152, (b->ncell[i] + 1023) / 1024)), 256, 0, b->stream>>>(b->dinst, i);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

@@ -42,18 +42,10 @@ __global__ void __launch_bounds__(NT, MINB) k_fused(Geo G, int stage, fused::Sta
   }
 }
 
-// Max wave speed of a state in double (timeStepping, FV_System2D.cpp:622-633): the first dt.
+// Max wave speed of a state in double (timeStepping, FV_System2D.cpp:622-633): the first dt.  Four
+// cells a thread at least, so that the first, unfiltered ones are few of them.
 __global__ void k_max_speed(Geo G, const double* __restrict__ q, StepState* st) {
-  const size_t nc = size_t(G.nx) * G.ny;
-  double ms = 0.0;
-  for (size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x; k < nc;
-       k += size_t(gridDim.x) * blockDim.x) {
-    const double r = q[k], u = q[nc + k] / r, v = q[2 * nc + k] / r;
-    const double p = (q[3 * nc + k] - 0.5 * (q[nc + k] * u + q[2 * nc + k] * v)) * G.g1;
-    const double c = sqrt(fabs(G.gamma * p / r));
-    ms = fmax(ms, fmax(fmax(u - c, fabs(u + c)), fmax(v - c, fabs(v + c))));
-  }
-  block_max_to(ms, &st->maxbits);
+  block_max_to(fused::grid_max_speed(G, q, &st->maxbits), &st->maxbits);
 }
 
 // Erosion of a route mask [rows][cols] along one axis: a bit stays set only where it is set on
@@ -202,7 +194,7 @@ int fv2d_fused_setup(hteno_solver* s) {
 int fv2d_fused_prepare(hteno_solver* s, const Geo& G, double* scratch) {
   s->router_steps = 0;  // a new state: the next step classifies (route masks are per state)
   if (s->audit) cudaMemsetAsync(s->audit, 0, 7 * sizeof(unsigned long long), s->stream);
-  k_max_speed<<<304, 256, 0, s->stream>>>(G, s->q, s->dstate);
+  k_max_speed<<<unsigned(std::min<size_t>(8 * 152, (s->ncell + 1023) / 1024)), 256, 0, s->stream>>>(G, s->q, s->dstate);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(s, e, "max speed");
   if (s->tile_variant >= 0) return HTENO_OK;

@@ -38,7 +38,7 @@ int hermite2d_prepare(hteno_solver* s) {
   const size_t nc = size_t(G.nx) * G.ny;
   if (s->cfg.precision == HTENO_PREC_MIXED) {
     const WorkH<float> W = carve_h<float>(s->work, G.nx, G.ny);
-    kh_prim_f<<<unsigned((nc + 255) / 256), 256, 0, s->stream>>>(G, s->q, W.qt, W.primt, s->dstate);
+    kh_prim_f<<<unsigned(std::min<size_t>(8 * 152, (nc + 255) / 256)), 256, 0, s->stream>>>(G, s->q, W.qt, W.primt, s->dstate);
   } else
     hermite2d_fp64_prim(s, G);
   return cuda_error(s, cudaGetLastError(), "kh_prim");
