@@ -34,14 +34,21 @@ namespace {
 
 constexpr uint32_t kWaitLimit = 1u << 22;  // polls of an mbarrier before giving up
 
+// Training, one tile of 128 rows at a time.  The transposed operands (rows = features or outputs,
+// K = the tile's rows) have their core matrices kTK = 144 bytes apart along K instead of 128: eight
+// consecutive rows write one 16-byte line of each core matrix, and with 128 the four core matrices
+// that a warp writes would fall on the same banks.
+constexpr int kTK = 144, kTGroup = 16 * kTK;  // bytes per core matrix along K, per group of 8 rows
 struct Smem {
-  alignas(128) unsigned char at[128 * 128 * 2];  // A operand of the weight gradients (rows = outputs)
+  // A operand of the weight gradients: 32 outputs.  The products read 128 rows (9 KB further each
+  // 32): what lies there goes to accumulator rows that nothing reads.
+  alignas(128) unsigned char at[4 * kTGroup];
   alignas(128) unsigned char x[128 * 16 * 2];
-  alignas(128) unsigned char xt[16 * 128 * 2];
+  alignas(128) unsigned char xt[2 * kTGroup];
   alignas(128) unsigned char h1[128 * 32 * 2];
-  alignas(128) unsigned char h1t[32 * 128 * 2];
+  alignas(128) unsigned char h1t[4 * kTGroup];
   alignas(128) unsigned char h2[128 * 32 * 2];
-  alignas(128) unsigned char h2t[32 * 128 * 2];
+  alignas(128) unsigned char h2t[4 * kTGroup];
   alignas(128) unsigned char dz3[128 * 16 * 2];
   alignas(128) unsigned char dz2[128 * 32 * 2];
   alignas(128) unsigned char w1[32 * 16 * 2];
@@ -51,13 +58,14 @@ struct Smem {
   alignas(128) unsigned char w2t[32 * 32 * 2];
   float b1[32], b2[32], b3[16];
   // bias gradients and loss, one slot per warp (summed in warp order at the end: deterministic)
-  float gb1[4][32], gb2[4][32], gb3[4][16];
+  float gb1[4][32], gb2[4][32], gb3[4][4];
   float loss[4];
   alignas(8) uint64_t mbar;
   uint32_t tmem;
   static constexpr bool kTrain = true;
   static constexpr uint32_t kTmemCols = 256;
 };
+static_assert(sizeof(Smem) >= 16 * kTGroup, "the A operand's 128 rows lie inside the structure");
 
 // Shared memory of the inference kernels (the forward pass only).  A CTA runs kCT tiles of 128
 // rows at once, so that each issue-wait-load round trip of a layer serves 512 rows; a tile's X,
@@ -88,29 +96,31 @@ __device__ __forceinline__ uint64_t desc_k(const unsigned char* base, int K, int
   return tc::sdesc(tc::smem_u32(base) + uint32_t(kstep) * 256u, 128u, uint32_t(K / 8) * 128u);
 }
 
+// Transposed operand: byte offset of (r, k), and the descriptor of K step kstep (16 of K).
+__device__ __forceinline__ uint32_t tmaj(int r, int k) {
+  return uint32_t((r >> 3) * kTGroup + (k >> 3) * kTK + (r & 7) * 16 + (k & 7) * 2);
+}
+__device__ __forceinline__ uint64_t desc_t(const unsigned char* base, int kstep) {
+  return tc::sdesc(tc::smem_u32(base) + uint32_t(kstep) * 2u * kTK, kTK, kTGroup);
+}
+
+// Row-major BF16 [rows][K] image to the operand layout, 16 bytes (8 of K) at a time.
+__device__ __forceinline__ void put_image(unsigned char* dst, const void* img, int rows, int K) {
+  for (int e = threadIdx.x; e < rows * K / 8; e += blockDim.x) {
+    const int r = e / (K / 8), g = e % (K / 8);
+    *reinterpret_cast<uint4*>(dst + tc::kmaj(r, 8 * g, K)) = static_cast<const uint4*>(img)[e];
+  }
+}
+
 // Copies the BF16 weight images into the operand layouts and the FP32 biases.
 template <typename SM>
 __device__ void load_weights(SM& S, const Weights& W) {
-  const __nv_bfloat16* w1 = reinterpret_cast<const __nv_bfloat16*>(W.w1);
-  for (int e = threadIdx.x; e < 32 * 16; e += blockDim.x) {
-    const int r = e / 16, k = e % 16;
-    *reinterpret_cast<__nv_bfloat16*>(S.w1 + tc::kmaj(r, k, 16)) = w1[e];
-    if constexpr (SM::kTrain)
-      *reinterpret_cast<__nv_bfloat16*>(S.w3t + tc::kmaj(r, k, 16)) =
-          reinterpret_cast<const __nv_bfloat16*>(W.w3t)[e];
-  }
-  for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
-    const int r = e / 32, k = e % 32;
-    *reinterpret_cast<__nv_bfloat16*>(S.w2 + tc::kmaj(r, k, 32)) =
-        reinterpret_cast<const __nv_bfloat16*>(W.w2)[e];
-    if constexpr (SM::kTrain)
-      *reinterpret_cast<__nv_bfloat16*>(S.w2t + tc::kmaj(r, k, 32)) =
-          reinterpret_cast<const __nv_bfloat16*>(W.w2t)[e];
-  }
-  for (int e = threadIdx.x; e < 16 * 32; e += blockDim.x) {
-    const int r = e / 32, k = e % 32;
-    *reinterpret_cast<__nv_bfloat16*>(S.w3 + tc::kmaj(r, k, 32)) =
-        reinterpret_cast<const __nv_bfloat16*>(W.w3)[e];
+  put_image(S.w1, W.w1, 32, 16);
+  put_image(S.w2, W.w2, 32, 32);
+  put_image(S.w3, W.w3, 16, 32);
+  if constexpr (SM::kTrain) {
+    put_image(S.w3t, W.w3t, 32, 16);
+    put_image(S.w2t, W.w2t, 32, 32);
   }
   for (int e = threadIdx.x; e < 32; e += blockDim.x) {
     S.b1[e] = W.b1[e];
@@ -135,19 +145,97 @@ __device__ __forceinline__ void before_issue() {
   __syncthreads();
 }
 
-__device__ __forceinline__ float rbf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// Forward pass of the tile whose inputs are in S.x / S.xt; leaves z1..z3 per thread.
-// keep_t: also store H1^T / H2^T (needed by the weight gradients).
-template <typename SM>
-__device__ __forceinline__ bool forward(SM& S, uint32_t tbase, uint32_t& phase, float* h1,
-                                        float* h2, float* z3, bool keep_t, uint32_t limit) {
+// The sums over the warp of each of 32 columns, lane c's result being column c's: halves of the
+// columns change sides at each step, 31 shuffles instead of 160 for 32 warp_sum, the same additions.
+__device__ __forceinline__ float column_sums(float* v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < o; ++j) {
+      const float send = up ? v[j] : v[j + o], keep = up ? v[j + o] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
+}
+
+// Two floats -> two BF16 (round to nearest even), lo to the lower address; and back.
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+__device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+
+// This thread's 32 values, packed in w, as row `row` of a K-major operand (dst, unless null) and as
+// column `row` of a transposed one.
+__device__ __forceinline__ void put_row32(unsigned char* dst, unsigned char* dst_t, int row, const uint32_t* w) {
+  if (dst != nullptr) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+      *reinterpret_cast<uint4*>(dst + tc::kmaj(row, 8 * g, 32)) =
+          make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+  }
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    *reinterpret_cast<uint16_t*>(dst_t + tmaj(2 * c, row)) = uint16_t(w[c]);
+    *reinterpret_cast<uint16_t*>(dst_t + tmaj(2 * c + 1, row)) = uint16_t(w[c] >> 16);
+  }
+}
+
+// A hidden layer of this thread's row (training): bias and ReLU on the accumulator row at taddr, the
+// BF16 operands of the next layer and of the weight gradient; returns where the ReLU passes.
+__device__ __forceinline__ uint32_t hidden_train(uint32_t taddr, const float* b, unsigned char* dst,
+                                                 unsigned char* dst_t, int row) {
+  float h[32];
+  tc::tmem_ld16(taddr, h);
+  tc::tmem_ld16(taddr + 16, h + 16);
+  uint32_t w[16], pass = 0u;
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    h[c] = fmaxf(h[c] + b[c], 0.0f);
+    pass |= h[c] > 0.f ? 1u << c : 0u;
+  }
+#pragma unroll
+  for (int c = 0; c < 16; ++c) w[c] = pack_bf16(h[2 * c], h[2 * c + 1]);
+  put_row32(dst, dst_t, row, w);
+  return pass;
+}
+
+// The error terms of a hidden layer: the accumulator row at taddr where the ReLU passed, as operands
+// (dst may be null); returns this warp's sum of column `lane` of the rounded terms (bias gradient).
+__device__ __forceinline__ float error_train(uint32_t taddr, uint32_t pass, unsigned char* dst,
+                                             unsigned char* dst_t, int row) {
+  float d[32];
+  tc::tmem_ld16(taddr, d);
+  tc::tmem_ld16(taddr + 16, d + 16);
+  uint32_t w[16];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) d[c] = (pass >> c) & 1u ? d[c] : 0.f;
+#pragma unroll
+  for (int c = 0; c < 16; ++c) w[c] = pack_bf16(d[2 * c], d[2 * c + 1]);
+  put_row32(dst, dst_t, row, w);
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    d[2 * c] = bf_lo(w[c]);
+    d[2 * c + 1] = bf_hi(w[c]);
+  }
+  return column_sums(d);
+}
+
+// Forward pass of the tile whose inputs are in S.x / S.xt: the logits z3 of this thread's row and
+// where its two hidden layers' ReLUs pass; H1, H2 and their transposes stay in shared memory.
+__device__ __forceinline__ bool forward(Smem& S, uint32_t tbase, uint32_t& phase, uint32_t* pass1,
+                                        uint32_t* pass2, float* z3, uint32_t limit) {
   const int row = threadIdx.x;
   const uint32_t lane_addr = tbase + (uint32_t(threadIdx.x & ~31) << 16);
   before_issue();
@@ -157,15 +245,7 @@ __device__ __forceinline__ bool forward(SM& S, uint32_t tbase, uint32_t& phase, 
     tc::commit(&S.mbar);
   }
   if (!wait_mma(S, phase, limit)) return false;
-  tc::tmem_ld16(lane_addr + C_D1, h1);
-  tc::tmem_ld16(lane_addr + C_D1 + 16, h1 + 16);
-#pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    h1[c] = fmaxf(h1[c] + S.b1[c], 0.0f);
-    tc::st_bf16(S.h1, tc::kmaj(row, c, 32), h1[c]);
-    if constexpr (SM::kTrain)
-      if (keep_t) tc::st_bf16(S.h1t, tc::kmaj(c, row, 128), h1[c]);
-  }
+  *pass1 = hidden_train(lane_addr + C_D1, S.b1, S.h1, S.h1t, row);
   before_issue();
   if (threadIdx.x == 0) {
     tc::fence_after();
@@ -174,15 +254,7 @@ __device__ __forceinline__ bool forward(SM& S, uint32_t tbase, uint32_t& phase, 
     tc::commit(&S.mbar);
   }
   if (!wait_mma(S, phase, limit)) return false;
-  tc::tmem_ld16(lane_addr + C_D2, h2);
-  tc::tmem_ld16(lane_addr + C_D2 + 16, h2 + 16);
-#pragma unroll
-  for (int c = 0; c < 32; ++c) {
-    h2[c] = fmaxf(h2[c] + S.b2[c], 0.0f);
-    tc::st_bf16(S.h2, tc::kmaj(row, c, 32), h2[c]);
-    if constexpr (SM::kTrain)
-      if (keep_t) tc::st_bf16(S.h2t, tc::kmaj(c, row, 128), h2[c]);
-  }
+  *pass2 = hidden_train(lane_addr + C_D2, S.b2, S.h2, S.h2t, row);
   before_issue();
   if (threadIdx.x == 0) {
     tc::fence_after();
@@ -281,30 +353,17 @@ __device__ __forceinline__ bool forward_rows(SmemC& S, uint32_t tbase, uint32_t&
   return true;
 }
 
-// Writes one input row (6 features, bf16 bits) into S.x and S.xt.
+// Everything of a launch that does not need the weights.
 template <typename SM>
-__device__ __forceinline__ void put_input(SM& S, int row, const uint16_t* f) {
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const uint16_t bits = k < 6 ? f[k] : uint16_t(0);
-    *reinterpret_cast<uint16_t*>(S.x + tc::kmaj(row, k, 16)) = bits;
-    if constexpr (SM::kTrain) *reinterpret_cast<uint16_t*>(S.xt + tc::kmaj(k, row, 128)) = bits;
-  }
-}
-
-template <typename SM>
-__device__ void setup(SM& S, const Weights& W) {
+__device__ void setup(SM& S) {
   if constexpr (SM::kTrain) {
-    for (int e = threadIdx.x; e < int(sizeof(S.at) / 16); e += blockDim.x)
-      reinterpret_cast<uint4*>(S.at)[e] = make_uint4(0, 0, 0, 0);
-  }
-  load_weights(S, W);
-  if constexpr (SM::kTrain) {
-    for (int e = threadIdx.x; e < 4 * 32; e += blockDim.x) {
-      S.gb1[e / 32][e % 32] = 0.f;
-      S.gb2[e / 32][e % 32] = 0.f;
-      if (e % 32 < 16) S.gb3[e / 32][e % 32] = 0.f;
-    }
+    // the constant zeros of the operands: features 6..15 of X and X^T, outputs 3..15 of dZ3
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(S.x + tc::kmaj(threadIdx.x, 8, 16)) = zero;
+    *reinterpret_cast<uint4*>(S.dz3 + tc::kmaj(threadIdx.x, 8, 16)) = zero;
+    for (int e = threadIdx.x; e < 10 * 16; e += blockDim.x)
+      *reinterpret_cast<uint4*>(S.xt + tmaj(6 + e / 16, 8 * (e % 16))) = zero;
+    if (threadIdx.x < 16) S.gb3[threadIdx.x / 4][threadIdx.x % 4] = 0.f;
     if (threadIdx.x < 4) S.loss[threadIdx.x] = 0.f;
   }
   if (threadIdx.x == 0) {
@@ -312,10 +371,20 @@ __device__ void setup(SM& S, const Weights& W) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x < 32) tc::tmem_alloc(&S.tmem, SM::kTmemCols);
+}
+template <typename SM>
+__device__ void setup(SM& S, const Weights& W) {
+  setup(S);
+  load_weights(S, W);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
 }
+
+// Programmatic dependent launch: wait for the previous kernel of the stream to complete (at once if
+// this one was launched without the attribute), and let the next one start its own set-up.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename SM>
 __device__ void teardown(SM& S, uint32_t tbase) {
@@ -326,8 +395,13 @@ __device__ void teardown(SM& S, uint32_t tbase) {
 }
 
 // Gradient of the mean BCE loss over `n_total` rows: each CTA writes its partial gradient (padded
-// layout) to Gp[blockIdx.x] and its partial loss sum to Lp[blockIdx.x]; k_reduce_grad adds the
-// partials in CTA order, so the gradient does not depend on the order in which CTAs finish.
+// layout) to Gp[blockIdx.x] and its partial loss sum to Lp[blockIdx.x]; the next kernel adds the
+// partials in CTA order, so the gradient does not depend on the order in which CTAs finish.  A batch
+// is a tile or two per CTA, so the time is one tile's chain: six tensor-core round trips and the
+// conversions between them, in one warp per scheduler.  Hence operand rows in 16-byte stores, the
+// transposed ones without bank conflicts, bias gradients by column_sums, set-up and input loads
+// before the previous kernel has completed.  Batches of 16384 rows, alone from cold caches: 16.3 -> 11.4
+// us; a whole batch with its sums and update 34 -> 17.4 us.
 // `limit`: polls of each tensor-core completion wait before the kernel gives up.
 __global__ void __launch_bounds__(128) k_train(Weights W, const uint16_t* __restrict__ X,
                                                const uint8_t* __restrict__ Y, long n, long n_total,
@@ -335,109 +409,106 @@ __global__ void __launch_bounds__(128) k_train(Weights W, const uint16_t* __rest
                                                int* __restrict__ err, uint32_t limit) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Smem& S = *reinterpret_cast<Smem*>(smem_raw);
-  setup(S, W);
-  const uint32_t tbase = S.tmem;
-  const uint32_t lane_addr = tbase + (uint32_t(threadIdx.x & ~31) << 16);
+  setup(S);
   const int row = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float inv_n = 1.0f / float(n_total);
+  const long ntiles = (n + 127) / 128;
+  uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+  uint32_t y = 0;
+  auto fetch = [&](long t) {
+    const long r = t * 128 + row;
+    const bool valid = t < ntiles && r < n;
+    raw = valid ? *reinterpret_cast<const uint4*>(X + r * 8) : make_uint4(0u, 0u, 0u, 0u);
+    y = valid ? Y[r] : 0u;
+  };
+  fetch(blockIdx.x);  // (the rows are not written by the kernel before this one, the weights are)
+  grid_wait();
+  grid_release();
+  load_weights(S, W);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tbase = S.tmem;
+  const uint32_t lane_addr = tbase + (uint32_t(threadIdx.x & ~31) << 16);
   uint32_t phase = 0;
   bool ok = true;
   int tiles_done = 0;
-  const long ntiles = (n + 127) / 128;
+  float gb1 = 0.f, gb2 = 0.f;  // bias gradients of hidden unit `lane`, this warp's rows
   for (long t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++tiles_done) {
-    const long r = t * 128 + row;
-    const bool valid = r < n;
-    uint16_t f[6] = {0, 0, 0, 0, 0, 0};
-    uint8_t y = 0;
-    if (valid) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(X + r * 8);
-      const uint16_t* p = reinterpret_cast<const uint16_t*>(&raw);
+    const bool valid = t * 128 + row < n;
+    const uint32_t f[3] = {raw.x, raw.y, raw.z}, yb = y;
+    *reinterpret_cast<uint4*>(S.x + tc::kmaj(row, 0, 16)) = make_uint4(f[0], f[1], f[2], 0u);
 #pragma unroll
-      for (int k = 0; k < 6; ++k) f[k] = p[k];
-      y = Y[r];
-    }
-    put_input(S, row, f);
-    float h1[32], h2[32], z3[3];
-    ok = forward(S, tbase, phase, h1, h2, z3, true, limit);
+    for (int k = 0; k < 6; ++k)
+      *reinterpret_cast<uint16_t*>(S.xt + tmaj(k, row)) = uint16_t(f[k / 2] >> (16 * (k & 1)));
+    fetch(t + gridDim.x);
+    uint32_t pass1, pass2;
+    float z3[3];
+    ok = forward(S, tbase, phase, &pass1, &pass2, z3, limit);
     if (!ok) break;
     // loss and dZ3
     float dz3[3], l = 0.f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float yk = float((y >> k) & 1);
+      const float yk = float((yb >> k) & 1u);
       const float z = z3[k];
       const float pk = 1.0f / (1.0f + __expf(-z));
       l += fmaxf(z, 0.f) - z * yk + log1pf(__expf(-fabsf(z)));
       dz3[k] = valid ? (pk - yk) * inv_n : 0.f;
     }
     if (!valid) l = 0.f;
-    l = warp_sum(l);
-    if (lane == 0) S.loss[warp] += l;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const float v = k < 3 ? dz3[k] : 0.f;
-      tc::st_bf16(S.dz3, tc::kmaj(row, k, 16), v);
-      tc::st_bf16(S.at, tc::kmaj(k, row, 128), v);
-    }
-    // bias gradients sum the same BF16-rounded error terms the matrix products use
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float s = warp_sum(rbf(dz3[k]));
-      if (lane == 0) S.gb3[warp][k] += s;
-    }
+    const uint32_t w01 = pack_bf16(dz3[0], dz3[1]), w2 = pack_bf16(dz3[2], 0.f);
+    *reinterpret_cast<uint4*>(S.dz3 + tc::kmaj(row, 0, 16)) = make_uint4(w01, w2, 0u, 0u);
+    *reinterpret_cast<uint16_t*>(S.at + tmaj(0, row)) = uint16_t(w01);
+    *reinterpret_cast<uint16_t*>(S.at + tmaj(1, row)) = uint16_t(w01 >> 16);
+    *reinterpret_cast<uint16_t*>(S.at + tmaj(2, row)) = uint16_t(w2);
     before_issue();
     if (threadIdx.x == 0) {
       tc::fence_after();
       tc::mma_bf16(tbase + C_DH2, desc_k(S.dz3, 16, 0), desc_k(S.w3t, 16, 0), tc::idesc_bf16(128, 32), 0);
       for (int s = 0; s < 8; ++s)
-        tc::mma_bf16(tbase + C_GW3, desc_k(S.at, 128, s), desc_k(S.h2t, 128, s), tc::idesc_bf16(128, 32),
+        tc::mma_bf16(tbase + C_GW3, desc_t(S.at, s), desc_t(S.h2t, s), tc::idesc_bf16(128, 32),
                      (tiles_done > 0 || s > 0) ? 1 : 0);
       tc::commit(&S.mbar);
     }
+    // while the products run: the loss, and the bias gradients, which sum the same BF16-rounded
+    // error terms the matrix products use
+    l = warp_sum(l);
+    const float g3[3] = {warp_sum(bf_lo(w01)), warp_sum(bf_hi(w01)), warp_sum(bf_lo(w2))};
+    if (lane == 0) {
+      S.loss[warp] += l;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) S.gb3[warp][k] += g3[k];
+    }
     if (!(ok = wait_mma(S, phase, limit))) break;
     // dZ2
-    float d[32];
-    tc::tmem_ld16(lane_addr + C_DH2, d);
-    tc::tmem_ld16(lane_addr + C_DH2 + 16, d + 16);
-#pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      const float v = h2[c] > 0.f ? d[c] : 0.f;
-      tc::st_bf16(S.dz2, tc::kmaj(row, c, 32), v);
-      tc::st_bf16(S.at, tc::kmaj(c, row, 128), v);
-      const float s = warp_sum(rbf(v));
-      if (lane == 0) S.gb2[warp][c] += s;
-    }
+    gb2 += error_train(lane_addr + C_DH2, pass2, S.dz2, S.at, row);
     before_issue();
     if (threadIdx.x == 0) {
       tc::fence_after();
       for (int s = 0; s < 2; ++s)
         tc::mma_bf16(tbase + C_DH1, desc_k(S.dz2, 32, s), desc_k(S.w2t, 32, s), tc::idesc_bf16(128, 32), s);
       for (int s = 0; s < 8; ++s)
-        tc::mma_bf16(tbase + C_GW2, desc_k(S.at, 128, s), desc_k(S.h1t, 128, s), tc::idesc_bf16(128, 32),
+        tc::mma_bf16(tbase + C_GW2, desc_t(S.at, s), desc_t(S.h1t, s), tc::idesc_bf16(128, 32),
                      (tiles_done > 0 || s > 0) ? 1 : 0);
       tc::commit(&S.mbar);
     }
     if (!(ok = wait_mma(S, phase, limit))) break;
     // dZ1
-    tc::tmem_ld16(lane_addr + C_DH1, d);
-    tc::tmem_ld16(lane_addr + C_DH1 + 16, d + 16);
-#pragma unroll
-    for (int c = 0; c < 32; ++c) {
-      const float v = h1[c] > 0.f ? d[c] : 0.f;
-      tc::st_bf16(S.at, tc::kmaj(c, row, 128), v);
-      const float s = warp_sum(rbf(v));
-      if (lane == 0) S.gb1[warp][c] += s;
-    }
+    gb1 += error_train(lane_addr + C_DH1, pass1, nullptr, S.at, row);
     before_issue();
     if (threadIdx.x == 0) {
       tc::fence_after();
       for (int s = 0; s < 8; ++s)
-        tc::mma_bf16(tbase + C_GW1, desc_k(S.at, 128, s), desc_k(S.xt, 128, s), tc::idesc_bf16(128, 16),
+        tc::mma_bf16(tbase + C_GW1, desc_t(S.at, s), desc_t(S.xt, s), tc::idesc_bf16(128, 16),
                      (tiles_done > 0 || s > 0) ? 1 : 0);
       tc::commit(&S.mbar);
     }
     if (!(ok = wait_mma(S, phase, limit))) break;
   }
+  S.gb1[warp][lane] = gb1;
+  S.gb2[warp][lane] = gb2;
+  __syncthreads();
   if (!ok) {
     if (threadIdx.x == 0) atomicExch(err, 1);
     // give in-flight MMAs a bounded chance to finish before the columns are released
@@ -445,24 +516,30 @@ __global__ void __launch_bounds__(128) k_train(Weights W, const uint16_t* __rest
   }
   // this CTA's partial gradient, every entry of the padded layout written once: rows of the
   // accumulators live in lanes 0..31 (warp 0).  The padded entries are exact zeros (zero input
-  // columns 6..15, zero output rows 3..15); a CTA without a completed tile writes zeros.
+  // columns 6..15, output rows 3..15); a CTA without a completed tile writes zeros.
   if (threadIdx.x < 32) {
     const bool have = ok && tiles_done > 0;
     float* g = Gp + size_t(blockIdx.x) * kParams;
     float v[16];
+    auto put = [&](float* dst, bool keep) {
+#pragma unroll
+      for (int c = 0; c < 16; c += 4)
+        *reinterpret_cast<float4*>(dst + c) =
+            keep ? make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
     for (int h = 0; h < 2; ++h) {
       if (have) tc::tmem_ld16(lane_addr + C_GW3 + 16 * h, v);
-      if (row < 16)
-        for (int c = 0; c < 16; ++c) g[kOffW3 + row * 32 + 16 * h + c] = have ? v[c] : 0.f;
+      if (row < 16) put(g + kOffW3 + row * 32 + 16 * h, have && row < 3);
       if (have) tc::tmem_ld16(lane_addr + C_GW2 + 16 * h, v);
-      for (int c = 0; c < 16; ++c) g[kOffW2 + row * 32 + 16 * h + c] = have ? v[c] : 0.f;
+      put(g + kOffW2 + row * 32 + 16 * h, have);
     }
     if (have) tc::tmem_ld16(lane_addr + C_GW1, v);
-    for (int c = 0; c < 16; ++c) g[kOffW1 + row * 16 + c] = have ? v[c] : 0.f;
+    put(g + kOffW1 + row * 16, have);
     g[kOffB1 + row] = have ? ((S.gb1[0][row] + S.gb1[1][row]) + S.gb1[2][row]) + S.gb1[3][row] : 0.f;
     g[kOffB2 + row] = have ? ((S.gb2[0][row] + S.gb2[1][row]) + S.gb2[2][row]) + S.gb2[3][row] : 0.f;
     if (row < 16)
-      g[kOffB3 + row] = have ? ((S.gb3[0][row] + S.gb3[1][row]) + S.gb3[2][row]) + S.gb3[3][row] : 0.f;
+      g[kOffB3 + row] =
+          have && row < 3 ? ((S.gb3[0][row] + S.gb3[1][row]) + S.gb3[2][row]) + S.gb3[3][row] : 0.f;
     if (row == 0) Lp[blockIdx.x] = have ? ((S.loss[0] + S.loss[1]) + S.loss[2]) + S.loss[3] : 0.f;
   }
   teardown(S, tbase);
@@ -725,18 +802,18 @@ __global__ void __launch_bounds__(128, 4) k_route_rows(Weights W, const uint4* _
   teardown(S, tbase);
 }
 
-// Adam on the FP32 master parameters (padded layout), then the BF16 images.
-__global__ void k_adam(float* __restrict__ P, float* __restrict__ G, float* __restrict__ M,
-                       float* __restrict__ V, float lr, float b1, float b2, float eps, int t) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kParams) return;
-  const float g = G[i];
-  const float m = b1 * M[i] + (1.f - b1) * g;
-  const float v = b2 * V[i] + (1.f - b2) * g * g;
-  M[i] = m;
-  V[i] = v;
-  const float mh = m / (1.f - powf(b1, float(t))), vh = v / (1.f - powf(b2, float(t)));
-  P[i] -= lr * mh / (sqrtf(vh) + eps);
+// The sum of p[b * stride], b < n, added in order of b, 32 loads in flight.
+__device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int n) {
+  float s = 0.f;
+  for (int b = 0; b < n; b += 32) {
+    float v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = b + j < n ? p[size_t(b + j) * stride] : 0.f;
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (b + j < n) s += v[j];
+  }
+  return s;
 }
 
 // G = the sum of the nblk per-CTA partial gradients, added in CTA order; *loss += the sum of the
@@ -744,43 +821,63 @@ __global__ void k_adam(float* __restrict__ P, float* __restrict__ G, float* __re
 __global__ void k_reduce_grad(const float* __restrict__ Gp, const float* __restrict__ Lp, int nblk,
                               float* __restrict__ G, float* __restrict__ loss) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < kParams) {
-    float s = 0.f;
-    for (int b = 0; b < nblk; ++b) s += Gp[size_t(b) * kParams + i];
-    G[i] = s;
-  } else if (i == kParams) {
-    float s = 0.f;
-    for (int b = 0; b < nblk; ++b) s += Lp[b];
-    *loss += s;
-  }
+  if (i < kParams) G[i] = ordered_sum(Gp + i, kParams, nblk);
+  else if (i == kParams) *loss += ordered_sum(Lp, 1, nblk);
 }
 
-__global__ void k_images(const float* __restrict__ P, Weights W) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+// Parameter i's (value p) entries of the device images.
+__device__ __forceinline__ void put_images(const Weights& W, int i, float p) {
   __nv_bfloat16* w1 = reinterpret_cast<__nv_bfloat16*>(W.w1);
   __nv_bfloat16* w2 = reinterpret_cast<__nv_bfloat16*>(W.w2);
   __nv_bfloat16* w3 = reinterpret_cast<__nv_bfloat16*>(W.w3);
   __nv_bfloat16* w3t = reinterpret_cast<__nv_bfloat16*>(W.w3t);
   __nv_bfloat16* w2t = reinterpret_cast<__nv_bfloat16*>(W.w2t);
-  if (e < 32 * 16) {
-    const int r = e / 16, k = e % 16;
-    w1[e] = __float2bfloat16_rn(k < 6 ? P[kOffW1 + e] : 0.f);
-    w3t[e] = __float2bfloat16_rn(k < 3 ? P[kOffW3 + k * 32 + r] : 0.f);  // W3^T[j][k]
+  if (i < kOffB1) {
+    w1[i] = __float2bfloat16_rn(i % 16 < 6 ? p : 0.f);
+  } else if (i < kOffW2) {
+    W.b1[i - kOffB1] = p;
+  } else if (i < kOffB2) {
+    const int e = i - kOffW2;
+    w2[e] = __float2bfloat16_rn(p);
+    w2t[(e % 32) * 32 + e / 32] = __float2bfloat16_rn(p);  // W2^T[i][j]
+  } else if (i < kOffW3) {
+    W.b2[i - kOffB2] = p;
+  } else if (i < kOffB3) {
+    const int e = i - kOffW3, r = e / 32, k = e % 32;
+    w3[e] = __float2bfloat16_rn(r < 3 ? p : 0.f);
+    w3t[k * 16 + r] = __float2bfloat16_rn(r < 3 ? p : 0.f);  // W3^T[j][k]
+  } else {
+    W.b3[i - kOffB3] = i - kOffB3 < 3 ? p : 0.f;
   }
-  if (e < 32 * 32) {
-    const int r = e / 32, k = e % 32;
-    w2[e] = __float2bfloat16_rn(P[kOffW2 + e]);
-    w2t[e] = __float2bfloat16_rn(P[kOffW2 + k * 32 + r]);  // W2^T[i][j]
-  }
-  if (e < 16 * 32) {
-    const int r = e / 32;
-    w3[e] = __float2bfloat16_rn(r < 3 ? P[kOffW3 + e] : 0.f);
-  }
-  if (e < 32) {
-    W.b1[e] = P[kOffB1 + e];
-    W.b2[e] = P[kOffB2 + e];
-    if (e < 16) W.b3[e] = e < 3 ? P[kOffB3 + e] : 0.f;
-  }
+}
+__global__ void k_images(const float* __restrict__ P, Weights W) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kParams) put_images(W, i, P[i]);
+}
+
+// After k_train, one thread per parameter: the gradient (the partials added in CTA order, as
+// k_reduce_grad), Adam on the FP32 master parameters (padded layout) and the images of the new value;
+// one thread more for the loss.  Bound by latency (34 blocks of 64 threads, the partials from L2, 32 loads
+// in flight each).  Alone from cold caches the three kernels that did this took 9.9 + 4 + 4 us, this one 11.
+__global__ void __launch_bounds__(64) k_adam(const float* __restrict__ Gp, const float* __restrict__ Lp, int nblk,
+                                             float* __restrict__ P, float* __restrict__ M, float* __restrict__ V,
+                                             float* __restrict__ loss, Weights W, float lr, float b1, float b2,
+                                             float eps, int t) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  grid_wait();
+  grid_release();
+  if (i == kParams) *loss += ordered_sum(Lp, 1, nblk);
+  if (i >= kParams) return;
+  const float m0 = M[i], v0 = V[i], p0 = P[i];
+  const float g = ordered_sum(Gp + i, kParams, nblk);
+  const float m = b1 * m0 + (1.f - b1) * g;
+  const float v = b2 * v0 + (1.f - b2) * g * g;
+  M[i] = m;
+  V[i] = v;
+  const float mh = m / (1.f - powf(b1, float(t))), vh = v / (1.f - powf(b2, float(t)));
+  const float p = p0 - lr * mh / (sqrtf(vh) + eps);
+  P[i] = p;
+  put_images(W, i, p);
 }
 
 // Converts float rows [n][6] to the bf16 training layout [n][8].
@@ -876,8 +973,25 @@ void from_padded(const float* p, float* c) {
   for (int k = 0; k < 3; ++k) c[1376 + k] = p[kOffB3 + k];
 }
 
+// Launch with programmatic stream serialization: the kernel may start while the one before it in the
+// stream ends, and calls grid_wait before it touches what that one reads or writes.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(unsigned(grid));
+  c.blockDim = dim3(unsigned(block));
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 int refresh_images(hteno_mlp* m) {
-  k_images<<<4, 256, 0, m->stream>>>(m->P, m->W);
+  k_images<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->P, m->W);
   return merr(m, cudaGetLastError(), "weight images");
 }
 
@@ -1040,13 +1154,13 @@ int hteno_mlp_train(hteno_mlp* m, const uint16_t* x, const uint8_t* y, long n, i
       const long nb = std::min(batch, n - off);
       const long tiles = (nb + 127) / 128;
       const int grid = int(std::min<long>(tiles, 2L * m->sms));
-      k_train<<<grid, 128, mlp::smem_bytes(), m->stream>>>(m->W, x + off * 8, y + off, nb, nb, m->Gp,
-                                                           m->Lp, m->err, m->wait_limit);
-      k_reduce_grad<<<(kParams + 256) / 256, 256, 0, m->stream>>>(m->Gp, m->Lp, grid, m->G, m->loss);
       ++m->t;
-      k_adam<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->P, m->G, m->M, m->V, lr, 0.9f, 0.999f,
-                                                           1e-8f, m->t);
-      k_images<<<4, 256, 0, m->stream>>>(m->P, m->W);
+      cudaError_t e = launch_early(k_train, grid, 128, mlp::smem_bytes(), m->stream, m->W, x + off * 8, y + off, nb,
+                                   nb, m->Gp, m->Lp, m->err, m->wait_limit);
+      if (e == cudaSuccess)
+        e = launch_early(k_adam, (kParams + 64) / 64, 64, 0, m->stream, m->Gp, m->Lp, grid, m->P, m->M, m->V,
+                         m->loss, m->W, lr, 0.9f, 0.999f, 1e-8f, m->t);
+      if (e != cudaSuccess) return merr(m, e, "train launch");
     }
     int rc = merr(m, cudaGetLastError(), "train launch");
     if (rc) return rc;
