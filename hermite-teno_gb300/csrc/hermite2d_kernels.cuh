@@ -9,6 +9,7 @@
 
 #include "hermite_limit.cuh"
 #include "hteno_internal.h"
+#include "mixed_pairs.cuh"
 
 namespace hteno {
 
@@ -442,13 +443,16 @@ template <typename T, int DIR>
 __global__ void __launch_bounds__(kHFluxThreads) kh_flux(GeoH G, const T* __restrict__ fc,
                                                         const T* __restrict__ froe,
                                                         T* __restrict__ F, const StepState* st) {
+  // In float bound by instruction issue (66 % of the slots, 4600 per warp of which GL3 half): GL3 and the
+  // back-projection take both sides of a face in packed pairs (2048^2: 700 -> 518 us, the same bits).
   // GL3 values of the 24 face arrays at the 3 Gauss points, per thread, in shared memory: for
-  // float [array][point][thread] (a warp's accesses fall in 32 distinct banks); for double
-  // [thread][array][point] with a one-value pad per thread (par::gl3 writes 3 contiguous values;
-  // the odd stride of 73 values spreads a warp's 8-byte accesses over all banks)
-  constexpr int kSgT = std::is_same<T, double>::value ? 73 : 72;
-  __shared__ T sg[kHFluxThreads * kSgT];
-  auto gat = [&](int a, int m) -> T& {
+  // float the (minus, plus) pairs as [pair][point][thread] (a warp's accesses fall in distinct banks);
+  // for double [thread][array][point] with a one-value pad per thread (par::gl3 writes 3 contiguous
+  // values; the odd stride of 73 values spreads a warp's 8-byte accesses over all banks)
+  typedef typename std::conditional<std::is_same<T, double>::value, double, f2>::type Sg;
+  constexpr int kSgT = std::is_same<T, double>::value ? 73 : 36;
+  __shared__ Sg sg[kHFluxThreads * kSgT];
+  auto gat = [&](int a, int m) -> Sg& {
     if constexpr (std::is_same<T, double>::value) return sg[threadIdx.x * kSgT + a * 3 + m];
     else return sg[(a * 3 + m) * kHFluxThreads + threadIdx.x];
   };
@@ -471,12 +475,25 @@ __global__ void __launch_bounds__(kHFluxThreads) kh_flux(GeoH G, const T* __rest
   size_t nb[5];
 #pragma unroll
   for (int m = 0; m < 5; ++m) nb[m] = fidx(t - 2 + m);
-  for (int a = 0; a < 24; ++a) {
-    T u5[5];
+  if constexpr (std::is_same<T, double>::value) {
+    for (int a = 0; a < 24; ++a) {
+      T u5[5];
 #pragma unroll
-    for (int m = 0; m < 5; ++m) u5[m] = fc[size_t(a) * nface + nb[m]];
-    if constexpr (std::is_same<T, double>::value) par::gl3(g_dev, u5, &gat(a, 0));
-    else gl3(c_dev, u5, gat(a, 0), gat(a, 1), gat(a, 2));
+      for (int m = 0; m < 5; ++m) u5[m] = fc[size_t(a) * nface + nb[m]];
+      par::gl3(g_dev, u5, &gat(a, 0));
+    }
+  } else {
+    // pair a: field a % 4 of kind a / 4 (u, normal and tangential derivative), both sides of the face
+    for (int a = 0; a < 12; ++a) {
+      const T* fa = fc + size_t(8 * (a / 4) + a % 4) * nface;
+      f2 u5[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) u5[m] = pack(fa[nb[m]], fa[4 * nface + nb[m]]);
+      const Gl3f g = gl3_pair<true>(c_dev, u5[0], u5[1], u5[2], u5[3], u5[4]);
+      gat(a, 0) = g.a;
+      gat(a, 1) = g.b;
+      gat(a, 2) = g.c;
+    }
   }
   const size_t o = nb[2];
   T acc[12];
@@ -517,9 +534,15 @@ __global__ void __launch_bounds__(kHFluxThreads) kh_flux(GeoH G, const T* __rest
     for (int m = 0; m < 3; ++m) {
       T X[6][4];
 #pragma unroll
-      for (int a = 0; a < 6; ++a) {
-        T c[4] = {gat(4 * a + 0, m), gat(4 * a + 1, m), gat(4 * a + 2, m), gat(4 * a + 3, m)};
-        roe_right(R, DIR, c, X[a]);
+      for (int a = 0; a < 3; ++a) {
+        const f2 c[4] = {gat(4 * a + 0, m), gat(4 * a + 1, m), gat(4 * a + 2, m), gat(4 * a + 3, m)};
+        f2 x[4];
+        right2(R, DIR, c, x);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          X[2 * a][k] = lo(x[k]);
+          X[2 * a + 1][k] = hi(x[k]);
+        }
       }
       T fu[4], fn[4], ft[4];
       rusanov2(gm, g1, DIR, R, X[0], X[1], fu);
