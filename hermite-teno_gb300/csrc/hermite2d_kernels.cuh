@@ -15,6 +15,9 @@ namespace hteno {
 
 constexpr int kHFaceThreads = 128;
 constexpr int kHFluxThreads = 64;
+// Blocks per SM that the face kernel's registers are cut for: in float 5, 6, 7 blocks (96, 80, 72
+// registers, a few spilled) took 413, 408, 405 us at 2048^2, unbounded 130-136.
+template <typename T> constexpr int kHFaceBlocks = std::is_same<T, float>::value ? 7 : 1;
 
 struct GeoH {
   int nx, ny;
@@ -313,8 +316,12 @@ __global__ void __launch_bounds__(256) kh_limit(GeoH G, HermiteK<T> K, const T* 
   }
 }
 
+// Characteristic reconstruction of every face: HTENO of value and derivative from u and the moment along
+// the sweep, TENO5 of the cross moment.  In float bound by instruction issue (67 % of the slots; FMA pipe
+// 62 %, ALU 46 %): projections of two cells and both sides of a reconstruction in packed pairs, the
+// weights per cut-off pattern in shared memory.  2048^2: 440 -> 405 us, the same bits.
 template <typename T, int DIR>
-__global__ void __launch_bounds__(kHFaceThreads) kh_faces(GeoH G, HermiteK<T> K,
+__global__ void __launch_bounds__(kHFaceThreads, kHFaceBlocks<T>) kh_faces(GeoH G, HermiteK<T> K,
                                                          const T* __restrict__ q,
                                                          const T* __restrict__ v,
                                                          const T* __restrict__ w,
@@ -322,6 +329,9 @@ __global__ void __launch_bounds__(kHFaceThreads) kh_faces(GeoH G, HermiteK<T> K,
                                                          T* __restrict__ fc, T* __restrict__ froe,
                                                          const StepState* st) {
   if (st && st->done) return;
+  __shared__ typename std::conditional<std::is_same<T, double>::value, char, HermiteTab>::type tab;
+  __shared__ typename std::conditional<std::is_same<T, double>::value, char[28][1], f2[28][kHFaceThreads]>::type cv;
+  if constexpr (!std::is_same<T, double>::value) load_hermite_tab(tab, K, c_dev);
   const int nf = DIR == 1 ? G.nx + 1 : G.ny + 1;
   const int nt = DIR == 1 ? G.ny : G.nx;
   const long idx = blockIdx.x * long(blockDim.x) + threadIdx.x;
@@ -381,62 +391,51 @@ __global__ void __launch_bounds__(kHFaceThreads) kh_faces(GeoH G, HermiteK<T> K,
       }
     }
     par::eig_store(E, froe + o, nface);
-    return;
-  }
-  const Roe2<T> R = roe2<T>(T(G.g1), prim[3 * nc + ca], prim[ca], prim[nc + ca], prim[2 * nc + ca],
-                            prim[3 * nc + cb], prim[cb], prim[nc + cb], prim[2 * nc + cb]);
-  {
-    T A[4][4], B[4][4];
+  } else {
+    const Roe2<T> R = roe2<T>(T(G.g1), prim[3 * nc + ca], prim[ca], prim[nc + ca], prim[2 * nc + ca],
+                              prim[3 * nc + cb], prim[cb], prim[nc + cb], prim[2 * nc + cb]);
+    const LeftRows L = left_rows(R, DIR);
+    // characteristic values of cells f + c0, f + c0 + 1 (pairs) of the conserved fields x
+    auto project = [&](const T* x, int c0, f2* c) {
+      const size_t a = cell(f + c0), b = cell(f + c0 + 1);
+      const f2 w[4] = {pack(x[a], x[b]), pack(x[nc + a], x[nc + b]), pack(x[2 * nc + a], x[2 * nc + b]),
+                       pack(x[3 * nc + a], x[3 * nc + b])};
+      project2(L, DIR, w, c);
+    };
+    // the pairs wait in shared memory (per thread), one field's at a time in registers
+    auto put = [&](int k, const T* x, int c0) {
+      f2 c[4];
+      project(x, c0, c);
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const size_t c = cell(f - 2 + m);
-      T a4[4] = {q[c], q[nc + c], q[2 * nc + c], q[3 * nc + c]};
-      T b4[4] = {mn[c], mn[nc + c], mn[2 * nc + c], mn[3 * nc + c]};
-      T ca4[4], cb4[4];
-      roe_left(R, DIR, a4, ca4);
-      roe_left(R, DIR, b4, cb4);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        A[r][m] = ca4[r];
-        B[r][m] = cb4[r];
-      }
-    }
-#pragma unroll
+      for (int r = 0; r < 4; ++r) cv[4 * k + r][threadIdx.x] = c[r];
+    };
+    put(0, q, -2);
+    put(1, q, 0);
+    put(2, mn, -2);
+    put(3, mn, 0);
+    put(4, mt, -3);
+    put(5, mt, -1);
+    put(6, mt, 1);
+#pragma unroll 1
     for (int r = 0; r < 4; ++r) {
-      T h[4];
-      hermite_recon(c_dev, K, 0, A[r], B[r], h);
-      fc[(0 * 4 + r) * nface + o] = h[0];
-      fc[(1 * 4 + r) * nface + o] = h[1];
-      fc[(2 * 4 + r) * nface + o] = h[2];
-      fc[(3 * 4 + r) * nface + o] = h[3];
+      auto get = [&](int k) { return cv[4 * k + r][threadIdx.x]; };
+      const HtenoSides h = hteno_sides(tab, K.dif, get(0), get(1), get(2), get(3));
+      fc[(0 * 4 + r) * nface + o] = lo(h.u);
+      fc[(1 * 4 + r) * nface + o] = hi(h.u);
+      fc[(2 * 4 + r) * nface + o] = lo(h.d);
+      fc[(3 * 4 + r) * nface + o] = hi(h.d);
+      const f2 u = teno5_sides(c_dev, tab, get(4), get(5), get(6));
+      fc[(4 * 4 + r) * nface + o] = lo(u);
+      fc[(5 * 4 + r) * nface + o] = hi(u);
     }
+    froe[0 * nface + o] = R.vxm;
+    froe[1 * nface + o] = R.vym;
+    froe[2 * nface + o] = R.hm;
+    froe[3 * nface + o] = R.qm;
+    froe[4 * nface + o] = R.cm;
+    froe[5 * nface + o] = R.rcm;
+    froe[6 * nface + o] = R.b1;
   }
-  {
-    T C[4][6];
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const size_t c = cell(f - 3 + m);
-      T c4[4] = {mt[c], mt[nc + c], mt[2 * nc + c], mt[3 * nc + c]};
-      T cc[4];
-      roe_left(R, DIR, c4, cc);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) C[r][m] = cc[r];
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      T a, b;
-      lagrange_recon(c_dev, HTENO_RECON_TENO5, C[r], a, b);
-      fc[(4 * 4 + r) * nface + o] = a;
-      fc[(5 * 4 + r) * nface + o] = b;
-    }
-  }
-  froe[0 * nface + o] = R.vxm;
-  froe[1 * nface + o] = R.vym;
-  froe[2 * nface + o] = R.hm;
-  froe[3 * nface + o] = R.qm;
-  froe[4 * nface + o] = R.cm;
-  froe[5 * nface + o] = R.rcm;
-  froe[6 * nface + o] = R.b1;
 }
 
 template <typename T, int DIR>
