@@ -34,6 +34,8 @@ __device__ __forceinline__ void block_max_to(double v, unsigned long long* bits)
 // Start of one step of timeStepping() (FV_System2D.cpp:622-645): stop when t >= t_final,
 // otherwise dt = dt_scale / max wave speed, clipped to t_final.
 __global__ void k_begin_step(StepState* st) {
+  grid_release();
+  grid_wait();
   if (st->done) return;
   if (!(st->t < st->t_final)) {
     st->done = 1;
@@ -47,6 +49,8 @@ __global__ void k_begin_step(StepState* st) {
 }
 
 __global__ void k_end_step(StepState* st) {
+  grid_release();
+  grid_wait();
   if (st->done) return;
   st->t += st->dt;
   st->steps += 1;

@@ -47,7 +47,7 @@ int fv2d_prepare(hteno_solver* s) {
 namespace {
 
 void launch_step(hteno_solver* s, const Geo& G) {
-  k_begin_step<<<1, 1, 0, s->stream>>>(s->dstate);
+  launch_early(s->early, k_begin_step, 1, 1, 0, s->stream, s->dstate);
   if (s->cfg.precision == HTENO_PREC_MIXED) {
     fv2d_fused_step(s, G, static_cast<double*>(s->work));
   } else {
@@ -55,7 +55,7 @@ void launch_step(hteno_solver* s, const Geo& G) {
     if (s->fused64) fv2d_fp64_fused_step(s, G, W);
     else for (int stage = 1; stage <= 3; ++stage) fv2d_fp64_stage(s, G, W, stage, s->q, nullptr);
   }
-  k_end_step<<<1, 1, 0, s->stream>>>(s->dstate);
+  launch_early(s->early, k_end_step, 1, 1, 0, s->stream, s->dstate);
 }
 
 // A plain FP64 step of a small grid is 20 launches on two streams of ~10-30 us each, which the host
@@ -66,10 +66,12 @@ constexpr int kGraphSteps = 4;
 constexpr size_t kGraphCells = size_t(1) << 15;
 
 // (a stream that the caller is capturing takes the launches themselves)
-bool graphed(const hteno_solver* s) {
+bool capturing(const hteno_solver* s) {
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-  return s->cfg.precision == HTENO_PREC_FP64 && !s->fused64 && !s->timing && s->ncell <= kGraphCells &&
-         cudaStreamIsCapturing(s->stream, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s->stream, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
+}
+bool graphed(const hteno_solver* s) {
+  return s->cfg.precision == HTENO_PREC_FP64 && !s->fused64 && !s->timing && s->ncell <= kGraphCells && !capturing(s);
 }
 
 cudaError_t ensure_graph(hteno_solver* s, const Geo& G) {
@@ -104,7 +106,11 @@ int fv2d_step_async(hteno_solver* s, int nsteps) {
       if (el != cudaSuccess) return cuda_error(s, el, "fv2d graph launch");
     }
   }
+  // a mixed step is 5 kernels in one stream, each of which starts while the one before it ends (24 steps
+  // of 96 x 80 with the small tiles: 1.88 -> 1.18 ms)
+  s->early = s->cfg.precision == HTENO_PREC_MIXED && !s->timing && !capturing(s);
   for (; left > 0; --left) launch_step(s, G);
+  s->early = false;
   return cuda_error(s, cudaGetLastError(), "fv2d step launch");
 }
 

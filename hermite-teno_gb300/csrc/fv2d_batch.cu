@@ -52,8 +52,8 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_stage(const BInst* __restric
   static_assert(sizeof(Geo) % 4 == 0, "copied by words");
   for (int w = threadIdx.x; w < int(sizeof(Geo) / 4); w += NT)
     reinterpret_cast<uint32_t*>(&geo)[w] = reinterpret_cast<const uint32_t*>(&I.G)[w];
-  if (tma_ok) fused::tma_setup(S);
   __syncthreads();
+  fused::tile_setup(c_dev, geo, S, tma_ok);
   fused::StageArgs a;
   if (stage == 0) a = fused::StageArgs{I.q, nullptr, I.q2, nullptr};
   else if (stage == 1) a = fused::StageArgs{I.q, nullptr, I.q1, I.st};
@@ -429,7 +429,7 @@ int hteno_batch_set_state(hteno_batch* b, int i, const double* q, int where) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->dstate + i, &s, sizeof(StepState), cudaMemcpyHostToDevice, b->stream);
   if (e == cudaSuccess) {
-    k_inst_max_speed<<<unsigned(std::min<size_t>(8 * 152, (b->ncell[i] + 1023) / 1024)), 256, 0, b->stream>>>(b->dinst, i);
+    k_inst_max_speed<<<unsigned(std::min<size_t>(8 * 152, (b->ncell[i] + 255) / 256)), 256, 0, b->stream>>>(b->dinst, i);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

@@ -25,14 +25,16 @@ std::mutex g_mu;
 template <int TX, int TY, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_fused(Geo G, int stage, fused::StageArgs a,
                                                     const __grid_constant__ CUtensorMap tm, int has_tm) {
-  if (a.st && a.st->done) return;
+  grid_release();
   extern __shared__ __align__(128) unsigned char smem[];
   auto& S = *reinterpret_cast<fused::Smem<TX, TY>*>(smem);
   a.tmap = has_tm && (tc::smem_u32(&S.c[0][0]) & 127u) == 0 ? &tm : nullptr;
+  fused::tile_setup(c_dev, G, S, a.tmap != nullptr);
+  grid_wait();
+  if (a.st && a.st->done) return;
   // an audited step that runs (not past the stop time) counts once
   if (stage == 1 && a.audit && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
     atomicAdd(a.audit + 6, 1ull);
-  if (a.tmap) fused::tma_setup(S);
   int bad = 0;
   const double ms = fused::tile_stage<TX, TY, NT>(c_dev, G, blockIdx.x * TX, blockIdx.y * TY,
                                                   stage, a, S, bad);
@@ -42,8 +44,8 @@ __global__ void __launch_bounds__(NT, MINB) k_fused(Geo G, int stage, fused::Sta
   }
 }
 
-// Max wave speed of a state in double (timeStepping, FV_System2D.cpp:622-633): the first dt.  Four
-// cells a thread at least, so that the first, unfiltered ones are few of them.
+// Max wave speed of a state in double (timeStepping, FV_System2D.cpp:622-633): the first dt.  Up to
+// 8 blocks an SM: a thread's first, unfiltered cells are all there is of a small grid, few of a large one.
 __global__ void k_max_speed(Geo G, const double* __restrict__ q, StepState* st) {
   block_max_to(fused::grid_max_speed(G, q, &st->maxbits), &st->maxbits);
 }
@@ -80,17 +82,17 @@ struct Variant {
   int tx, ty, nt;
   size_t smem;
   const char* name;
-  void (*launch)(cudaStream_t, const Geo&, int, const fused::StageArgs&, const CUtensorMap*);
+  void (*launch)(cudaStream_t, bool early, const Geo&, int, const fused::StageArgs&, const CUtensorMap*);
   cudaError_t (*prepare)();
 };
 
 template <int TX, int TY, int NT, int MINB>
-void launch_v(cudaStream_t cs, const Geo& G, int stage, const fused::StageArgs& a, const CUtensorMap* tm) {
+void launch_v(cudaStream_t cs, bool early, const Geo& G, int stage, const fused::StageArgs& a, const CUtensorMap* tm) {
   const dim3 grid(unsigned((G.nx + TX - 1) / TX), unsigned((G.ny + TY - 1) / TY));
   CUtensorMap none;
   std::memset(&none, 0, sizeof(none));
-  k_fused<TX, TY, NT, MINB><<<grid, NT, fused::smem_bytes<TX, TY>(), cs>>>(G, stage, a, tm ? *tm : none,
-                                                                          tm ? 1 : 0);
+  launch_early(early, k_fused<TX, TY, NT, MINB>, grid, NT, fused::smem_bytes<TX, TY>(), cs, G, stage, a,
+               tm ? *tm : none, tm ? 1 : 0);
 }
 
 template <int TX, int TY, int NT, int MINB>
@@ -103,10 +105,14 @@ cudaError_t prepare_v() {
   { TX, TY, NT, fused::smem_bytes<TX, TY>(), "fused_" #TX "x" #TY "_" #NT "_b" #MINB,               \
     launch_v<TX, TY, NT, MINB>, prepare_v<TX, TY, NT, MINB> }
 
+// The last three are for grids that leave SMs idle: a tile is one serial chain of six phases, so less of
+// it per thread is faster although halos are computed more often (96 x 80, cold: 32 x 16 43 us, 16 x 8
+// with 128 threads 25, with 256 20, 8 x 8 18; 4096^2: 2.8, 4.9, 6.2, 6-9.5 ms).
 const Variant kVariants[] = {
     HTENO_VARIANT(32, 16, 256, 1), HTENO_VARIANT(32, 8, 256, 1),  HTENO_VARIANT(16, 16, 256, 1),
     HTENO_VARIANT(64, 8, 256, 1),  HTENO_VARIANT(32, 32, 512, 1), HTENO_VARIANT(16, 8, 128, 1),
-    HTENO_VARIANT(32, 16, 256, 3), HTENO_VARIANT(64, 8, 256, 3),
+    HTENO_VARIANT(32, 16, 256, 3), HTENO_VARIANT(64, 8, 256, 3),  HTENO_VARIANT(16, 8, 256, 1),
+    HTENO_VARIANT(8, 8, 128, 1),   HTENO_VARIANT(8, 8, 256, 1),
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
@@ -146,7 +152,7 @@ void launch_stage(hteno_solver* s, const Geo& G, int stage, const fused::StageAr
   const int kind = trace_kind(s, stage == 2 || stage == 3 ? "fused_s23" : "fused_s1", bytes,
                               (kFacesFlops + fluxf) * nf + kUpdateFlops * nc);
   trace_begin(s, kind);
-  V.launch(s->stream, G, stage, a, tm);
+  V.launch(s->stream, s->early, G, stage, a, tm);
   trace_end(s);
 }
 
@@ -194,7 +200,7 @@ int fv2d_fused_setup(hteno_solver* s) {
 int fv2d_fused_prepare(hteno_solver* s, const Geo& G, double* scratch) {
   s->router_steps = 0;  // a new state: the next step classifies (route masks are per state)
   if (s->audit) cudaMemsetAsync(s->audit, 0, 7 * sizeof(unsigned long long), s->stream);
-  k_max_speed<<<unsigned(std::min<size_t>(8 * 152, (s->ncell + 1023) / 1024)), 256, 0, s->stream>>>(G, s->q, s->dstate);
+  k_max_speed<<<unsigned(std::min<size_t>(8 * 152, (s->ncell + 255) / 256)), 256, 0, s->stream>>>(G, s->q, s->dstate);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(s, e, "max speed");
   if (s->tile_variant >= 0) return HTENO_OK;
@@ -206,9 +212,9 @@ int fv2d_fused_prepare(hteno_solver* s, const Geo& G, double* scratch) {
   int best = 0;
   float best_ms = 3.4e38f;
   for (int v = 0; v < kNumVariants; ++v) {
-    kVariants[v].launch(s->stream, G, 0, args, nullptr);  // warm
+    kVariants[v].launch(s->stream, false, G, 0, args, nullptr);  // warm
     cudaEventRecord(a, s->stream);
-    for (int r = 0; r < 3; ++r) kVariants[v].launch(s->stream, G, 0, args, nullptr);
+    for (int r = 0; r < 3; ++r) kVariants[v].launch(s->stream, false, G, 0, args, nullptr);
     cudaEventRecord(b, s->stream);
     e = cudaEventSynchronize(b);
     if (e != cudaSuccess) break;

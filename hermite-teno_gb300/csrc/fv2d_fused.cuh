@@ -54,6 +54,9 @@ struct Shape {
   static constexpr int YF = TY + 1, YC = TX + 4;  // y faces: rows 0..TY, columns -2..TX+1
   static constexpr int XN = XF * XR, YN = YF * YC;
   static constexpr int FN = XN > YN ? XN : YN;
+  // floats that the TMA box (Box) takes beyond c, fx, fy (8 x 8 tiles)
+  static constexpr int BOX = (TX + 8) * (TY + 6) * 8 - 8 * FN - 4 * TY * (TX + 1) - 4 * (TY + 1) * TX;
+  static constexpr int REST = BOX > 0 ? BOX : 1;
 };
 
 template <int TX, int TY>
@@ -64,6 +67,7 @@ struct Smem {
   alignas(128) float c[8][Shape<TX, TY>::FN];
   float fx[4][TY][TX + 1];
   float fy[4][TY + 1][TX];
+  float box_rest[Shape<TX, TY>::REST];
   float wtab[2][8][3];  // TENO weights per cut-off pattern, minus and plus side
   double rd[2];         // 1 / dx, 1 / dy
   alignas(8) uint64_t bar;  // completion of the TMA box
@@ -78,7 +82,7 @@ struct Box {
 };
 template <int TX, int TY>
 __device__ __forceinline__ double (*stage_box(Smem<TX, TY>& S))[Box<TX, TY>::Y][Box<TX, TY>::X] {
-  static_assert(Box<TX, TY>::kBytes <= sizeof(S.c) + sizeof(S.fx) + sizeof(S.fy), "TMA box fits");
+  static_assert(Box<TX, TY>::kBytes <= sizeof(S.c) + sizeof(S.fx) + sizeof(S.fy) + sizeof(S.box_rest), "TMA box fits");
   return reinterpret_cast<double (*)[Box<TX, TY>::Y][Box<TX, TY>::X]>(&S.c[0][0]);
 }
 // This thread's share of the largest wave speed of nc cells; the whole block calls it.
@@ -336,21 +340,30 @@ __device__ __forceinline__ bool tame_state(float r, float mx, float my, float e,
   return r >= lo && r <= hi && p >= lo && p <= hi && u * u + v * v <= 64.0f * (gamma * p * ir);
 }
 
-// The block's TMA mbarrier (S.bar), initialised once per launch before its tile when a
-// tensor map may be used.
+// What a block sets up before it reads the state: the weight tables, 1 / dx and 1 / dy, and (where a
+// tensor map may be used) the TMA mbarrier.  The whole block calls it; a barrier of the tile follows
+// before anything but thread 0's own box copy uses them (so that thread 0 need not wait for the tables).
 template <int TX, int TY>
-__device__ __forceinline__ void tma_setup(Smem<TX, TY>& S) {
-  if (threadIdx.x == 0) {
-    tc::mbar_init(&S.bar, 1);
-    tc::fence_mbar_init();
+__device__ __forceinline__ void tile_setup(const DevConst& C, const Geo& G, Smem<TX, TY>& S, bool tma) {
+  const int tid = threadIdx.x, e = tid - 64;
+  if (e >= 0 && e < 48) {
+    const int side = e / 24, pat = (e % 24) / 3, k = e % 3;
+    S.wtab[side][pat][k] = side ? C.f_wtab_p[pat][k] : C.f_wtab_m[pat][k];
   }
-  __syncthreads();
+  if (tid == 0) {
+    S.rd[0] = G.rdx;
+    S.rd[1] = G.rdy;
+    if (tma) {
+      tc::mbar_init(&S.bar, 1);
+      tc::fence_mbar_init();
+    }
+  }
 }
 
 // The tile at (i0, j0) of grid G.  Every thread of the block must call it (barriers inside).
 // Returns this thread's max wave speed over the cells it updated (stage 3) and ORs health flags
 // into *bad (bit 2: the tile's TMA copy did not complete within the bounded wait; the tile is
-// left unwritten).  One tile a block: the box copy's mbarrier (tma_setup ran) is in its first phase.
+// left unwritten).  One tile a block: the box copy's mbarrier (tile_setup ran) is in its first phase.
 template <int TX, int TY, int NT>
 __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, int i0, int j0,
                                              int stage, const StageArgs& a, Smem<TX, TY>& S,
@@ -365,14 +378,6 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
   const float g1 = float(G.g1);
   const int tid = threadIdx.x;
 
-  if (tid < 48) {
-    const int side = tid / 24, pat = (tid % 24) / 3, k = tid % 3;
-    S.wtab[side][pat][k] = side ? C.f_wtab_p[pat][k] : C.f_wtab_m[pat][k];
-  }
-  if (tid == 0) {
-    S.rd[0] = G.rdx;
-    S.rd[1] = G.rdy;
-  }
   // A: state and primitives of the tile and its halo (ghosts as the boundary routine fills them)
   const bool ghosts = G.bc >= HTENO_BC_TAYLOR;
   const double tm = a.st ? a.st->t : G.t0;
@@ -386,6 +391,7 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
       tc::mbar_arrive_expect_tx(&S.bar, Box<TX, TY>::kBytes);
       tc::tma_load_3d(&box[0][0][0], a.tmap, i0 - 4, j0 - 3, 0, &S.bar);
     }
+    __syncthreads();  // the mbarrier is set up
     // bounded wait; on giving up (never expected) the block flags the step, waits once more
     // for its copy in flight, and leaves this tile unwritten
     const bool late = __syncthreads_or(!tc::mbar_wait(&S.bar, 0u, kTmaWaitLimit));

@@ -11,6 +11,7 @@
 
 #include "../../include/hteno.h"
 #include "device_math.cuh"
+#include "launch.cuh"
 
 namespace hteno {
 
@@ -73,6 +74,7 @@ struct hteno_solver {
   hteno::StepState* hstate = nullptr;  // pinned host mirror
 
   int launches_per_step = 0;
+  bool early = false;     // mixed FV 2D: this run's steps use programmatic dependent launches
   int tile_variant = -1;  // mixed FV 2D: tile shape picked by the tuner (-1: not yet)
   // mixed FV 2D: TMA tensor maps (CUtensorMap, 128 bytes each) of the three stage inputs, made
   // for the tile shape tmap_variant; tma false (HTENO_TMA=0) loads every tile cell by cell

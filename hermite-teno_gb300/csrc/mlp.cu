@@ -24,6 +24,7 @@
 
 #include "fv2d_fused.cuh"
 #include "hteno_internal.h"
+#include "launch.cuh"
 #include "mlp_internal.cuh"
 
 struct hteno_mlp;
@@ -380,11 +381,6 @@ __device__ void setup(SM& S, const Weights& W) {
   __syncthreads();
   tc::fence_after();
 }
-
-// Programmatic dependent launch: wait for the previous kernel of the stream to complete (at once if
-// this one was launched without the attribute), and let the next one start its own set-up.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename SM>
 __device__ void teardown(SM& S, uint32_t tbase) {
@@ -973,23 +969,6 @@ void from_padded(const float* p, float* c) {
   for (int k = 0; k < 3; ++k) c[1376 + k] = p[kOffB3 + k];
 }
 
-// Launch with programmatic stream serialization: the kernel may start while the one before it in the
-// stream ends, and calls grid_wait before it touches what that one reads or writes.
-template <typename... P, typename... A>
-cudaError_t launch_early(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c = {};
-  c.gridDim = dim3(unsigned(grid));
-  c.blockDim = dim3(unsigned(block));
-  c.dynamicSmemBytes = smem;
-  c.stream = st;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, P(args)...);
-}
-
 int refresh_images(hteno_mlp* m) {
   k_images<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->P, m->W);
   return merr(m, cudaGetLastError(), "weight images");
@@ -1155,10 +1134,10 @@ int hteno_mlp_train(hteno_mlp* m, const uint16_t* x, const uint8_t* y, long n, i
       const long tiles = (nb + 127) / 128;
       const int grid = int(std::min<long>(tiles, 2L * m->sms));
       ++m->t;
-      cudaError_t e = launch_early(k_train, grid, 128, mlp::smem_bytes(), m->stream, m->W, x + off * 8, y + off, nb,
+      cudaError_t e = launch_early(true, k_train, grid, 128, mlp::smem_bytes(), m->stream, m->W, x + off * 8, y + off, nb,
                                    nb, m->Gp, m->Lp, m->err, m->wait_limit);
       if (e == cudaSuccess)
-        e = launch_early(k_adam, (kParams + 64) / 64, 64, 0, m->stream, m->Gp, m->Lp, grid, m->P, m->M, m->V,
+        e = launch_early(true, k_adam, (kParams + 64) / 64, 64, 0, m->stream, m->Gp, m->Lp, grid, m->P, m->M, m->V,
                          m->loss, m->W, lr, 0.9f, 0.999f, 1e-8f, m->t);
       if (e != cudaSuccess) return merr(m, e, "train launch");
     }
