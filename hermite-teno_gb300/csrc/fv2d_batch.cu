@@ -44,9 +44,9 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_stage(const BInst* __restric
   extern __shared__ __align__(128) unsigned char smem[];
   auto& S = *reinterpret_cast<fused::Smem<TX, TY>*>(smem);
   __shared__ Geo geo;
+  grid_release();
   const int4 job = jobs[blockIdx.x];
   const BInst& I = inst[job.x];
-  if (stage != 0 && I.st->done) return;  // uniform over the block
   // TMA box copies (tensor maps in the instance records, global memory): one mbarrier per block
   const bool tma_ok = stage != 0 && (tc::smem_u32(&S.c[0][0]) & 127u) == 0;
   static_assert(sizeof(Geo) % 4 == 0, "copied by words");
@@ -54,6 +54,8 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_stage(const BInst* __restric
     reinterpret_cast<uint32_t*>(&geo)[w] = reinterpret_cast<const uint32_t*>(&I.G)[w];
   __syncthreads();
   fused::tile_setup(c_dev, geo, S, tma_ok);
+  grid_wait();
+  if (stage != 0 && I.st->done) return;  // uniform over the block
   fused::StageArgs a;
   if (stage == 0) a = fused::StageArgs{I.q, nullptr, I.q2, nullptr};
   else if (stage == 1) a = fused::StageArgs{I.q, nullptr, I.q1, I.st};
@@ -70,6 +72,8 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_stage(const BInst* __restric
 }
 
 __global__ void k_batch_begin(StepState* st, int n) {
+  grid_release();
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   StepState* s = st + i;
@@ -86,6 +90,8 @@ __global__ void k_batch_begin(StepState* st, int n) {
 }
 
 __global__ void k_batch_end(StepState* st, int n) {
+  grid_release();
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || st[i].done) return;
   st[i].t += st[i].dt;
@@ -115,7 +121,7 @@ struct BVariant {
 
 template <int TX, int TY, int NT, int MINB>
 void blaunch(cudaStream_t cs, int njobs, const BInst* inst, const int4* jobs, int stage) {
-  k_batch_stage<TX, TY, NT, MINB><<<njobs, NT, fused::smem_bytes<TX, TY>(), cs>>>(inst, jobs, stage);
+  launch_early(stage != 0, k_batch_stage<TX, TY, NT, MINB>, njobs, NT, fused::smem_bytes<TX, TY>(), cs, inst, jobs, stage);
 }
 
 template <int TX, int TY, int NT, int MINB>
@@ -192,10 +198,10 @@ int bcuda(hteno_batch* b, cudaError_t e, const char* what) {
 void launch_step(hteno_batch* b, cudaStream_t cs) {
   const int v = b->variant;
   const unsigned nb = unsigned((b->n + 127) / 128);
-  k_batch_begin<<<nb, 128, 0, cs>>>(b->dstate, b->n);
+  launch_early(true, k_batch_begin, nb, 128, 0, cs, b->dstate, b->n);
   for (int stage = 1; stage <= 3; ++stage)
     kBVariants[v].launch(cs, b->njobs[v], b->dinst, b->jobs[v], stage);
-  k_batch_end<<<nb, 128, 0, cs>>>(b->dstate, b->n);
+  launch_early(true, k_batch_end, nb, 128, 0, cs, b->dstate, b->n);
 }
 
 // Tile-shape tuner: each candidate evaluates the residual of every instance (into the stage-2
