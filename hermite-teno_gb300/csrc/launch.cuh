@@ -13,6 +13,14 @@ namespace hteno {
 // was launched without the attribute).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A pointer that the compiler knows only from here on.  Loads through const __restrict__ parameters count
+// as loads of constants and might move above grid_wait: kernels launched early pass such parameters
+// through this after it.
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 
 // kernel<<<grid, block, smem, st>>>(args...), early or (a stream under capture, timed launches) not.
 template <typename... P, typename... A>

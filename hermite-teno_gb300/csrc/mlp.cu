@@ -862,6 +862,8 @@ __global__ void __launch_bounds__(64) k_adam(const float* __restrict__ Gp, const
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   grid_wait();
   grid_release();
+  Gp = after_wait(Gp);
+  Lp = after_wait(Lp);
   if (i == kParams) *loss += ordered_sum(Lp, 1, nblk);
   if (i >= kParams) return;
   const float m0 = M[i], v0 = V[i], p0 = P[i];
