@@ -105,14 +105,16 @@ cudaError_t prepare_v() {
   { TX, TY, NT, fused::smem_bytes<TX, TY>(), "fused_" #TX "x" #TY "_" #NT "_b" #MINB,               \
     launch_v<TX, TY, NT, MINB>, prepare_v<TX, TY, NT, MINB> }
 
-// The last three are for grids that leave SMs idle: a tile is one serial chain of six phases, so less of
+// 32 x 15: 528 and 544 flux faces of a 32 x 16 tile take 256 threads three rounds, the last nearly empty;
+// 495 and 512 take two (1024^2 172.7 -> 166.4 us a stage; 24 x 20 the same, 30 x 16 170.6, 288 threads 177.8).
+// The three before it are for grids that leave SMs idle: a tile is one serial chain of six phases, so less of
 // it per thread is faster although halos are computed more often (96 x 80, cold: 32 x 16 43 us, 16 x 8
 // with 128 threads 25, with 256 20, 8 x 8 18; 4096^2: 2.8, 4.9, 6.2, 6-9.5 ms).
 const Variant kVariants[] = {
     HTENO_VARIANT(32, 16, 256, 1), HTENO_VARIANT(32, 8, 256, 1),  HTENO_VARIANT(16, 16, 256, 1),
     HTENO_VARIANT(64, 8, 256, 1),  HTENO_VARIANT(32, 32, 512, 1), HTENO_VARIANT(16, 8, 128, 1),
     HTENO_VARIANT(32, 16, 256, 3), HTENO_VARIANT(64, 8, 256, 3),  HTENO_VARIANT(16, 8, 256, 1),
-    HTENO_VARIANT(8, 8, 128, 1),   HTENO_VARIANT(8, 8, 256, 1),
+    HTENO_VARIANT(8, 8, 128, 1),   HTENO_VARIANT(8, 8, 256, 1),   HTENO_VARIANT(32, 15, 256, 3),
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 

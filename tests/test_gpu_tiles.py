@@ -28,10 +28,10 @@ def test_small_tiles_same_bits(hteno_lib, cuda, nx, ny, bc, flux, recon):
 
     q = ic.four_quadrant(nx, ny, 11)
     want, t, _ = run(hteno_lib, q, 0, 6, bc=bc, flux=flux, recon=recon)
-    for tile in (8, 9, 10):
+    for tile in (8, 9, 10, 11):
         got, tg, tma = run(hteno_lib, q, tile, 6, bc=bc, flux=flux, recon=recon)
         np.testing.assert_array_equal(got, want)
-        assert tg == t and (tma > 0) == ((nx, ny) == (96, 80))
+        assert tg == t and (tma > 0) == ((nx, ny) == (96, 80))  # (an interior tile, nx even)
 
 
 def test_captured_steps(hteno_lib, cuda):
