@@ -465,15 +465,6 @@ __device__ __forceinline__ T max_speed2(T g, const T* w, int dir) {
   return fmax(w[dir] - c, fabs(w[dir] + c));
 }
 
-// Schemes::SSPRK::RungeKuttaIII (Schemes_SSPRK.cpp:3-15), always in double and without
-// contraction, so the stage combination rounds exactly like the reference.
-__device__ __forceinline__ double ssprk3(double q0, double qn, double rhs, double dt, int stage) {
-  if (stage == 1) return __dadd_rn(q0, __dmul_rn(dt, rhs));
-  if (stage == 2)
-    return __dadd_rn(__dmul_rn(0.75, q0), __dmul_rn(0.25, __dadd_rn(qn, __dmul_rn(rhs, dt))));
-  return __ddiv_rn(__dadd_rn(q0, __dmul_rn(2.0, __dadd_rn(qn, __dmul_rn(dt, rhs)))), 3.0);
-}
-
 // ---------------------------------------------------------------------------------------------
 // Equations::Euler1D (3 conserved variables)
 // ---------------------------------------------------------------------------------------------

@@ -151,9 +151,5 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void st_bf16(unsigned char* base, uint32_t off, float v) {
-  *reinterpret_cast<__nv_bfloat16*>(base + off) = __float2bfloat16_rn(v);
-}
-
 }  // namespace tc
 }  // namespace hteno
