@@ -809,7 +809,8 @@ __global__ void __launch_bounds__(128, 4) k_route_rows(Weights W, const uint4* _
   teardown(S, tbase);
 }
 
-// The sum of p[b * stride], b < n, added in order of b, 32 loads in flight.
+// The sum of p[b * stride], b < n, added in order of b, 32 loads in flight.  (Two training epochs of 1e6
+// rows: 2.18 ms; with 16 in flight 2.26; with 128 2.80, the longer code being fetched cold at each launch.)
 __device__ __forceinline__ float ordered_sum(const float* p, size_t stride, int n) {
   float s = 0.f;
   for (int b = 0; b < n; b += 32) {
