@@ -267,7 +267,7 @@ def batch_path(hteno, torch, stream, steps, world):
     return {"value": cells * steps * world / (ms / 1e3) / 1e6, "unit": UNIT, "ms_per_step": ms / steps,
             "instances": len(cfgs), "cells": cells, "steps": steps, "tile": list(tile),
             "min_steps_done": min(done), "unhealthy_instances": int(sum(1 for s in status if s)),
-            "note": "one persistent launch per RK stage over all instances' tiles, a step replayed "
+            "note": "one launch per RK stage over all instances' tiles, a step replayed "
                     "as one CUDA graph; FP32 reconstruction/fluxes, FP64 state; "
                     "unhealthy_instances: grids whose state reached a non-positive density or "
                     "pressure in some RK stage, which the plain FP64 solver (the reference's "
