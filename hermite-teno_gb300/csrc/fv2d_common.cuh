@@ -27,9 +27,9 @@ struct Geo {
 // state of interior cell (0, 6) where x < 1/6 + tan(pi/6) (y_top + (1 + m) dy + 20 t), of cell
 // (nx - 7, 6) elsewhere (m = j - ny); the x ghosts of every row copy its first / last column.
 // Positions are computed with explicitly rounded operations, as the reference's expressions
-// round them, in any translation unit.
-__device__ __forceinline__ void bc_state(const Geo& G, const double* __restrict__ q, int i, int j,
-                                         double t, double* out) {
+// round them, in any translation unit.  (q is not __restrict__: kernels launched early read what the
+// kernel before them writes.)
+__device__ __forceinline__ void bc_state(const Geo& G, const double* q, int i, int j, double t, double* out) {
   const size_t nc = size_t(G.nx) * G.ny;
   auto ld = [&](int ii, int jj) {
     const size_t k = size_t(jj) * G.nx + ii;

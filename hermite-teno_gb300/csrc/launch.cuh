@@ -13,9 +13,11 @@ namespace hteno {
 // was launched without the attribute).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// A pointer that the compiler knows only from here on.  Loads through const __restrict__ parameters count
-// as loads of constants and might move above grid_wait: kernels launched early pass such parameters
-// through this after it.
+// A pointer that the compiler knows only from here on.  A load through a const __restrict__ parameter or
+// by __ldg counts as one of memory that nobody writes while the kernel lives: it may take the path that is
+// not kept coherent, and a load through any __restrict__ parameter may move above grid_wait.  A kernel
+// launched early reads what an earlier kernel writes by plain loads only, through pointers that pass this
+// after grid_wait.
 template <typename T>
 __device__ __forceinline__ T* after_wait(T* p) {
   asm volatile("" : "+l"(p)::"memory");

@@ -876,6 +876,10 @@ __global__ void __launch_bounds__(64) k_adam(const float* __restrict__ Gp, const
   grid_release();
   Gp = after_wait(Gp);
   Lp = after_wait(Lp);
+  P = after_wait(P);
+  M = after_wait(M);
+  V = after_wait(V);
+  loss = after_wait(loss);
   if (i == kParams) *loss += ordered_sum(Lp, 1, nblk);
   if (i >= kParams) return;
   const float m0 = M[i], v0 = V[i], p0 = P[i];
