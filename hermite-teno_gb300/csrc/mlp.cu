@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(128) k_train(Weights W, const uint16_t* __rest
     raw = valid ? *reinterpret_cast<const uint4*>(X + r * 8) : make_uint4(0u, 0u, 0u, 0u);
     y = valid ? Y[r] : 0u;
   };
-  fetch(blockIdx.x);  // (the rows are not written by the kernel before this one, the weights are)
+  fetch(blockIdx.x);  // before the wait: launched early only behind k_adam, which writes the weights but no rows
   grid_wait();
   grid_release();
   load_weights(S, W);
@@ -1152,7 +1152,9 @@ int hteno_mlp_train(hteno_mlp* m, const uint16_t* x, const uint8_t* y, long n, i
       const long tiles = (nb + 127) / 128;
       const int grid = int(std::min<long>(tiles, 2L * m->sms));
       ++m->t;
-      cudaError_t e = launch_early(true, k_train, grid, 128, mlp::smem_bytes(), m->stream, m->W, x + off * 8, y + off, nb,
+      // an epoch's first batch waits for whatever is before it: k_train reads rows before its grid_wait,
+      // and the kernel before it may be the one that wrote them; the later batches follow k_adam
+      cudaError_t e = launch_early(off > 0, k_train, grid, 128, mlp::smem_bytes(), m->stream, m->W, x + off * 8, y + off, nb,
                                    nb, m->Gp, m->Lp, m->err, m->wait_limit);
       if (e == cudaSuccess)
         e = launch_early(true, k_adam, (kParams + 64) / 64, 64, 0, m->stream, m->Gp, m->Lp, grid, m->P, m->M, m->V,

@@ -76,3 +76,14 @@ def test_early_stage_reads_its_state_after_the_wait():
     ghost = src["fv2d_common.cuh"]
     head = ghost[ghost.index("void bc_state("):]
     assert "__restrict__" not in head[:head.index("{")]
+
+
+def test_train_reads_the_callers_rows_only_behind_a_full_dependency():
+    """k_train fetches its first rows before grid_wait.  The kernel before an epoch's first batch may be
+    the caller's that wrote them, so that batch is not launched early; the later ones follow k_adam,
+    which does not write rows."""
+    text = sources()["mlp.cu"]
+    early = re.findall(r"launch_early\(\s*([^,]+),\s*k_train\b", text)
+    assert early == ["off > 0"]
+    _, body = kernel({"mlp.cu": text}, "k_adam")
+    assert not re.search(r"\b[XY]\b", body)
