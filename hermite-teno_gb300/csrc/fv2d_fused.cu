@@ -7,6 +7,7 @@
 #include <cstring>
 
 #include "fv2d_fused.cuh"
+#include "tile_rule.h"
 
 namespace hteno {
 namespace {
@@ -110,7 +111,8 @@ cudaError_t prepare_v() {
 // 495 and 512 take two (1024^2 172.7 -> 166.4 us a stage; 24 x 20 the same, 30 x 16 170.6, 288 threads 177.8).
 // The three before it are for grids that leave SMs idle: a tile is one serial chain of six phases, so less of
 // it per thread is faster although halos are computed more often (96 x 80, cold: 32 x 16 43 us, 16 x 8
-// with 128 threads 25, with 256 20, 8 x 8 18; 4096^2: 2.8, 4.9, 6.2, 6-9.5 ms).
+// with 128 threads 25, with 256 20, 8 x 8 18; 4096^2: 2.8, 4.9, 6.2, 6-9.5 ms).  tile_rule.h says which are
+// timed for a grid.
 const Variant kVariants[] = {
     HTENO_VARIANT(32, 16, 256, 1), HTENO_VARIANT(32, 8, 256, 1),  HTENO_VARIANT(16, 16, 256, 1),
     HTENO_VARIANT(64, 8, 256, 1),  HTENO_VARIANT(32, 32, 512, 1), HTENO_VARIANT(16, 8, 128, 1),
@@ -212,18 +214,31 @@ int fv2d_fused_prepare(hteno_solver* s, const Geo& G, double* scratch) {
     return set_error(s, HTENO_ERR_CUDA, "tuner events");
   fused::StageArgs args{s->q, nullptr, scratch, nullptr};
   args.skip_uniform = false;  // time the full work, not the (mostly uniform) initial state
-  int best = 0;
-  float best_ms = 3.4e38f;
-  for (int v = 0; v < kNumVariants; ++v) {
-    kVariants[v].launch(s->stream, false, G, 0, args, nullptr);  // warm
+  int best = 0, sms = 0, list[kNumVariants];
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+  const long tiles = long((G.nx + 31) / 32) * ((G.ny + 15) / 16);
+  const int candidates = tile_candidates(tiles, sms, list);
+  float best_ms = 3.4e38f;  // per launch
+  // device time of n launches of variant v; negative after an error
+  auto timed = [&](int v, int n) {
     cudaEventRecord(a, s->stream);
-    for (int r = 0; r < 3; ++r) kVariants[v].launch(s->stream, false, G, 0, args, nullptr);
+    for (int r = 0; r < n; ++r) kVariants[v].launch(s->stream, false, G, 0, args, nullptr);
     cudaEventRecord(b, s->stream);
+    float ms = -1.f;
     e = cudaEventSynchronize(b);
-    if (e != cudaSuccess) break;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, a, b);
-    if (ms < best_ms) {
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
+    return ms;
+  };
+  for (int k = 0; k < candidates && e == cudaSuccess; ++k) {
+    const int v = list[k];
+    if (tiles > sms) {
+      const float first = timed(v, 1);
+      if (e != cudaSuccess || (k > 0 && tile_dropped(tiles, sms, first, best_ms))) continue;
+    } else {
+      kVariants[v].launch(s->stream, false, G, 0, args, nullptr);  // warm
+    }
+    const float ms = timed(v, 3) / 3.f;
+    if (e == cudaSuccess && ms < best_ms) {
       best_ms = ms;
       best = v;
     }

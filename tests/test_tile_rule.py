@@ -1,0 +1,76 @@
+"""Which tile shapes a new mixed FV 2D solver times (tile_rule.h), and what that costs it."""
+from __future__ import annotations
+
+import os
+import subprocess
+import time
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "hermite-teno_gb300" / "csrc"
+SMALL, BIG = {8, 9, 10}, {3, 4, 6, 7, 11}  # a chain per idle SM; three blocks an SM or more than 512 cells
+
+
+def test_candidates(tmp_path):
+    src = tmp_path / "rule.cpp"
+    src.write_text('#include <cstdio>\n#include <initializer_list>\n#include "tile_rule.h"\nint main() {\n'
+                   "  for (long t : {1l, 15l, 101l, 102l, 152l, 153l, 304l, 305l, 32768l}) {\n"
+                   "    int v[12];\n    const int n = hteno::tile_candidates(t, 152, v);\n"
+                   '    std::printf("%ld:", t);\n'
+                   '    for (int k = 0; k < n; ++k) std::printf(" %d", v[k]);\n'
+                   '    std::printf("\\n");\n  }\n}\n')
+    exe = tmp_path / "rule"
+    subprocess.run(["g++", "-std=c++17", "-I", str(CSRC), str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+    lists = {int(k): [int(x) for x in v.split()] for k, v in (ln.split(":") for ln in out.splitlines())}
+    for tiles, c in lists.items():
+        assert len(set(c)) == len(c) <= 9 and set(c) <= set(range(12))
+        assert bool(SMALL & set(c)) == (3 * tiles <= 2 * 152)
+        assert bool(BIG & set(c)) == (tiles > 152)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [256, 1024, 2048])
+def test_choosing_a_tile_costs_few_stages(hteno_lib, cuda, n):
+    """A new solver's first state beyond what it costs with a given shape, in stages of the shape chosen.
+    With eight shapes timed at every size this was 41 to 46 stages, with all twelve 69 to 72; the lists
+    of the rule come to 19 to 28."""
+    h = hteno_lib
+    from hteno import ic
+
+    q = cuda.from_numpy(ic.four_quadrant(n, n, 3)).cuda()
+    cfg = h.config(dims=2, nx=n, ny=n, precision=h.PREC_MIXED, flux=1)
+
+    def first_state(tile):
+        if tile:
+            os.environ["HTENO_FV2D_TILE"] = tile
+        try:
+            ts = []
+            for _ in range(7):
+                cuda.cuda.synchronize()
+                t0 = time.perf_counter()
+                with h.Solver(cfg) as s:
+                    s.set_state(q)
+                    t1 = time.perf_counter()
+                ts.append(t1 - t0)
+            return sorted(ts)[3]
+        finally:
+            os.environ.pop("HTENO_FV2D_TILE", None)
+
+    first_state("0")  # the first solver of the process
+    cost = first_state("") - first_state("0")
+    os.environ["HTENO_UNIFORM_SKIP"] = "0"  # as the timed stages: full work in constant regions too
+    try:
+        with h.Solver(cfg) as s:
+            s.set_state(q)
+            s.step(10)
+            ts = []
+            for _ in range(5):
+                t0 = time.perf_counter()
+                s.step_async(20)
+                s.sync()
+                ts.append((time.perf_counter() - t0) / 60)
+    finally:
+        os.environ.pop("HTENO_UNIFORM_SKIP")
+    assert cost <= 40 * sorted(ts)[2], (cost, sorted(ts)[2])
