@@ -63,7 +63,6 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_stage(const BInst* __restric
   else a = fused::StageArgs{I.q2, I.q, I.q, I.st};
   a.skip_uniform = stage != 0;  // stage 0 only times tile shapes: the full work
   a.tmap = tma_ok && I.has_tm ? &I.tm[stage - 1] : nullptr;
-  a.after_wait();
   int bad = 0;
   const double ms = fused::tile_stage<TX, TY, NT>(c_dev, geo, job.y, job.z, stage, a, S, bad);
   if (stage == 3) {

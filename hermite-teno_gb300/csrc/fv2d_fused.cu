@@ -32,7 +32,6 @@ __global__ void __launch_bounds__(NT, MINB) k_fused(Geo G, int stage, fused::Sta
   a.tmap = has_tm && (tc::smem_u32(&S.c[0][0]) & 127u) == 0 ? &tm : nullptr;
   fused::tile_setup(c_dev, G, S, a.tmap != nullptr);
   grid_wait();
-  a.after_wait();
   if (a.st && a.st->done) return;
   // an audited step that runs (not past the stop time) counts once
   if (stage == 1 && a.audit && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)

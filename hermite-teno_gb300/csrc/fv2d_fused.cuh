@@ -326,14 +326,6 @@ struct StageArgs {
   // tensor map of qin ([4][ny][nx] doubles, box Box<TX, TY>) for TMA staging of interior tiles;
   // null: every tile loads cell by cell
   const CUtensorMap* tmap = nullptr;
-
-  // What kernels before this one write, as pointers known from here on (launch.cuh: after grid_wait).
-  __device__ __forceinline__ void after_wait() {
-    qin = hteno::after_wait(qin);
-    qbase = hteno::after_wait(qbase);
-    mx = hteno::after_wait(mx);
-    my = hteno::after_wait(my);
-  }
 };
 
 // A float state whose fluxes stay finite through the characteristic round trip: density and
@@ -441,10 +433,10 @@ __device__ __forceinline__ double tile_stage(const DevConst& C, const Geo& G, in
     } else {
       const int gi = cmap(i0 - 3 + x, G.nx, G.bc), gj = cmap(j0 - 3 + y, G.ny, G.bc);
       const size_t k = size_t(gj) * G.nx + gi;
-      r = d2f(a.qin[k]);
-      mx = d2f(a.qin[nc + k]);
-      my = d2f(a.qin[2 * nc + k]);
-      e = d2f(a.qin[3 * nc + k]);
+      r = d2f(load_behind(a.qin + k));
+      mx = d2f(load_behind(a.qin + nc + k));
+      my = d2f(load_behind(a.qin + 2 * nc + k));
+      e = d2f(load_behind(a.qin + 3 * nc + k));
     }
     S.q[0][y][x] = r;
     S.q[1][y][x] = mx;
