@@ -218,10 +218,12 @@ int fv2d_fused_prepare(hteno_solver* s, const Geo& G, double* scratch) {
   const long tiles = long((G.nx + 31) / 32) * ((G.ny + 15) / 16);
   const int candidates = tile_candidates(tiles, sms, list);
   float best_ms = 3.4e38f;  // per launch
-  // device time of n launches of variant v; negative after an error
+  // device time of n launches of variant v; negative after an error.  Launched early, as the steps are:
+  // the waiting blocks of the next launch take part of each SM, which costs shapes with several blocks an
+  // SM most (384 x 336, timed by plain launches: shape 11, 1085 us per six steps; shape 4 takes 918).
   auto timed = [&](int v, int n) {
     cudaEventRecord(a, s->stream);
-    for (int r = 0; r < n; ++r) kVariants[v].launch(s->stream, false, G, 0, args, nullptr);
+    for (int r = 0; r < n; ++r) kVariants[v].launch(s->stream, true, G, 0, args, nullptr);
     cudaEventRecord(b, s->stream);
     float ms = -1.f;
     e = cudaEventSynchronize(b);
