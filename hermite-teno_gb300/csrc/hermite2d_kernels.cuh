@@ -9,6 +9,7 @@
 
 #include "hermite_limit.cuh"
 #include "hteno_internal.h"
+#include "limit_rule.h"
 #include "mixed_pairs.cuh"
 
 namespace hteno {
@@ -215,8 +216,8 @@ constexpr int kLimC = 16, kLimWarm = 24;
 template <typename T, bool kStaged>
 __global__ void __launch_bounds__(256) kh_limit(GeoH G, HermiteK<T> K, const T* __restrict__ q,
                                                 const double* __restrict__ v, const double* __restrict__ w,
-                                                T* __restrict__ vt, T* __restrict__ wt, int lines, int nbx,
-                                                const StepState* st) {
+                                                T* __restrict__ vt, T* __restrict__ wt, int lines, int segx, int segy,
+                                                int nbx, const StepState* st) {
   if (st->done) return;
   __shared__ T last[256];  // the limited value of each segment's last cell
   const bool xd = int(blockIdx.x) < nbx;
@@ -224,10 +225,10 @@ __global__ void __launch_bounds__(256) kh_limit(GeoH G, HermiteK<T> K, const T* 
   const int nl = xd ? G.ny : G.nx;  // number of lines
   const int n = xd ? G.nx : G.ny;   // length of a line
   const int nlb = (nl + lines - 1) / lines;
-  const int e = b / nlb, seg = threadIdx.x / lines, segs = blockDim.x / lines;
+  const int e = b / nlb, seg = threadIdx.x / lines, segs = xd ? segx : segy;
   const int l0 = (b - e * nlb) * lines, line = l0 + int(threadIdx.x) - seg * lines;
   const int len = (n + segs - 1) / segs, c0 = min(n, seg * len), c1 = min(n, c0 + len);
-  const bool live = line < nl && c0 < c1;
+  const bool live = line < nl && c0 < c1;  // (no thread of a segment past the direction's number)
   const size_t field = size_t(e) * G.nx * G.ny;
   const size_t base = field + (xd ? size_t(line) * G.nx : size_t(line));
   const size_t step = xd ? 1 : size_t(G.nx);
@@ -691,28 +692,19 @@ GeoH geo_of(const hteno_solver* s) {
   return G;
 }
 
-// The limiter's launch: lines per block and segments per line.  32 lines x 8 segments (coalesced)
-// while that gives the chip's 608 sub-partitions two warps each or more; else 16 lines x 8 segments: a
-// small grid is bound by the length of a chain, and twice the blocks, of one warp per sub-partition,
-// put its warps on more of the chip.  Segments have at least 16 cells, about what a repeated sweep takes to agree.
-// Measured at 2048^2 in float 0.55 -> 0.27 ms a launch (one warp per line group before, its block's
-// three other warps staging the lines), at 300 x 211 in double 2.42 -> 0.43 ms.
+// The limiter's launch (limit_rule.h).
 template <typename T>
 void launch_limit(hteno_solver* s, const GeoH& G, const HermiteK<T>& K, const WorkH<T>& W) {
-  const int nx = G.nx, ny = G.ny;
-  auto blocks = [&](int nl, int lines) { return 4 * ((nl + lines - 1) / lines); };
-  const bool wide = (blocks(nx, 32) + blocks(ny, 32)) * 8 >= 2 * 608;
-  const int lines = wide ? 32 : 16;
-  const int segs = std::max(2, std::min(8, std::min(nx, ny) / 32 * 2));
-  const int nbx = blocks(ny, lines), nby = blocks(nx, lines);
-  const unsigned threads = unsigned(lines * segs);  // whole warps
+  const LimitShape L = limit_shape(G.nx, G.ny);
+  const int nbx = 4 * ((G.ny + L.lines - 1) / L.lines), nby = 4 * ((G.nx + L.lines - 1) / L.lines);
+  const unsigned threads = unsigned(L.lines * std::max(L.segx, L.segy));  // whole warps
   constexpr bool staged = std::is_same<T, float>::value;
-  if (wide && staged)
-    kh_limit<T, staged><<<unsigned(nbx + nby), threads, 0, s->stream>>>(G, K, W.qt, s->v, s->w, W.vt, W.wt, lines,
-                                                                       nbx, s->dstate);
+  if (L.wide && staged)
+    kh_limit<T, staged><<<unsigned(nbx + nby), threads, 0, s->stream>>>(G, K, W.qt, s->v, s->w, W.vt, W.wt, L.lines,
+                                                                       L.segx, L.segy, nbx, s->dstate);
   else
-    kh_limit<T, false><<<unsigned(nbx + nby), threads, 0, s->stream>>>(G, K, W.qt, s->v, s->w, W.vt, W.wt, lines,
-                                                                      nbx, s->dstate);
+    kh_limit<T, false><<<unsigned(nbx + nby), threads, 0, s->stream>>>(G, K, W.qt, s->v, s->w, W.vt, W.wt, L.lines,
+                                                                      L.segx, L.segy, nbx, s->dstate);
 }
 
 template <typename T>
