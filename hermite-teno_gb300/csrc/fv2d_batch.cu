@@ -11,6 +11,7 @@
 #include <new>
 
 #include "fv2d_fused.cuh"
+#include "speed_rule.h"
 
 struct hteno_batch;
 
@@ -106,9 +107,9 @@ __global__ void k_batch_set_target(StepState* st, int n, double t_final) {
 }
 
 // Max wave speed of one instance's state (the first dt after set_state), double.
-__global__ void k_inst_max_speed(const BInst* __restrict__ inst, int i) {
+__global__ void k_inst_max_speed(const BInst* __restrict__ inst, int i, bool filter) {
   const BInst& I = inst[i];
-  block_max_to(fused::grid_max_speed(I.G, I.q, &I.st->maxbits), &I.st->maxbits);
+  block_max_to(fused::grid_max_speed(I.G, I.q, &I.st->maxbits, filter), &I.st->maxbits);
 }
 
 struct BVariant {
@@ -435,7 +436,8 @@ int hteno_batch_set_state(hteno_batch* b, int i, const double* q, int where) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->dstate + i, &s, sizeof(StepState), cudaMemcpyHostToDevice, b->stream);
   if (e == cudaSuccess) {
-    k_inst_max_speed<<<unsigned(std::min<size_t>(8 * 152, (b->ncell[i] + 255) / 256)), 256, 0, b->stream>>>(b->dinst, i);
+    const SpeedLaunch l = speed_launch(b->ncell[i], false);
+    k_inst_max_speed<<<l.blocks, 256, 0, b->stream>>>(b->dinst, i, l.filter);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

@@ -7,6 +7,7 @@
 #include <cstring>
 
 #include "fv2d_fused.cuh"
+#include "speed_rule.h"
 #include "tile_rule.h"
 
 namespace hteno {
@@ -45,10 +46,9 @@ __global__ void __launch_bounds__(NT, MINB) k_fused(Geo G, int stage, fused::Sta
   }
 }
 
-// Max wave speed of a state in double (timeStepping, FV_System2D.cpp:622-633): the first dt.  Up to
-// 8 blocks an SM: a thread's first, unfiltered cells are all there is of a small grid, few of a large one.
-__global__ void k_max_speed(Geo G, const double* __restrict__ q, StepState* st) {
-  block_max_to(fused::grid_max_speed(G, q, &st->maxbits), &st->maxbits);
+// Max wave speed of a state in double (timeStepping, FV_System2D.cpp:622-633): the first dt.
+__global__ void k_max_speed(Geo G, const double* __restrict__ q, StepState* st, bool filter) {
+  block_max_to(fused::grid_max_speed(G, q, &st->maxbits, filter), &st->maxbits);
 }
 
 // Erosion of a route mask [rows][cols] along one axis: a bit stays set only where it is set on
@@ -204,7 +204,8 @@ int fv2d_fused_setup(hteno_solver* s) {
 int fv2d_fused_prepare(hteno_solver* s, const Geo& G, double* scratch) {
   s->router_steps = 0;  // a new state: the next step classifies (route masks are per state)
   if (s->audit) cudaMemsetAsync(s->audit, 0, 7 * sizeof(unsigned long long), s->stream);
-  k_max_speed<<<unsigned(std::min<size_t>(8 * 152, (s->ncell + 255) / 256)), 256, 0, s->stream>>>(G, s->q, s->dstate);
+  const SpeedLaunch l = speed_launch(s->ncell, false);
+  k_max_speed<<<l.blocks, 256, 0, s->stream>>>(G, s->q, s->dstate, l.filter);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(s, e, "max speed");
   if (s->tile_variant >= 0) return HTENO_OK;

@@ -85,19 +85,30 @@ __device__ __forceinline__ double (*stage_box(Smem<TX, TY>& S))[Box<TX, TY>::Y][
   static_assert(Box<TX, TY>::kBytes <= sizeof(S.c) + sizeof(S.fx) + sizeof(S.fy) + sizeof(S.box_rest), "TMA box fits");
   return reinterpret_cast<double (*)[Box<TX, TY>::Y][Box<TX, TY>::X]>(&S.c[0][0]);
 }
-// This thread's share of the largest wave speed of nc cells; the whole block calls it.
-__device__ __forceinline__ double grid_max_speed(const Geo& G, const double* __restrict__ q, unsigned long long* bits) {
+// This thread's share of the largest wave speed of the grid's cells, every cell evaluated or (filter) only
+// those that may be the fastest; the whole block calls it (speed_rule.h).
+__device__ __forceinline__ double grid_max_speed(const Geo& G, const double* __restrict__ q, unsigned long long* bits,
+                                                 bool filter) {
   __shared__ unsigned found;
   const size_t nc = size_t(G.nx) * G.ny;
+  auto speed = [&](const double* c) {
+    const double u = c[1] / c[0], v = c[2] / c[0];
+    const double p = (c[3] - 0.5 * (c[1] * u + c[2] * v)) * G.g1;
+    const double a = sqrt(fabs(G.gamma * p / c[0]));
+    return fmax(fmax(u - a, fabs(u + a)), fmax(v - a, fabs(v + a)));
+  };
+  if (!filter) {  // a cell a thread
+    const size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    if (k >= nc) return 0.0;
+    const double c[4] = {q[k], q[nc + k], q[2 * nc + k], q[3 * nc + k]};
+    return fmax(0.0, speed(c));
+  }
   mix::SpeedFilter F(&found, bits, G.g1, G.gamma, nc);
   double ms = 0.0;
   for (size_t k = F.k; k < F.end; k += blockDim.x) {
     const double c[4] = {q[k], q[nc + k], q[2 * nc + k], q[3 * nc + k]};
     if (!F.may_exceed(c)) continue;
-    const double u = c[1] / c[0], v = c[2] / c[0];
-    const double p = (c[3] - 0.5 * (c[1] * u + c[2] * v)) * G.g1;
-    const double a = sqrt(fabs(G.gamma * p / c[0]));
-    const double m = fmax(fmax(u - a, fabs(u + a)), fmax(v - a, fabs(v + a)));
+    const double m = speed(c);
     ms = fmax(ms, m);
     F.add(c, m);
   }

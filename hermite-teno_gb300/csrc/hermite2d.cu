@@ -12,6 +12,7 @@
 //                       the unlimited stage values, which v, w keep: the limited ones go to vt, wt.
 // Boundaries are zero-gradient (the reference's Hermite 2D rhs).  T = double or float.
 #include "hermite2d_kernels.cuh"
+#include "speed_rule.h"
 
 namespace hteno {
 
@@ -38,7 +39,8 @@ int hermite2d_prepare(hteno_solver* s) {
   const size_t nc = size_t(G.nx) * G.ny;
   if (s->cfg.precision == HTENO_PREC_MIXED) {
     const WorkH<float> W = carve_h<float>(s->work, G.nx, G.ny);
-    kh_prim_f<<<unsigned(std::min<size_t>(8 * 152, (nc + 255) / 256)), 256, 0, s->stream>>>(G, s->q, W.qt, W.primt, s->dstate);
+    const SpeedLaunch l = speed_launch(nc, true);
+    kh_prim_f<<<l.blocks, 256, 0, s->stream>>>(G, s->q, W.qt, W.primt, s->dstate, l.filter);
   } else
     hermite2d_fp64_prim(s, G);
   return cuda_error(s, cudaGetLastError(), "kh_prim");

@@ -145,15 +145,34 @@ __global__ void kh_prim(GeoH G, const double* __restrict__ q, double* __restrict
 // So they are first computed from refined float reciprocals and roots (14 FP64 operations, relative
 // errors below 2^-41), which round to the same floats unless a value lies that close to the middle of
 // two of them; there, in odd ranges and for the speed (SpeedFilter) cell_prim decides.  Now 0.25 ms.
+// Small grids take cell_prim in every cell (speed_rule.h).
 __device__ __forceinline__ bool float_sure(double x) {
   const unsigned lo = unsigned(__double2loint(x)) & 0x1fffffffu;  // the bits a float drops
   const int e = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
   return (lo - (0x10000000u - 16384u) > 32768u && e > -100 && e < 100) || x == 0.0;
 }
 __global__ void kh_prim_f(GeoH G, const double* __restrict__ q, float* __restrict__ qt,
-                          float* __restrict__ primt, StepState* st) {
+                          float* __restrict__ primt, StepState* st, bool filter) {
   __shared__ unsigned found;
   const size_t nc = size_t(G.nx) * G.ny;
+  if (!filter) {  // a cell a thread
+    const size_t k = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+    double m = 0.0;
+    if (k < nc) {
+      const double qq[4] = {q[k], q[nc + k], q[2 * nc + k], q[3 * nc + k]};
+      double u, v, p, h, sr;
+      cell_prim(G.g1, qq, u, v, p, h, sr);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) qt[e * nc + k] = mix::d2f(qq[e]);
+      primt[k] = mix::d2f(u);
+      primt[nc + k] = mix::d2f(v);
+      primt[2 * nc + k] = mix::d2f(h);
+      primt[3 * nc + k] = mix::d2f(sr);
+      m = cell_max_speed(G.gamma, qq[0], u, v, p);
+    }
+    block_max_to(m, &st->maxbits);
+    return;
+  }
   mix::SpeedFilter F(&found, &st->maxbits, G.g1, G.gamma, nc);
   const float g1f = 1.0f + fabsf(float(G.g1));
   double ms = 0.0;
