@@ -1,6 +1,7 @@
 // Packed pieces (f32x2.cuh) that the mixed FV 2D and Hermite 2D kernels share: GL3 of both sides of a
 // face, the Roe projection of two cells, the back-projection of both sides.  Each half gets the bits of
-// the scalar function of device_math.cuh.
+// the scalar function of device_math.cuh or hermite_math.cuh, which the pointwise entry points run
+// (tests/cuda/packed_pairs.cu compares them).
 #pragma once
 
 #include "device_math.cuh"
@@ -73,9 +74,9 @@ __device__ __forceinline__ void load_hermite_tab(HermiteTab& S, const HermiteK<f
 }
 
 // HTENO (Schemes_Hermite.cpp:295-379; hermite_recon of hermite_math.cuh, kind 0) of both sides of a face:
-// U, V the cell pairs (0, 1), (2, 3) of the averages, A, B of the derivatives.  Every product and sum rounds as the compiler contracts the scalar function in
-// a unit where it may (checked on 8e9 values): the first of two products is fused, in S and on the minus
-// side of brkd's second bracket the other one.
+// U, V the cell pairs (0, 1), (2, 3) of the averages, A, B of the derivatives.  Every product and sum rounds
+// as the compiler contracts the scalar function in a unit where it may: the first of two products is fused,
+// in S and on the minus side of brkd's second bracket the other one.
 struct HtenoSides {
   f2 u, d;  // (minus, plus) values and derivatives
 };
