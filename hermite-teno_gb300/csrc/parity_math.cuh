@@ -97,7 +97,9 @@ __device__ __forceinline__ fp quot(fp a, const Den& d) {
 // constant in two parts, Brisebarre & Muller, IEEE Trans. Computers 57(2), 2008.)  The value that is
 // rounded is off by less than 2^-104 of itself, 2^-51 ulp, while a / c, a quotient by an integer with
 // the odd part d, lies 1/(2d) ulp or more from every midpoint of two doubles (d <= 315 here): no
-// rounding can differ.  Zeros keep their sign; other operands outside quot's range take the division.
+// rounding can differ.  +0 stays +0, and -0 keeps its sign where the low part is positive; where it is
+// negative (6720, 1680) -0 would give +0: callers pass absolute values there.  Other operands outside quot's
+// range take the division.
 __device__ __forceinline__ fp quot_lit(fp a, double c, Lit hi) {
   if (mid_range(a.v) || zero_bits(a.v)) return fma(a.v, lit(hi).v, (a * lit(Lit(hi + 1))).v);
   return divide(a.v, c);
