@@ -29,7 +29,7 @@ namespace par {
 
 enum Lit : int {
   kOne, kNegZero, kHalf, kNegHalf, kQuarter, kNegQuarter, kThreeQuarters, kThreeHalves, kTwo, kNegTwo, kThree,
-  kFour, kNegFour, kSix, kTwelve, kThirteenTwelfths, kEpsz, kEps6, k6908, k51001, k67923, k38947, k8209, k104963,
+  kFour, kNegFour, kSix, kThirteenTwelfths, kEpsz, kEps6, k6908, k51001, k67923, k38947, k8209, k104963,
   k299076, k179098, k231153, kDiv5040, kDiv5040Lo, kDiv6, kDiv6Lo, kDiv24, kDiv24Lo, kDiv3, kDiv3Lo, k23, k26,
   // Schemes::Hermite's full-stencil indicators
   k1029270, k2129184, k1099914, k281121, k494958, k1099445, k4317056, k2118166, kDiv6720, kDiv6720Lo, k3156862, k13189240,
@@ -39,7 +39,7 @@ enum Lit : int {
 };
 static __device__ double g_lit[kLitCount] = {
     1.0, -0.0, 0.5, -0.5, 0.25, -0.25, 0.75, 1.5, 2.0, -2.0, 3.0,
-    4.0, -4.0, 6.0, 12.0, 13.0 / 12.0, 1e-40, 1e-6, 6908.0, 51001.0, 67923.0, 38947.0, 8209.0, 104963.0,
+    4.0, -4.0, 6.0, 13.0 / 12.0, 1e-40, 1e-6, 6908.0, 51001.0, 67923.0, 38947.0, 8209.0, 104963.0,
     299076.0, 179098.0, 231153.0, 1.0 / 5040.0, 0x1.a01a01a01a01ap-73, 1.0 / 6.0, 0x1.5555555555555p-57,
     1.0 / 24.0, 0x1.5555555555555p-59, 1.0 / 3.0, 0x1.5555555555555p-56, 23.0, 26.0,
     1029270.0, 2129184.0, 1099914.0, 281121.0, 494958.0, 1099445.0, 4317056.0, 2118166.0, 1.0 / 6720.0,

@@ -338,7 +338,9 @@ void launch_stages(hteno_solver* s, const Geo1& G, cudaStream_t cs) {
 void launch_step(hteno_solver* s, const Geo1& G, cudaStream_t cs) {
   if (s->cfg.precision == HTENO_PREC_FP64) {
     // 4 faces a block (a third of them computed twice) while that is at most a warp per SM
-    // sub-partition; then 16 (a fifteenth)
+    // sub-partition; then 16 (a fifteenth).  32 steps, 4 / 16 faces, HLLC and Rusanov: 400 cells 1.75 / 1.82 ms (HLLC),
+    // 1824 1.80 / 1.84, 1.63 / 1.63; 2000 1.97 / 1.83, 1.72 / 1.55; 2400 2.23 / 2.47, 1.90 / 2.30; 3500 2.77 / 2.76,
+    // 2.43 / 2.43; 5000 3.68 / 3.86, 3.27 / 3.33; 7000 5.22 / 4.93, 4.46 / 4.31; 10000 7.58 / 6.29, 6.51 / 5.39.
     if (G.nx <= 3 * 608) launch_stages<4>(s, G, cs);
     else launch_stages<16>(s, G, cs);
     return;

@@ -61,7 +61,10 @@ void launch_step(hteno_solver* s, const Geo& G) {
 // A plain FP64 step of a small grid is 20 launches on two streams of ~10-30 us each, which the host
 // issues hardly faster than they run: runs of kGraphSteps steps are captured once into a graph (the
 // solver's buffers are fixed; dt, t and the stop live on the device) and replayed.  Larger grids'
-// launches outlast their issue.  64 x 48, 24 steps with state copies: 7.5 -> 6.2 ms with the blocks of update_threads.
+// launches outlast their issue.  64 x 48, 24 steps with state copies: 7.5 -> 6.2 ms with the blocks of
+// update_threads.  Eight steps, launched / replayed, four quadrants and periodic waves: 64^2 2.70 / 2.43, 2.52 / 2.25
+// ms; 128^2 6.40 / 6.15, 5.30 / 5.07; 181^2 10.76 / 10.69, 9.81 / 9.54; 200^2 12.48 / 12.42, 12.02 / 11.79;
+// 230^2 16.35 / 16.59, 13.93 / 14.63; 320^2 24.18 / 23.59, 25.79 / 25.57.
 constexpr int kGraphSteps = 4;
 constexpr size_t kGraphCells = size_t(1) << 15;
 

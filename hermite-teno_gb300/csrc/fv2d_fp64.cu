@@ -928,7 +928,9 @@ __global__ void __launch_bounds__(NT, 2) kp_stage64(Geo G, int stage, const doub
 }  // namespace
 
 // Threads per block of the cell kernels: small blocks while they give each of the chip's 608
-// sub-partitions two warps or fewer (a block of 256 would put two on each of its SM's).
+// sub-partitions two warps or fewer (a block of 256 would put two on each of its SM's).  Eight steps with
+// blocks of 256 / 64: 24^2 1.158 / 1.113 ms, 64^2 2.478 / 2.430, 128^2 6.196 / 6.155, 181^2 10.71 / 10.69, 200^2
+// 12.48 / 12.42, 256^2 17.73 / 17.70.
 static unsigned update_threads(size_t nc) { return nc <= size_t(32) * 1216 ? 64 : 256; }
 
 int fv2d_fp64_setup(hteno_solver* s) {
@@ -1035,7 +1037,10 @@ void fv2d_fp64_stage(hteno_solver* s, const Geo& G, const Work<double>& W, int s
                     cudaStreamWaitEvent(s->side_stream, s->fork_ev, 0) == cudaSuccess;
   cudaStream_t ys = fork ? s->side_stream : cs;
   // 8 lanes per face (about 5 times the work in a seventh of the sequence) while the faces of both
-  // directions give the chip's 608 sub-partitions less than three quarters of a warp each
+  // directions give the chip's 608 sub-partitions less than three quarters of a warp each.  Eight steps, a
+  // thread / 8 lanes a face, four quadrants and periodic waves: 64^2 3.87 / 2.43, 3.27 / 2.25 ms; 78^2 3.94 / 3.65,
+  // 3.30 / 3.28; 84^2 3.94 / 4.01, 3.28 / 3.51; 96^2 3.98 / 4.81, 3.27 / 4.37; 100^2 5.81 / 5.18, 5.04 / 4.71 (a
+  // second wave of blocks of a thread a face begins); 128^2 6.16 / 7.60, 5.07 / 7.31.
   const bool lanes = nxf + nyf <= 32l * 456;
   trace_begin(s, kf_x);
   if (lanes && !gx) {

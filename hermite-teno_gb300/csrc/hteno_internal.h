@@ -92,7 +92,11 @@ struct hteno_solver {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   bool side = true;
-  cudaGraphExec_t step_graph = nullptr;  // 1D schemes: a run of steps replayed as one graph
+  // FV 1D, Hermite 1D and small plain FP64 FV 2D grids: a run of steps replayed as one graph.  It holds the
+  // buffers, the geometry, uniform_skip, side, the lane rule and the block sizes of its capture, all of them
+  // fixed at create (fused64 and timing bypass it; dt, t and the stop live on the device): a call that
+  // came to change one of them would have to drop the graph.
+  cudaGraphExec_t step_graph = nullptr;
   // learned routing (mixed FV 2D): classifier, threshold, audit period, masks, audit sums
   hteno_mlp* router = nullptr;
   float router_thr = 0.9f;

@@ -105,7 +105,7 @@ __device__ __forceinline__ fp quot_lit(fp a, double c, Lit hi) {
   return divide(a.v, c);
 }
 
-// Schemes::SSPRK::RungeKuttaIII (Schemes_SSPRK.cpp:3-15): hteno::ssprk3's operations
+// Schemes::SSPRK::RungeKuttaIII (Schemes_SSPRK.cpp:3-15)
 __device__ __forceinline__ double rk3(fp q0, fp qn, fp rhs, fp dt, int stage) {
   if (stage == 1) return (q0 + dt * rhs).v;
   const fp x = qn + rhs * dt;
@@ -281,8 +281,8 @@ __device__ __forceinline__ int teno_decide(const fp* v, const fp* SI, bool impro
   // equal whatever tau is, and the cut-off keeps all candidates (pattern 7) -- decided without
   // tau, same bits.  (Equal values alone do not suffice: 3u - 4u + u can leave a rounding
   // residue in one indicator.)
-  // The full arithmetic below gives pattern 7 on such a window too (three equal ratios), so the
-  // shortcut is taken only when every active lane of the warp can take it: a warp never runs both.
+  // The full arithmetic below gives pattern 7 on such a window too (three equal ratios): a thread that
+  // returns here only saves it.
   if (zero_bits(SI[0].v) && zero_bits(SI[1].v) && zero_bits(SI[2].v)) return 7;
   double tau;
   if (!improved) {

@@ -211,7 +211,7 @@ int hteno_residual(hteno_solver* s, const double* q, double* rhs);
 /* n independent FV::System2D instances (FV_System2D.h:12-20), each with its own config (dims 2,
  * scheme FV, precision HTENO_PREC_MIXED; grid sizes may differ and need not be square), advanced
  * together: each instance keeps its own time, dt and stop test exactly as its own
- * timeStepping() loop would (FV_System2D.cpp:614-651).  One persistent launch per RK stage
+ * timeStepping() loop would (FV_System2D.cpp:614-651).  One launch per RK stage
  * covers the tiles of every instance; a whole step is captured once in a CUDA graph and
  * replayed; the tile shape is picked by timing the candidates on the batch itself (first step,
  * or hteno_batch_tile).  No reference counterpart for the batching itself: the reference runs
