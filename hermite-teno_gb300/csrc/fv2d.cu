@@ -77,8 +77,17 @@ bool graphed(const hteno_solver* s) {
   return s->cfg.precision == HTENO_PREC_FP64 && !s->fused64 && !s->timing && s->ncell <= kGraphCells && !capturing(s);
 }
 
+// While it lives, this thread may make calls that a capture elsewhere (the caller's, on another stream or in
+// another thread) would refuse and be invalidated by: creating a stream, instantiating a graph.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 cudaError_t ensure_graph(hteno_solver* s, const Geo& G) {
   if (s->step_graph) return cudaSuccess;
+  const RelaxedCapture relaxed;
   cudaStream_t cap, own = s->stream;
   cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
   if (e != cudaSuccess) return e;
