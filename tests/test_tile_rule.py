@@ -80,8 +80,8 @@ def test_choosing_a_tile_costs_few_stages(hteno_lib, cuda, n):
 @pytest.mark.parametrize("nx,ny", [(256, 192), (384, 336)])
 def test_shape_chosen_is_the_fastest_in_steps(hteno_lib, cuda, nx, ny):
     """Grids of less than one and about two tiles an SM, where a shape that is faster in plain launches is
-    14 to 18 % slower in the early launches of a step: steps with the shape chosen take at most 1.08
-    times those with the best of the shapes that win on such grids.  (Smooth data: the shapes are timed
+    14 to 18 % slower in the early launches of a step: steps with the shape chosen (the median of three new
+    solvers) take at most 1.08 times those with the best of the shapes that win on such grids.  (Smooth data: the shapes are timed
     doing the full work, while steps skip the tiles of constant regions.)"""
     h = hteno_lib
     from hteno import ic
@@ -99,7 +99,7 @@ def test_shape_chosen_is_the_fastest_in_steps(hteno_lib, cuda, nx, ny):
         s.set_state(q)
         return s
 
-    tiles = ("", "2", "4", "5", "9", "11")
+    tiles = ("", "", "", "2", "4", "5", "9", "11")
     solvers = [solver(t) for t in tiles]
     best = [1e9] * len(tiles)
     for _ in range(9):
@@ -110,4 +110,4 @@ def test_shape_chosen_is_the_fastest_in_steps(hteno_lib, cuda, nx, ny):
             best[k] = min(best[k], time.perf_counter() - t0)
     for s in solvers:
         s.close()
-    assert best[0] <= 1.08 * min(best[1:]), dict(zip(tiles, best))
+    assert sorted(best[:3])[1] <= 1.08 * min(best[3:]), list(zip(tiles, best))
