@@ -27,7 +27,7 @@ __device__ __forceinline__ void cell_prim(double g1, const double* qd, double* w
   const par::fp q[4] = {qd[0], qd[1], qd[2], qd[3]};
   const par::Den d = par::den_of(q[0]);
   const par::fp u = par::quot(q[1], d), v = par::quot(q[2], d);
-  const par::fp p = par::scaled(par::kNegHalf, q[1] * u + q[2] * v, q[3]) * g1;  // par::primitive's pressure
+  const par::fp p = par::minus_half(q[1] * u + q[2] * v, q[3]) * g1;  // par::primitive's pressure
   w[0] = qd[0];
   w[1] = u.v;
   w[2] = v.v;

@@ -105,13 +105,18 @@ __device__ __forceinline__ fp quot_lit(fp a, double c, Lit hi) {
   return divide(a.v, c);
 }
 
+// q0 + 2 x where 2 x overflows by itself, whatever q0 is
+static __device__ __noinline__ double plus_twice_huge(double x, double q0) { return __dadd_rn(q0, __dmul_rn(2.0, x)); }
+
 // Schemes::SSPRK::RungeKuttaIII (Schemes_SSPRK.cpp:3-15)
 __device__ __forceinline__ double rk3(fp q0, fp qn, fp rhs, fp dt, int stage) {
   if (stage == 1) return (q0 + dt * rhs).v;
   const fp x = qn + rhs * dt;
   // (the quarter rounds where it is subnormal: not folded into the sum)
   if (stage == 2) return (lit(kThreeQuarters) * q0 + lit(kQuarter) * x).v;
-  return quot_lit(scaled(kTwo, x, q0), 3.0, kDiv3).v;
+  fp s = scaled(kTwo, x, q0);
+  if (__builtin_expect((unsigned(__double2hiint(x.v)) & 0x7ff00000u) == 0x7fe00000u, 0)) s = plus_twice_huge(x.v, q0.v);
+  return quot_lit(s, 3.0, kDiv3).v;
 }
 // x <= 0, on the integer pipes
 __device__ __forceinline__ bool nonpositive_bits(double x) {
@@ -554,6 +559,15 @@ static __device__ __noinline__ void gl3(const DevConst& C, const double* ud, dou
 
 // ---- Equations::Euler2D ---------------------------------------------------------------------
 
+// y - x / 2, the energy less the kinetic part, in one operation.  Where the half may be subnormal the reference
+// rounds it first.  That can reach the result only if y is below 2^-968 (the half is below 2^-1021 there):
+// such y take the separate operations.  The test needs y alone, on the integer pipes beside the chain.
+__device__ __forceinline__ bool tiny(fp y) { return (unsigned(__double2hiint(y.v)) & 0x7fffffffu) < (123u << 20); }  // 2^-900
+static __device__ __noinline__ double minus_half_tiny(double x, double y) { return __dsub_rn(y, __dmul_rn(0.5, x)); }
+__device__ __forceinline__ fp minus_half(fp x, fp y) {
+  if (__builtin_expect(tiny(y), 0)) return minus_half_tiny(x.v, y.v);
+  return scaled(kNegHalf, x, y);
+}
 __device__ __forceinline__ fp operator/(fp a, fp b) { return fp(a.v / b.v); }
 __device__ __forceinline__ fp sqrt_abs(fp a) { return fp(sqrt(fabs(a.v))); }
 __device__ __forceinline__ fp max_(fp a, fp b) { return fp(fmax(a.v, b.v)); }
@@ -563,7 +577,7 @@ __device__ __forceinline__ void primitive(double g1, const fp* q, const Den& d, 
   w[0] = q[0];
   w[1] = quot(q[1], d);
   w[2] = quot(q[2], d);
-  w[3] = scaled(kNegHalf, q[1] * w[1] + q[2] * w[2], q[3]) * g1;
+  w[3] = minus_half(q[1] * w[1] + q[2] * w[2], q[3]) * g1;
 }
 __device__ __forceinline__ void primitive(double g1, const double* q, double* w) {
   const fp qf[4] = {q[0], q[1], q[2], q[3]};
@@ -837,7 +851,7 @@ __device__ __forceinline__ double max_speed2(double g, const double* w) {
 __device__ __forceinline__ void primitive1(double g1, const fp* q, const Den& d, fp* w) {  // :18-23
   w[0] = q[0];
   w[1] = quot(q[1], d);
-  w[2] = scaled(kNegHalf, q[1] * w[1], q[2]) * g1;
+  w[2] = (q[2] - lit(kHalf) * q[1] * w[1]) * g1;  // (the half beside the quotient's chain)
 }
 
 // eigen1DEuler (FV_System1D.cpp:121-156), eigenvectors :55-89 as full row-major 3x3 matrices
